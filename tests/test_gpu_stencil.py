@@ -1,0 +1,117 @@
+"""The assembled 27-point operator of the structured numbering: A x and
+A^T x against the oracle and against the element-wise apply (scatter
+"atomic"), and the solve on it.
+
+Bars: 1e-12 relative L2 (FP64), as for every stored apply; each row is a sum
+of at most 64 pair products whose pairs carry 2^-47, 64 * 2^-47 = 4.5e-13.
+"""
+import numpy as np
+import pytest
+
+from helpers import kat_problem, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-12
+# one element, single rows, a row longer than a block, ragged, several blocks
+DIMS = [(1, 1, 1), (1, 2, 1), (2, 1, 3), (31, 1, 2), (9, 7, 5), (300, 2, 3), (33, 17, 21)]
+
+
+def oracle_bb(oracle, prob, aH, aM):
+    m = prob.mesh
+    bb, _, _ = oracle.assemble(prob.variant, m.xx, m.yy, m.zz, m.iss, prob.vel, prob.lam,
+                               prob.pdec, prob.q, kod=m.kod, robin_alpha=prob.robin_alpha,
+                               aH=aH, aM=aM, want_b=False, want_diag=False)
+    return bb
+
+
+@pytest.mark.parametrize("dims", DIMS)
+def test_apply_matches_oracle(vdr, oracle, gpu_lib, dims):
+    prob = vdr.problems.rotation_shear(*dims, seed=81)
+    prob.pdec[:] = 0.2
+    aH, aM = 2.0, 7.0
+    bb = oracle_bb(oracle, prob, aH, aM)
+    x = np.random.default_rng(3).standard_normal(prob.mesh.nnode)
+    with vdr.Solver(prob, aH=aH, aM=aM) as s:
+        s.apply(x)  # the rows are assembled from the second apply on
+        for tr in (False, True):
+            ref, _ = oracle.matvec0(prob.mesh.iss, bb, prob.bc, x, transpose=tr)
+            y = s.apply(x, transpose=tr)
+            assert rel_l2(y, ref) < TOL, (dims, tr)
+            assert np.all(y[prob.bc == 1] == 0.0)
+
+
+def test_dirichlet_values_scale_and_nonfinite(vdr, oracle, gpu_lib):
+    """Whatever lies on Dirichlet nodes is ignored; inputs of any magnitude
+    keep their relative accuracy; a non-finite entry reaches exactly the
+    rows that the element-wise apply gives it to."""
+    prob = vdr.problems.rotation_shear(13, 6, 5, seed=82)
+    m = prob.mesh
+    free = np.flatnonzero(prob.bc == 0)
+    bb = oracle_bb(oracle, prob, 2.0, 7.0)
+    rng = np.random.default_rng(4)
+    with vdr.Solver(prob, aH=2.0, aM=7.0) as s, \
+            vdr.Solver(prob, vdr.Options(scatter="atomic"), aH=2.0, aM=7.0) as e:
+        x = rng.standard_normal(m.nnode)
+        s.apply(x)
+        ref, _ = oracle.matvec0(m.iss, bb, prob.bc, x)
+        for fill in (np.nan, np.inf, 1e300):
+            xd = np.where(prob.bc == 1, fill, x)
+            assert rel_l2(s.apply(xd), ref) < TOL
+        for scale in (1e-250, 1e-30, 1e30, 1e250):
+            assert rel_l2(s.apply(x * scale) / scale, ref) < TOL
+        for bad in (np.nan, np.inf):
+            xb = x.copy()
+            xb[free[len(free) // 2]] = bad
+            for tr in (False, True):
+                a, b = s.apply(xb, transpose=tr), e.apply(xb, transpose=tr)
+                ok = np.isfinite(b)
+                assert np.array_equal(ok, np.isfinite(a))
+                assert rel_l2(a[ok], b[ok]) < TOL
+
+
+@pytest.mark.parametrize("solver", ["bicgstab", "bicg"])
+@pytest.mark.parametrize("dims", [(1, 1, 1), (2, 1, 3), (19, 13, 11), (70, 40, 30)])
+def test_solve_matches_element_wise(vdr, gpu_lib, dims, solver):
+    """Both to 1e-12: their distance is bounded by the residuals times the
+    condition of the theta-step operator (below 1e3 here)."""
+    prob = vdr.problems.rotation_shear(*dims, seed=83)
+    if np.all(prob.bc == 1):
+        prob.bc[:] = 0
+    xs = []
+    for scatter in ("auto", "atomic"):
+        with vdr.Solver(prob, vdr.Options(scatter=scatter, solver=solver), aH=2.0,
+                        aM=0.3 * max(dims)) as s:
+            b = s.assemble_rhs(3.0, 0.3 * max(dims), np.linspace(0, 1, prob.mesh.nnode))
+            x, it, err, st = s.solve(b, tol=1e-12, itmax=2000)
+            assert st == 0 and err <= 1e-12
+            xs.append(x)
+    assert rel_l2(xs[0], xs[1]) < 1e-9
+
+
+def test_operator_follows_fields_and_mask(vdr, oracle, gpu_lib):
+    prob = vdr.problems.rotation_shear(9, 8, 6, seed=84)
+    m = prob.mesh
+    x = np.random.default_rng(5).standard_normal(m.nnode)
+    with vdr.Solver(prob, aH=2.0, aM=7.0) as s:
+        s.apply(x)
+        s.apply(x)
+        prob.vel *= -0.5
+        prob.lam *= 3.0
+        prob.bc[:] = vdr.problems.inflow_mask(m, prob.vel)
+        s.set_fields(prob.vel, prob.lam, prob.pdec, prob.q)
+        s.set_dirichlet(prob.bc)
+        ref, _ = oracle.matvec0(m.iss, oracle_bb(oracle, prob, 2.0, 7.0), prob.bc, x)
+        for _ in range(2):  # element-wise, then from the new rows
+            assert rel_l2(s.apply(x), ref) < TOL
+
+
+def test_recorded_case(vdr, oracle, gpu_lib):
+    prob = kat_problem(vdr)
+    bb = oracle_bb(oracle, prob, 2.0, 0.03)
+    x = np.random.default_rng(6).standard_normal(prob.mesh.nnode)
+    with vdr.Solver(prob, aH=2.0, aM=0.03) as s:
+        s.apply(x)
+        for tr in (False, True):
+            ref, _ = oracle.matvec0(prob.mesh.iss, bb, prob.bc, x, transpose=tr)
+            assert rel_l2(s.apply(x, transpose=tr), ref) < TOL

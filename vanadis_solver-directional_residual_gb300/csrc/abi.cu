@@ -359,6 +359,15 @@ void invalidate(Handle &h) {
   h.op64_valid = h.op32_valid = h.diag_valid = false;
   h.mass_valid = false;
   h.aos_valid = h.phi_valid = false;
+  if (h.st_state > 0) h.st_state = 0;
+  h.st_applies = 0;
+}
+
+// Single applies: the rows are assembled at the second apply of an operator.
+// Summing them moves 732 bytes a node where an apply then saves 308, so the
+// third apply has paid for it; one apply per operator stays element-wise.
+cudaError_t rows_for_apply(Handle &h) {
+  return ++h.st_applies >= 2 ? ensure_stencil(h) : cudaSuccess;
 }
 
 // d64[c][p] = src[c][perm[p]] (perm null: identity), d32 the FP32 copy.
@@ -397,6 +406,7 @@ void free_handle(Handle &h) {
   dfree(h.xx); dfree(h.yy); dfree(h.zz);
   dfree(h.xx32); dfree(h.yy32); dfree(h.zz32);
   dfree(h.conn); dfree(h.mask); dfree(h.emask);
+  dfree(h.st_S); dfree(h.st_nm); dfree(h.st_x);
   dfree(h.vel); dfree(h.lam); dfree(h.pdec); dfree(h.q);
   dfree(h.vel32); dfree(h.lam32); dfree(h.pdec32); dfree(h.robin);
   dfree(h.A64); dfree(h.A32); dfree(h.diag); dfree(h.dinv);
@@ -713,8 +723,12 @@ int vdr_apply_device(vdr_handle *H, const double *x, double *y, int transpose) {
     return VDR_BAD_ARGUMENT;
   }
   if ((st = ensure_operator(h))) return st;
-  cudaError_t e;
-  if ((e = cudaMemsetAsync(y, 0, sizeof(double) * h.N, h.stream)))
+  cudaError_t e = rows_for_apply(h);
+  if (!e && stencil_ready(h)) {
+    e = launch_stencil_apply(h, transpose != 0, false, x, y, nullptr, nullptr, h.stream);
+    return e ? cuda_fail(e, "apply") : VDR_OK;
+  }
+  if (e || (e = cudaMemsetAsync(y, 0, sizeof(double) * h.N, h.stream)))
     return cuda_fail(e, "memset");
   if ((e = launch_apply(h, transpose != 0, x, y, nullptr, nullptr, h.stream)))
     return cuda_fail(e, "apply");
@@ -731,7 +745,8 @@ int vdr_apply_accumulate_device(vdr_handle *H, const double *x, double *y,
     return VDR_BAD_ARGUMENT;
   }
   if ((st = ensure_operator(h))) return st;
-  cudaError_t e = launch_apply(h, transpose != 0, x, y, nullptr, nullptr, h.stream);
+  cudaError_t e = rows_for_apply(h);
+  if (!e) e = launch_apply(h, transpose != 0, x, y, nullptr, nullptr, h.stream);
   return e ? cuda_fail(e, "apply") : VDR_OK;
 }
 

@@ -299,6 +299,7 @@ int solve_gcr_device(Handle &h, const double *b, double *x, double tol,
     return VDR_BAD_ARGUMENT;
   }
   cudaError_t e = ensure_solver_workspace(h, 8);  // KState, events
+  if (!e) e = ensure_stencil(h);
   if (e) return cuda_fail(e, "solver workspace");
   cudaStream_t s = h.stream;
   const int g = gcr_grid(h.N);
@@ -369,7 +370,8 @@ int solve_gcr_device(Handle &h, const double *b, double *x, double tol,
                                    ((uintptr_t)h.gcr_work << 2) ^ (uintptr_t)m ^
                                    ((uintptr_t)(prec ? prec->ctx : nullptr) << 3) ^
                                    ((uintptr_t)h.apply_mode << 8) ^
-                                   ((uintptr_t)h.scatter << 12));
+                                   ((uintptr_t)h.scatter << 12) ^
+                                   ((uintptr_t)stencil_ready(h) << 16));
   long per_cycle = 0;
   if (!h.gcr_graph || h.gcr_key != key) {
     if (h.gcr_graph) cudaGraphExecDestroy(h.gcr_graph);

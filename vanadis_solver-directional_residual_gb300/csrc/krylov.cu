@@ -25,6 +25,7 @@
 #include <cstring>
 
 #include "dfloat.cuh"
+#include "stencil.cuh"
 #include "vdr_internal.h"
 
 namespace vdr {
@@ -103,6 +104,7 @@ struct Vec {
   const unsigned char *m;
   double *x, *r, *rh, *p, *v, *ph, *s, *sh, *t;  // BiCGStab
   double *rr, *pp, *z, *zz;                      // BiCG (r, p, x shared)
+  float2 *php, *shp;  // p^ and s^ as pairs (assembled operator)
 };
 
 // Grid-stride loops unrolled U times with every load of the U elements
@@ -132,8 +134,9 @@ template <bool BICG>
 __global__ void __launch_bounds__(RED_THREADS) k_start(Vec a) {
   double v[3] = {0.0, 0.0, 0.0};
   double bv[U], rv[U], dv[U];
+  int em = 0;
   VLOOP(bv[u] = ok ? a.b[i] : 0.0; rv[u] = ok ? a.r[i] : 0.0;
-        dv[u] = (ok && BICG) ? a.dinv[i] : 0.0;,
+        dv[u] = (ok && (BICG || a.php)) ? a.dinv[i] : 0.0;,
         const double ri = bv[u] - rv[u];
         a.r[i] = ri;
         if (BICG) {
@@ -142,8 +145,13 @@ __global__ void __launch_bounds__(RED_THREADS) k_start(Vec a) {
         } else {
           a.rh[i] = ri;
         }
+        if (a.php) em = max(em, df_exp(ri) + df_exp(dv[u]) - 1022);
         v[0] += bv[u] * bv[u];
         v[1] += ri * ri;)
+  if (a.php) {
+    em = __reduce_max_sync(FULL, em);
+    if ((threadIdx.x & 31) == 0) atomicMax(&a.st->pmax, em);
+  }
   double o[3];
   if (grid_sum<3>(v, a.partials, &a.st->ticket, o)) {
     KState *st = a.st;
@@ -448,7 +456,206 @@ Vec make_vec(Handle &h, const double *b, double *x) {
   a.pp = a.ph;
   a.z = a.v;
   a.zz = a.t;
+  if (h.st_x) {
+    a.php = h.st_x + stencil_pad(h);
+    a.shp = a.php + N + 2 * stencil_pad(h);
+  }
   return a;
+}
+
+// ---- BiCGStab on the assembled rows (stencil.cuh) ----
+// With the rows assembled a node's product is one thread's sum, so the
+// iteration needs four kernels, no cleared outputs and no atomics:
+//   bst_v   v = A p^ with (rh, v)                      -> alpha
+//   bst_s   s = r - alpha v, s^ = D^-1 s with ||s||, (rh, s)
+//   bst_t   t = A s^ with (t, s), (t, t), (rh, t)      -> omega, next rho
+//   bst_p   x, r, the next p and p^ in one pass with ||r||
+// The next rho is (rh, r) = (rh, s) - omega (rh, t), known before r is
+// formed, which lets the direction update share the pass over x and r.
+// p^ and s^ exist only as the products' inputs, pairs scaled by the largest
+// exponent of the direction before (a direction would have to grow 2^100
+// times in one iteration to leave the pairs' range, which then reads as a
+// breakdown).  610 bytes per node and iteration against 1,024 E + ~240 N
+// element-wise; each kernel's last block adds the block partials in a fixed
+// order.
+__global__ void __launch_bounds__(RED_THREADS) bst_first(Vec a) {
+  KState *st = a.st;
+  if (st->done) return;
+  const int e = st->pmax, shift = e - 1023;
+  double rv[U], dv[U];
+  unsigned char mv[U];
+  VLOOP(rv[u] = ok ? a.r[i] : 0.0; dv[u] = ok ? a.dinv[i] : 0.0; mv[u] = ok ? a.m[i] : 1;,
+        a.p[i] = rv[u];
+        a.php[i] = mv[u] ? make_float2(0.f, 0.f) : stencil_pair(rv[u] * dv[u], shift);)
+  if (blockIdx.x == 0 && threadIdx.x == 0) st->pexp = e;
+}
+
+template <bool KEEP>
+__global__ void __launch_bounds__(RED_THREADS, 4) bst_v(Vec a, StencilView w) {
+  if (a.st->done) return;
+  const int shift = a.st->pexp - 1023;
+  double v[1] = {0.0};
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n;
+       i += (long)gridDim.x * blockDim.x) {
+    const double o = stencil_row_pairs<KEEP>(w, i, a.php, shift);
+    a.v[i] = o;
+    v[0] += a.rh[i] * o;
+  }
+  double o[1];
+  if (grid_sum<1>(v, a.partials, &a.st->ticket, o)) {
+    KState *st = a.st;
+    if (o[0] == 0.0 || !finite(o[0])) {
+      st->status = VDR_BREAKDOWN;
+      st->reason = 2;
+      st->done = 1;
+    } else {
+      st->alpha = st->rho / o[0];
+    }
+  }
+}
+
+__global__ void __launch_bounds__(RED_THREADS) bst_s(Vec a) {
+  if (a.st->done) return;
+  const double al = a.st->alpha;
+  const int shift = a.st->pexp - 1023;
+  double v[2] = {0.0, 0.0};
+  double rv[U], vv[U], dv[U], hv[U];
+  unsigned char mv[U];
+  VLOOP(rv[u] = ok ? a.r[i] : 0.0; vv[u] = ok ? a.v[i] : 0.0;
+        dv[u] = ok ? a.dinv[i] : 0.0; hv[u] = ok ? a.rh[i] : 0.0; mv[u] = ok ? a.m[i] : 1;,
+        const double si = rv[u] - al * vv[u];
+        a.s[i] = si;
+        a.shp[i] = mv[u] ? make_float2(0.f, 0.f) : stencil_pair(si * dv[u], shift);
+        v[0] += si * si;
+        v[1] += hv[u] * si;)
+  double o[2];
+  if (grid_sum<2>(v, a.partials, &a.st->ticket, o)) {
+    KState *st = a.st;
+    st->snrm = sqrt(o[0]) / sqrt(st->bnrm2);
+    st->rhs = o[1];
+    if (st->snrm <= st->tol) st->sconv = 1;
+  }
+}
+
+template <bool KEEP>
+__global__ void __launch_bounds__(RED_THREADS, 4) bst_t(Vec a, StencilView w) {
+  if (a.st->done || a.st->sconv) return;
+  const int shift = a.st->pexp - 1023;
+  double v[3] = {0.0, 0.0, 0.0};
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n;
+       i += (long)gridDim.x * blockDim.x) {
+    const double o = stencil_row_pairs<KEEP>(w, i, a.shp, shift);
+    a.t[i] = o;
+    v[0] += o * a.s[i];
+    v[1] += o * o;
+    v[2] += a.rh[i] * o;
+  }
+  double o[3];
+  if (grid_sum<3>(v, a.partials, &a.st->ticket, o)) {
+    KState *st = a.st;
+    if (o[1] == 0.0 || !finite(o[1]) || !finite(o[0])) {
+      st->status = VDR_BREAKDOWN;
+      st->reason = 3;
+      st->done = 1;
+    } else {
+      st->omega = o[0] / o[1];
+      st->rho_next = st->rhs - st->omega * o[2];
+    }
+  }
+}
+
+__global__ void __launch_bounds__(RED_THREADS) bst_p(Vec a) {
+  KState *stc = a.st;
+  if (stc->done) return;
+  const double al = stc->alpha;
+  if (stc->sconv) {  // s met the tolerance: x += alpha p^, r = s
+    double v[1] = {0.0};
+    double xv[U], pv[U], sv[U], dv[U];
+    unsigned char mv[U];
+    VLOOP(xv[u] = ok ? a.x[i] : 0.0; pv[u] = ok ? a.p[i] : 0.0; dv[u] = ok ? a.dinv[i] : 0.0;
+          sv[u] = ok ? a.s[i] : 0.0; mv[u] = ok ? a.m[i] : 1;,
+          if (!mv[u]) a.x[i] = xv[u] + dv[u] * (al * pv[u]);
+          a.r[i] = sv[u];)
+    double o[1];
+    if (grid_sum<1>(v, a.partials, &a.st->ticket, o)) {
+      KState *st = a.st;
+      st->iter += 1;
+      st->err = st->snrm;
+      st->status = VDR_OK;
+      st->done = 1;
+    }
+    return;
+  }
+  const double om = stc->omega, rho1 = stc->rho_next;
+  const double beta = (rho1 / stc->rho) * (al / om);
+  const int e = stc->pmax, shift = e - 1023;
+  int em = 0;
+  double v[1] = {0.0};
+  double xv[U], pv[U], sv[U], tv[U], vv[U], dv[U];
+  unsigned char mv[U];
+  VLOOP(xv[u] = ok ? a.x[i] : 0.0; pv[u] = ok ? a.p[i] : 0.0; sv[u] = ok ? a.s[i] : 0.0;
+        tv[u] = ok ? a.t[i] : 0.0; vv[u] = ok ? a.v[i] : 0.0; dv[u] = ok ? a.dinv[i] : 0.0;
+        mv[u] = ok ? a.m[i] : 1;,
+        const double ri = sv[u] - om * tv[u];
+        const double pi = ri + beta * (pv[u] - om * vv[u]);
+        if (!mv[u]) a.x[i] = xv[u] + dv[u] * (al * pv[u] + om * sv[u]);
+        a.r[i] = ri;
+        a.p[i] = pi;
+        const double hi = mv[u] ? 0.0 : pi * dv[u];
+        a.php[i] = stencil_pair(hi, shift);
+        em = max(em, df_exp(hi));
+        v[0] += ri * ri;)
+  em = __reduce_max_sync(FULL, em);
+  if ((threadIdx.x & 31) == 0) atomicMax(&stc->pmax_next, em);
+  __threadfence();
+  double o[1];
+  if (grid_sum<1>(v, a.partials, &a.st->ticket, o)) {
+    KState *st = a.st;
+    st->iter += 1;
+    st->pexp = e;
+    st->pmax = atomicExch(&st->pmax_next, 0);
+    st->rho_old = st->rho;
+    st->rho = rho1;
+    st->err = sqrt(o[0]) / sqrt(st->bnrm2);
+    if (!(st->err == st->err) || !finite(rho1)) {
+      st->status = VDR_BREAKDOWN;
+      st->reason = 5;
+      st->done = 1;
+    } else if (st->err <= st->tol) {
+      st->status = VDR_OK;
+      st->done = 1;
+    } else if (rho1 == 0.0 || om == 0.0) {
+      st->status = VDR_BREAKDOWN;
+      st->reason = rho1 == 0.0 ? 1 : 4;
+      st->done = 1;
+    } else if (st->iter >= st->itmax) {
+      st->status = VDR_NOT_CONVERGED;
+      st->done = 1;
+    } else if (st->stall_window > 0) {
+      if (st->err < 0.99 * st->best_err) {
+        st->best_err = st->err;
+        st->since_best = 0;
+      } else if (++st->since_best >= st->stall_window) {
+        st->status = VDR_NOT_CONVERGED;
+        st->reason = 6;  // stalled
+        st->done = 1;
+      }
+    }
+  }
+}
+
+cudaError_t launch_stencil_iteration(Handle &h, const Vec &a, cudaStream_t s) {
+  const StencilView w = stencil_view(h);
+  const bool keep = stencil_keep(h);
+  const int gv = red_grid(h.N);
+  const int gs = std::min(gv, device_sm_count() * 4);
+  if (keep) bst_v<true><<<gs, RED_THREADS, 0, s>>>(a, w);
+  else bst_v<false><<<gs, RED_THREADS, 0, s>>>(a, w);
+  bst_s<<<gv, RED_THREADS, 0, s>>>(a);
+  if (keep) bst_t<true><<<gs, RED_THREADS, 0, s>>>(a, w);
+  else bst_t<false><<<gs, RED_THREADS, 0, s>>>(a, w);
+  bst_p<<<gv, RED_THREADS, 0, s>>>(a);
+  return cudaGetLastError();
 }
 
 // The fused FP64 BiCGStab iteration (defined below with the fused kernels).
@@ -459,6 +666,8 @@ cudaError_t launch_iteration(Handle &h, int method, const Vec &a,
   const int g = red_grid(h.N);
   cudaStream_t s = h.stream;
   cudaError_t e;
+  if (method == VDR_SOLVER_BICGSTAB && !prec && stencil_ready(h))
+    return launch_stencil_iteration(h, a, s);
   if (method == VDR_SOLVER_BICGSTAB && !prec && h.fused64)
     return launch_fused64_iteration(h, a, s);
   if (method == VDR_SOLVER_BICGSTAB) {
@@ -520,6 +729,7 @@ cudaError_t ensure_solver_workspace(Handle &h, int nvec) {
 
 // Kernels of one captured iteration.
 long launches_graph_nodes(Handle &h, int method, const Precond *prec) {
+  if (method == VDR_SOLVER_BICGSTAB && !prec && stencil_ready(h)) return 4;
   if (method == VDR_SOLVER_BICGSTAB && !prec && h.fused64) return 2 + 2 * apply_launches(h);
   long n = (method == VDR_SOLVER_BICGSTAB ? 5 : 3) +
            (method != VDR_SOLVER_BICGSTAB && can_apply_both(h) ? 1 : 2) *
@@ -539,6 +749,7 @@ int solve_device(Handle &h, int method, const double *b, double *x,
                  const Precond *prec, int stall_window, double *hist,
                  int max_hist, int *n_hist) {
   cudaError_t e = ensure_solver_workspace(h, 8);
+  if (!e && !h.apply_fp32) e = ensure_stencil(h);
   if (e) return cuda_fail(e, "solver workspace");
   cudaStream_t s = h.stream;
   Vec a = make_vec(h, b, x);
@@ -591,10 +802,12 @@ int solve_device(Handle &h, int method, const double *b, double *x,
   // graph captured for other sizes (buffers reused by a smaller mesh) is
   // captured again
   const long long size_key = ((long long)h.N << 32) | (unsigned)h.E;
+  const bool rows = stencil_ready(h);
   const bool fusable = method == VDR_SOLVER_BICGSTAB && !prec;
   for (int attempt = 0; attempt < 2; attempt++) {
     const bool fused = fusable && h.fused64;
-    const void *fkey = (const void *)((uintptr_t)key ^ ((uintptr_t)fused << 20));
+    const void *fkey = (const void *)((uintptr_t)key ^ ((uintptr_t)fused << 20) ^
+                                      ((uintptr_t)rows << 21));
     if (h.graph_exec[slot] && h.graph_key[slot] == fkey && h.graph_size[slot] == size_key)
       break;
     if (h.graph_exec[slot]) cudaGraphExecDestroy(h.graph_exec[slot]);
@@ -623,7 +836,7 @@ int solve_device(Handle &h, int method, const double *b, double *x,
     }
     // a cooperative launch that the capture or the graph refuses: the
     // five-kernel iteration instead
-    if (fused) {
+    if (fused && !rows) {
       cudaGetLastError();
       h.fused64 = false;
       e = cudaSuccess;
@@ -632,7 +845,11 @@ int solve_device(Handle &h, int method, const double *b, double *x,
     if (e) return cuda_fail(e, "capture");
     return cuda_fail(e2 ? e2 : cudaErrorUnknown, "end capture");
   }
-  if (fusable && h.fused64) {  // the first search direction p = r, p^ = D^-1 r, v = 0
+  if (fusable && rows) {  // the first search direction and its pairs
+    bst_first<<<g, RED_THREADS, 0, s>>>(a);
+    count_launches(1);
+    if ((e = cudaGetLastError())) return cuda_fail(e, "first direction");
+  } else if (fusable && h.fused64) {  // the first search direction p = r, p^ = D^-1 r, v = 0
     bs_p<<<g, RED_THREADS, 0, s>>>(a);
     count_launches(1);
     if ((e = cudaGetLastError())) return cuda_fail(e, "first direction");
@@ -1612,6 +1829,7 @@ int solve_mixed_device(Handle &h, int method, const double *b, double *x,
                        double tol, double inner_tol, int max_outer,
                        int inner_itmax, MixedStats *ms) {
   cudaError_t e = ensure_solver_workspace(h, 11);
+  if (!e) e = ensure_stencil(h);
   if (e) return cuda_fail(e, "solver workspace");
   cudaStream_t s = h.stream;
   double *r = h.work + 8 * (size_t)h.N;

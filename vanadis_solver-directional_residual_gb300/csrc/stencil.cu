@@ -1,0 +1,176 @@
+// stencil.cu -- assembly of the 27-point operator (stencil.cuh) from the
+// double-float element store, and its plain applies.
+#include "stencil.cuh"
+
+#include <algorithm>
+
+namespace vdr {
+namespace {
+
+constexpr int slot_of(int a, int b, int c) {
+  return 4 * c + (b ? (a ? 2 : 3) : (a ? 1 : 0));
+}
+constexpr int slot_x(int s) { return ((s + 1) & 2) ? 1 : 0; }
+constexpr int slot_y(int s) { return (s & 2) ? 1 : 0; }
+constexpr int slot_z(int s) { return (s & 4) ? 1 : 0; }
+
+// acc += (h, l), the error terms gathered in acc.c.
+__device__ __forceinline__ void acc_pair(DfAcc &acc, float h, float l) {
+  df_acc_add(acc, Df2{h, l});
+}
+
+// Row n of P A P: the sum of its row in each of the up to eight elements
+// around it, TwoSum per entry (error ~2^-47 of the largest element entry, as
+// the sums of an element-wise apply).  One thread per node: an element's
+// row i is read by exactly one thread, so the store is read once (512 E
+// bytes) and 220 N written: 1.23 ms at 8.4M elements (5.0 TB/s).
+__global__ void __launch_bounds__(256, 2) stencil_assemble(
+    const float4 *__restrict__ Ahi, const float4 *__restrict__ Alo,
+    const unsigned char *__restrict__ emask, int nax, int nay, int naz, float2 *S,
+    unsigned *nm) {
+  const int E = (nax - 1) * (nay - 1) * (naz - 1), N = nax * nay * naz;
+  for (long n = (long)blockIdx.x * blockDim.x + threadIdx.x; n < N;
+       n += (long)gridDim.x * blockDim.x) {
+    const unsigned r = (unsigned)n / (unsigned)nax;
+    const int i = (int)((unsigned)n - r * (unsigned)nax);
+    const int k = (int)(r / (unsigned)nay), j = (int)(r - (unsigned)k * (unsigned)nay);
+    DfAcc acc[27];
+#pragma unroll
+    for (int t = 0; t < 27; t++) acc[t] = DfAcc{0.f, 0.f};
+    unsigned m = 0u;
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+      const int ex = (e & 1) - 1, ey = ((e >> 1) & 1) - 1, ez = (e >> 2) - 1;
+      const int ei = i + ex, ej = j + ey, ek = k + ez;
+      if (ei < 0 || ei >= nax - 1 || ej < 0 || ej >= nay - 1 || ek < 0 || ek >= naz - 1)
+        continue;
+      const long p = ei + (long)(nax - 1) * (ej + (long)(nay - 1) * ek);
+      const int own = slot_of(-ex, -ey, -ez);
+      const unsigned dm = __ldg(emask + p);
+      if ((dm >> own) & 1u) continue;  // a Dirichlet row
+      float4 h[2], l[2];
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        h[q] = __ldcs(Ahi + (size_t)(2 * own + q) * E + p);
+        l[q] = __ldcs(Alo + (size_t)(2 * own + q) * E + p);
+      }
+#pragma unroll
+      for (int s = 0; s < 8; s++) {
+        const int t = 9 * (slot_z(s) + ez + 1) + 3 * (slot_y(s) + ey + 1) + slot_x(s) + ex + 1;
+        const float4 &hq = h[s >> 2], &lq = l[s >> 2];
+        const int w = s & 3;
+        const float hv = w == 0 ? hq.x : w == 1 ? hq.y : w == 2 ? hq.z : hq.w;
+        const float lv = w == 0 ? lq.x : w == 1 ? lq.y : w == 2 ? lq.z : lq.w;
+        if (!((dm >> s) & 1u)) {
+          acc_pair(acc[t], hv, lv);
+          m |= 1u << t;
+        }
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < 27; t++) {
+      const Df2 a = df_norm(acc[t]);
+      S[(size_t)t * N + n] = make_float2(a.h, a.l);
+    }
+    nm[n] = m;
+  }
+}
+
+// y = A x or A^T x, or y += with ACC, any FP64 x.  Here every thread splits
+// its 27 gathered values and scales each plane by itself, which makes it
+// bound by instruction issue (0.75 ms at 8.5M nodes, 94 us at 1.08M: about
+// the element-wise apply's time); the Krylov iterations split once per node.
+template <bool TRANS, bool ACC, bool KEEP>
+__global__ void __launch_bounds__(256, 4) stencil_apply(const StencilView v,
+                                                        const double *__restrict__ x,
+                                                        double *__restrict__ y,
+                                                        const int *skip, const int *skip2) {
+  if (skip && *(volatile const int *)skip) return;
+  if (skip2 && *(volatile const int *)skip2) return;
+  for (long n = (long)blockIdx.x * blockDim.x + threadIdx.x; n < v.N;
+       n += (long)gridDim.x * blockDim.x) {
+    const double o = stencil_row<TRANS, KEEP>(v, n, x);
+    y[n] = ACC ? y[n] + o : o;
+  }
+}
+
+template <bool TRANS, bool ACC>
+void apply_keep(const Handle &h, bool keep, int grid, const StencilView &v, const double *x,
+                double *y, const int *skip, const int *skip2, cudaStream_t s) {
+  if (keep)
+    stencil_apply<TRANS, ACC, true><<<grid, 256, 0, s>>>(v, x, y, skip, skip2);
+  else
+    stencil_apply<TRANS, ACC, false><<<grid, 256, 0, s>>>(v, x, y, skip, skip2);
+}
+
+}  // namespace
+
+StencilView stencil_view(const Handle &h) {
+  StencilView v;
+  v.S = h.st_S;
+  v.nm = h.st_nm;
+  v.N = h.N;
+  v.nax = h.nax;
+  v.pl = h.nax * h.nay;
+  return v;
+}
+
+bool stencil_keep(const Handle &h) { return 220.0 * h.N < 80.0e6; }
+
+bool stencil_ready(const Handle &h) {
+  return h.st_state == 1 && h.apply_mode == VDR_APPLY_STORED && !h.apply_fp32 &&
+         !h.gate_active && h.storage == VDR_STORE_DF;
+}
+
+cudaError_t ensure_stencil(Handle &h) {
+  if (h.st_state != 0 || !h.op64_valid || h.apply_mode != VDR_APPLY_STORED ||
+      h.storage != VDR_STORE_DF || h.opt.scatter != VDR_SCATTER_AUTO || h.perm_d || !h.Ahi ||
+      !h.emask || h.nax < 2 || h.nay < 2 || h.naz < 2)
+    return cudaSuccess;
+  const size_t N = (size_t)h.N;
+  if (!h.st_S) {
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || 240 * N > free_b / 2 ||
+        cudaMalloc(&h.st_S, sizeof(float2) * 27 * N) ||
+        cudaMalloc(&h.st_nm, sizeof(unsigned) * N) ||
+        cudaMalloc(&h.st_x, sizeof(float2) * 2 * (N + 2 * stencil_pad(h))) ||
+        cudaMemsetAsync(h.st_x, 0, sizeof(float2) * 2 * (N + 2 * stencil_pad(h)), h.stream)) {
+      cudaGetLastError();  // no room for the rows: the element-wise apply stays
+      cudaFree(h.st_S);
+      cudaFree(h.st_nm);
+      cudaFree(h.st_x);
+      h.st_S = nullptr;
+      h.st_nm = nullptr;
+      h.st_x = nullptr;
+      h.st_state = -1;
+      return cudaSuccess;
+    }
+  }
+  const long need = (h.N + 255L) / 256;
+  const int grid = (int)std::min<long>(need, (long)device_sm_count() * 32);
+  stencil_assemble<<<grid, 256, 0, h.stream>>>(h.Ahi, h.Alo, h.emask, h.nax, h.nay, h.naz,
+                                               h.st_S, h.st_nm);
+  count_launches(1);
+  const cudaError_t e = cudaGetLastError();
+  if (!e) h.st_state = 1;
+  return e;
+}
+
+cudaError_t launch_stencil_apply(const Handle &h, bool transpose, bool accumulate,
+                                 const double *x, double *y, const int *skip,
+                                 const int *skip2, cudaStream_t s) {
+  const StencilView v = stencil_view(h);
+  const bool keep = stencil_keep(h);
+  const int grid = (int)((h.N + 255L) / 256);
+  if (transpose) {
+    if (accumulate) apply_keep<true, true>(h, keep, grid, v, x, y, skip, skip2, s);
+    else apply_keep<true, false>(h, keep, grid, v, x, y, skip, skip2, s);
+  } else {
+    if (accumulate) apply_keep<false, true>(h, keep, grid, v, x, y, skip, skip2, s);
+    else apply_keep<false, false>(h, keep, grid, v, x, y, skip, skip2, s);
+  }
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+}  // namespace vdr

@@ -35,6 +35,11 @@ struct KState {
   unsigned int ticket;
   unsigned int pad2;
   unsigned int bar_count, bar_gen;  // grid barrier of the fused inner kernels
+  // the assembled-operator iteration: (rh, s), the next rho, the exponent that
+  // its pair vectors are scaled by, the largest exponents of the last
+  // direction and of the one being formed
+  double rhs, rho_next;
+  int pexp, pmax, pmax_next;
 };
 
 // A right preconditioner for BiCGStab beyond Jacobi: `enqueue` adds
@@ -210,6 +215,14 @@ struct Handle {
   int *flag = nullptr;     // device flag: an entry left the FP32 range
   double *diag = nullptr;  // [N] assembled diagonal, 1 on Dirichlet nodes
   double *dinv = nullptr;  // [N] 1/diag (the Jacobi preconditioner)
+
+  // the assembled 27-point operator of the structured numbering (stencil.cuh):
+  // st_state 0 not formed, 1 valid for the current operator, -1 no device
+  // memory for it; st_applies: single applies of the current operator
+  float2 *st_S = nullptr;       // [27][N]
+  unsigned *st_nm = nullptr;    // [N]
+  float2 *st_x = nullptr;       // two padded pair vectors: p^ and s^
+  int st_state = 0, st_applies = 0;
 
   // solver workspace
   double *work = nullptr;
@@ -397,6 +410,18 @@ cudaError_t launch_mask_vec(double *v, const unsigned char *mask, int N,
                             cudaStream_t s);
 cudaError_t launch_bc_to_mask(const int *bc, unsigned char *mask, int N,
                               cudaStream_t s);
+
+// ---- the assembled operator (stencil.cu) ----
+// Sums the element matrices into the 27-point rows on the handle's stream
+// unless they are current or the handle cannot have them (the double-float
+// store on the canonical structured numbering, scatter AUTO, device memory);
+// called before work that applies the operator several times.
+cudaError_t ensure_stencil(Handle &h);
+bool stencil_ready(const Handle &h);
+// y (+)= A x or A^T x from the assembled rows.
+cudaError_t launch_stencil_apply(const Handle &h, bool transpose, bool accumulate,
+                                 const double *x, double *y, const int *skip,
+                                 const int *skip2, cudaStream_t s);
 
 // ---- the 16-bit inner operator (half.cu) ----
 // Builds A^ = P A P D^-1 in the binary16 store from the current FP64
