@@ -115,3 +115,37 @@ def test_recorded_case(vdr, oracle, gpu_lib):
         for tr in (False, True):
             ref, _ = oracle.matvec0(prob.mesh.iss, bb, prob.bc, x, transpose=tr)
             assert rel_l2(s.apply(x, transpose=tr), ref) < TOL
+
+
+# node counts at the edges of the whole-solve kernel's launch shapes: one
+# cluster of 64, 128 and 192 threads a CTA (1024, 2048, 3072 nodes and one
+# plane more), grids of 128, 256, 512, 768 and 1024 threads a CTA on 152 SMs,
+# and the first size that runs as separate kernels
+SHAPES = [(15, 15, 3), (15, 15, 4), (15, 7, 15), (15, 15, 8), (15, 15, 11), (15, 15, 12),
+          (75, 31, 7), (75, 31, 8), (75, 31, 15), (75, 63, 15), (75, 63, 16), (75, 63, 23),
+          (75, 63, 31), (75, 63, 32)]
+
+
+@pytest.mark.parametrize("dims", SHAPES)
+def test_whole_solve_launch_shapes(vdr, gpu_lib, dims):
+    """From a warm and from a zero start, to 1e-11 against the element-wise
+    solve (distance bounded as above), and the reported residual against the
+    true one."""
+    torch = pytest.importorskip("torch")
+    prob = vdr.problems.rotation_shear(*dims, seed=85)
+    N, aM = prob.mesh.nnode, 0.3 * max(dims)
+    told = torch.tensor(np.cos(0.37 * np.arange(N)), device="cuda")
+    xs = {}
+    for scatter in ("auto", "atomic"):
+        with vdr.Solver(prob, vdr.Options(scatter=scatter), aH=2.0, aM=aM) as s:
+            b = torch.empty(N, dtype=torch.float64, device="cuda")
+            s.assemble_rhs_device(b, 3.0, aM, told)
+            for x0 in ("zero", "warm"):
+                x = torch.zeros_like(b) if x0 == "zero" else told.clone()
+                it, err, st = s.solve_device(b, x, tol=1e-11, itmax=2000)
+                assert st == 0 and err <= 1e-11, (dims, scatter, x0)
+                assert s.true_residual_device(b * torch.tensor(prob.bc == 0, device="cuda"),
+                                              x) < 2e-11
+                xs[scatter, x0] = x.cpu().numpy()
+    for x0 in ("zero", "warm"):
+        assert rel_l2(xs["auto", x0], xs["atomic", x0]) < 1e-8

@@ -25,6 +25,7 @@
 #include <cstring>
 
 #include "dfloat.cuh"
+#include "reduce.cuh"
 #include "stencil.cuh"
 #include "vdr_internal.h"
 
@@ -33,28 +34,20 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
+// Block sum of NQ <= 4 values, valid in warp 0.
 template <int NQ>
 __device__ __forceinline__ void block_sum(double (&v)[NQ]) {
-  __shared__ double sm[RED_THREADS / 32][MAXQ];
-#pragma unroll
-  for (int q = 0; q < NQ; q++)
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
-      v[q] += __shfl_xor_sync(FULL, v[q], off);
+  __shared__ double sm[RED_THREADS / 32][4];
+  static_assert(RED_THREADS == 256, "one fold over eight warps");
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const double f = warp_sums<NQ>(v, l);
   __syncthreads();
-  if (l == 0)
-#pragma unroll
-    for (int q = 0; q < NQ; q++) sm[w][q] = v[q];
+  if ((l & 7) == 0 && (l >> 3) < NQ) sm[w][l >> 3] = f;
   __syncthreads();
   if (w == 0) {
+    const double c = fold8((l >> 3) < NQ ? sm[l & 7][l >> 3] : 0.0);
 #pragma unroll
-    for (int q = 0; q < NQ; q++) {
-      v[q] = (l < (int)(blockDim.x >> 5)) ? sm[l][q] : 0.0;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1)
-        v[q] += __shfl_xor_sync(FULL, v[q], off);
-    }
+    for (int q = 0; q < NQ; q++) v[q] = __shfl_sync(FULL, c, 8 * q);
   }
 }
 
@@ -105,6 +98,7 @@ struct Vec {
   double *x, *r, *rh, *p, *v, *ph, *s, *sh, *t;  // BiCGStab
   double *rr, *pp, *z, *zz;                      // BiCG (r, p, x shared)
   float2 *php, *shp;  // p^ and s^ as pairs (assembled operator)
+  double *w;          // A^T rh (assembled operator, in p^'s place)
 };
 
 // Grid-stride loops unrolled U times with every load of the U elements
@@ -134,7 +128,7 @@ template <bool BICG>
 __global__ void __launch_bounds__(RED_THREADS) k_start(Vec a) {
   double v[3] = {0.0, 0.0, 0.0};
   double bv[U], rv[U], dv[U];
-  int em = 0;
+  int em = 0, er = 0;
   VLOOP(bv[u] = ok ? a.b[i] : 0.0; rv[u] = ok ? a.r[i] : 0.0;
         dv[u] = (ok && (BICG || a.php)) ? a.dinv[i] : 0.0;,
         const double ri = bv[u] - rv[u];
@@ -145,12 +139,19 @@ __global__ void __launch_bounds__(RED_THREADS) k_start(Vec a) {
         } else {
           a.rh[i] = ri;
         }
-        if (a.php) em = max(em, df_exp(ri) + df_exp(dv[u]) - 1022);
+        if (a.php) {
+          em = max(em, df_exp(ri) + df_exp(dv[u]) - 1022);
+          er = max(er, df_exp(ri));
+        }
         v[0] += bv[u] * bv[u];
         v[1] += ri * ri;)
   if (a.php) {
     em = __reduce_max_sync(FULL, em);
-    if ((threadIdx.x & 31) == 0) atomicMax(&a.st->pmax, em);
+    er = __reduce_max_sync(FULL, er);
+    if ((threadIdx.x & 31) == 0) {
+      atomicMax(&a.st->pmax, em);
+      atomicMax(&a.st->rmax, er);
+    }
   }
   double o[3];
   if (grid_sum<3>(v, a.partials, &a.st->ticket, o)) {
@@ -459,75 +460,84 @@ Vec make_vec(Handle &h, const double *b, double *x) {
   if (h.st_x) {
     a.php = h.st_x + stencil_pad(h);
     a.shp = a.php + N + 2 * stencil_pad(h);
+    a.w = a.ph;
   }
   return a;
 }
 
 // ---- BiCGStab on the assembled rows (stencil.cuh) ----
 // With the rows assembled a node's product is one thread's sum, so the
-// iteration needs four kernels, no cleared outputs and no atomics:
-//   bst_v   v = A p^ with (rh, v)                      -> alpha
-//   bst_s   s = r - alpha v, s^ = D^-1 s with ||s||, (rh, s)
-//   bst_t   t = A s^ with (t, s), (t, t), (rh, t)      -> omega, next rho
-//   bst_p   x, r, the next p and p^ in one pass with ||r||
-// The next rho is (rh, r) = (rh, s) - omega (rh, t), known before r is
-// formed, which lets the direction update share the pass over x and r.
+// iteration needs three kernels, no cleared outputs and no atomics:
+//   bst_v   v = A p^, s = r - alpha v, s^ = D^-1 s with (s, s), (rh, s)
+//   bst_t   t = A s^ with (t, s), (t, t), (rh, t)     -> omega, next rho
+//   bst_p   x, r, the next p and p^ with (r, r), (w, p^)  -> next alpha
+// w = A^T rh, formed once, gives alpha = rho / (w, p^) before the product it
+// scales; the next rho is (rh, s) - omega (rh, t), known before r is formed.
 // p^ and s^ exist only as the products' inputs, pairs scaled by the largest
 // exponent of the direction before (a direction would have to grow 2^100
 // times in one iteration to leave the pairs' range, which then reads as a
-// breakdown).  610 bytes per node and iteration against 1,024 E + ~240 N
+// breakdown).  618 bytes per node and iteration against 1,024 E + ~240 N
 // element-wise; each kernel's last block adds the block partials in a fixed
 // order.
+
+// p = rh = r; p^ and rh as pairs (rh in s^'s place, for w).
 __global__ void __launch_bounds__(RED_THREADS) bst_first(Vec a) {
   KState *st = a.st;
   if (st->done) return;
-  const int e = st->pmax, shift = e - 1023;
+  const int e = st->pmax, er = st->rmax;
   double rv[U], dv[U];
   unsigned char mv[U];
   VLOOP(rv[u] = ok ? a.r[i] : 0.0; dv[u] = ok ? a.dinv[i] : 0.0; mv[u] = ok ? a.m[i] : 1;,
         a.p[i] = rv[u];
-        a.php[i] = mv[u] ? make_float2(0.f, 0.f) : stencil_pair(rv[u] * dv[u], shift);)
+        a.shp[i] = mv[u] ? make_float2(0.f, 0.f) : stencil_pair(rv[u], er - 1023);
+        a.php[i] = mv[u] ? make_float2(0.f, 0.f) : stencil_pair(rv[u] * dv[u], e - 1023);)
   if (blockIdx.x == 0 && threadIdx.x == 0) st->pexp = e;
+}
+
+// The alpha of the direction whose (w, p^) is wp.
+__device__ __forceinline__ void bst_alpha(KState *st, double wp) {
+  if (wp == 0.0 || !finite(wp)) {
+    st->status = VDR_BREAKDOWN;
+    st->reason = 2;
+    st->done = 1;
+  } else {
+    st->alpha = st->rho / wp;
+  }
+}
+
+// w = A^T rh with (w, p^).
+__global__ void __launch_bounds__(RED_THREADS, 4) bst_w(Vec a, StencilView w) {
+  if (a.st->done) return;
+  const int shift = a.st->rmax - 1023;
+  double v[1] = {0.0};
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n;
+       i += (long)gridDim.x * blockDim.x) {
+    const double o = stencil_row_pairs<true, false>(w, i, a.shp, shift);
+    a.w[i] = o;
+    if (!a.m[i]) v[0] += o * (a.p[i] * a.dinv[i]);
+  }
+  double o[1];
+  if (grid_sum<1>(v, a.partials, &a.st->ticket, o)) bst_alpha(a.st, o[0]);
 }
 
 template <bool KEEP>
 __global__ void __launch_bounds__(RED_THREADS, 4) bst_v(Vec a, StencilView w) {
   if (a.st->done) return;
   const int shift = a.st->pexp - 1023;
-  double v[1] = {0.0};
+  const double al = a.st->alpha;
+  double v[2] = {0.0, 0.0};
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n;
        i += (long)gridDim.x * blockDim.x) {
-    const double o = stencil_row_pairs<KEEP>(w, i, a.php, shift);
+    const double ri = a.r[i], di = a.dinv[i], hi = a.rh[i];
+    const bool mi = a.m[i] != 0;
+    const double o = stencil_row_pairs<false, KEEP>(w, i, a.php, shift);
+    const double si = ri - al * o;
     a.v[i] = o;
-    v[0] += a.rh[i] * o;
+    a.s[i] = si;
+    a.shp[i] = mi ? make_float2(0.f, 0.f) : stencil_pair(si * di, shift);
+    v[0] += si * si;
+    v[1] += hi * si;
   }
-  double o[1];
-  if (grid_sum<1>(v, a.partials, &a.st->ticket, o)) {
-    KState *st = a.st;
-    if (o[0] == 0.0 || !finite(o[0])) {
-      st->status = VDR_BREAKDOWN;
-      st->reason = 2;
-      st->done = 1;
-    } else {
-      st->alpha = st->rho / o[0];
-    }
-  }
-}
-
-__global__ void __launch_bounds__(RED_THREADS) bst_s(Vec a) {
-  if (a.st->done) return;
-  const double al = a.st->alpha;
-  const int shift = a.st->pexp - 1023;
-  double v[2] = {0.0, 0.0};
-  double rv[U], vv[U], dv[U], hv[U];
-  unsigned char mv[U];
-  VLOOP(rv[u] = ok ? a.r[i] : 0.0; vv[u] = ok ? a.v[i] : 0.0;
-        dv[u] = ok ? a.dinv[i] : 0.0; hv[u] = ok ? a.rh[i] : 0.0; mv[u] = ok ? a.m[i] : 1;,
-        const double si = rv[u] - al * vv[u];
-        a.s[i] = si;
-        a.shp[i] = mv[u] ? make_float2(0.f, 0.f) : stencil_pair(si * dv[u], shift);
-        v[0] += si * si;
-        v[1] += hv[u] * si;)
   double o[2];
   if (grid_sum<2>(v, a.partials, &a.st->ticket, o)) {
     KState *st = a.st;
@@ -544,11 +554,12 @@ __global__ void __launch_bounds__(RED_THREADS, 4) bst_t(Vec a, StencilView w) {
   double v[3] = {0.0, 0.0, 0.0};
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n;
        i += (long)gridDim.x * blockDim.x) {
-    const double o = stencil_row_pairs<KEEP>(w, i, a.shp, shift);
+    const double si = a.s[i], hi = a.rh[i];
+    const double o = stencil_row_pairs<false, KEEP>(w, i, a.shp, shift);
     a.t[i] = o;
-    v[0] += o * a.s[i];
+    v[0] += o * si;
     v[1] += o * o;
-    v[2] += a.rh[i] * o;
+    v[2] += hi * o;
   }
   double o[3];
   if (grid_sum<3>(v, a.partials, &a.st->ticket, o)) {
@@ -564,18 +575,19 @@ __global__ void __launch_bounds__(RED_THREADS, 4) bst_t(Vec a, StencilView w) {
   }
 }
 
-__global__ void __launch_bounds__(RED_THREADS) bst_p(Vec a) {
+// Two nodes in flight per thread and 64 registers: the pass is bound by the
+// FP64 pipe (nine operations a node) about as much as by its 97 bytes, and
+// wants warps more than loads per thread.
+__global__ void __launch_bounds__(RED_THREADS, 4) bst_p(Vec a) {
   KState *stc = a.st;
   if (stc->done) return;
   const double al = stc->alpha;
-  if (stc->sconv) {  // s met the tolerance: x += alpha p^, r = s
+  const long stride = (long)gridDim.x * blockDim.x;
+  const long i00 = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (stc->sconv) {  // s met the tolerance: x += alpha p^
     double v[1] = {0.0};
-    double xv[U], pv[U], sv[U], dv[U];
-    unsigned char mv[U];
-    VLOOP(xv[u] = ok ? a.x[i] : 0.0; pv[u] = ok ? a.p[i] : 0.0; dv[u] = ok ? a.dinv[i] : 0.0;
-          sv[u] = ok ? a.s[i] : 0.0; mv[u] = ok ? a.m[i] : 1;,
-          if (!mv[u]) a.x[i] = xv[u] + dv[u] * (al * pv[u]);
-          a.r[i] = sv[u];)
+    for (long i = i00; i < a.n; i += stride)
+      if (!a.m[i]) a.x[i] += a.dinv[i] * (al * a.p[i]);
     double o[1];
     if (grid_sum<1>(v, a.partials, &a.st->ticket, o)) {
       KState *st = a.st;
@@ -590,26 +602,45 @@ __global__ void __launch_bounds__(RED_THREADS) bst_p(Vec a) {
   const double beta = (rho1 / stc->rho) * (al / om);
   const int e = stc->pmax, shift = e - 1023;
   int em = 0;
-  double v[1] = {0.0};
-  double xv[U], pv[U], sv[U], tv[U], vv[U], dv[U];
-  unsigned char mv[U];
-  VLOOP(xv[u] = ok ? a.x[i] : 0.0; pv[u] = ok ? a.p[i] : 0.0; sv[u] = ok ? a.s[i] : 0.0;
-        tv[u] = ok ? a.t[i] : 0.0; vv[u] = ok ? a.v[i] : 0.0; dv[u] = ok ? a.dinv[i] : 0.0;
-        mv[u] = ok ? a.m[i] : 1;,
-        const double ri = sv[u] - om * tv[u];
-        const double pi = ri + beta * (pv[u] - om * vv[u]);
-        if (!mv[u]) a.x[i] = xv[u] + dv[u] * (al * pv[u] + om * sv[u]);
-        a.r[i] = ri;
-        a.p[i] = pi;
-        const double hi = mv[u] ? 0.0 : pi * dv[u];
-        a.php[i] = stencil_pair(hi, shift);
-        em = max(em, df_exp(hi));
-        v[0] += ri * ri;)
+  double v[2] = {0.0, 0.0};
+  constexpr int UP = 2;
+  for (long i0 = i00; i0 < a.n; i0 += UP * stride) {
+    double xv[UP], pv[UP], sv[UP], tv[UP], vv[UP], dv[UP], wv[UP];
+    unsigned char mv[UP];
+#pragma unroll
+    for (int u = 0; u < UP; u++) {
+      const long i = i0 + u * stride;
+      const bool ok = i < a.n;
+      xv[u] = ok ? a.x[i] : 0.0;
+      pv[u] = ok ? a.p[i] : 0.0;
+      sv[u] = ok ? a.s[i] : 0.0;
+      tv[u] = ok ? a.t[i] : 0.0;
+      vv[u] = ok ? a.v[i] : 0.0;
+      dv[u] = ok ? a.dinv[i] : 0.0;
+      wv[u] = ok ? a.w[i] : 0.0;
+      mv[u] = ok ? a.m[i] : 1;
+    }
+#pragma unroll
+    for (int u = 0; u < UP; u++) {
+      const long i = i0 + u * stride;
+      if (i >= a.n) continue;
+      const double ri = sv[u] - om * tv[u];
+      const double pi = ri + beta * (pv[u] - om * vv[u]);
+      if (!mv[u]) a.x[i] = xv[u] + dv[u] * (al * pv[u] + om * sv[u]);
+      a.r[i] = ri;
+      a.p[i] = pi;
+      const double hi = mv[u] ? 0.0 : pi * dv[u];
+      a.php[i] = stencil_pair(hi, shift);
+      em = max(em, df_exp(hi));
+      v[0] += ri * ri;
+      v[1] += wv[u] * hi;
+    }
+  }
   em = __reduce_max_sync(FULL, em);
   if ((threadIdx.x & 31) == 0) atomicMax(&stc->pmax_next, em);
   __threadfence();
-  double o[1];
-  if (grid_sum<1>(v, a.partials, &a.st->ticket, o)) {
+  double o[2];
+  if (grid_sum<2>(v, a.partials, &a.st->ticket, o)) {
     KState *st = a.st;
     st->iter += 1;
     st->pexp = e;
@@ -641,20 +672,19 @@ __global__ void __launch_bounds__(RED_THREADS) bst_p(Vec a) {
         st->done = 1;
       }
     }
+    if (!st->done) bst_alpha(st, o[1]);
   }
 }
 
 cudaError_t launch_stencil_iteration(Handle &h, const Vec &a, cudaStream_t s) {
   const StencilView w = stencil_view(h);
   const bool keep = stencil_keep(h);
-  const int gv = red_grid(h.N);
-  const int gs = std::min(gv, device_sm_count() * 4);
+  const int gs = std::min(red_grid(h.N), device_sm_count() * 4);
   if (keep) bst_v<true><<<gs, RED_THREADS, 0, s>>>(a, w);
   else bst_v<false><<<gs, RED_THREADS, 0, s>>>(a, w);
-  bst_s<<<gv, RED_THREADS, 0, s>>>(a);
   if (keep) bst_t<true><<<gs, RED_THREADS, 0, s>>>(a, w);
   else bst_t<false><<<gs, RED_THREADS, 0, s>>>(a, w);
-  bst_p<<<gv, RED_THREADS, 0, s>>>(a);
+  bst_p<<<gs, RED_THREADS, 0, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -729,7 +759,7 @@ cudaError_t ensure_solver_workspace(Handle &h, int nvec) {
 
 // Kernels of one captured iteration.
 long launches_graph_nodes(Handle &h, int method, const Precond *prec) {
-  if (method == VDR_SOLVER_BICGSTAB && !prec && stencil_ready(h)) return 4;
+  if (method == VDR_SOLVER_BICGSTAB && !prec && stencil_ready(h)) return 3;
   if (method == VDR_SOLVER_BICGSTAB && !prec && h.fused64) return 2 + 2 * apply_launches(h);
   long n = (method == VDR_SOLVER_BICGSTAB ? 5 : 3) +
            (method != VDR_SOLVER_BICGSTAB && can_apply_both(h) ? 1 : 2) *
@@ -756,6 +786,25 @@ int solve_device(Handle &h, int method, const double *b, double *x,
   const int g = red_grid(h.N);
   const long long launches0 = launches_so_far();
   h.last = vdr_solve_stats{};
+
+  if (method == VDR_SOLVER_BICGSTAB && !prec && !hist && resident_fits(h)) {
+    if (!(e = launch_resident(h, b, x, tol, itmax, stall_window))) {
+      if ((e = cudaMemcpyAsync(&h.h_st[0], h.st, sizeof(KState), cudaMemcpyDeviceToHost, s)) ||
+          (e = cudaStreamSynchronize(s)))
+        return cuda_fail(e, "solve");
+      const KState &fin = h.h_st[0];
+      const int status = fin.done ? fin.status : VDR_NOT_CONVERGED;
+      h.last.iterations = fin.iter;
+      h.last.status = status;
+      h.last.kernel_launches = 1;
+      h.last.breakdown = (status == VDR_BREAKDOWN || fin.reason == 6) ? fin.reason : 0;
+      if (iter) *iter = fin.iter;
+      if (err) *err = fin.err;
+      return status;
+    }
+    cudaGetLastError();  // no cooperative launch here: the iteration as kernels
+    h.resident = false;
+  }
 
   // KState scalars the kernels read: tol, itmax (ticket stays 0 between uses).
   KState init{};
@@ -847,7 +896,8 @@ int solve_device(Handle &h, int method, const double *b, double *x,
   }
   if (fusable && rows) {  // the first search direction and its pairs
     bst_first<<<g, RED_THREADS, 0, s>>>(a);
-    count_launches(1);
+    bst_w<<<std::min(g, device_sm_count() * 4), RED_THREADS, 0, s>>>(a, stencil_view(h));
+    count_launches(2);
     if ((e = cudaGetLastError())) return cuda_fail(e, "first direction");
   } else if (fusable && h.fused64) {  // the first search direction p = r, p^ = D^-1 r, v = 0
     bs_p<<<g, RED_THREADS, 0, s>>>(a);

@@ -1,0 +1,597 @@
+// resident.cu -- a whole BiCGStab solve in one launch, for meshes whose rows
+// and vectors fit on the chip (one node per thread, at most 1024 per SM).
+//
+// At these sizes an iteration moves little data: what it costs is launches,
+// FP64 sums on a pipe that takes 16 cycles per warp instruction, and waits
+// (31 us per iteration at 2,800 nodes with four launches, of which the
+// products are 2 us).  Here a node's vector entries stay in its thread's
+// registers for the whole solve and only p^ and s^ (a pair each) are handed
+// to the neighbours.  The CTAs meet three times per iteration:
+//
+//   v = A p^, s = r - alpha v, s^ out             | (s,s), (rh,s)
+//   t = A s^                                       | (t,s), (t,t), (rh,t)
+//   x, r, p, p^ out                                | (r,r), (w,p^)
+//
+// with w = A^T rh formed once, so that alpha = rho / (w, p^) is known before
+// the product that it scales, and the next rho is (rh,s) - omega (rh,t).
+// Sums: per warp by a transposing butterfly (5-6 FP64 adds for up to four
+// quantities), then one warp per CTA adds all partials in the same order, so
+// all CTAs hold bit-identical scalars and take the same exit.  Divisions run
+// on that warp only (on every warp they took longer than the products).
+//
+// CLUSTER: up to 16 CTAs of at most 192 nodes in one cluster; p^, s^ and the
+// partials lie in shared memory and are read across the cluster, the
+// meetings are cluster barriers.  IN_REGS, IN_SMEM: a cooperative grid, one
+// CTA per SM, p^ and s^ through L2, meetings at a counter (bounded waits:
+// VDR_TIMEOUT, reason 7); a node's 27 pairs stay in registers up to 512
+// threads, in shared memory (216 bytes a thread) above.  Per iteration,
+// cluster / grid: 8.1 us at 448 nodes, 9.6 / 12 at 1,170, 11 / 12.5 at 2,800,
+// 19.5 / 12.8 at 7,000 (reads across a cluster are slow in number), then 14.1
+// at 18,500, 20 at 75,000, 26 at 100,000, 31 at 148,000; four kernels per
+// iteration: 31 at 2,800, 53 at 100,000.
+#include <cuda_runtime.h>
+#include <math.h>
+
+#include <algorithm>
+
+#include "reduce.cuh"
+#include "stencil.cuh"
+
+namespace vdr {
+namespace {
+
+constexpr long long RES_LIMIT = 2000000000LL;  // ~1 s of clocks
+constexpr int RES_NB = 5;                      // at most 32 RES_NB CTAs in the grid
+constexpr int CLUSTER_MAX = 16;
+
+enum { CLUSTER, IN_REGS, IN_SMEM };
+// partial sums' places: (s,s) (rh,s) | (t,s) (t,t) (rh,t) | (r,r) (w,p^)
+enum { AT_C = 0, AT_D = 2, AT_A = 5, SLOTS = 7 };
+
+struct ResArgs {
+  StencilView w;
+  const double *b, *dinv;
+  const unsigned char *m;
+  double *x;
+  float2 *php, *shp;  // the grid's p^ and s^
+  KState *st;
+  double *part;  // [SLOTS][gridDim]
+  int *ipart;    // [3][gridDim]: largest exponents
+  double tol;
+  int itmax, window;
+};
+
+struct ResShared {
+  double s[SLOTS][32];  // this CTA's sums, per warp
+  int e[3][32];
+  double tot[6];  // totals, or scalars made of them
+  int etot[2];
+  int ok;
+};
+
+// ---- thread-block clusters
+__device__ __forceinline__ void cluster_meet() {
+  asm volatile(
+      "barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
+          : "memory");
+}
+__device__ __forceinline__ unsigned cluster_addr(const void *p, int cta) {
+  unsigned a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;"
+      : "=r"(a)
+      : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(cta));
+  return a;
+}
+__device__ __forceinline__ double cluster_f64(unsigned a) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ int cluster_s32(unsigned a) {
+  int v;
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 cluster_pair(unsigned a) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a)
+               : "memory");
+  return v;
+}
+
+// A meeting of all CTAs.  Each leaves its sums of Q quantities at place SLOT
+// (and NE largest exponents at place ES); what any thread wrote before is
+// visible to all after.  Then the totals of the R quantities from place READ
+// on (R = 0: none) are in sh.tot and the largest exponents in sh.etot, and
+// `scalars` runs on warp 0 with them there, its results in sh for all
+// threads.  No place is written again before a meeting that follows its
+// reads.
+template <int MODE, int T, int Q, int NE, int R, int SLOT, int READ, int ES, typename F>
+__device__ __forceinline__ bool meet(ResShared &sh, const ResArgs &a, const double (&v)[Q],
+                                     const int (&em)[NE > 0 ? NE : 1], unsigned &target,
+                                     F scalars) {
+  constexpr int nw = T / 32;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int B = (int)gridDim.x;
+  const double f = warp_sums<Q>(v, lane);
+  if ((lane & 7) == 0 && (lane >> 3) < Q) sh.s[SLOT + (lane >> 3)][w] = f;
+#pragma unroll
+  for (int k = 0; k < NE; k++) {
+    const int e = __reduce_max_sync(FULLR, em[k]);
+    if (lane == 0) sh.e[ES + k][w] = e;
+  }
+  constexpr int RP = R > 0 ? R : 1, R4 = RP < 4 ? RP : 4;
+  double tot[RP];
+  int etot[NE > 0 ? NE : 1] = {0};
+  if (MODE == CLUSTER) {
+    cluster_meet();
+    if (R == 0 && NE == 0) return true;
+    if (w == 0) {  // all warps' sums of all CTAs, every load before the adds
+      constexpr int NI = (CLUSTER_MAX * nw + 31) / 32;
+      double in[NI][RP];
+      int ein[NI][NE > 0 ? NE : 1];
+#pragma unroll
+      for (int i = 0; i < NI; i++) {
+        const int j = lane + 32 * i, c = min(j / nw, B - 1), u = j % nw;
+        const unsigned at = cluster_addr(&sh.s[READ][u], c);
+        if (R > 0)
+#pragma unroll
+          for (int k = 0; k < RP; k++)
+            in[i][k] = cluster_f64(at + (unsigned)(k * sizeof sh.s[0]));
+#pragma unroll
+        for (int k = 0; k < NE; k++) ein[i][k] = cluster_s32(cluster_addr(&sh.e[ES + k][u], c));
+      }
+#pragma unroll
+      for (int k = 0; k < RP; k++) tot[k] = 0.0;
+#pragma unroll
+      for (int i = 0; i < NI; i++) {
+        const bool mine = lane + 32 * i < B * nw;
+        if (R > 0 && (i == 0 || 32 * i < B * nw))
+#pragma unroll
+          for (int k = 0; k < RP; k++) tot[k] += mine ? in[i][k] : 0.0;
+#pragma unroll
+        for (int k = 0; k < NE; k++) etot[k] = max(etot[k], ein[i][k]);
+      }
+    }
+  } else {
+    target += gridDim.x;
+    __syncthreads();
+    if (w == 0) {
+      const int q = lane >> 3, sub = lane & 7;
+      double c = 0.0;
+      for (int k = sub; k < nw; k += 8) c += sh.s[SLOT + (q < Q ? q : 0)][k];
+      c = fold8(c);
+      if (sub == 0 && q < Q) __stcg(a.part + (size_t)(SLOT + q) * B + blockIdx.x, c);
+#pragma unroll
+      for (int k = 0; k < NE; k++) {
+        const int e = __reduce_max_sync(FULLR, lane < nw ? sh.e[ES + k][lane] : 0);
+        if (lane == 0) __stcg(a.ipart + (size_t)(ES + k) * B + blockIdx.x, e);
+      }
+      __syncwarp();
+      unsigned *bar = &a.st->bar_count;
+      if (lane == 0)
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+      __syncwarp();
+      // the whole warp polls: with one lane polling, what followed ran split
+      // (13 us more per iteration at 145 CTAs)
+      const long long t0 = clock64();
+      bool met, late = false;
+      do {
+        unsigned seen;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+        met = (int)(seen - target) >= 0;
+        late = clock64() - t0 > RES_LIMIT;
+      } while (!__all_sync(FULLR, met || late));
+      if (lane == 0) sh.ok = met;
+      if (R > 0) {
+        double in[RES_NB][RP];  // every load before the first add
+#pragma unroll
+        for (int i = 0; i < RES_NB; i++)
+#pragma unroll
+          for (int k = 0; k < RP; k++)
+            in[i][k] = __ldcg(a.part + (size_t)(READ + k) * B + min(lane + 32 * i, B - 1));
+#pragma unroll
+        for (int k = 0; k < RP; k++) tot[k] = lane < B ? in[0][k] : 0.0;
+#pragma unroll
+        for (int i = 1; i < RES_NB; i++)
+          if (32 * i < B)
+#pragma unroll
+            for (int k = 0; k < RP; k++) tot[k] += lane + 32 * i < B ? in[i][k] : 0.0;
+      }
+#pragma unroll
+      for (int k = 0; k < NE; k++)
+#pragma unroll
+        for (int i = 0; i < RES_NB; i++)
+          etot[k] =
+              max(etot[k], __ldcg(a.ipart + (size_t)(ES + k) * B + min(lane + 32 * i, B - 1)));
+    }
+  }
+  if (w == 0) {
+    if (R > 0) {
+      double u[R4];
+#pragma unroll
+      for (int k = 0; k < R4; k++) u[k] = tot[k];
+      const double g = warp_sums<R4>(u, lane);
+      if ((lane & 7) == 0 && (lane >> 3) < R4) sh.tot[lane >> 3] = g;
+      if (R > 4) {
+        const double u1[1] = {tot[RP - 1]};
+        const double g1 = warp_sums<1>(u1, lane);
+        if (lane == 0) sh.tot[4] = g1;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < NE; k++) {
+      const int e = __reduce_max_sync(FULLR, etot[k]);
+      if (lane == 0) sh.etot[k] = e;
+    }
+    __syncwarp();
+    if (R > 0) scalars(lane);
+  }
+  __syncthreads();
+  return MODE == CLUSTER || sh.ok != 0;
+}
+
+__device__ __forceinline__ void res_timeout(KState *st) {
+  if (threadIdx.x == 0) {
+    st->status = VDR_TIMEOUT;
+    st->reason = 7;
+    st->done = 1;
+  }
+}
+
+__device__ __forceinline__ double row_value(const DfAcc &acc, int shift) {
+  double o = df_to_double(acc.s, acc.c);
+  if (!df_scale(o, shift)) o = ldexp(o, shift);
+  return o;
+}
+
+__device__ __forceinline__ float2 masked_pair(bool msk, double d, int shift) {
+  return msk ? make_float2(0.f, 0.f) : stencil_pair(d, shift);
+}
+
+template <int MODE, int T>
+__global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
+  extern __shared__ float2 dyn[];  // CLUSTER: p^ and s^, [2][T]; IN_SMEM: rows, [27][T]
+  __shared__ ResShared sh;
+  const int N = a.w.N, n = (int)(blockIdx.x * T + threadIdx.x);
+  const bool on = n < N;
+  unsigned target = 0;
+  const int none[1] = {0};
+  const auto nothing = [](int) {};
+  double x = 0.0, r = 0.0, p = 0.0, v = 0.0, s = 0.0, t = 0.0, rh = 0.0, wn = 0.0;
+  const double di = on ? a.dinv[n] : 0.0;
+  const bool msk = on ? a.m[n] != 0 : true;
+
+  // the node's row, and in a cluster where its neighbours' entries lie (its
+  // own where there is none: the row holds a zero)
+  float2 A[MODE == IN_SMEM ? 1 : 27];
+  unsigned nb[MODE == CLUSTER ? 27 : 1];
+#pragma unroll
+  for (int k = 0; k < 27; k++) {
+    const float2 e = on ? __ldcg(a.w.S + (size_t)k * N + n) : make_float2(0.f, 0.f);
+    if (MODE == IN_SMEM) dyn[k * T + threadIdx.x] = e;
+    else A[MODE == IN_SMEM ? 0 : k] = e;
+    if (MODE == CLUSTER) {
+      const int q = n + stencil_off(k, a.w.nax, a.w.pl);
+      const int u = q >= 0 && q < (int)gridDim.x * T ? q : n;
+      nb[MODE == CLUSTER ? k : 0] = cluster_addr(dyn + u % T, u / T);
+    }
+  }
+  if (MODE == CLUSTER) {
+    dyn[threadIdx.x] = dyn[T + threadIdx.x] = make_float2(0.f, 0.f);
+    cluster_meet();  // every CTA runs before its memory is read
+  }
+  // the entries handed out: which = 0 p^, 1 s^
+  const auto put = [&](int which, float2 e) {
+    if (MODE == CLUSTER) dyn[which * T + threadIdx.x] = e;
+    else if (on) (which ? a.shp : a.php)[n] = e;
+  };
+  const auto get = [&](int which, int k) {
+    if (MODE == CLUSTER)
+      return cluster_pair(nb[MODE == CLUSTER ? k : 0] + (unsigned)(which * T * sizeof(float2)));
+    return __ldcg((which ? a.shp : a.php) + (on ? n : 0) + stencil_off(k, a.w.nax, a.w.pl));
+  };
+  const auto row = [&](int which, int shift) {
+    DfAcc acc{0.f, 0.f};
+    constexpr int G = MODE == IN_SMEM ? 9 : 27;  // entries in flight
+#pragma unroll
+    for (int z = 0; z < 27; z += G) {
+      float2 xv[G];
+#pragma unroll
+      for (int c = 0; c < G; c++) xv[c] = get(which, z + c);
+#pragma unroll
+      for (int c = 0; c < G; c++) {
+        const float2 e = MODE == IN_SMEM ? dyn[(z + c) * T + threadIdx.x]
+                                         : A[MODE == IN_SMEM ? 0 : z + c];
+        df_fma_acc(acc, e.x, e.y, xv[c].x, xv[c].y);
+      }
+    }
+    return row_value(acc, shift);
+  };
+
+  // x masked in place; r = b - A x (A x skipped when x is zero)
+  {
+    x = msk ? 0.0 : a.x[n];
+    const double z[1] = {0.0};
+    const int e1[1] = {df_exp(x)};
+    if (!meet<MODE, T, 1, 1, 0, AT_C, AT_C, 2>(sh, a, z, e1, target, nothing))
+      return res_timeout(a.st);
+  }
+  const int ex = sh.etot[0];
+  if (ex) {
+    put(0, masked_pair(msk, x, ex - 1023));
+    const double z[1] = {0.0};
+    if (!meet<MODE, T, 1, 0, 0, AT_D, AT_D, 0>(sh, a, z, none, target, nothing))
+      return res_timeout(a.st);
+    v = row(0, ex - 1023);
+  }
+  {
+    const double bi = msk ? 0.0 : a.b[n];
+    r = bi - (msk ? 0.0 : v);
+    rh = p = r;
+    const double q[2] = {bi * bi, r * r};
+    const int em[2] = {df_exp(r), df_exp(msk ? 0.0 : r * di)};
+    if (!meet<MODE, T, 2, 2, 2, AT_A, AT_A, 0>(sh, a, q, em, target, nothing))
+      return res_timeout(a.st);
+  }
+  const double bnrm2 = sh.tot[0];
+  double rho = sh.tot[1], rr2 = rho;
+  // ||r|| <= tol ||b|| as squares; a NaN or overflowed sum is told apart first
+  const double thr = a.tol * a.tol * bnrm2;
+  const int er = sh.etot[0];
+  int pexp = sh.etot[1];
+  int iter = 0, status = VDR_NOT_CONVERGED, reason = 0, since = 0;
+  double best2 = INFINITY;
+  bool done = false;
+  if (bnrm2 == 0.0) {  // b = 0: the solution is x = 0
+    x = 0.0;
+    status = VDR_OK;
+    rr2 = 0.0;
+    done = true;
+  } else if (!isfinite(bnrm2) || !isfinite(rr2)) {
+    status = VDR_BREAKDOWN;
+    reason = 5;
+    done = true;
+  } else if (rr2 <= thr) {
+    status = VDR_OK;
+    done = true;
+  } else if (a.itmax <= 0) {
+    done = true;
+  }
+  double al = 0.0, iwp = 0.0;
+  // alpha = rho / (w, p^) and 1 / (w, p^), on two lanes of one division
+  const auto alpha_of = [&](int lane, double wp) {
+    const double d = (lane ? 1.0 : rho) / wp;
+    if (lane < 2) sh.tot[2 + lane] = d;
+  };
+  if (!done) {
+    // p^ = D^-1 r, and w = A^T rh (the neighbours' rows, from L2)
+    put(0, masked_pair(msk, p * di, pexp - 1023));
+    put(1, masked_pair(msk, rh, er - 1023));
+    double q[1] = {0.0};
+    if (!meet<MODE, T, 1, 0, 0, AT_C, AT_C, 0>(sh, a, q, none, target, nothing))
+      return res_timeout(a.st);
+    DfAcc acc{0.f, 0.f};
+    for (int z = 0; z < 27; z += 9)
+#pragma unroll
+      for (int c = 0; c < 9; c++) {
+        const int k = z + c, o = n + stencil_off(k, a.w.nax, a.w.pl);
+        if (!on || o < 0 || o >= N) continue;
+        const float2 e = __ldcg(a.w.S + (size_t)(26 - k) * N + o);
+        float2 xv;
+        if (MODE == CLUSTER)
+          xv = cluster_pair(cluster_addr(dyn + T + o % T, o / T));
+        else
+          xv = __ldcg(a.shp + o);
+        df_fma_acc(acc, e.x, e.y, xv.x, xv.y);
+      }
+    wn = row_value(acc, er - 1023);
+    if (!msk) q[0] = wn * (p * di);
+    if (!meet<MODE, T, 1, 0, 1, AT_D, AT_D, 0>(sh, a, q, none, target,
+                                            [&](int lane) { alpha_of(lane, sh.tot[0]); }))
+      return res_timeout(a.st);
+    if (sh.tot[0] == 0.0 || !isfinite(sh.tot[0])) {
+      status = VDR_BREAKDOWN;
+      reason = 2;
+      done = true;
+    }
+    al = sh.tot[2];
+    iwp = sh.tot[3];
+  }
+  int pmax = pexp;
+  while (!done) {
+    const int shift = pexp - 1023;
+    v = row(0, shift);
+    s = r - al * v;
+    put(1, masked_pair(msk, s * di, shift));
+    {
+      const double q[2] = {s * s, rh * s};
+      if (!meet<MODE, T, 2, 0, 0, AT_C, AT_C, 0>(sh, a, q, none, target, nothing))
+        return res_timeout(a.st);
+    }
+    t = row(1, shift);
+    // omega = ts / tt and beta = (rho' / rho) (alpha / omega) = (rhs tt / ts -
+    // rht) / (w, p^), rho' = rhs - omega rht: ts / tt and tt / ts on two
+    // lanes of one division.
+    {
+      const double q[3] = {t * s, t * t, rh * t};
+      if (!meet<MODE, T, 3, 0, 5, AT_D, AT_C, 0>(sh, a, q, none, target, [&](int lane) {
+            const double ts = sh.tot[2], tt = sh.tot[3], rhs = sh.tot[1], rht = sh.tot[4];
+            const double num = lane ? tt : ts, den = lane ? ts : tt, d = num / den;
+            const double e = lane ? (rhs * d - rht) * iwp : rhs - d * rht;
+            __syncwarp();
+            if (lane == 0) {
+              sh.tot[1] = d;
+              sh.tot[4] = e;
+            } else if (lane == 1) {
+              sh.tot[5] = e;
+            }
+          }))
+        return res_timeout(a.st);
+    }
+    const double ss = sh.tot[0], om = sh.tot[1], ts = sh.tot[2], tt = sh.tot[3],
+                 rho1 = sh.tot[4], beta = sh.tot[5];
+    if (ss <= thr) {  // s met the tolerance: x += alpha p^
+      if (!msk) x += di * (al * p);
+      iter++;
+      rr2 = ss;
+      status = VDR_OK;
+      break;
+    }
+    if (tt == 0.0 || !isfinite(tt) || !isfinite(ts)) {
+      status = VDR_BREAKDOWN;
+      reason = 3;
+      break;
+    }
+    if (!msk) x += di * (al * p + om * s);
+    r = s - om * t;
+    p = r + beta * (p - om * v);
+    const double ph = msk ? 0.0 : p * di;
+    put(0, stencil_pair(ph, pmax - 1023));
+    rho = rho1;
+    {
+      const double q[2] = {r * r, wn * ph};
+      const int em[1] = {df_exp(ph)};
+      if (!meet<MODE, T, 2, 1, 2, AT_A, AT_A, 0>(sh, a, q, em, target,
+                                              [&](int lane) { alpha_of(lane, sh.tot[1]); }))
+        return res_timeout(a.st);
+    }
+    pexp = pmax;
+    pmax = sh.etot[0];
+    rr2 = sh.tot[0];
+    const double wp = sh.tot[1];
+    al = sh.tot[2];
+    iwp = sh.tot[3];
+    iter++;
+    if (!(rr2 == rr2) || !isfinite(rho1)) {
+      status = VDR_BREAKDOWN;
+      reason = 5;
+      done = true;
+    } else if (rr2 <= thr) {
+      status = VDR_OK;
+      done = true;
+    } else if (rho1 == 0.0 || om == 0.0) {
+      status = VDR_BREAKDOWN;
+      reason = rho1 == 0.0 ? 1 : 4;
+      done = true;
+    } else if (iter >= a.itmax) {
+      done = true;
+    } else if (a.window > 0) {
+      if (rr2 < 0.9801 * best2) {  // a 1 % drop of the norm
+        best2 = rr2;
+        since = 0;
+      } else if (++since >= a.window) {
+        reason = 6;  // stalled
+        done = true;
+      }
+    }
+    if (!done && (wp == 0.0 || !isfinite(wp))) {
+      status = VDR_BREAKDOWN;
+      reason = 2;
+      done = true;
+    }
+  }
+  if (on) a.x[n] = x;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    KState *st = a.st;
+    st->iter = iter;
+    st->err = bnrm2 > 0.0 ? sqrt(rr2) / sqrt(bnrm2) : 0.0;
+    st->status = status;
+    st->reason = reason;
+    st->done = 1;
+  }
+  if (MODE == CLUSTER) cluster_meet();  // no CTA leaves while its memory is read
+}
+
+// One launch of `grid` CTAs: one cluster, or a cooperative grid.
+template <int MODE, int T>
+cudaError_t launch_one(int grid, const ResArgs &a, cudaStream_t s) {
+  const auto kern = resident_bicgstab<MODE, T>;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(T);
+  cfg.stream = s;
+  cudaError_t e;
+  cudaLaunchAttribute attr[1];
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (MODE == CLUSTER) {
+    cfg.dynamicSmemBytes = sizeof(float2) * 2 * T;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)grid;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    if (grid > 8 &&
+        (e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)))
+      return e;
+  } else {
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    if (MODE == IN_SMEM) {
+      cfg.dynamicSmemBytes = sizeof(float2) * 27 * T;
+      if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)cfg.dynamicSmemBytes)))
+        return e;
+    }
+  }
+  return cudaLaunchKernelEx(&cfg, kern, a);
+}
+
+// The smallest power of two of CTAs of T threads that holds N nodes.
+int cluster_ctas(int N, int T) {
+  int c = 1;
+  while ((long)c * T < N) c *= 2;
+  return c;
+}
+
+}  // namespace
+
+bool resident_fits(const Handle &h) {
+  return h.resident && stencil_ready(h) &&
+         h.N <= 1024L * std::min(device_sm_count(), 32 * RES_NB);
+}
+
+cudaError_t launch_resident(Handle &h, const double *b, double *x, double tol, int itmax,
+                            int stall_window) {
+  cudaError_t e;
+  if ((e = cudaMemsetAsync(&h.st->bar_count, 0, sizeof(unsigned), h.stream))) return e;
+  ResArgs a{};
+  a.w = stencil_view(h);
+  a.b = b;
+  a.dinv = h.dinv;
+  a.m = h.mask;
+  a.x = x;
+  a.php = h.st_x + stencil_pad(h);
+  a.shp = a.php + h.N + 2 * stencil_pad(h);
+  a.st = h.st;
+  a.part = h.partials;
+  a.ipart = reinterpret_cast<int *>(h.partials + SLOTS * 32 * RES_NB);
+  a.tol = tol;
+  a.itmax = itmax;
+  a.window = stall_window;
+  const int N = h.N, sms = std::min(device_sm_count(), 32 * RES_NB);
+  const auto blocks = [&](int T) { return (N + T - 1) / T; };
+  // the fewest threads per CTA that hold a node each: with few warps per SM
+  // the FP64 pipe and the sums are the shortest
+  cudaStream_t s = h.stream;
+  e = cudaErrorNotSupported;
+  if (h.resident_cluster && N <= 192 * CLUSTER_MAX) {
+    if (N <= 64 * CLUSTER_MAX) e = launch_one<CLUSTER, 64>(cluster_ctas(N, 64), a, s);
+    else if (N <= 128 * CLUSTER_MAX) e = launch_one<CLUSTER, 128>(CLUSTER_MAX, a, s);
+    else e = launch_one<CLUSTER, 192>(CLUSTER_MAX, a, s);
+    if (e) {  // no cluster of this size here: the grid
+      cudaGetLastError();
+      h.resident_cluster = false;
+    }
+  }
+  if (e) {
+    if (blocks(128) <= sms) e = launch_one<IN_REGS, 128>(blocks(128), a, s);
+    else if (blocks(256) <= sms) e = launch_one<IN_REGS, 256>(blocks(256), a, s);
+    else if (blocks(512) <= sms) e = launch_one<IN_REGS, 512>(blocks(512), a, s);
+    else if (blocks(768) <= sms) e = launch_one<IN_SMEM, 768>(blocks(768), a, s);
+    else e = launch_one<IN_SMEM, 1024>(blocks(1024), a, s);
+  }
+  if (!e) count_launches(1);
+  return e;
+}
+
+}  // namespace vdr

@@ -102,19 +102,21 @@ __device__ __forceinline__ double stencil_row(const StencilView &v, long n,
 // one power of two per vector, with zeros for a plane and a row beyond both
 // ends (stencil_pad), so that the 27 products need no mask, no index clamp
 // and no split: the rows hold zeros wherever no coupling exists.
-template <bool KEEP>
+// A^T reads its neighbours' rows at shifted places, which stay inside S.
+template <bool TRANS, bool KEEP>
 __device__ __forceinline__ double stencil_row_pairs(const StencilView &v, long n,
                                                     const float2 *xp, int shift) {
   DfAcc acc{0.f, 0.f};
-  const float2 *s = v.S + n;
 #pragma unroll
   for (int z = 0; z < 3; z++) {
     float2 a[9], xv[9];
 #pragma unroll
     for (int c = 0; c < 9; c++) {
+      const int k = 9 * z + c;
+      const long q = n + ((z - 1) * v.pl + (c / 3 - 1) * v.nax + (c % 3 - 1));
+      const float2 *s = TRANS ? v.S + (size_t)(26 - k) * v.N + q : v.S + (size_t)k * v.N + n;
       a[c] = KEEP ? __ldcg(s) : __ldcs(s);
-      s += v.N;
-      xv[c] = xp[n + ((z - 1) * v.pl + (c / 3 - 1) * v.nax + (c % 3 - 1))];
+      xv[c] = xp[q];
     }
 #pragma unroll
     for (int c = 0; c < 9; c++) df_fma_acc(acc, a[c].x, a[c].y, xv[c].x, xv[c].y);

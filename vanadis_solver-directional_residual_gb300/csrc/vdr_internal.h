@@ -37,9 +37,9 @@ struct KState {
   unsigned int bar_count, bar_gen;  // grid barrier of the fused inner kernels
   // the assembled-operator iteration: (rh, s), the next rho, the exponent that
   // its pair vectors are scaled by, the largest exponents of the last
-  // direction and of the one being formed
+  // direction, of the one being formed and of the first residual
   double rhs, rho_next;
-  int pexp, pmax, pmax_next;
+  int pexp, pmax, pmax_next, rmax;
 };
 
 // A right preconditioner for BiCGStab beyond Jacobi: `enqueue` adds
@@ -223,6 +223,8 @@ struct Handle {
   unsigned *st_nm = nullptr;    // [N]
   float2 *st_x = nullptr;       // two padded pair vectors: p^ and s^
   int st_state = 0, st_applies = 0;
+  bool resident = true;  // whole solves in one launch (resident.cu) ...
+  bool resident_cluster = true;  // ... of one cluster where they fit
 
   // solver workspace
   double *work = nullptr;
@@ -422,6 +424,13 @@ bool stencil_ready(const Handle &h);
 cudaError_t launch_stencil_apply(const Handle &h, bool transpose, bool accumulate,
                                  const double *x, double *y, const int *skip,
                                  const int *skip2, cudaStream_t s);
+
+// ---- whole solves in one launch (resident.cu) ----
+// BiCGStab with Jacobi on the assembled rows, where they fit in L2; the
+// outcome is in h.st.  An error means that nothing ran.
+bool resident_fits(const Handle &h);
+cudaError_t launch_resident(Handle &h, const double *b, double *x, double tol, int itmax,
+                            int stall_window);
 
 // ---- the 16-bit inner operator (half.cu) ----
 // Builds A^ = P A P D^-1 in the binary16 store from the current FP64
