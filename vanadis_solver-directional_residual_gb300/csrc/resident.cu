@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
   const auto get = [&](int which, int k) {
     if (MODE == CLUSTER)
       return cluster_pair(nb[MODE == CLUSTER ? k : 0] + (unsigned)(which * T * sizeof(float2)));
-    return __ldcg((which ? a.shp : a.php) + (on ? n : 0) + stencil_off(k, a.w.nax, a.w.pl));
+    return (which ? a.shp : a.php)[(on ? n : 0) + stencil_off(k, a.w.nax, a.w.pl)];
   };
   const auto row = [&](int which, int shift) {
     DfAcc acc{0.f, 0.f};
