@@ -149,3 +149,36 @@ def test_whole_solve_launch_shapes(vdr, gpu_lib, dims):
                 xs[scatter, x0] = x.cpu().numpy()
     for x0 in ("zero", "warm"):
         assert rel_l2(xs["auto", x0], xs["atomic", x0]) < 1e-8
+
+
+# the mixed solve's inner kernel: odd node counts, then 128 to 1024 threads of
+# one pair of nodes and 768 / 1024 threads of two (152 SMs), the last with its
+# neighbours across the edge, and the separate kernels beyond
+MIXED_SHAPES = [(2, 2, 2), (4, 2, 6), (15, 15, 3), (75, 31, 15), (75, 31, 16), (75, 63, 15),
+                (75, 63, 16), (75, 63, 31), (75, 63, 32), (75, 63, 63), (76, 62, 64),
+                (75, 63, 95), (75, 127, 63), (75, 127, 64)]
+
+
+@pytest.mark.parametrize("dims", MIXED_SHAPES)
+def test_mixed_launch_shapes(vdr, gpu_lib, dims):
+    """The refinement on the binary16 rows reaches the FP64 tolerance (its
+    true residual recomputed in FP64) and the FP64 solve's solution: both to
+    1e-10, apart by at most the residuals times the condition (below 1e3)."""
+    torch = pytest.importorskip("torch")
+    prob = vdr.problems.rotation_shear(*dims, seed=86)
+    N, aM = prob.mesh.nnode, 0.3 * max(dims)
+    if np.all(prob.bc == 1):
+        prob.bc[:] = 0
+    told = torch.tensor(np.cos(0.37 * np.arange(N)), device="cuda")
+    xs = []
+    for precision in ("mixed", "fp64"):
+        with vdr.Solver(prob, vdr.Options(precision=precision), aH=2.0, aM=aM) as s:
+            b = torch.empty(N, dtype=torch.float64, device="cuda")
+            s.assemble_rhs_device(b, 3.0, aM, told)
+            x = torch.zeros_like(b)
+            it, err, st = s.solve_device(b, x, tol=1e-10, itmax=2000)
+            assert st == 0 and err <= 1e-10, (dims, precision, st, err)
+            free = torch.tensor(prob.bc == 0, device="cuda")
+            assert s.true_residual_device(b * free, x) < 1.1e-10
+            xs.append(x.cpu().numpy())
+    assert rel_l2(xs[0], xs[1]) < 1e-7

@@ -15,7 +15,7 @@ OBJ_DIR = os.path.join(HERE, "_build")
 LIB_PATH = os.path.join(LIB_DIR, "libvdr.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
-SOURCES = ["element.cu", "apply.cu", "half.cu", "stencil.cu", "resident.cu", "krylov.cu", "abi.cu", "noalloc.cu",
+SOURCES = ["element.cu", "apply.cu", "half.cu", "stencil.cu", "resident.cu", "half_rows.cu", "krylov.cu", "abi.cu", "noalloc.cu",
            "block.cu", "block_tc.cu", "unet.cu", "gcr.cu", "batch.cu", "tune.cu", "txtio.cpp"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",

@@ -336,6 +336,17 @@ int ensure_operator32(Handle &h) {
   return VDR_OK;
 }
 
+// The mixed solve's inner operator: binary16 assembled rows where the handle
+// can have them (BiCGStab), the element-wise FP32 or binary16 store otherwise.
+int ensure_inner(Handle &h, int method) {
+  if (method == VDR_SOLVER_BICGSTAB) {
+    int st = ensure_operator(h);
+    if (st || (st = ensure_half_rows(h))) return st;
+    if (half_rows_ready(h)) return VDR_OK;
+  }
+  return ensure_operator32(h);
+}
+
 // The solve of vdr_solve, vdr_solve_device and vdr_time_steps: FP64
 // Krylov, or (VDR_PRECISION_MIXED) FP64 refinement around FP32-operator
 // inner solves to the same FP64 tolerance; *iter counts inner iterations.
@@ -343,12 +354,12 @@ int solve_by_option(Handle &h, int method, const double *b, double *x,
                     double tol, int itmax, int *iter, double *err) {
   if (h.opt.precision != VDR_PRECISION_MIXED)
     return solve_device(h, method, b, x, tol, itmax, iter, err);
-  int st = ensure_operator32(h);
+  int st = ensure_inner(h, method);
   if (st) return st;
   // each correction to 1e-5, or to 1e-3 with the binary16 operator, whose
   // rounding (2^-11 per element) a tighter inner solve cannot get past
   MixedStats ms;
-  st = solve_mixed_device(h, method, b, x, tol, h.use_half ? 1e-3 : 1e-5, 20,
+  st = solve_mixed_device(h, method, b, x, tol, half_rows_ready(h) || h.use_half ? 1e-3 : 1e-5, 20,
                           itmax, &ms);
   if (iter) *iter = ms.inner;
   if (err) *err = ms.err;
@@ -360,6 +371,7 @@ void invalidate(Handle &h) {
   h.mass_valid = false;
   h.aos_valid = h.phi_valid = false;
   if (h.st_state > 0) h.st_state = 0;
+  if (h.hr_state > 0) h.hr_state = 0;
   h.st_applies = 0;
 }
 
@@ -407,6 +419,9 @@ void free_handle(Handle &h) {
   dfree(h.xx32); dfree(h.yy32); dfree(h.zz32);
   dfree(h.conn); dfree(h.mask); dfree(h.emask);
   dfree(h.st_S); dfree(h.st_nm); dfree(h.st_x);
+  if (h.hr_H) cudaFree(h.hr_H);
+  dfree(h.hr_e); dfree(h.hr_vec);
+  if (h.hr_graph) cudaGraphExecDestroy(h.hr_graph);
   dfree(h.vel); dfree(h.lam); dfree(h.pdec); dfree(h.q);
   dfree(h.vel32); dfree(h.lam32); dfree(h.pdec32); dfree(h.robin);
   dfree(h.A64); dfree(h.A32); dfree(h.diag); dfree(h.dinv);
@@ -904,15 +919,15 @@ int vdr_solve_mixed_device(vdr_handle *H, const double *b, double *x,
     set_error("vdr_solve_mixed_device: bad arguments");
     return VDR_BAD_ARGUMENT;
   }
-  if ((st = ensure_operator(h)) || (st = ensure_operator32(h))) return st;
+  const int method = h.opt.solver == VDR_SOLVER_BICG ? VDR_SOLVER_BICG
+                                                     : VDR_SOLVER_BICGSTAB;
+  if ((st = ensure_operator(h)) || (st = ensure_inner(h, method))) return st;
   if ((st = ensure_io(H))) return st;
   double *bm = H->io + 2 * (size_t)h.N;
   cudaError_t e = cudaMemcpyAsync(bm, b, sizeof(double) * h.N,
                                   cudaMemcpyDeviceToDevice, h.stream);
   if (!e) e = launch_mask_vec(bm, h.mask, h.N, h.stream);
   if (e) return cuda_fail(e, "rhs copy");
-  const int method = h.opt.solver == VDR_SOLVER_BICG ? VDR_SOLVER_BICG
-                                                     : VDR_SOLVER_BICGSTAB;
   MixedStats ms;
   st = solve_mixed_device(h, method, bm, x, tol, inner_tol, max_outer,
                           inner_itmax, &ms);

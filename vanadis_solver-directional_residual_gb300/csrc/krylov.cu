@@ -965,6 +965,43 @@ __global__ void __launch_bounds__(RED_THREADS) k_residual(Vec a, double *r,
   }
 }
 
+// The same on the assembled rows: x split once per node into pairs scaled by
+// its largest exponent, then r = b - A x and both norms in one pass (264 bytes
+// a node; the apply that splits every gathered value by itself is bound by
+// instruction issue).
+__global__ void __launch_bounds__(RED_THREADS) bst_xmax(Vec a, int *ex) {
+  int em = 0;
+  double xv[U];
+  VLOOP(xv[u] = ok ? a.x[i] : 0.0;, em = max(em, df_exp(xv[u]));)
+  em = __reduce_max_sync(FULL, em);
+  if ((threadIdx.x & 31) == 0) atomicMax(ex, em);
+}
+__global__ void __launch_bounds__(RED_THREADS) bst_xsplit(Vec a, const int *ex) {
+  const int shift = *ex - 1023;
+  if (*ex == 0) return;
+  double xv[U];
+  VLOOP(xv[u] = ok ? a.x[i] : 0.0;, a.php[i] = stencil_pair(xv[u], shift);)
+}
+__global__ void __launch_bounds__(RED_THREADS, 4) bst_residual(Vec a, StencilView w, double *r,
+                                                               const int *ex, double *out) {
+  const int e = *ex;  // 0: x is zero
+  double v[2] = {0.0, 0.0};
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n;
+       i += (long)gridDim.x * blockDim.x) {
+    const double bi = a.b[i];
+    const double ax = e ? stencil_row_pairs<false, false>(w, i, a.php, e - 1023) : 0.0;
+    const double ri = bi - ax;
+    r[i] = ri;
+    v[0] += ri * ri;
+    v[1] += bi * bi;
+  }
+  double o[2];
+  if (grid_sum<2>(v, a.partials, &a.st->ticket, o)) {
+    out[0] = o[1] > 0.0 ? sqrt(o[0]) / sqrt(o[1]) : 0.0;
+    out[1] = sqrt(o[0]);
+  }
+}
+
 // x += d
 __global__ void __launch_bounds__(RED_THREADS) k_axpy1(Vec a, const double *d) {
   double xv[U], dv[U];
@@ -986,19 +1023,6 @@ struct Vec32 {
   const unsigned char *m;
   float *b, *x, *r, *rh, *p, *v, *ph, *s, *sh, *t;
 };
-
-__device__ __forceinline__ void dot_acc(DfAcc &a, float x, float y) {
-  const float p = __fmul_rn(x, y);
-  const float e = __fmaf_rn(x, y, -p);
-  const float t = __fadd_rn(a.s, p);
-  const float bp = __fsub_rn(t, a.s);
-  const float err = __fadd_rn(__fsub_rn(a.s, __fsub_rn(t, bp)), __fsub_rn(p, bp));
-  a.s = t;
-  a.c = __fadd_rn(a.c, __fadd_rn(err, e));
-}
-__device__ __forceinline__ double dot_val(const DfAcc &a) {
-  return df_to_double(a.s, a.c);
-}
 
 // x = 0, r = rh = b, rho = ||b||^2.
 __global__ void __launch_bounds__(RED_THREADS) k32_start(Vec32 a) {
@@ -1895,19 +1919,30 @@ int solve_mixed_device(Handle &h, int method, const double *b, double *x,
     return cuda_fail(e, "mask x");
   // The stored FP32 operator runs its inner BiCGStab on FP32 vectors.
   const bool f32v = h.apply_mode == VDR_APPLY_STORED && method == VDR_SOLVER_BICGSTAB;
-  if (f32v && !h.dinv32 && (e = cudaMalloc(&h.dinv32, sizeof(float) * (size_t)h.N)))
+  const bool hr = f32v && half_rows_ready(h);
+  if (f32v && !hr && !h.dinv32 && (e = cudaMalloc(&h.dinv32, sizeof(float) * (size_t)h.N)))
     return cuda_fail(e, "FP32 diagonal");
-  if (f32v && !h.work32 &&
+  if (f32v && !hr && !h.work32 &&
       (e = cudaMalloc(&h.work32, sizeof(float) * 10 * (size_t)h.N)))
     return cuda_fail(e, "FP32 workspace");
   for (int outer = 0; outer <= max_outer; outer++) {
     h.apply_fp32 = false;
-    if ((e = cudaMemsetAsync(r, 0, sizeof(double) * h.N, s)) ||
-        (e = launch_apply(h, false, x, r, outer == 0 ? &h.st->x_zero : nullptr,
-                          nullptr, s)))
-      return cuda_fail(e, "outer residual");
-    k_residual<<<g, RED_THREADS, 0, s>>>(a, r, scal);
-    count_launches(1);
+    if (stencil_ready(h)) {
+      int *ex = reinterpret_cast<int *>(scal + 2);
+      if ((e = cudaMemsetAsync(ex, 0, sizeof(int), s))) return cuda_fail(e, "outer residual");
+      bst_xmax<<<g, RED_THREADS, 0, s>>>(a, ex);
+      bst_xsplit<<<g, RED_THREADS, 0, s>>>(a, ex);
+      bst_residual<<<std::min(g, device_sm_count() * 4), RED_THREADS, 0, s>>>(
+          a, stencil_view(h), r, ex, scal);
+      count_launches(3);
+    } else {
+      if ((e = cudaMemsetAsync(r, 0, sizeof(double) * h.N, s)) ||
+          (e = launch_apply(h, false, x, r, outer == 0 ? &h.st->x_zero : nullptr, nullptr, s)))
+        return cuda_fail(e, "outer residual");
+      k_residual<<<g, RED_THREADS, 0, s>>>(a, r, scal);
+      count_launches(1);
+    }
+    if ((e = cudaGetLastError())) return cuda_fail(e, "outer residual");
     double rr[2] = {0.0, 0.0};  // ||r||/||b||, ||r||
     if ((e = cudaMemcpyAsync(rr, scal, 2 * sizeof(double), cudaMemcpyDeviceToHost, s)) ||
         (e = cudaStreamSynchronize(s)))
@@ -1927,7 +1962,11 @@ int solve_mixed_device(Handle &h, int method, const double *b, double *x,
     int it = 0;
     double ierr = 0.0;
     const double itol = std::max(inner_tol, 0.5 * tol / rel);
-    if (f32v) {
+    if (hr) {
+      if (!(1.0 / rr[1] < INFINITY)) break;  // ||r|| at the denormal floor
+      const int ist = solve_half_rows(h, r, rr[1], x, itol, inner_itmax, &it, &ierr);
+      if (ist == VDR_CUDA_ERROR || ist == VDR_BAD_ARGUMENT) return ist;
+    } else if (f32v) {
       // d solves A32 d = r / ||r|| on FP32 vectors; x += ||r|| d in FP64
       if (!(1.0 / rr[1] < INFINITY)) break;  // ||r|| at the denormal floor
       Vec32 a32 = make_vec32(h);

@@ -3,6 +3,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "dfloat.cuh"
+
 namespace vdr {
 
 constexpr unsigned FULLR = 0xffffffffu;
@@ -29,6 +31,20 @@ __device__ __forceinline__ double warp_sums(const double (&v)[Q], int lane) {
   const double d0 = (up ? v2 : v[0]) + __shfl_xor_sync(FULLR, up ? v[0] : v2, 16);
   const double d1 = (up ? v3 : v[1 % Q]) + __shfl_xor_sync(FULLR, up ? v[1 % Q] : v3, 16);
   return fold8((uq ? d1 : d0) + __shfl_xor_sync(FULLR, uq ? d0 : d1, 8));
+}
+
+// a += x * y, the product exact, and the sum's value.
+__device__ __forceinline__ void dot_acc(DfAcc &a, float x, float y) {
+  const float p = __fmul_rn(x, y);
+  const float e = __fmaf_rn(x, y, -p);
+  const float t = __fadd_rn(a.s, p);
+  const float bp = __fsub_rn(t, a.s);
+  const float err = __fadd_rn(__fsub_rn(a.s, __fsub_rn(t, bp)), __fsub_rn(p, bp));
+  a.s = t;
+  a.c = __fadd_rn(a.c, __fadd_rn(err, e));
+}
+__device__ __forceinline__ double dot_val(const DfAcc &a) {
+  return df_to_double(a.s, a.c);
 }
 
 }  // namespace vdr

@@ -34,19 +34,11 @@
 
 #include <algorithm>
 
-#include "reduce.cuh"
+#include "meet.cuh"
 #include "stencil.cuh"
 
 namespace vdr {
 namespace {
-
-constexpr long long RES_LIMIT = 2000000000LL;  // ~1 s of clocks
-constexpr int RES_NB = 5;                      // at most 32 RES_NB CTAs in the grid
-constexpr int CLUSTER_MAX = 16;
-
-enum { CLUSTER, IN_REGS, IN_SMEM };
-// partial sums' places: (s,s) (rh,s) | (t,s) (t,t) (rh,t) | (r,r) (w,p^)
-enum { AT_C = 0, AT_D = 2, AT_A = 5, SLOTS = 7 };
 
 struct ResArgs {
   StencilView w;
@@ -55,181 +47,10 @@ struct ResArgs {
   double *x;
   float2 *php, *shp;  // the grid's p^ and s^
   KState *st;
-  double *part;  // [SLOTS][gridDim]
-  int *ipart;    // [3][gridDim]: largest exponents
+  MeetArgs mt;
   double tol;
   int itmax, window;
 };
-
-struct ResShared {
-  double s[SLOTS][32];  // this CTA's sums, per warp
-  int e[3][32];
-  double tot[6];  // totals, or scalars made of them
-  int etot[2];
-  int ok;
-};
-
-// ---- thread-block clusters
-__device__ __forceinline__ void cluster_meet() {
-  asm volatile(
-      "barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
-          : "memory");
-}
-__device__ __forceinline__ unsigned cluster_addr(const void *p, int cta) {
-  unsigned a;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;"
-      : "=r"(a)
-      : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(cta));
-  return a;
-}
-__device__ __forceinline__ double cluster_f64(unsigned a) {
-  double v;
-  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ int cluster_s32(unsigned a) {
-  int v;
-  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ float2 cluster_pair(unsigned a) {
-  float2 v;
-  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a)
-               : "memory");
-  return v;
-}
-
-// A meeting of all CTAs.  Each leaves its sums of Q quantities at place SLOT
-// (and NE largest exponents at place ES); what any thread wrote before is
-// visible to all after.  Then the totals of the R quantities from place READ
-// on (R = 0: none) are in sh.tot and the largest exponents in sh.etot, and
-// `scalars` runs on warp 0 with them there, its results in sh for all
-// threads.  No place is written again before a meeting that follows its
-// reads.
-template <int MODE, int T, int Q, int NE, int R, int SLOT, int READ, int ES, typename F>
-__device__ __forceinline__ bool meet(ResShared &sh, const ResArgs &a, const double (&v)[Q],
-                                     const int (&em)[NE > 0 ? NE : 1], unsigned &target,
-                                     F scalars) {
-  constexpr int nw = T / 32;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int B = (int)gridDim.x;
-  const double f = warp_sums<Q>(v, lane);
-  if ((lane & 7) == 0 && (lane >> 3) < Q) sh.s[SLOT + (lane >> 3)][w] = f;
-#pragma unroll
-  for (int k = 0; k < NE; k++) {
-    const int e = __reduce_max_sync(FULLR, em[k]);
-    if (lane == 0) sh.e[ES + k][w] = e;
-  }
-  constexpr int RP = R > 0 ? R : 1, R4 = RP < 4 ? RP : 4;
-  double tot[RP];
-  int etot[NE > 0 ? NE : 1] = {0};
-  if (MODE == CLUSTER) {
-    cluster_meet();
-    if (R == 0 && NE == 0) return true;
-    if (w == 0) {  // all warps' sums of all CTAs, every load before the adds
-      constexpr int NI = (CLUSTER_MAX * nw + 31) / 32;
-      double in[NI][RP];
-      int ein[NI][NE > 0 ? NE : 1];
-#pragma unroll
-      for (int i = 0; i < NI; i++) {
-        const int j = lane + 32 * i, c = min(j / nw, B - 1), u = j % nw;
-        const unsigned at = cluster_addr(&sh.s[READ][u], c);
-        if (R > 0)
-#pragma unroll
-          for (int k = 0; k < RP; k++)
-            in[i][k] = cluster_f64(at + (unsigned)(k * sizeof sh.s[0]));
-#pragma unroll
-        for (int k = 0; k < NE; k++) ein[i][k] = cluster_s32(cluster_addr(&sh.e[ES + k][u], c));
-      }
-#pragma unroll
-      for (int k = 0; k < RP; k++) tot[k] = 0.0;
-#pragma unroll
-      for (int i = 0; i < NI; i++) {
-        const bool mine = lane + 32 * i < B * nw;
-        if (R > 0 && (i == 0 || 32 * i < B * nw))
-#pragma unroll
-          for (int k = 0; k < RP; k++) tot[k] += mine ? in[i][k] : 0.0;
-#pragma unroll
-        for (int k = 0; k < NE; k++) etot[k] = max(etot[k], ein[i][k]);
-      }
-    }
-  } else {
-    target += gridDim.x;
-    __syncthreads();
-    if (w == 0) {
-      const int q = lane >> 3, sub = lane & 7;
-      double c = 0.0;
-      for (int k = sub; k < nw; k += 8) c += sh.s[SLOT + (q < Q ? q : 0)][k];
-      c = fold8(c);
-      if (sub == 0 && q < Q) __stcg(a.part + (size_t)(SLOT + q) * B + blockIdx.x, c);
-#pragma unroll
-      for (int k = 0; k < NE; k++) {
-        const int e = __reduce_max_sync(FULLR, lane < nw ? sh.e[ES + k][lane] : 0);
-        if (lane == 0) __stcg(a.ipart + (size_t)(ES + k) * B + blockIdx.x, e);
-      }
-      __syncwarp();
-      unsigned *bar = &a.st->bar_count;
-      if (lane == 0)
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-      __syncwarp();
-      // the whole warp polls: with one lane polling, what followed ran split
-      // (13 us more per iteration at 145 CTAs)
-      const long long t0 = clock64();
-      bool met, late = false;
-      do {
-        unsigned seen;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
-        met = (int)(seen - target) >= 0;
-        late = clock64() - t0 > RES_LIMIT;
-      } while (!__all_sync(FULLR, met || late));
-      if (lane == 0) sh.ok = met;
-      if (R > 0) {
-        double in[RES_NB][RP];  // every load before the first add
-#pragma unroll
-        for (int i = 0; i < RES_NB; i++)
-#pragma unroll
-          for (int k = 0; k < RP; k++)
-            in[i][k] = __ldcg(a.part + (size_t)(READ + k) * B + min(lane + 32 * i, B - 1));
-#pragma unroll
-        for (int k = 0; k < RP; k++) tot[k] = lane < B ? in[0][k] : 0.0;
-#pragma unroll
-        for (int i = 1; i < RES_NB; i++)
-          if (32 * i < B)
-#pragma unroll
-            for (int k = 0; k < RP; k++) tot[k] += lane + 32 * i < B ? in[i][k] : 0.0;
-      }
-#pragma unroll
-      for (int k = 0; k < NE; k++)
-#pragma unroll
-        for (int i = 0; i < RES_NB; i++)
-          etot[k] =
-              max(etot[k], __ldcg(a.ipart + (size_t)(ES + k) * B + min(lane + 32 * i, B - 1)));
-    }
-  }
-  if (w == 0) {
-    if (R > 0) {
-      double u[R4];
-#pragma unroll
-      for (int k = 0; k < R4; k++) u[k] = tot[k];
-      const double g = warp_sums<R4>(u, lane);
-      if ((lane & 7) == 0 && (lane >> 3) < R4) sh.tot[lane >> 3] = g;
-      if (R > 4) {
-        const double u1[1] = {tot[RP - 1]};
-        const double g1 = warp_sums<1>(u1, lane);
-        if (lane == 0) sh.tot[4] = g1;
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < NE; k++) {
-      const int e = __reduce_max_sync(FULLR, etot[k]);
-      if (lane == 0) sh.etot[k] = e;
-    }
-    __syncwarp();
-    if (R > 0) scalars(lane);
-  }
-  __syncthreads();
-  return MODE == CLUSTER || sh.ok != 0;
-}
 
 __device__ __forceinline__ void res_timeout(KState *st) {
   if (threadIdx.x == 0) {
@@ -314,14 +135,14 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
     x = msk ? 0.0 : a.x[n];
     const double z[1] = {0.0};
     const int e1[1] = {df_exp(x)};
-    if (!meet<MODE, T, 1, 1, 0, AT_C, AT_C, 2>(sh, a, z, e1, target, nothing))
+    if (!meet<MODE, T, 1, 1, 0, AT_C, AT_C, 2>(sh, a.mt, z, e1, target, nothing))
       return res_timeout(a.st);
   }
   const int ex = sh.etot[0];
   if (ex) {
     put(0, masked_pair(msk, x, ex - 1023));
     const double z[1] = {0.0};
-    if (!meet<MODE, T, 1, 0, 0, AT_D, AT_D, 0>(sh, a, z, none, target, nothing))
+    if (!meet<MODE, T, 1, 0, 0, AT_D, AT_D, 0>(sh, a.mt, z, none, target, nothing))
       return res_timeout(a.st);
     v = row(0, ex - 1023);
   }
@@ -331,7 +152,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
     rh = p = r;
     const double q[2] = {bi * bi, r * r};
     const int em[2] = {df_exp(r), df_exp(msk ? 0.0 : r * di)};
-    if (!meet<MODE, T, 2, 2, 2, AT_A, AT_A, 0>(sh, a, q, em, target, nothing))
+    if (!meet<MODE, T, 2, 2, 2, AT_A, AT_A, 0>(sh, a.mt, q, em, target, nothing))
       return res_timeout(a.st);
   }
   const double bnrm2 = sh.tot[0];
@@ -369,7 +190,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
     put(0, masked_pair(msk, p * di, pexp - 1023));
     put(1, masked_pair(msk, rh, er - 1023));
     double q[1] = {0.0};
-    if (!meet<MODE, T, 1, 0, 0, AT_C, AT_C, 0>(sh, a, q, none, target, nothing))
+    if (!meet<MODE, T, 1, 0, 0, AT_C, AT_C, 0>(sh, a.mt, q, none, target, nothing))
       return res_timeout(a.st);
     DfAcc acc{0.f, 0.f};
     for (int z = 0; z < 27; z += 9)
@@ -387,7 +208,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
       }
     wn = row_value(acc, er - 1023);
     if (!msk) q[0] = wn * (p * di);
-    if (!meet<MODE, T, 1, 0, 1, AT_D, AT_D, 0>(sh, a, q, none, target,
+    if (!meet<MODE, T, 1, 0, 1, AT_D, AT_D, 0>(sh, a.mt, q, none, target,
                                             [&](int lane) { alpha_of(lane, sh.tot[0]); }))
       return res_timeout(a.st);
     if (sh.tot[0] == 0.0 || !isfinite(sh.tot[0])) {
@@ -406,7 +227,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
     put(1, masked_pair(msk, s * di, shift));
     {
       const double q[2] = {s * s, rh * s};
-      if (!meet<MODE, T, 2, 0, 0, AT_C, AT_C, 0>(sh, a, q, none, target, nothing))
+      if (!meet<MODE, T, 2, 0, 0, AT_C, AT_C, 0>(sh, a.mt, q, none, target, nothing))
         return res_timeout(a.st);
     }
     t = row(1, shift);
@@ -415,7 +236,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
     // lanes of one division.
     {
       const double q[3] = {t * s, t * t, rh * t};
-      if (!meet<MODE, T, 3, 0, 5, AT_D, AT_C, 0>(sh, a, q, none, target, [&](int lane) {
+      if (!meet<MODE, T, 3, 0, 5, AT_D, AT_C, 0>(sh, a.mt, q, none, target, [&](int lane) {
             const double ts = sh.tot[2], tt = sh.tot[3], rhs = sh.tot[1], rht = sh.tot[4];
             const double num = lane ? tt : ts, den = lane ? ts : tt, d = num / den;
             const double e = lane ? (rhs * d - rht) * iwp : rhs - d * rht;
@@ -452,7 +273,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
     {
       const double q[2] = {r * r, wn * ph};
       const int em[1] = {df_exp(ph)};
-      if (!meet<MODE, T, 2, 1, 2, AT_A, AT_A, 0>(sh, a, q, em, target,
+      if (!meet<MODE, T, 2, 1, 2, AT_A, AT_A, 0>(sh, a.mt, q, em, target,
                                               [&](int lane) { alpha_of(lane, sh.tot[1]); }))
         return res_timeout(a.st);
     }
@@ -563,8 +384,7 @@ cudaError_t launch_resident(Handle &h, const double *b, double *x, double tol, i
   a.php = h.st_x + stencil_pad(h);
   a.shp = a.php + h.N + 2 * stencil_pad(h);
   a.st = h.st;
-  a.part = h.partials;
-  a.ipart = reinterpret_cast<int *>(h.partials + SLOTS * 32 * RES_NB);
+  a.mt = meet_args(h);
   a.tol = tol;
   a.itmax = itmax;
   a.window = stall_window;

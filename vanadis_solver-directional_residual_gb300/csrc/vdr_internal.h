@@ -223,6 +223,13 @@ struct Handle {
   unsigned *st_nm = nullptr;    // [N]
   float2 *st_x = nullptr;       // two padded pair vectors: p^ and s^
   int st_state = 0, st_applies = 0;
+  // its binary16 rows for the mixed solve (half_rows.cu): 27 half planes, a
+  // scale per row, FP32 vectors; hr_state as st_state, 2 = out of range
+  void *hr_H = nullptr;
+  signed char *hr_e = nullptr;
+  float *hr_vec = nullptr;
+  int hr_state = 0, hr_graph_iters = 0;
+  cudaGraphExec_t hr_graph = nullptr;
   bool resident = true;  // whole solves in one launch (resident.cu) ...
   bool resident_cluster = true;  // ... of one cluster where they fit
 
@@ -424,6 +431,16 @@ bool stencil_ready(const Handle &h);
 cudaError_t launch_stencil_apply(const Handle &h, bool transpose, bool accumulate,
                                  const double *x, double *y, const int *skip,
                                  const int *skip2, cudaStream_t s);
+
+// ---- the mixed solve's inner operator on assembled rows (half_rows.cu) ----
+// Forms the binary16 rows for the current operator where it can (the handle
+// has assembled rows and VDR_MIXED_HALF); half_rows_ready tells.
+int ensure_half_rows(Handle &h);
+bool half_rows_ready(const Handle &h);
+// One correction of the refinement: y from A^ y = res / rnorm to `tol`, x +=
+// rnorm D^-1 y.
+int solve_half_rows(Handle &h, const double *res, double rnorm, double *x, double tol,
+                    int itmax, int *iter, double *err);
 
 // ---- whole solves in one launch (resident.cu) ----
 // BiCGStab with Jacobi on the assembled rows, where they fit in L2; the
