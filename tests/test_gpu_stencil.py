@@ -182,3 +182,38 @@ def test_mixed_launch_shapes(vdr, gpu_lib, dims):
             assert s.true_residual_device(b * free, x) < 1.1e-10
             xs.append(x.cpu().numpy())
     assert rel_l2(xs[0], xs[1]) < 1e-7
+
+
+BICG_SHAPES = [(1, 1, 1), (2, 1, 3), (15, 15, 3), (75, 31, 7), (75, 31, 8), (75, 31, 16),
+               (75, 63, 15), (75, 63, 16), (75, 63, 31), (75, 63, 32)]
+
+
+@pytest.mark.parametrize("dims", BICG_SHAPES)
+def test_dropin_launch_shapes(vdr, oracle, gpu_lib, dims):
+    """kernel_dbcg_simple_ at the launch shapes of the whole-solve BiCG (128 to
+    1024 threads a CTA, then separate kernels), sizes going up and down so that
+    its buffers are reused: solution to 1e-9 of the oracle's BiCG at 1e-12, and
+    to the tolerance where elements are listed in another order (the
+    element-wise path)."""
+    prob = vdr.problems.rotation_shear(*dims, seed=87)
+    m, aM = prob.mesh, 0.3 * max(dims)
+    if np.all(prob.bc == 1):
+        prob.bc[:] = 0
+    told = np.cos(0.37 * np.arange(m.nnode))
+    bb, b, diag = oracle.assemble(prob.variant, m.xx, m.yy, m.zz, m.iss, prob.vel, prob.lam,
+                                  prob.pdec, prob.q, kod=m.kod, robin_alpha=0.0, aH=2.0,
+                                  aM=aM, cf=3.0, rM=aM, t_old=told, nthreads=8)
+    b[prob.bc == 1] = 0.0
+    diag[prob.bc == 1] = 1.0
+    x0 = np.where(prob.bc == 1, 0.0, told)
+    ref, _, _, st = oracle.bicgstab(b, x0, bb, m.iss, diag, prob.bc, tol=1e-12, itmax=5000)
+    assert st == 0
+    args = (m.nax, m.nay, m.naz, prob.bc)
+    x, it, err = vdr.kernel_dbcg_simple(m.nnode, b, x0, 1e-11, 5000, bb, m.iss, diag, *args)
+    assert err <= 1e-11 and rel_l2(x, ref) < 1e-9
+    E = m.nelem
+    perm = np.random.default_rng(7).permutation(E)
+    x2, it2, err2 = vdr.kernel_dbcg_simple(
+        m.nnode, b, x0, 1e-11, 5000, np.ascontiguousarray(bb.reshape(E, 64)[perm]).ravel(),
+        np.ascontiguousarray(m.iss.reshape(8, E)[:, perm]).ravel(), diag, *args)
+    assert err2 <= 1e-11 and rel_l2(x2, ref) < 1e-9

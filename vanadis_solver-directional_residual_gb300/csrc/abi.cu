@@ -1390,6 +1390,7 @@ int legacy_prepare(Legacy &L, int N, int E) {
     dfree(h.Ahi); h.Ahi = nullptr;
     dfree(h.Alo); h.Alo = nullptr;
     dfree(h.conn); h.conn = nullptr;
+    dfree(h.emask); h.emask = nullptr;
     dfree(h.diag); h.diag = nullptr;
     dfree(h.dinv); h.dinv = nullptr;
     dfree(h.mask); h.mask = nullptr;
@@ -1415,7 +1416,7 @@ int legacy_prepare(Legacy &L, int N, int E) {
     const size_t cN = std::max(N, L.capN), cE = std::max(E, L.capE);
     if ((e = dalloc(&h.Ahi, cE * 16)) ||
         (e = dalloc(&h.Alo, cE * 16)) || (e = dalloc(&h.conn, cE * 8)) ||
-        (e = dalloc(&h.diag, cN)) || (e = dalloc(&h.dinv, cN)) ||
+        (e = dalloc(&h.emask, cE)) || (e = dalloc(&h.diag, cN)) || (e = dalloc(&h.dinv, cN)) ||
         (e = dalloc(&h.mask, cN)) ||
         (e = dalloc(&L.bb, cE * 64)) || (e = dalloc(&L.b, cN)) ||
         (e = dalloc(&L.x, cN)) || (e = dalloc(&L.iss, cE * 8)) ||
@@ -1478,8 +1479,8 @@ void kernel_dbcg_simple_(int *Np, double *B, double *X, double *TOLp,
       break;
     }
     if ((e = cudaMemsetAsync(L.bad, 0, sizeof(int), s)) ||
-        (e = launch_legacy_conn(L.iss, (int)E, N, bc_dirichlet ? L.bc : nullptr,
-                                h.conn, L.bad, s)) ||
+        (e = launch_legacy_conn(L.iss, (int)E, N, (int)nax, (int)nay,
+                                bc_dirichlet ? L.bc : nullptr, h.conn, L.bad, s)) ||
         (e = launch_legacy_bb_df(L.bb, (int)E, h.Ahi, h.Alo, L.bad, s)) ||
         (e = launch_diag_fix(h.diag, h.dinv, nullptr, N, s)) ||
         (e = cudaMemcpyAsync(&bad, L.bad, sizeof(int), cudaMemcpyDeviceToHost, s)) ||
@@ -1499,6 +1500,17 @@ void kernel_dbcg_simple_(int *Np, double *B, double *X, double *TOLp,
   }
   if (bad & 1) {
     set_error("kernel_dbcg_simple_: ISS entry outside 1..N");
+    *ERRp = inf;
+    return;
+  }
+  // on the reference's own numbering the solve runs on assembled rows
+  const bool canonical = !(bad & 8) && (long)nax * nay * naz == N;
+  h.nax = canonical ? (int)nax : 0;
+  h.nay = canonical ? (int)nay : 0;
+  h.naz = canonical ? (int)naz : 0;
+  if (h.st_state > 0) h.st_state = 0;
+  if (canonical && (e = launch_emask(h))) {
+    cuda_fail(e, "kernel_dbcg_simple_: masks");
     *ERRp = inf;
     return;
   }

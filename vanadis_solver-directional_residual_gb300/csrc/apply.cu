@@ -602,13 +602,19 @@ __global__ void export_bb_kernel(const float4 *__restrict__ Ahi,
   }
 }
 
-__global__ void legacy_conn_kernel(const int *__restrict__ iss, int E, int N,
+__global__ void legacy_conn_kernel(const int *__restrict__ iss, int E, int N, int nax, int nay,
                                    const int *__restrict__ bc,
                                    int *__restrict__ conn, int *bad) {
   const long total = (long)E * 8;
+  bool other = false;  // an entry that is not the canonical numbering's
   for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (long)gridDim.x * blockDim.x) {
     const int n = iss[t] - 1;
+    const unsigned s = (unsigned)(t / E), p = (unsigned)(t - (long)s * E), s2 = s & 3;
+    const unsigned r = p / (unsigned)(nax - 1), i = p - r * (unsigned)(nax - 1);
+    const unsigned k = r / (unsigned)(nay - 1), j = r - k * (unsigned)(nay - 1);
+    other |= n != (int)(i + (s2 == 1 || s2 == 2) +
+                        nax * (j + (s2 >> 1) + (long)nay * (k + (s >> 2))));
     if (n < 0 || n >= N) {
       atomicOr(bad, 1);
       conn[t] = MASK_BIT;  // node 0, masked: never read or written
@@ -616,6 +622,7 @@ __global__ void legacy_conn_kernel(const int *__restrict__ iss, int E, int N,
     }
     conn[t] = (bc && bc[n] == 1) ? (n | MASK_BIT) : n;
   }
+  if (other) atomicOr(bad, 8);
 }
 
 __global__ void mask_conn_kernel(int *__restrict__ conn, long total,
@@ -874,10 +881,10 @@ cudaError_t launch_export_bb(const Handle &h, double *bb, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_legacy_conn(const int *iss_ref, int E, int N, const int *bc,
-                               int *conn, int *bad, cudaStream_t s) {
+cudaError_t launch_legacy_conn(const int *iss_ref, int E, int N, int nax, int nay,
+                               const int *bc, int *conn, int *bad, cudaStream_t s) {
   legacy_conn_kernel<<<grid_for((long)E * 8, 256, 16), 256, 0, s>>>(
-      iss_ref, E, N, bc, conn, bad);
+      iss_ref, E, N, nax, nay, bc, conn, bad);
   count_launches(1);
   return cudaGetLastError();
 }

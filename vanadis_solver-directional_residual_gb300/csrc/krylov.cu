@@ -787,8 +787,8 @@ int solve_device(Handle &h, int method, const double *b, double *x,
   const long long launches0 = launches_so_far();
   h.last = vdr_solve_stats{};
 
-  if (method == VDR_SOLVER_BICGSTAB && !prec && !hist && resident_fits(h)) {
-    if (!(e = launch_resident(h, b, x, tol, itmax, stall_window))) {
+  if (!prec && !hist && resident_fits(h)) {
+    if (!(e = launch_resident(h, method, b, x, tol, itmax, stall_window))) {
       if ((e = cudaMemcpyAsync(&h.h_st[0], h.st, sizeof(KState), cudaMemcpyDeviceToHost, s)) ||
           (e = cudaStreamSynchronize(s)))
         return cuda_fail(e, "solve");

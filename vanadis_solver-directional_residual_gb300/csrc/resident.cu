@@ -324,10 +324,186 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
   if (MODE == CLUSTER) cluster_meet();  // no CTA leaves while its memory is read
 }
 
-// One launch of `grid` CTAs: one cluster, or a cooperative grid.
+// Jacobi BiCG in the same form (a cooperative grid): p and p~ handed out, A p
+// from the node's row and A^T p~ from its column (in shared memory up to 512
+// threads, from L2 above), then (A p, p~), then (r,r) and (D^-1 r, r~).  b is
+// taken as it is (the drop-in's may be nonzero on Dirichlet rows, where x
+// stays zero).
 template <int MODE, int T>
+__global__ void __launch_bounds__(T, 1) resident_bicg(ResArgs a) {
+  extern __shared__ float2 dyn[];  // [27][T]: columns, or rows (IN_SMEM)
+  __shared__ ResShared sh;
+  const int N = a.w.N, n = (int)(blockIdx.x * T + threadIdx.x);
+  const bool on = n < N;
+  unsigned target = 0;
+  const int none[1] = {0};
+  const auto nothing = [](int) {};
+  const auto column = [&](int k) {  // A's entry of neighbour k with this node
+    const int q = n + stencil_off(k, a.w.nax, a.w.pl);
+    return on && q >= 0 && q < N ? __ldcg(a.w.S + (size_t)(26 - k) * N + q)
+                                 : make_float2(0.f, 0.f);
+  };
+  float2 A[MODE == IN_REGS ? 27 : 1];
+#pragma unroll
+  for (int k = 0; k < 27; k++) {
+    const float2 e = on ? __ldcg(a.w.S + (size_t)k * N + n) : make_float2(0.f, 0.f);
+    if (MODE == IN_REGS) A[MODE == IN_REGS ? k : 0] = e;
+    dyn[k * T + threadIdx.x] = MODE == IN_REGS ? column(k) : e;
+  }
+  const double di = on ? a.dinv[n] : 0.0;
+  const bool msk = on ? a.m[n] != 0 : true;
+  double x = 0.0, r, rr, p = 0.0, pp = 0.0, z = 0.0, zz = 0.0;
+  const float2 *gp = a.php + (on ? n : 0), *gs = a.shp + (on ? n : 0);
+  const auto row = [&](int shift) {
+    DfAcc acc{0.f, 0.f};
+#pragma unroll
+    for (int g = 0; g < 27; g += 9) {
+      float2 xv[9];
+#pragma unroll
+      for (int c = 0; c < 9; c++) xv[c] = gp[stencil_off(g + c, a.w.nax, a.w.pl)];
+#pragma unroll
+      for (int c = 0; c < 9; c++) {
+        const float2 e = MODE == IN_REGS ? A[MODE == IN_REGS ? g + c : 0]
+                                         : dyn[(g + c) * T + threadIdx.x];
+        df_fma_acc(acc, e.x, e.y, xv[c].x, xv[c].y);
+      }
+    }
+    return row_value(acc, shift);
+  };
+  const auto trans = [&](int shift) {
+    DfAcc acc{0.f, 0.f};
+#pragma unroll
+    for (int g = 0; g < 27; g += 9) {
+      float2 xv[9], e[9];
+#pragma unroll
+      for (int c = 0; c < 9; c++) {
+        xv[c] = gs[stencil_off(g + c, a.w.nax, a.w.pl)];
+        e[c] = MODE == IN_REGS ? dyn[(g + c) * T + threadIdx.x] : column(g + c);
+      }
+#pragma unroll
+      for (int c = 0; c < 9; c++) df_fma_acc(acc, e[c].x, e[c].y, xv[c].x, xv[c].y);
+    }
+    return row_value(acc, shift);
+  };
+
+  {
+    x = msk ? 0.0 : a.x[n];
+    const double q[1] = {0.0};
+    const int e1[1] = {df_exp(x)};
+    if (!meet<MODE, T, 1, 1, 0, AT_C, AT_C, 2>(sh, a.mt, q, e1, target, nothing))
+      return res_timeout(a.st);
+  }
+  const int ex = sh.etot[0];
+  if (ex) {
+    if (on) a.php[n] = masked_pair(msk, x, ex - 1023);
+    const double q[1] = {0.0};
+    if (!meet<MODE, T, 1, 0, 0, AT_D, AT_D, 0>(sh, a.mt, q, none, target, nothing))
+      return res_timeout(a.st);
+    z = row(ex - 1023);
+  }
+  {
+    const double bi = on ? a.b[n] : 0.0;
+    r = bi - (msk ? 0.0 : z);
+    rr = r;
+    const double q[3] = {bi * bi, r * r, (r * di) * rr};
+    const int e1[1] = {df_exp(msk ? 0.0 : r * di)};
+    if (!meet<MODE, T, 3, 1, 3, AT_A - 1, AT_A - 1, 0>(sh, a.mt, q, e1, target, nothing))
+      return res_timeout(a.st);
+  }
+  const double bnrm2 = sh.tot[0], thr = a.tol * a.tol * bnrm2;
+  double rr2 = sh.tot[1], bknum = sh.tot[2], bk = 0.0;
+  int pexp = sh.etot[0], qexp = pexp;
+  int iter = 0, status = VDR_NOT_CONVERGED, reason = 0;
+  bool done = false;
+  if (bnrm2 == 0.0) {  // b = 0: the solution is x = 0
+    x = 0.0;
+    rr2 = 0.0;
+    status = VDR_OK;
+    done = true;
+  } else if (!isfinite(bnrm2) || !isfinite(rr2)) {
+    status = VDR_BREAKDOWN;
+    reason = 5;
+    done = true;
+  } else if (rr2 <= thr) {
+    status = VDR_OK;
+    done = true;
+  } else if (a.itmax <= 0) {
+    done = true;
+  }
+  while (!done) {
+    p = msk ? 0.0 : r * di + bk * p;
+    pp = msk ? 0.0 : rr * di + bk * pp;
+    if (on) {
+      a.php[n] = stencil_pair(p, pexp - 1023);
+      a.shp[n] = stencil_pair(pp, qexp - 1023);
+    }
+    {
+      const double q[1] = {0.0};
+      if (!meet<MODE, T, 1, 0, 0, AT_C, AT_C, 0>(sh, a.mt, q, none, target, nothing))
+        return res_timeout(a.st);
+    }
+    z = row(pexp - 1023);
+    zz = trans(qexp - 1023);
+    {
+      const double q[1] = {z * pp};
+      const int em[2] = {df_exp(p), df_exp(pp)};
+      if (!meet<MODE, T, 1, 2, 1, AT_C, AT_C, 0>(sh, a.mt, q, em, target, [&](int lane) {
+            const double d = bknum / sh.tot[0];
+            if (lane == 0) sh.tot[1] = d;
+          }))
+        return res_timeout(a.st);
+    }
+    const double ak = sh.tot[1];
+    pexp = sh.etot[0];
+    qexp = sh.etot[1];
+    if (!isfinite(ak)) {
+      status = VDR_BREAKDOWN;
+      reason = 2;
+      break;
+    }
+    x += ak * p;
+    r -= ak * z;
+    rr -= ak * zz;
+    {
+      const double q[2] = {r * r, (r * di) * rr};
+      if (!meet<MODE, T, 2, 0, 2, AT_D, AT_D, 0>(sh, a.mt, q, none, target, [&](int lane) {
+            const double d = sh.tot[1] / bknum;
+            if (lane == 0) sh.tot[2] = d;
+          }))
+        return res_timeout(a.st);
+    }
+    rr2 = sh.tot[0];
+    bknum = sh.tot[1];
+    bk = sh.tot[2];
+    iter++;
+    if (!(rr2 == rr2)) {
+      status = VDR_BREAKDOWN;
+      reason = 5;
+      done = true;
+    } else if (rr2 <= thr) {
+      status = VDR_OK;
+      done = true;
+    } else if (iter >= a.itmax) {
+      done = true;
+    }
+  }
+  if (on) a.x[n] = x;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    KState *st = a.st;
+    st->iter = iter;
+    st->err = bnrm2 > 0.0 ? sqrt(rr2) / sqrt(bnrm2) : 0.0;
+    st->status = status;
+    st->reason = reason;
+    st->done = 1;
+  }
+}
+
+// One launch of `grid` CTAs: one cluster, or a cooperative grid.
+template <int MODE, int T, bool BICG = false>
 cudaError_t launch_one(int grid, const ResArgs &a, cudaStream_t s) {
-  const auto kern = resident_bicgstab<MODE, T>;
+  void (*kern)(ResArgs);
+  if constexpr (BICG) kern = resident_bicg<MODE, T>;
+  else kern = resident_bicgstab<MODE, T>;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(T);
@@ -347,7 +523,7 @@ cudaError_t launch_one(int grid, const ResArgs &a, cudaStream_t s) {
   } else {
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
-    if (MODE == IN_SMEM) {
+    if (MODE == IN_SMEM || BICG) {
       cfg.dynamicSmemBytes = sizeof(float2) * 27 * T;
       if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)cfg.dynamicSmemBytes)))
@@ -371,8 +547,8 @@ bool resident_fits(const Handle &h) {
          h.N <= 1024L * std::min(device_sm_count(), 32 * RES_NB);
 }
 
-cudaError_t launch_resident(Handle &h, const double *b, double *x, double tol, int itmax,
-                            int stall_window) {
+cudaError_t launch_resident(Handle &h, int method, const double *b, double *x, double tol,
+                            int itmax, int stall_window) {
   cudaError_t e;
   if ((e = cudaMemsetAsync(&h.st->bar_count, 0, sizeof(unsigned), h.stream))) return e;
   ResArgs a{};
@@ -394,6 +570,14 @@ cudaError_t launch_resident(Handle &h, const double *b, double *x, double tol, i
   // the FP64 pipe and the sums are the shortest
   cudaStream_t s = h.stream;
   e = cudaErrorNotSupported;
+  if (method == VDR_SOLVER_BICG) {
+    if (blocks(128) <= sms) e = launch_one<IN_REGS, 128, true>(blocks(128), a, s);
+    else if (blocks(256) <= sms) e = launch_one<IN_REGS, 256, true>(blocks(256), a, s);
+    else if (blocks(512) <= sms) e = launch_one<IN_REGS, 512, true>(blocks(512), a, s);
+    else e = launch_one<IN_SMEM, 1024, true>(blocks(1024), a, s);
+    if (!e) count_launches(1);
+    return e;
+  }
   if (h.resident_cluster && N <= 192 * CLUSTER_MAX) {
     if (N <= 64 * CLUSTER_MAX) e = launch_one<CLUSTER, 64>(cluster_ctas(N, 64), a, s);
     else if (N <= 128 * CLUSTER_MAX) e = launch_one<CLUSTER, 128>(CLUSTER_MAX, a, s);

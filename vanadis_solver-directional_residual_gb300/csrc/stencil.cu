@@ -127,14 +127,21 @@ cudaError_t ensure_stencil(Handle &h) {
       h.storage != VDR_STORE_DF || h.opt.scatter != VDR_SCATTER_AUTO || h.perm_d || !h.Ahi ||
       !h.emask || h.nax < 2 || h.nay < 2 || h.naz < 2)
     return cudaSuccess;
-  const size_t N = (size_t)h.N;
-  if (!h.st_S) {
+  const size_t N = (size_t)h.N, len = 2 * (N + 2 * stencil_pad(h));
+  if (N > h.st_rows || len > h.st_len) {
+    cudaFree(h.st_S);
+    cudaFree(h.st_nm);
+    cudaFree(h.st_x);
+    h.st_S = nullptr;
+    h.st_nm = nullptr;
+    h.st_x = nullptr;
+    h.st_rows = h.st_len = 0;
+    h.st_nax = 0;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || 240 * N > free_b / 2 ||
         cudaMalloc(&h.st_S, sizeof(float2) * 27 * N) ||
         cudaMalloc(&h.st_nm, sizeof(unsigned) * N) ||
-        cudaMalloc(&h.st_x, sizeof(float2) * 2 * (N + 2 * stencil_pad(h))) ||
-        cudaMemsetAsync(h.st_x, 0, sizeof(float2) * 2 * (N + 2 * stencil_pad(h)), h.stream)) {
+        cudaMalloc(&h.st_x, sizeof(float2) * len)) {
       cudaGetLastError();  // no room for the rows: the element-wise apply stays
       cudaFree(h.st_S);
       cudaFree(h.st_nm);
@@ -145,13 +152,21 @@ cudaError_t ensure_stencil(Handle &h) {
       h.st_state = -1;
       return cudaSuccess;
     }
+    h.st_rows = N;
+    h.st_len = len;
+  }
+  cudaError_t e;
+  if (h.st_nax != h.nax || h.st_pl != h.nax * h.nay) {
+    if ((e = cudaMemsetAsync(h.st_x, 0, sizeof(float2) * h.st_len, h.stream))) return e;
+    h.st_nax = h.nax;
+    h.st_pl = h.nax * h.nay;
   }
   const long need = (h.N + 255L) / 256;
   const int grid = (int)std::min<long>(need, (long)device_sm_count() * 32);
   stencil_assemble<<<grid, 256, 0, h.stream>>>(h.Ahi, h.Alo, h.emask, h.nax, h.nay, h.naz,
                                                h.st_S, h.st_nm);
   count_launches(1);
-  const cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if (!e) h.st_state = 1;
   return e;
 }

@@ -222,6 +222,8 @@ struct Handle {
   float2 *st_S = nullptr;       // [27][N]
   unsigned *st_nm = nullptr;    // [N]
   float2 *st_x = nullptr;       // two padded pair vectors: p^ and s^
+  size_t st_rows = 0, st_len = 0;  // nodes and pairs that they hold room for
+  int st_nax = 0, st_pl = 0;    // the strides that st_x's pads are zero for
   int st_state = 0, st_applies = 0;
   // its binary16 rows for the mixed solve (half_rows.cu): 27 half planes, a
   // scale per row, FP32 vectors; hr_state as st_state, 2 = out of range
@@ -407,8 +409,10 @@ cudaError_t launch_export_bb(const Handle &h, double *bb, cudaStream_t s);
 // outside the store window (use launch_legacy_bb instead).
 cudaError_t launch_legacy_bb_df(const double *bb_ref, int E, float4 *Ahi, float4 *Alo,
                                 int *bad, cudaStream_t s);
-cudaError_t launch_legacy_conn(const int *iss_ref, int E, int N, const int *bc,
-                               int *conn, int *bad, cudaStream_t s);
+// (bit 3 of *bad unless iss is the canonical numbering of nax x nay nodes a
+// plane)
+cudaError_t launch_legacy_conn(const int *iss_ref, int E, int N, int nax, int nay,
+                               const int *bc, int *conn, int *bad, cudaStream_t s);
 // diag = 1 on Dirichlet nodes (when mask != null); dinv = 1/diag.
 cudaError_t launch_diag_fix(double *diag, double *dinv,
                             const unsigned char *mask, int N, cudaStream_t s);
@@ -443,11 +447,11 @@ int solve_half_rows(Handle &h, const double *res, double rnorm, double *x, doubl
                     int itmax, int *iter, double *err);
 
 // ---- whole solves in one launch (resident.cu) ----
-// BiCGStab with Jacobi on the assembled rows, where they fit in L2; the
-// outcome is in h.st.  An error means that nothing ran.
+// BiCGStab or BiCG with Jacobi on the assembled rows, where a node per thread
+// fits on the device; the outcome is in h.st.  An error means that nothing ran.
 bool resident_fits(const Handle &h);
-cudaError_t launch_resident(Handle &h, const double *b, double *x, double tol, int itmax,
-                            int stall_window);
+cudaError_t launch_resident(Handle &h, int method, const double *b, double *x, double tol,
+                            int itmax, int stall_window);
 
 // ---- the 16-bit inner operator (half.cu) ----
 // Builds A^ = P A P D^-1 in the binary16 store from the current FP64
