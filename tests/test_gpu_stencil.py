@@ -217,3 +217,45 @@ def test_dropin_launch_shapes(vdr, oracle, gpu_lib, dims):
         m.nnode, b, x0, 1e-11, 5000, np.ascontiguousarray(bb.reshape(E, 64)[perm]).ravel(),
         np.ascontiguousarray(m.iss.reshape(8, E)[:, perm]).ravel(), diag, *args)
     assert err2 <= 1e-11 and rel_l2(x2, ref) < 1e-9
+
+
+def test_many_meshes_on_assembled_rows(vdr, oracle, gpu_lib):
+    """Uneven meshes in one handle, a mesh of one element and one of a single
+    row among them: every mesh's solution against the element-wise segmented
+    solve (scatter "atomic") and its true residual by the oracle; a non-finite
+    source stays in its own mesh; a second solve at another tolerance."""
+    torch = pytest.importorskip("torch")
+    P = vdr.problems
+    probs = [P.rotation_cube(7, 91), P.rotation_shear(1, 1, 1, seed=92),
+             P.rotation_cube(12, 93), P.rotation_shear(19, 1, 2, seed=94),
+             P.rotation_shear(40, 31, 9, seed=95)]
+    union = P.concat(probs)
+    off, aM = union.mesh.node_off, 10.0
+    bad_mesh = 2
+    out = {}
+    for scatter in ("auto", "atomic"):
+        with vdr.Solver(union, vdr.Options(scatter=scatter), aH=2.0, aM=aM) as s:
+            s.set_segments(off)
+            told = torch.tensor(np.cos(0.37 * np.arange(union.mesh.nnode)), device="cuda")
+            b = torch.empty_like(told)
+            s.assemble_rhs_device(b, 3.0, aM, told)
+            b *= torch.tensor(union.bc == 0, device="cuda")
+            for tol in (1e-6, 1e-12):
+                x = torch.zeros_like(b)
+                its, errs, sts, st = s.solve_segmented_device(b, x, tol=tol, itmax=2000)
+                assert st == 0 and np.all(sts == 0) and np.all(errs <= tol)
+            out[scatter] = (x.cpu().numpy(), b.cpu().numpy())
+            bad = b.clone()
+            bad[int(off[bad_mesh]) + 900] = float("inf")
+            y = torch.zeros_like(b)
+            _, _, sts, _ = s.solve_segmented_device(bad, y, tol=1e-12, itmax=2000)
+            assert np.all(np.delete(sts, bad_mesh) == 0)
+            keep = np.r_[0:off[bad_mesh], off[bad_mesh + 1]:off[-1]]
+            assert rel_l2(y.cpu().numpy()[keep], out[scatter][0][keep]) < 1e-9
+    x, b = out["auto"]
+    for m, p in enumerate(probs):
+        sl = slice(off[m], off[m + 1])
+        assert rel_l2(x[sl], out["atomic"][0][sl]) < 1e-9, m
+        ax, _ = oracle.matvec0(p.mesh.iss, oracle_bb(oracle, p, 2.0, aM), p.bc, x[sl])
+        nb = np.linalg.norm(b[sl])
+        assert np.linalg.norm(b[sl] - ax) <= 2e-12 * nb or nb == 0.0, m

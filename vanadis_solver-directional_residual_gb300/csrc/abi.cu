@@ -372,6 +372,7 @@ void invalidate(Handle &h) {
   h.aos_valid = h.phi_valid = false;
   if (h.st_state > 0) h.st_state = 0;
   if (h.hr_state > 0) h.hr_state = 0;
+  h.seg_rows = false;
   h.st_applies = 0;
 }
 
@@ -422,6 +423,7 @@ void free_handle(Handle &h) {
   if (h.hr_H) cudaFree(h.hr_H);
   dfree(h.hr_e); dfree(h.hr_vec);
   if (h.hr_graph) cudaGraphExecDestroy(h.hr_graph);
+  dfree(h.seg_mesh); dfree(h.seg_x);
   dfree(h.vel); dfree(h.lam); dfree(h.pdec); dfree(h.q);
   dfree(h.vel32); dfree(h.lam32); dfree(h.pdec32); dfree(h.robin);
   dfree(h.A64); dfree(h.A32); dfree(h.diag); dfree(h.dinv);

@@ -917,6 +917,12 @@ cudaError_t launch_emask(Handle &h) {
   return cudaGetLastError();
 }
 
+cudaError_t launch_element_masks(Handle &h) {
+  emask_kernel<<<grid_for(h.E, 256, 8), 256, 0, h.stream>>>(h.conn, h.E, h.emask);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_mask_conn(int *conn, int E, const unsigned char *mask,
                              cudaStream_t s) {
   mask_conn_kernel<<<grid_for((long)E * 8, 256, 16), 256, 0, s>>>(

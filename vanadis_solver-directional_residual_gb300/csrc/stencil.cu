@@ -23,57 +23,78 @@ __device__ __forceinline__ void acc_pair(DfAcc &acc, float h, float l) {
 // around it, TwoSum per entry (error ~2^-47 of the largest element entry, as
 // the sums of an element-wise apply).  One thread per node: an element's
 // row i is read by exactly one thread, so the store is read once (512 E
-// bytes) and 220 N written: 1.23 ms at 8.4M elements (5.0 TB/s).
+// bytes) and 220 N written: 1.23 ms at 8.4M elements (5.0 TB/s).  The mesh's
+// elements lie from e0 on in the store of E, `l` is the node's number in it.
+__device__ __forceinline__ void assemble_node(const float4 *__restrict__ Ahi,
+                                              const float4 *__restrict__ Alo,
+                                              const unsigned char *__restrict__ emask, int E,
+                                              long e0, int nax, int nay, int naz, unsigned l,
+                                              long n, long N, float2 *S, unsigned *nm) {
+  const unsigned r = l / (unsigned)nax;
+  const int i = (int)(l - r * (unsigned)nax);
+  const int k = (int)(r / (unsigned)nay), j = (int)(r - (unsigned)k * (unsigned)nay);
+  DfAcc acc[27];
+#pragma unroll
+  for (int t = 0; t < 27; t++) acc[t] = DfAcc{0.f, 0.f};
+  unsigned m = 0u;
+#pragma unroll
+  for (int e = 0; e < 8; e++) {
+    const int ex = (e & 1) - 1, ey = ((e >> 1) & 1) - 1, ez = (e >> 2) - 1;
+    const int ei = i + ex, ej = j + ey, ek = k + ez;
+    if (ei < 0 || ei >= nax - 1 || ej < 0 || ej >= nay - 1 || ek < 0 || ek >= naz - 1)
+      continue;
+    const long p = e0 + ei + (long)(nax - 1) * (ej + (long)(nay - 1) * ek);
+    const int own = slot_of(-ex, -ey, -ez);
+    const unsigned dm = __ldg(emask + p);
+    if ((dm >> own) & 1u) continue;  // a Dirichlet row
+    float4 h[2], lo[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      h[q] = __ldcs(Ahi + (size_t)(2 * own + q) * E + p);
+      lo[q] = __ldcs(Alo + (size_t)(2 * own + q) * E + p);
+    }
+#pragma unroll
+    for (int s = 0; s < 8; s++) {
+      const int t = 9 * (slot_z(s) + ez + 1) + 3 * (slot_y(s) + ey + 1) + slot_x(s) + ex + 1;
+      const float4 &hq = h[s >> 2], &lq = lo[s >> 2];
+      const int w = s & 3;
+      const float hv = w == 0 ? hq.x : w == 1 ? hq.y : w == 2 ? hq.z : hq.w;
+      const float lv = w == 0 ? lq.x : w == 1 ? lq.y : w == 2 ? lq.z : lq.w;
+      if (!((dm >> s) & 1u)) {
+        acc_pair(acc[t], hv, lv);
+        m |= 1u << t;
+      }
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < 27; t++) {
+    const Df2 a = df_norm(acc[t]);
+    S[(size_t)t * N + n] = make_float2(a.h, a.l);
+  }
+  nm[n] = m;
+}
+
 __global__ void __launch_bounds__(256, 2) stencil_assemble(
     const float4 *__restrict__ Ahi, const float4 *__restrict__ Alo,
     const unsigned char *__restrict__ emask, int nax, int nay, int naz, float2 *S,
     unsigned *nm) {
   const int E = (nax - 1) * (nay - 1) * (naz - 1), N = nax * nay * naz;
   for (long n = (long)blockIdx.x * blockDim.x + threadIdx.x; n < N;
-       n += (long)gridDim.x * blockDim.x) {
-    const unsigned r = (unsigned)n / (unsigned)nax;
-    const int i = (int)((unsigned)n - r * (unsigned)nax);
-    const int k = (int)(r / (unsigned)nay), j = (int)(r - (unsigned)k * (unsigned)nay);
-    DfAcc acc[27];
-#pragma unroll
-    for (int t = 0; t < 27; t++) acc[t] = DfAcc{0.f, 0.f};
-    unsigned m = 0u;
-#pragma unroll
-    for (int e = 0; e < 8; e++) {
-      const int ex = (e & 1) - 1, ey = ((e >> 1) & 1) - 1, ez = (e >> 2) - 1;
-      const int ei = i + ex, ej = j + ey, ek = k + ez;
-      if (ei < 0 || ei >= nax - 1 || ej < 0 || ej >= nay - 1 || ek < 0 || ek >= naz - 1)
-        continue;
-      const long p = ei + (long)(nax - 1) * (ej + (long)(nay - 1) * ek);
-      const int own = slot_of(-ex, -ey, -ez);
-      const unsigned dm = __ldg(emask + p);
-      if ((dm >> own) & 1u) continue;  // a Dirichlet row
-      float4 h[2], l[2];
-#pragma unroll
-      for (int q = 0; q < 2; q++) {
-        h[q] = __ldcs(Ahi + (size_t)(2 * own + q) * E + p);
-        l[q] = __ldcs(Alo + (size_t)(2 * own + q) * E + p);
-      }
-#pragma unroll
-      for (int s = 0; s < 8; s++) {
-        const int t = 9 * (slot_z(s) + ez + 1) + 3 * (slot_y(s) + ey + 1) + slot_x(s) + ex + 1;
-        const float4 &hq = h[s >> 2], &lq = l[s >> 2];
-        const int w = s & 3;
-        const float hv = w == 0 ? hq.x : w == 1 ? hq.y : w == 2 ? hq.z : hq.w;
-        const float lv = w == 0 ? lq.x : w == 1 ? lq.y : w == 2 ? lq.z : lq.w;
-        if (!((dm >> s) & 1u)) {
-          acc_pair(acc[t], hv, lv);
-          m |= 1u << t;
-        }
-      }
-    }
-#pragma unroll
-    for (int t = 0; t < 27; t++) {
-      const Df2 a = df_norm(acc[t]);
-      S[(size_t)t * N + n] = make_float2(a.h, a.l);
-    }
-    nm[n] = m;
-  }
+       n += (long)gridDim.x * blockDim.x)
+    assemble_node(Ahi, Alo, emask, E, 0, nax, nay, naz, (unsigned)n, n, N, S, nm);
+}
+
+// The same for many meshes side by side (one row of blocks per mesh).
+__global__ void __launch_bounds__(256, 2) stencil_assemble_meshes(
+    const float4 *__restrict__ Ahi, const float4 *__restrict__ Alo,
+    const unsigned char *__restrict__ emask, int E, long N,
+    const SegMesh *__restrict__ meshes, float2 *S, unsigned *nm) {
+  const SegMesh g = meshes[blockIdx.y];
+  const int count = g.nax * g.nay * g.naz;
+  for (int l = (int)(blockIdx.x * blockDim.x + threadIdx.x); l < count;
+       l += (int)(gridDim.x * blockDim.x))
+    assemble_node(Ahi, Alo, emask, E, g.e0, g.nax, g.nay, g.naz, (unsigned)l, g.n0 + (long)l,
+                  N, S, nm);
 }
 
 // y = A x or A^T x, or y += with ACC, any FP64 x.  Here every thread splits
@@ -122,39 +143,55 @@ bool stencil_ready(const Handle &h) {
          !h.gate_active && h.storage == VDR_STORE_DF;
 }
 
+// Room for the rows of the handle's nodes and for `len` pairs in *x (its
+// present length in *have; a new one is not zeroed).  False where the device
+// has no room for them: the element-wise apply stays.
+static bool row_storage(Handle &h, float2 **x, size_t *have, size_t len) {
+  const size_t N = (size_t)h.N;
+  const bool rows = N > h.st_rows, vec = len > *have;
+  if (!rows && !vec) return true;
+  if (rows) {
+    cudaFree(h.st_S);
+    cudaFree(h.st_nm);
+    h.st_S = nullptr;
+    h.st_nm = nullptr;
+    h.st_rows = 0;
+  }
+  if (vec) {
+    cudaFree(*x);
+    *x = nullptr;
+    *have = 0;
+    h.st_nax = 0;  // its pads are to be zeroed
+  }
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
+      (rows ? 220 * N : 0) + (vec ? sizeof(float2) * len : 0) <= free_b / 2 &&
+      (!rows || (!cudaMalloc(&h.st_S, sizeof(float2) * 27 * N) &&
+                 !cudaMalloc(&h.st_nm, sizeof(unsigned) * N))) &&
+      (!vec || !cudaMalloc(x, sizeof(float2) * len))) {
+    if (rows) h.st_rows = N;
+    if (vec) *have = len;
+    return true;
+  }
+  cudaGetLastError();
+  cudaFree(h.st_S);
+  cudaFree(h.st_nm);
+  cudaFree(*x);
+  h.st_S = nullptr;
+  h.st_nm = nullptr;
+  *x = nullptr;
+  *have = h.st_rows = 0;
+  h.st_state = -1;
+  return false;
+}
+
 cudaError_t ensure_stencil(Handle &h) {
   if (h.st_state != 0 || !h.op64_valid || h.apply_mode != VDR_APPLY_STORED ||
       h.storage != VDR_STORE_DF || h.opt.scatter != VDR_SCATTER_AUTO || h.perm_d || !h.Ahi ||
       !h.emask || h.nax < 2 || h.nay < 2 || h.naz < 2)
     return cudaSuccess;
   const size_t N = (size_t)h.N, len = 2 * (N + 2 * stencil_pad(h));
-  if (N > h.st_rows || len > h.st_len) {
-    cudaFree(h.st_S);
-    cudaFree(h.st_nm);
-    cudaFree(h.st_x);
-    h.st_S = nullptr;
-    h.st_nm = nullptr;
-    h.st_x = nullptr;
-    h.st_rows = h.st_len = 0;
-    h.st_nax = 0;
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || 240 * N > free_b / 2 ||
-        cudaMalloc(&h.st_S, sizeof(float2) * 27 * N) ||
-        cudaMalloc(&h.st_nm, sizeof(unsigned) * N) ||
-        cudaMalloc(&h.st_x, sizeof(float2) * len)) {
-      cudaGetLastError();  // no room for the rows: the element-wise apply stays
-      cudaFree(h.st_S);
-      cudaFree(h.st_nm);
-      cudaFree(h.st_x);
-      h.st_S = nullptr;
-      h.st_nm = nullptr;
-      h.st_x = nullptr;
-      h.st_state = -1;
-      return cudaSuccess;
-    }
-    h.st_rows = N;
-    h.st_len = len;
-  }
+  if (!row_storage(h, &h.st_x, &h.st_len, len)) return cudaSuccess;
   cudaError_t e;
   if (h.st_nax != h.nax || h.st_pl != h.nax * h.nay) {
     if ((e = cudaMemsetAsync(h.st_x, 0, sizeof(float2) * h.st_len, h.stream))) return e;
@@ -168,6 +205,27 @@ cudaError_t ensure_stencil(Handle &h) {
   count_launches(1);
   e = cudaGetLastError();
   if (!e) h.st_state = 1;
+  return e;
+}
+
+cudaError_t ensure_segment_rows(Handle &h) {
+  if (h.seg_rows || !h.seg_canonical || !h.op64_valid ||
+      h.apply_mode != VDR_APPLY_STORED || h.storage != VDR_STORE_DF ||
+      h.opt.scatter != VDR_SCATTER_AUTO || h.perm_d || !h.Ahi || h.st_state < 0)
+    return cudaSuccess;
+  cudaError_t e;
+  if (!h.emask && (e = cudaMalloc(&h.emask, (size_t)h.E))) return e;
+  size_t have = h.seg_x ? 2 * h.seg_pairs : 0;
+  const bool fresh = have == 0;
+  if (!row_storage(h, &h.seg_x, &have, 2 * h.seg_pairs)) return cudaSuccess;
+  if (fresh && (e = cudaMemsetAsync(h.seg_x, 0, sizeof(float2) * have, h.stream))) return e;
+  if ((e = launch_element_masks(h))) return e;
+  const int per = (int)std::max<long>(1, std::min<long>(64, (h.seg_largest + 255) / 256));
+  stencil_assemble_meshes<<<dim3((unsigned)per, (unsigned)(h.seg_off.size() - 1)), 256, 0,
+                            h.stream>>>(h.Ahi, h.Alo, h.emask, h.E, h.N, h.seg_mesh, h.st_S,
+                                        h.st_nm);
+  count_launches(1);
+  if (!(e = cudaGetLastError())) h.seg_rows = true;
   return e;
 }
 

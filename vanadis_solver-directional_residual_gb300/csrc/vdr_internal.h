@@ -149,6 +149,14 @@ struct GeoFactors {
   float2 *Ji = nullptr, *Dj = nullptr, *K = nullptr;
 };
 
+// One mesh of a handle that holds several: its first node and element, its
+// grid, and where its nodes lie in the padded pair vectors (node n at n +
+// shift).
+struct SegMesh {
+  int n0, nax, nay, naz;
+  long long e0, shift;
+};
+
 struct Handle {
   int N = 0, E = 0;
   int nax = 0, nay = 0, naz = 0;  // > 0 when the mesh is the canonical structured numbering
@@ -304,6 +312,13 @@ struct Handle {
   const void *seg_key = nullptr;
   long seg_graph_launches = 0;
   int *seg_of_elem = nullptr;         // [E] storage order
+  // every mesh in the canonical numbering: their grids, the assembled rows
+  // (in st_S, st_nm) and two pair vectors with zeros between the meshes
+  bool seg_canonical = false, seg_rows = false;
+  SegMesh *seg_mesh = nullptr;
+  float2 *seg_x = nullptr;
+  size_t seg_pairs = 0;
+  long seg_largest = 0;  // nodes of the largest mesh
   const int *gate_eseg = nullptr;     // apply gate while a segmented solve runs
   const int *gate_active = nullptr;
 
@@ -431,6 +446,9 @@ cudaError_t launch_bc_to_mask(const int *bc, unsigned char *mask, int N,
 // called before work that applies the operator several times.
 cudaError_t ensure_stencil(Handle &h);
 bool stencil_ready(const Handle &h);
+// The same for a handle of many meshes (h.seg_rows when they are current).
+cudaError_t ensure_segment_rows(Handle &h);
+cudaError_t launch_element_masks(Handle &h);
 // y (+)= A x or A^T x from the assembled rows.
 cudaError_t launch_stencil_apply(const Handle &h, bool transpose, bool accumulate,
                                  const double *x, double *y, const int *skip,
