@@ -27,10 +27,16 @@
 // output]: the second part comes from its own tensor (the upsampled copy)
 // through a second map, into its own slab.
 //
-// Weights: [tap][chunk][COUT][8] BF16 in the no-swizzle K-major layout
-// (core matrices of 8 output channels x 8 input channels), resident in
-// shared memory when all 27 taps fit next to the slab stages, else streamed
-// one tap at a time through a ring.
+// Weights: BF16 in the no-swizzle K-major layout (core matrices of 8 output
+// channels x 8 input channels).  Resident in shared memory when all 27 taps
+// fit next to the slab stages: [dy, dx][chunk][dz = 2, 1, 0][COUT][8], the
+// three z taps of a slab plane side by side, so that the plane's rows are
+// read once per (dy, dx) for all three output planes that they feed (9 (G +
+// 2) MMAs of N = 3 COUT per K step and tile instead of 27 G of N = COUT:
+// at N = 16 an MMA is bound by its 4 KB of A rows).  A pass over 129 x 129 x
+// 65 voxels, 16 -> 16 channels: 57 -> 36 us; the whole forward's kernels 614
+// -> 445 us.
+// Else [tap][chunk][COUT][8], streamed one tap at a time through a ring.
 //
 // Warp roles (192 threads): warp 0 = TMA / bulk-copy producer, warp 1 =
 // TMEM owner and MMA issuer, warps 2-5 = epilogue (TMEM -> registers ->
@@ -92,6 +98,12 @@ __host__ __device__ constexpr int stages_of(int cin1, int cin2, int cout) {
 __host__ __device__ constexpr int group_of(int cin1, int cin2, int cout) {
   return fit_group(cin1, cin2, cout, stages_of(cin1, cin2, cout));
 }
+// Whether all 27 taps' weights lie in shared memory (the Shape's RES).
+__host__ __device__ constexpr bool weights_resident(int cin1, int cin2, int cout) {
+  const int ns = stages_of(cin1, cin2, cout), G = group_of(cin1, cin2, cout);
+  return 27 * tap_bytes(cin1 + cin2, cout) +
+             ns * (slab_bytes(cin1, G) + slab_bytes(cin2, G)) <= BUDGET;
+}
 // Descriptor layout code of a K-major operand whose rows are `row_bytes`
 // wide: 32B, 64B or 128B swizzle.
 __host__ __device__ constexpr int swizzle_code(int row_bytes) {
@@ -118,7 +130,7 @@ struct Shape {
   static constexpr int SLAB = SLAB1 + SLAB2;
   static constexpr int TXB = PROWS * (G + 2) * 2 * (CIN1 + CIN2);  // bytes the boxes land
   static constexpr int WTAP = tap_bytes(CIN1 + CIN2, COUT);  // one tap's weights
-  static constexpr bool RES = 27 * WTAP + NS * SLAB <= BUDGET;
+  static constexpr bool RES = weights_resident(CIN1, CIN2, COUT);
   static constexpr int NW = RES ? 27 : 8;       // weight slots
   static constexpr int ACC = 2 * G * COUT;      // columns of the two accumulator sets
   static constexpr int TMEM_COLS =
@@ -269,43 +281,82 @@ __global__ void __launch_bounds__(THREADS, 1)
             tc::smem_desc_sw(sbase + S::SLAB1, SX * 2 * (CIN2 > 0 ? CIN2 : 16),
                              swizzle_code(CIN2 > 0 ? 2 * CIN2 : 32));
         const uint64_t bdd = tc::smem_desc(tc::smem_u32(wbuf), COUT * 16, 128);
+        const uint64_t b3d = tc::smem_desc(tc::smem_u32(wbuf), 3 * COUT * 16, 128);
+        if constexpr (S::RES) {
+          // Slab plane zs feeds output planes zs - 2, zs - 1 and zs with the
+          // taps dz = 2, 1 and 0: one MMA per (dy, dx) and K step with the
+          // three taps' weights side by side (N = 3 COUT) and the planes'
+          // accumulators, which lie side by side too.  Every plane still
+          // adds its taps in the order dz, dy, dx, K.
+#pragma unroll 1
+          for (int zs = 0; zs < S::G + 2; zs++) {
+            const int g0 = zs < 2 ? 0 : zs - 2, g1 = zs < S::G ? zs : S::G - 1;
+            const int nb = g1 - g0 + 1, blk = g0 - zs + 2;  // planes, first weight block
+            const uint32_t d0 = dtm + (uint32_t)(g0 * COUT);
+            const uint32_t idn = nb == 3 ? tc::idesc_bf16_f32(128, 3 * COUT)
+                                 : nb == 2 ? tc::idesc_bf16_f32(128, 2 * COUT) : IDESC;
+            const uint64_t bz = b3d + (uint64_t)((blk * COUT * 16) >> 4);
+            const uint64_t az1 = a1d + (uint64_t)(((uint32_t)zs * PROWS * 2 * CIN1) >> 4);
+            const uint64_t az2 =
+                a2d + (uint64_t)(((uint32_t)zs * PROWS * 2 * (CIN2 > 0 ? CIN2 : 16)) >> 4);
+#pragma unroll
+            for (int t9 = 0; t9 < 9; t9++) {
+              const int row = (t9 / 3) * SX + t9 % 3;
+              const uint64_t bt = bz + (uint64_t)((t9 * 3 * S::WTAP) >> 4);
+#pragma unroll
+              for (int j = 0; j < (CIN1 + CIN2) / 16; j++) {
+                const uint64_t ad =
+                    j < CIN1 / 16
+                        ? az1 + (uint64_t)((row * 2 * CIN1 + 32 * j) >> 4)
+                        : az2 + (uint64_t)((row * 2 * CIN2 + 32 * (j - CIN1 / 16)) >> 4);
+                const uint64_t bd = bt + (uint64_t)((2 * j * 3 * COUT * 16) >> 4);
+                if (t9 == 0 && j == 0 && zs < S::G) {
+                  // plane zs starts here: its columns are overwritten
+                  if (nb > 1)
+                    tc::mma_bf16(d0, ad, bd, nb == 3 ? tc::idesc_bf16_f32(128, 2 * COUT) : IDESC,
+                                 1u);
+                  tc::mma_bf16(dtm + (uint32_t)(zs * COUT), ad,
+                               bd + (uint64_t)(((nb - 1) * COUT * 16) >> 4), IDESC, 0u);
+                } else {
+                  tc::mma_bf16(d0, ad, bd, idn, 1u);
+                }
+              }
+            }
+          }
+        } else {
 #pragma unroll 3
-        for (int tap = 0; tap < 27; tap++) {
-          int w = tap;
-          if (!S::RES) {
-            w = (int)(wc % S::NW);
+          for (int tap = 0; tap < 27; tap++) {
+            const int w = (int)(wc % S::NW);
             if (!tc::mbar_wait(bar(B_WFULL + w), (uint32_t)(wc / S::NW) & 1u, WAIT_LIMIT)) {
               ok = false;
               break;
             }
             tc::fence_after();
-          }
-          const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;  // 0..2
-          const int row0 = (dz * SY + dy) * SX + dx;  // the tap's first slab row
-          const uint64_t bt = bdd + (uint64_t)((w * S::WTAP) >> 4);
-          // part 1: rows of 2 CIN1 bytes, K steps of 16 channels (32 bytes);
-          // plane g's rows start PROWS g rows further into the slab
-          const uint64_t at1 = a1d + (uint64_t)((row0 * 2 * CIN1) >> 4);
+            const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;  // 0..2
+            const int row0 = (dz * SY + dy) * SX + dx;  // the tap's first slab row
+            const uint64_t bt = bdd + (uint64_t)((w * S::WTAP) >> 4);
+            // part 1: rows of 2 CIN1 bytes, K steps of 16 channels (32 bytes);
+            // plane g's rows start PROWS g rows further into the slab
+            const uint64_t at1 = a1d + (uint64_t)((row0 * 2 * CIN1) >> 4);
 #pragma unroll
-          for (int j = 0; j < CIN1 / 16; j++)
-#pragma unroll
-            for (int g = 0; g < S::G; g++)
-              tc::mma_bf16(dtm + g * COUT,
-                           at1 + (uint64_t)((g * PROWS * 2 * CIN1 + 32 * j) >> 4),
-                           bt + (uint64_t)((2 * j * COUT * 16) >> 4), IDESC,
-                           (tap > 0 || j > 0) ? 1u : 0u);
-          if (CIN2 > 0) {
-            const uint64_t at2 = a2d + (uint64_t)((row0 * 2 * CIN2) >> 4);
-#pragma unroll
-            for (int j = 0; j < CIN2 / 16; j++)
+            for (int j = 0; j < CIN1 / 16; j++)
 #pragma unroll
               for (int g = 0; g < S::G; g++)
                 tc::mma_bf16(dtm + g * COUT,
-                             at2 + (uint64_t)((g * PROWS * 2 * CIN2 + 32 * j) >> 4),
-                             bt + (uint64_t)(((S::KC1 + 2 * j) * COUT * 16) >> 4), IDESC,
-                             1u);
-          }
-          if (!S::RES) {
+                             at1 + (uint64_t)((g * PROWS * 2 * CIN1 + 32 * j) >> 4),
+                             bt + (uint64_t)((2 * j * COUT * 16) >> 4), IDESC,
+                             (tap > 0 || j > 0) ? 1u : 0u);
+            if (CIN2 > 0) {
+              const uint64_t at2 = a2d + (uint64_t)((row0 * 2 * CIN2) >> 4);
+#pragma unroll
+              for (int j = 0; j < CIN2 / 16; j++)
+#pragma unroll
+                for (int g = 0; g < S::G; g++)
+                  tc::mma_bf16(dtm + g * COUT,
+                               at2 + (uint64_t)((g * PROWS * 2 * CIN2 + 32 * j) >> 4),
+                               bt + (uint64_t)(((S::KC1 + 2 * j) * COUT * 16) >> 4), IDESC,
+                               1u);
+            }
             tc::commit(bar(B_WEMPTY + w));
             wc++;
           }

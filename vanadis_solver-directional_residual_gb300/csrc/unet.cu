@@ -560,28 +560,40 @@ __host__ __device__ inline Dims coarse_of(const Dims &f) {
   return c;
 }
 
+// Eight channels (16 bytes) a thread.
 __global__ void pool_fwd(const bf16 *in, bf16 *out, Dims f, Dims c, int C,
                          const int *skip, const int *skip2) {
   if (skipped(skip, skip2)) return;
-  const long total = c.V * C;
+  const int c8 = C / 8;
+  const long total = c.V * c8;
   for (long idx = (long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += (long)gridDim.x * blockDim.x) {
-    const int ch = (int)(idx % C);
-    const long vc = idx / C;
-    const int X = (int)(vc % c.W), Y = (int)((vc / c.W) % c.H),
-              Z = (int)(vc / ((long)c.W * c.H));
-    float s = 0.f;
+    const int ch = (int)((unsigned)idx % (unsigned)c8);
+    const unsigned vc = (unsigned)(idx / c8);
+    const int X = (int)(vc % (unsigned)c.W), r = (int)(vc / (unsigned)c.W);
+    const int Y = r % c.H, Z = r / c.H;
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     int cnt = 0;
-    for (int k = 0; k < 2; k++)
-      for (int j = 0; j < 2; j++)
-        for (int i = 0; i < 2; i++) {
-          const int x = 2 * X + i, y = 2 * Y + j, z = 2 * Z + k;
-          if (x < f.W && y < f.H && z < f.D) {
-            s += __bfloat162float(in[((long)x + (long)f.W * (y + (long)f.H * z)) * C + ch]);
-            cnt++;
-          }
+#pragma unroll
+    for (int t = 0; t < 8; t++) {
+      const int x = 2 * X + (t & 1), y = 2 * Y + ((t >> 1) & 1), z = 2 * Z + (t >> 2);
+      if (x < f.W && y < f.H && z < f.D) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(
+                                  in + ((long)x + (long)f.W * (y + (long)f.H * z)) * C) + ch);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          s[2 * k] += bf_lo(w[k]);
+          s[2 * k + 1] += bf_hi(w[k]);
         }
-    out[idx] = __float2bfloat16_rn(s / (float)cnt);
+        cnt++;
+      }
+    }
+    uint32_t o[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      o[k] = pack2(s[2 * k] / (float)cnt, s[2 * k + 1] / (float)cnt);
+    reinterpret_cast<uint4 *>(out)[idx] = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 
@@ -720,9 +732,10 @@ __global__ void adam_kernel(float *th, const float *g, float *m, float *v, long 
 // BF16 copies of a conv layer's weights: wb (same layout) and wbt =
 // [27][CIN][COUT] with the tap flipped (the backward data pass).
 // wb[tap][co][ci] (forward), wbt[26 - tap][ci][co] (backward data pass) and
-// wtc[tap][ci/8][co][ci%8] (the tensor-core kernel's core-matrix order).
+// wtc[tap][ci/8][co][ci%8], or with the three z taps side by side (stack)
+// wtc[dy, dx][ci/8][2 - dz][co][ci%8] (the tensor-core kernel's orders).
 __global__ void pack_weights(const float *th, bf16 *wb, bf16 *wbt, bf16 *wtc, int cin,
-                             int cout) {
+                             int cout, int stack) {
   const long total = 27L * cin * cout;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long)gridDim.x * blockDim.x) {
@@ -732,7 +745,8 @@ __global__ void pack_weights(const float *th, bf16 *wb, bf16 *wbt, bf16 *wtc, in
     const bf16 b = __float2bfloat16_rn(th[i]);
     wb[i] = b;
     wbt[((long)(26 - tap) * cin + ci) * cout + co] = b;
-    wtc[(((long)tap * (cin / 8) + ci / 8) * cout + co) * 8 + (ci & 7)] = b;
+    const long chunk = (long)(stack ? tap % 9 : tap) * (cin / 8) + ci / 8;
+    wtc[((stack ? chunk * 3 + 2 - tap / 9 : chunk) * cout + co) * 8 + (ci & 7)] = b;
   }
 }
 
@@ -1283,11 +1297,11 @@ cudaError_t net_forward_tc(Net &n, const int *sk, const int *sk2, cudaStream_t s
   if ((e = conv_tc_launch<16, 0, 16>(n, L_E0A, n.a0, sk, sk2, s)) ||
       (e = conv_tc_launch<16, 0, 16>(n, L_E0B, n.s0, sk, sk2, s)))
     return e;
-  pool_fwd<<<grid_for(f1.V * 16, 256), 256, 0, s>>>(n.s0, n.p0, f0, f1, 16, sk, sk2);
+  pool_fwd<<<grid_for(f1.V * 2, 256), 256, 0, s>>>(n.s0, n.p0, f0, f1, 16, sk, sk2);
   if ((e = conv_tc_launch<16, 0, 32>(n, L_E1A, n.a1, sk, sk2, s)) ||
       (e = conv_tc_launch<32, 0, 32>(n, L_E1B, n.s1, sk, sk2, s)))
     return e;
-  pool_fwd<<<grid_for(f2.V * 32, 256), 256, 0, s>>>(n.s1, n.p1, f1, f2, 32, sk, sk2);
+  pool_fwd<<<grid_for(f2.V * 4, 256), 256, 0, s>>>(n.s1, n.p1, f1, f2, 32, sk, sk2);
   if ((e = conv_tc_launch<32, 0, 64>(n, L_BTA, n.a2, sk, sk2, s)) ||
       (e = conv_tc_launch<64, 0, 64>(n, L_BTB, n.b2, sk, sk2, s)))
     return e;
@@ -1319,10 +1333,10 @@ cudaError_t net_forward(Net &n, const int *sk, const int *sk2, cudaStream_t s) {
     return e;
   VDR_CONV(16, 0, 16, 0, n.x0, nullptr, L_E0A, n.a0)
   VDR_CONV(16, 0, 16, 0, n.a0, nullptr, L_E0B, n.s0)
-  pool_fwd<<<grid_for(n.d[1].V * 16, 256), 256, 0, s>>>(n.s0, n.p0, n.d[0], n.d[1], 16, sk, sk2);
+  pool_fwd<<<grid_for(n.d[1].V * 2, 256), 256, 0, s>>>(n.s0, n.p0, n.d[0], n.d[1], 16, sk, sk2);
   VDR_CONV(16, 0, 32, 1, n.p0, nullptr, L_E1A, n.a1)
   VDR_CONV(32, 0, 32, 1, n.a1, nullptr, L_E1B, n.s1)
-  pool_fwd<<<grid_for(n.d[2].V * 32, 256), 256, 0, s>>>(n.s1, n.p1, n.d[1], n.d[2], 32, sk, sk2);
+  pool_fwd<<<grid_for(n.d[2].V * 4, 256), 256, 0, s>>>(n.s1, n.p1, n.d[1], n.d[2], 32, sk, sk2);
   VDR_CONV(32, 0, 64, 2, n.p1, nullptr, L_BTA, n.a2)
   VDR_CONV(64, 0, 64, 2, n.a2, nullptr, L_BTB, n.b2)
   VDR_CONV(32, 64, 32, 1, n.s1, n.b2, L_D1A, n.a3)
@@ -1407,7 +1421,7 @@ cudaError_t pack_all(Net &n, cudaStream_t s) {
     const int cin = DEFS[l].cin1 + DEFS[l].cin2, cout = DEFS[l].cout;
     pack_weights<<<grid_for(layer_wsize(l), 256), 256, 0, s>>>(
         n.theta + n.woff[l], n.wb + n.woff[l], n.wbt + n.woff[l], n.wtc + n.woff[l], cin,
-        cout);
+        cout, convtc::weights_resident(DEFS[l].cin1, DEFS[l].cin2, cout));
   }
   count_launches(L_HEAD);
   return cudaGetLastError();
