@@ -259,3 +259,42 @@ def test_many_meshes_on_assembled_rows(vdr, oracle, gpu_lib):
         ax, _ = oracle.matvec0(p.mesh.iss, oracle_bb(oracle, p, 2.0, aM), p.bc, x[sl])
         nb = np.linalg.norm(b[sl])
         assert np.linalg.norm(b[sl] - ax) <= 2e-12 * nb or nb == 0.0, m
+
+
+@pytest.mark.parametrize("K", [16, 32, 64])
+@pytest.mark.parametrize("dims", [(1, 1, 1), (6, 2, 1), (7, 3, 30), (8, 7, 5), (15, 16, 9),
+                                  (33, 17, 12)])
+def test_block_solve_launch_shapes(vdr, oracle, gpu_lib, dims, K):
+    """The block solve on assembled rows where its tiles (8 or 16 nodes along
+    x, 4 or 8 along y), its blocks' shares of the planes and the last plane
+    end: every column's true residual by the oracle, and against the
+    element-wise solve (scatter "atomic"); columns of very different size, a
+    zero one, a start from a nonzero X."""
+    torch = pytest.importorskip("torch")
+    prob = vdr.problems.rotation_shear(*dims, seed=96)
+    m, aM, tol = prob.mesh, 10.0, 1e-11
+    rng = np.random.default_rng(sum(dims) + K)
+    B = rng.standard_normal((m.nnode, K)) * 10.0 ** rng.integers(-200, 200, K)
+    B[prob.bc == 1] = 0.0
+    B[:, 3] = 0.0
+    X0 = np.zeros_like(B)
+    X0[:, 5] = B[:, 5]
+    got = {}
+    for scatter in ("auto", "atomic"):
+        with vdr.Solver(prob, vdr.Options(scatter=scatter), aH=2.0, aM=aM) as s:
+            X = torch.tensor(X0, device="cuda")
+            _, _, errs, st = s.solve_block_device(torch.tensor(B, device="cuda"), X, tol=tol,
+                                                  inner_tol=1e-4)
+            torch.cuda.synchronize()
+            assert st == 0 and np.all(errs <= tol)
+            got[scatter] = X.cpu().numpy()
+    bb = oracle_bb(oracle, prob, 2.0, aM)
+    assert np.all(got["auto"][prob.bc == 1] == 0.0) and np.all(got["auto"][:, 3] == 0.0)
+    for k in range(K):
+        x, b = got["auto"][:, k], B[:, k]
+        if not b.any():
+            continue
+        scale = np.abs(b).max()
+        ax, _ = oracle.matvec0(m.iss, bb, prob.bc, x / scale)
+        assert np.linalg.norm(b / scale - ax) <= 1.01 * tol * np.linalg.norm(b / scale), k
+        assert rel_l2(x / scale, got["atomic"][:, k] / scale) < 1e-8, k

@@ -429,7 +429,7 @@ void free_handle(Handle &h) {
   dfree(h.A64); dfree(h.A32); dfree(h.diag); dfree(h.dinv);
   dfree(h.Ahi); dfree(h.Alo); dfree(h.flag); dfree(h.A16); dfree(h.e16);
   dfree(h.Aaos); dfree(h.phi); dfree(h.perm_d); dfree(h.dinv32); dfree(h.block_err);
-  dfree(h.bk_f); dfree(h.bk_d);
+  dfree(h.bk_f); dfree(h.bk_d); dfree(h.br_rows);
   if (h.bk_graph) cudaGraphExecDestroy(h.bk_graph);
   dfree(h.gcr_work); dfree(h.stage_d); dfree(h.drs); dfree(h.work32);
   dfree(h.Mhi); dfree(h.Mlo); dfree(h.Fvec); dfree(h.rhs_tmp); dfree(h.massw);

@@ -20,7 +20,9 @@
 // launch: per-column scalars (rho, alpha, omega, norms) in FP64, per-column
 // deterministic reductions, and a per-column "active" flag that freezes a
 // column once it meets its tolerance.  The outer loop refines each column
-// in FP64 (residual and update), as the single-RHS mixed solver does.
+// in FP64 (residual and update), as the single-RHS mixed solver does.  On the
+// canonical structured numbering the solve runs on assembled rows
+// (block_rows.cu) unless an apply variant was asked for.
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -28,13 +30,13 @@
 #include <atomic>
 #include <vector>
 
+#include "block_cols.cuh"
 #include "dfloat.cuh"
 #include "vdr_internal.h"
 
 namespace vdr {
 namespace {
 
-constexpr int BT = 512;  // threads per block of the block-vector kernels
 constexpr unsigned FULL = 0xffffffffu;
 
 // --------------------------------------------------------------- applies
@@ -765,33 +767,6 @@ __global__ void block_rhs(const double *__restrict__ phi,
   }
 }
 
-// ------------------------------------------------------ block Krylov state
-struct BState {
-  unsigned ticket;
-  int done, iter, itmax;
-  double tol;
-};
-// per-column arrays, each of length K (kept in one device buffer)
-struct BCols {
-  double *bnrm2, *err, *rho, *rho_old, *alpha, *omega, *snrm;
-  double *tol;  // the column's inner tolerance
-  int *active, *sconv, *status;
-};
-
-struct BVec {
-  long n;  // N*K
-  int K;
-  BState *st;
-  BCols c;
-  double *partials;  // [q][k][block]
-  const float *b, *dinv;  // dinv per node
-  const unsigned char *m; // per node
-  float *x, *r, *rh, *p, *v, *s, *t;
-  int kshift;               // K = 1 << kshift
-  const double *outer_err;  // per column FP64 residual of the refinement
-  double outer_tol;         // columns already at outer_tol stay inactive
-};
-
 // Per-column grid reduction: thread tid owns column tid % K (blockDim is a
 // multiple of K and the grid stride keeps the column).  Each block writes
 // its per-column sums of NQ quantities to partials[q][k][block]; the last
@@ -859,39 +834,6 @@ __device__ __forceinline__ bool col_grid_sum(double (&v)[NQ], const BVec &a,
   __syncthreads();
   if (tid == 0) a.st->ticket = 0u;
   return tid < K;
-}
-
-// Per-thread inner-product accumulation in double-float: exact FP32
-// products (two-product) summed with TwoSum, i.e. FP64-accurate inner
-// products without the FP64 pipe.
-__device__ __forceinline__ void dot_acc(DfAcc &acc, float a, float b) {
-  df_fma_acc(acc, a, 0.0f, b, 0.0f);
-}
-__device__ __forceinline__ double dot_val(const DfAcc &acc) {
-  return df_to_double(acc.s, acc.c);
-}
-
-// Grid-stride loops.  BLOOP: over the N*K block entries, one per thread per
-// trip (the FP64 glue kernels below).  ULOOP: over units of four
-// consecutive columns 4g .. 4g+3 of one node row (unit j = node * K/4 + g,
-// float4 loads and stores); the stride is a multiple of K/4, so a thread's
-// column group g = threadIdx.x % (K/4) never changes.
-#define BSTRIDE ((long)gridDim.x * blockDim.x)
-#define BLOOP(i)                                                      \
-  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; \
-       i += BSTRIDE)
-#define ULOOP(j)                                                           \
-  for (long j = (long)blockIdx.x * blockDim.x + threadIdx.x; j < (a.n >> 2); \
-       j += BSTRIDE)
-
-__device__ __forceinline__ float4 ld4(const float *p, long j) {
-  return reinterpret_cast<const float4 *>(p)[j];
-}
-__device__ __forceinline__ void st4(float *p, long j, float4 v) {
-  reinterpret_cast<float4 *>(p)[j] = v;
-}
-__device__ __forceinline__ float f4(const float4 &v, int c) {
-  return c == 0 ? v.x : (c == 1 ? v.y : (c == 2 ? v.z : v.w));
 }
 
 // col_grid_sum for threads that own four columns: each block first adds,
@@ -1526,13 +1468,6 @@ cudaError_t ensure_aos(Handle &h, bool scaled, float4 **out) {
   return cudaSuccess;
 }
 
-namespace {
-// device workspace of the block solve, carved from h.bk_f / h.bk_d
-constexpr int BK_COLS = 16 * 64;            // per-column doubles and ints
-constexpr int BK_PARTIALS = 2 * 64 * 2048;  // NQ x K x blocks
-constexpr int BK_MAX_GRID = 2048;
-}  // namespace
-
 // The bulk-copy wait's timeout path, end to end: VDR_TIMEOUT when a wait
 // that nothing completes ran out of its (about 1 ms) budget and the flag
 // reached the host; the context stays usable.
@@ -1615,6 +1550,14 @@ int solve_block_device(Handle &h, int K, int precision, const double *B,
   double *scale = colsd + 10 * 64;
   int *colsi = reinterpret_cast<int *>(colsd + 11 * 64);  // 3 x 64 ints + a flag
   a.c.tol = colsd + 13 * 64;
+  a.c.rho_next = colsd + 14 * 64;
+  BlockOuter o{};
+  o.err = outer_err;
+  o.scale = scale;
+  o.bb = colsd + 15 * 64;
+  o.rmax = reinterpret_cast<unsigned long long *>(colsd + 16 * 64);
+  o.bmax = o.rmax + 64;
+  o.xexp = reinterpret_cast<int *>(colsd + 18 * 64);
   a.c.active = colsi;
   a.c.sconv = colsi + 64;
   a.c.status = colsi + 128;
@@ -1635,9 +1578,13 @@ int solve_block_device(Handle &h, int K, int precision, const double *B,
   dinv_to_f32<<<grid_n(h.N, 256, 8), 256, 0, s>>>(h.dinv, h.dinv32, h.N);
   count_launches(1);
   if ((e = cudaGetLastError())) return cuda_fail(e, "block setup");
+  // the canonical structured numbering: the iteration on assembled rows
+  BlockRows rows{};
+  const bool on_rows = block_rows_usable(h, K, &rows);
   // The apply's operator copy carries the Jacobi scale (A D^-1).
   float4 *Aaos = nullptr;
-  if ((e = ensure_aos(h, true, &Aaos))) return cuda_fail(e, "block operator copy");
+  if ((!on_rows || (K == 64 && !h.blk_tuned)) && (e = ensure_aos(h, true, &Aaos)))
+    return cuda_fail(e, "block operator copy");
   if (K == 64 && !h.blk_tuned) {  // launch shape by measurement, before capture
     if ((e = cudaMemsetAsync(a.p, 0, sizeof(float) * 2 * n, s)))
       return cuda_fail(e, "block tuning");
@@ -1646,28 +1593,36 @@ int solve_block_device(Handle &h, int K, int precision, const double *B,
     if (h.bk_graph) cudaGraphExecDestroy(h.bk_graph);
     h.bk_graph = nullptr;
   }
-  const int gv = std::min(BK_MAX_GRID, grid_n(n, BT, 2));  // one wave
+  const int gv = std::min(BK_MAX_GRID, grid_n(on_rows ? n / 4 : n, BT, 2));  // one wave
+  if (on_rows) a.rh = bf;  // x = 0, so the right-hand side is the shadow residual too
   const int gm = grid_n(n, 256, 8);
   // the initial guess masked; a zero one makes the first residual B itself
   int *x_nonzero = colsi + 3 * 64;
   int x_nz_host = 1;
   if ((e = cudaMemsetAsync(x_nonzero, 0, sizeof(int), s))) return cuda_fail(e, "block setup");
-  bo_mask<<<gm, 256, 0, s>>>(n, a.kshift, X, h.mask, x_nonzero);
-  count_launches(1);
+  if (on_rows) {
+    if ((e = cudaMemsetAsync(o.xexp, 0, sizeof(int) * 64, s)) ||
+        (e = block_rows_mask(a, o, X, x_nonzero, gv, s)))
+      return cuda_fail(e, "block setup");
+  } else {
+    bo_mask<<<gm, 256, 0, s>>>(n, a.kshift, X, h.mask, x_nonzero);
+    count_launches(1);
+  }
   if ((e = cudaGetLastError()) ||
       (e = cudaMemcpyAsync(&x_nz_host, x_nonzero, sizeof(int), cudaMemcpyDeviceToHost, s)) ||
       (e = cudaStreamSynchronize(s)))
     return cuda_fail(e, "block setup");
 
-  // KI inner iterations per graph launch (8 kernels each)
+  // KI inner iterations per graph launch (8 kernels each, on rows 4)
   constexpr int KI = 4;
-  if (!h.bk_graph || h.bk_graph_split != split) {
+  if (!h.bk_graph || h.bk_graph_split != split || h.bk_graph_rows != rows.rows) {
     if (h.bk_graph) cudaGraphExecDestroy(h.bk_graph);
     h.bk_graph = nullptr;
     cudaGraph_t graph;
     if ((e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal)))
       return cuda_fail(e, "capture");
-    for (int it = 0; it < KI; it++) {
+    if (on_rows) e = block_rows_iterations(a, rows, KI, gv, s);
+    for (int it = 0; it < KI && !on_rows; it++) {
       bb_p<<<gv, BT, 0, s>>>(a);
       block_apply_launches_tf32(h, K, split, a.p, nullptr, a.v, Aaos,
                                 &st->done, s, true);
@@ -1679,13 +1634,14 @@ int solve_block_device(Handle &h, int K, int precision, const double *B,
       bb_xr<<<gv, BT, 0, s>>>(a);
       bb_tail<<<1, 64, 0, s>>>(a);
     }
-    count_launches(-2L * KI);  // the captured applies count at replay
+    if (!on_rows) count_launches(-2L * KI);  // the captured applies count at replay
     const cudaError_t e2 = cudaStreamEndCapture(s, &graph);
-    if (e2) return cuda_fail(e2, "end capture");
+    if (e || e2) return cuda_fail(e ? e : e2, "end capture");
     e = cudaGraphInstantiate(&h.bk_graph, graph, 0);
     cudaGraphDestroy(graph);
     if (e) return cuda_fail(e, "instantiate");
     h.bk_graph_split = split;
+    h.bk_graph_rows = rows.rows;
   }
 
   BState init{};
@@ -1696,13 +1652,20 @@ int solve_block_device(Handle &h, int K, int precision, const double *B,
   int status = VDR_NOT_CONVERGED;
   for (outer = 0;; outer++) {
     // FP64 residual of every column, its scale and relative norm
-    if ((e = cudaMemsetAsync(R, 0, sizeof(double) * n, s)) ||
-        ((outer > 0 || x_nz_host) && (e = launch_block_apply64(h, K, X, R, s))) ||
-        (e = cudaMemsetAsync(st, 0, sizeof(BState), s)))
-      return cuda_fail(e, "block residual");
-    bo_residual<<<gv, BT, 0, s>>>(a, B, R, mx);
-    bo_scale<<<gv, BT, 0, s>>>(a, B, R, bf, mx, scale, outer_err);
-    count_launches(2);
+    const bool zero_x = outer == 0 && !x_nz_host;
+    if ((e = cudaMemsetAsync(st, 0, sizeof(BState), s))) return cuda_fail(e, "block residual");
+    if (on_rows) {
+      if ((e = cudaMemsetAsync(o.rmax, 0, sizeof(*o.rmax) * 2 * 64, s)) ||
+          (e = block_rows_residual(a, rows, o, B, X, R, zero_x, outer == 0, gv, s)))
+        return cuda_fail(e, "block residual");
+    } else {
+      if ((e = cudaMemsetAsync(R, 0, sizeof(double) * n, s)) ||
+          (!zero_x && (e = launch_block_apply64(h, K, X, R, s))))
+        return cuda_fail(e, "block residual");
+      bo_residual<<<gv, BT, 0, s>>>(a, B, R, mx);
+      bo_scale<<<gv, BT, 0, s>>>(a, B, R, bf, mx, scale, outer_err);
+      count_launches(2);
+    }
     if ((e = cudaMemcpyAsync(herr.data(), outer_err, sizeof(double) * K,
                              cudaMemcpyDeviceToHost, s)) ||
         (e = cudaStreamSynchronize(s)))
@@ -1729,25 +1692,36 @@ int solve_block_device(Handle &h, int K, int precision, const double *B,
       htol[k] = herr[k] > 0.0 ? std::max(inner_tol, 0.5 * tol / herr[k]) : inner_tol;
     if ((e = cudaMemcpyAsync(a.c.tol, htol.data(), sizeof(double) * K,
                              cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemcpyAsync(st, &init, sizeof(BState), cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemsetAsync(a.x, 0, sizeof(float) * n, s)) ||
-        (e = cudaMemsetAsync(a.r, 0, sizeof(float) * n, s)))
+        (e = cudaMemcpyAsync(st, &init, sizeof(BState), cudaMemcpyHostToDevice, s)))
       return cuda_fail(e, "inner reset");
-    bb_start<<<gv, BT, 0, s>>>(a);
-    bb_finish_start<<<1, 64, 0, s>>>(a);
-    count_launches(2);
+    if (on_rows) {
+      if ((e = block_rows_begin(a, s))) return cuda_fail(e, "inner reset");
+    } else {
+      if ((e = cudaMemsetAsync(a.x, 0, sizeof(float) * n, s)) ||
+          (e = cudaMemsetAsync(a.r, 0, sizeof(float) * n, s)))
+        return cuda_fail(e, "inner reset");
+      bb_start<<<gv, BT, 0, s>>>(a);
+      bb_finish_start<<<1, 64, 0, s>>>(a);
+      count_launches(2);
+    }
     BState hs{};
     for (int c = 0; c * KI < inner_itmax + KI; c++) {
       if ((e = cudaGraphLaunch(h.bk_graph, s))) return cuda_fail(e, "graph");
-      count_launches(8L * KI);
+      count_launches((on_rows ? 4L : 8L) * KI);
       if ((e = cudaMemcpyAsync(&hs, st, sizeof(BState), cudaMemcpyDeviceToHost, s)) ||
           (e = cudaStreamSynchronize(s)))
         return cuda_fail(e, "inner state");
       if (hs.done) break;
     }
     total_inner += hs.iter;
-    bo_update<<<gm, 256, 0, s>>>(n, K, X, a.x, scale);
-    count_launches(1);
+    if (on_rows) {
+      if ((e = cudaMemsetAsync(o.xexp, 0, sizeof(int) * 64, s)) ||
+          (e = block_rows_update(a, o, X, gv, s)))
+        return cuda_fail(e, "update");
+    } else {
+      bo_update<<<gm, 256, 0, s>>>(n, K, X, a.x, scale);
+      count_launches(1);
+    }
     if ((e = cudaGetLastError())) return cuda_fail(e, "update");
   }
   if ((e = cudaStreamSynchronize(s))) return cuda_fail(e, "block solve");

@@ -60,6 +60,7 @@
 
 #include <atomic>
 
+#include "block_cols.cuh"
 #include "tc_ptx.cuh"
 #include "vdr_internal.h"
 
@@ -652,6 +653,22 @@ bool make_amap(CUtensorMap *m, const float *A, int nex, int ney, int nez) {
 }
 
 }  // namespace blocktc
+
+bool make_node_map(CUtensorMap *m, const float *base, int words, int nax, int nay, int naz,
+                   int bx, int by) {
+  blocktc::EncodeTiledFn fn = blocktc::encode_tiled();
+  if (!fn || !base || (reinterpret_cast<uintptr_t>(base) & 15)) return false;
+  const cuuint64_t row = 4 * (cuuint64_t)words;
+  const cuuint64_t dims[4] = {(cuuint64_t)words, (cuuint64_t)nax, (cuuint64_t)nay,
+                              (cuuint64_t)naz};
+  const cuuint64_t strides[3] = {row, row * nax, row * nax * nay};
+  const cuuint32_t box[4] = {(cuuint32_t)words, (cuuint32_t)bx, (cuuint32_t)by, 1};
+  const cuuint32_t es[4] = {1, 1, 1, 1};
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(base), dims, strides, box,
+            es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
+         CUDA_SUCCESS;
+}
 
 bool block_tc_supported(const Handle &h) {
   return h.nax > 1 && h.nay > 1 && h.naz > 1 && !h.perm_d && h.block_err &&

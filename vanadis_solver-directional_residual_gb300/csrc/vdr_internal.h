@@ -294,6 +294,9 @@ struct Handle {
   double *bk_d = nullptr;
   cudaGraphExec_t bk_graph = nullptr;
   bool bk_graph_split = false;
+  const void *bk_graph_rows = nullptr;  // the rows it reads, null: element matrices
+  float *br_rows = nullptr;  // 28 scaled FP32 entries per node (block_rows.cu)
+  size_t br_words = 0;
   bool block_tma = false;     // bulk-copy block apply
   bool block_tile = true;     // node-tile block apply on structured meshes (default)
   int blk_tc_mode = -1;       // K = 64 on the tile path: -1 by measurement, 0 node tile, 1 tcgen05
