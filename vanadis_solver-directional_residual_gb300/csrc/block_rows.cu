@@ -107,48 +107,9 @@ __device__ __forceinline__ bool col_sums(const D (&d)[NQ][4], const BVec &a, dou
   return true;
 }
 
-// Two columns at once (packed FP32 operations, each rounded as the single
-// one): half the instructions of the inner products.
-#define VDR_F32X2(OP, a, b)                                                    \
-  ({                                                                           \
-    float2 r_, a_ = a, b_ = b;                                                 \
-    asm(OP ".rn.f32x2 %0, %1, %2;"                                             \
-        : "=l"(reinterpret_cast<unsigned long long &>(r_))                     \
-        : "l"(reinterpret_cast<unsigned long long &>(a_)),                     \
-          "l"(reinterpret_cast<unsigned long long &>(b_)));                    \
-    r_;                                                                        \
-  })
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return VDR_F32X2("add", a, b); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return VDR_F32X2("mul", a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  float2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(reinterpret_cast<unsigned long long &>(r))
-      : "l"(reinterpret_cast<unsigned long long &>(a)),
-        "l"(reinterpret_cast<unsigned long long &>(b)),
-        "l"(reinterpret_cast<unsigned long long &>(c)));
-  return r;
-}
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
-  return fma2(b, make_float2(-1.f, -1.f), a);
-}
-// dot_acc of two columns; nx = -x.
-struct Dot2 {
-  float2 s, c;
-};
-__device__ __forceinline__ void dot_acc2(Dot2 &a, float2 x, float2 nx, float2 y) {
-  const float2 p = mul2(x, y);
-  const float2 ne = fma2(nx, y, p);  // -(x y - p), exact
-  const float2 t = add2(a.s, p);
-  const float2 bp = sub2(t, a.s);
-  const float2 err = add2(sub2(a.s, sub2(t, bp)), sub2(p, bp));
-  a.s = t;
-  a.c = add2(a.c, sub2(err, ne));
-}
 __device__ __forceinline__ float2 half_of(const float4 &v, int h) {
   return h ? make_float2(v.z, v.w) : make_float2(v.x, v.y);
 }
-__device__ __forceinline__ float2 neg2(float2 v) { return mul2(v, make_float2(-1.f, -1.f)); }
 
 __device__ __forceinline__ void fma4(float4 &o, float c, const float4 &x) {
   o.x = fmaf(c, x.x, o.x);
@@ -250,10 +211,10 @@ __global__ void __launch_bounds__(PT, 2) br_apply(const BVec a, const BlockRows 
   extern __shared__ __align__(128) unsigned char stage[];
   __shared__ __align__(8) uint64_t full[ST];
   if (a.st->done) return;
-  Dot2 d[NQ][2];
+  DfAccx2 d[NQ][2];
 #pragma unroll
   for (int q = 0; q < NQ; q++)
-    d[q][0] = d[q][1] = Dot2{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    d[q][0] = d[q][1] = DfAccx2{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
   const float4 *__restrict__ H = reinterpret_cast<const float4 *>(a.rh);
   float4 *__restrict__ Y = reinterpret_cast<float4 *>(SECOND ? a.t : a.v);
   const int l = threadIdx.x % L, pair = threadIdx.x / L;

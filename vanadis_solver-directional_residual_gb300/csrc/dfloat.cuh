@@ -196,4 +196,92 @@ __device__ __forceinline__ void df_acc_add(DfAcc &acc, Df2 a) {
   acc.c = __fadd_rn(acc.c, __fadd_rn(err, a.l));
 }
 
+// ---- two values at once: packed FP32 operations, each half rounded as the
+// single operation is, so every result has the same bits.  The FMA pipe does
+// no more per cycle; half the instructions leave issue slots to the loads,
+// conversions and integer work between them.
+#define VDR_F32X2(OP, a, b)                                                    \
+  ({                                                                           \
+    float2 r_, a_ = a, b_ = b;                                                 \
+    asm(OP ".rn.f32x2 %0, %1, %2;"                                             \
+        : "=l"(reinterpret_cast<unsigned long long &>(r_))                     \
+        : "l"(reinterpret_cast<unsigned long long &>(a_)),                     \
+          "l"(reinterpret_cast<unsigned long long &>(b_)));                    \
+    r_;                                                                        \
+  })
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return VDR_F32X2("add", a, b); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return VDR_F32X2("mul", a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<unsigned long long &>(r))
+      : "l"(reinterpret_cast<unsigned long long &>(a)),
+        "l"(reinterpret_cast<unsigned long long &>(b)),
+        "l"(reinterpret_cast<unsigned long long &>(c)));
+  return r;
+}
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  return fma2(b, make_float2(-1.f, -1.f), a);
+}
+__device__ __forceinline__ float2 neg2(float2 v) { return mul2(v, make_float2(-1.f, -1.f)); }
+
+struct Df2x2 {  // two pairs
+  float2 h, l;
+};
+struct DfAccx2 {  // two accumulators
+  float2 s, c;
+};
+// One pair in both halves, and its negative (which forms the products' errors
+// without negating the products).
+struct DfDup {
+  float2 h, nh, nl;
+};
+__device__ __forceinline__ DfDup df_dup(Df2 a) {
+  return DfDup{make_float2(a.h, a.h), make_float2(-a.h, -a.h), make_float2(-a.l, -a.l)};
+}
+// acc += p - ne by TwoSum (ne: the product's error, negative).
+__device__ __forceinline__ void df_sum2(DfAccx2 &acc, float2 p, float2 ne) {
+  const float2 t = add2(acc.s, p);
+  const float2 bp = sub2(t, acc.s);
+  const float2 err = add2(sub2(acc.s, sub2(t, bp)), sub2(p, bp));
+  acc.s = t;
+  acc.c = add2(acc.c, sub2(err, ne));
+}
+// df_acc of two columns.
+__device__ __forceinline__ void df_acc2(DfAccx2 &acc, const DfDup &a, const Df2x2 &b) {
+  const float2 p = mul2(a.h, b.h);
+  float2 ne = fma2(a.nh, b.h, p);
+  ne = fma2(a.nh, b.l, ne);
+  ne = fma2(a.nl, b.h, ne);
+  df_sum2(acc, p, ne);
+}
+// df_acc_add of two columns.
+__device__ __forceinline__ void df_acc_add2(DfAccx2 &acc, const Df2x2 &a) {
+  const float2 t = add2(acc.s, a.h);
+  const float2 bp = sub2(t, acc.s);
+  const float2 err = add2(sub2(acc.s, sub2(t, bp)), sub2(a.h, bp));
+  acc.s = t;
+  acc.c = add2(acc.c, add2(err, a.l));
+}
+// df_norm of two columns.
+__device__ __forceinline__ Df2x2 df_norm2(const DfAccx2 &a) {
+  const float2 s = add2(a.s, a.c);
+  const float2 bp = sub2(s, a.s);
+  return Df2x2{s, add2(sub2(a.s, sub2(s, bp)), sub2(a.c, bp))};
+}
+// df_mul of two columns.
+__device__ __forceinline__ Df2x2 df_mul2(const DfDup &a, const Df2x2 &b) {
+  const float2 p = mul2(a.h, b.h);
+  float2 ne = fma2(a.nh, b.h, p);
+  ne = fma2(a.nh, b.l, ne);
+  ne = fma2(a.nl, b.h, ne);
+  const float2 s = sub2(p, ne);
+  return Df2x2{s, neg2(add2(ne, sub2(s, p)))};
+}
+// dot_acc (reduce.cuh) of two columns; nx = -x.
+__device__ __forceinline__ void dot_acc2(DfAccx2 &a, float2 x, float2 nx, float2 y) {
+  const float2 p = mul2(x, y);
+  df_sum2(a, p, fma2(nx, y, p));
+}
+
 }  // namespace vdr

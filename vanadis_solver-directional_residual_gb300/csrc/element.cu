@@ -1088,25 +1088,34 @@ __device__ __forceinline__ Df2 df_point_tau_pairs(int variant, const float2 *sc,
                             range_bad);
 }
 
+// Strides in floats, chosen so that neither the points' stores (lane = point)
+// nor the rows' loads (one address per element, or one per element and row)
+// meet in a bank; with the plain strides of 256 and 512 bytes they did four
+// and eight times over.
 struct GeoBuildSmem {
-  // per element, point q, node j: detJ W_j and c_j (SPLIT: v.gradN_j + P N_j;
-  // otherwise aH v.gradN_j + (aH P + aM) N_j), read by the row lanes two
-  // nodes per 16-byte load
-  __align__(16) Df2 dw[ROWS_EPB][8][8];
-  __align__(16) Df2 c[ROWS_EPB][8][8];
+  static constexpr int Q = 20, DW = 8 * Q + 16, C = 8 * Q + 4, QT = 68;
+  // per element, point q, node j: detJ W_j as pairs at [DW le + Q q + 2 j], and
+  // c_j (SPLIT: v.gradN_j + P N_j; otherwise aH v.gradN_j + (aH P + aM) N_j),
+  // the hi parts at [C le + Q q + j], the lo parts 8 further
+  __align__(16) float dw[ROWS_EPB * DW];
+  __align__(16) float c[ROWS_EPB * C];
   __align__(16) Df2 told[ROWS_EPB][8];  // T_old at the nodes times 2^-shift
-  __align__(16) float4 qt[8][8][2];     // point q, node j: (N, dN/dxi), (dN/deta, dN/dzeta)
-  __align__(16) Df2 nt[8][8];           // N_j at point q
+  // point q, nodes j and j + 1: N, dN/dxi, dN/deta, dN/dzeta as (hi, hi, lo,
+  // lo) at [QT q + 8 j + 4 k]
+  __align__(16) float qt[8 * QT];
+  __align__(16) float nt[8][16];  // N_j at point q, the hi parts, the lo parts
 };
 
-// Two consecutive pairs (16-byte aligned) from shared memory.
-__device__ __forceinline__ void lds_pairs(const Df2 *p, Df2 &a, Df2 &b) {
+__device__ __forceinline__ Df2x2 lds_x2(const float *p) {
   const float4 v = *reinterpret_cast<const float4 *>(p);
-  a = Df2{v.x, v.y};
-  b = Df2{v.z, v.w};
+  return Df2x2{make_float2(v.x, v.y), make_float2(v.z, v.w)};
 }
-__device__ __forceinline__ void sts_pairs(Df2 *p, Df2 a, Df2 b) {
-  *reinterpret_cast<float4 *>(p) = make_float4(a.h, a.l, b.h, b.l);
+// Pairs j .. j + 3 (two and two) of eight stored as hi and lo parts.
+__device__ __forceinline__ void lds_x4(const float *p, Df2x2 &a, Df2x2 &b) {
+  const float4 h = *reinterpret_cast<const float4 *>(p);
+  const float4 l = *reinterpret_cast<const float4 *>(p + 8);
+  a = Df2x2{make_float2(h.x, h.y), make_float2(l.x, l.y)};
+  b = Df2x2{make_float2(h.z, h.w), make_float2(l.z, l.w)};
 }
 
 // The double-float build from the mesh's geometric factors.  With
@@ -1122,8 +1131,14 @@ __device__ __forceinline__ void sts_pairs(Df2 *p, Df2 a, Df2 b) {
 // products per entry (SPLIT: H and M apart, 1 + 16), then writes as
 // elem_build_df_kernel does.  A value outside the pairs' safe window sets
 // bit 2 of the flag (the host redoes the build with FP64 rows).
+// Bound by the FMA pipe (60 % busy) and by issue beside it: the pair products
+// run two nodes at a time (packed operations), the shared arrays are strided
+// so that no access meets another in a bank.  1.05 M elements with a
+// right-hand side from T_old 1.72 -> 1.37 ms, without one 1.22 -> 0.99; 8.4 M
+// 9.9 -> 8.4.  Blocks per SM: with the registers that 12 / 16 leave 1.40 / 8.79
+// ms (1.05 M / 8.4 M), 11 / 14 1.40 / 8.40, 10 / 12 1.37 / 8.41.
 template <bool SPLIT>
-__global__ void __launch_bounds__(64, SPLIT ? 12 : 16) elem_build_geo_kernel(OpArgs a, BuildArgs ba) {
+__global__ void __launch_bounds__(64, SPLIT ? 10 : 12) elem_build_geo_kernel(OpArgs a, BuildArgs ba) {
   __shared__ GeoBuildSmem sm;
   if (threadIdx.x < 8) {
     const int t = threadIdx.x;
@@ -1132,11 +1147,16 @@ __global__ void __launch_bounds__(64, SPLIT ? 12 : 16) elem_build_geo_kernel(OpA
                      gauss_coord<double>(t, 2), n, d0, d1, d2);
 #pragma unroll
     for (int j = 0; j < 8; j++) {
-      const Df2 N = df_from_double(n[j]), a0 = df_from_double(d0[j]);
-      const Df2 a1 = df_from_double(d1[j]), a2 = df_from_double(d2[j]);
-      sm.qt[t][j][0] = make_float4(N.h, N.l, a0.h, a0.l);
-      sm.qt[t][j][1] = make_float4(a1.h, a1.l, a2.h, a2.l);
-      sm.nt[t][j] = N;
+      const Df2 v[4] = {df_from_double(n[j]), df_from_double(d0[j]), df_from_double(d1[j]),
+                        df_from_double(d2[j])};
+      float *o = sm.qt + GeoBuildSmem::QT * t + 16 * (j / 2) + (j & 1);
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        o[4 * k] = v[k].h;
+        o[4 * k + 2] = v[k].l;
+      }
+      sm.nt[t][j] = v[0].h;
+      sm.nt[t][8 + j] = v[0].l;
     }
   }
   __syncthreads();
@@ -1188,33 +1208,35 @@ __global__ void __launch_bounds__(64, SPLIT ? 12 : 16) elem_build_geo_kernel(OpA
       df_acc(acc, di[3 * r + 2], vzd);
       w[r] = df_norm(acc);
     }
-    const Df2 cm = SPLIT ? pd : df_add(df_mul(aHd, pd), aMd);
+    const DfDup cm = df_dup(SPLIT ? pd : df_add(df_mul(aHd, pd), aMd));
+    const DfDup w0 = df_dup(w[0]), w1 = df_dup(w[1]), w2 = df_dup(w[2]);
+    const DfDup tau2 = df_dup(taud), dj2 = df_dup(djq);
+    float *dwq = sm.dw + GeoBuildSmem::DW * le + GeoBuildSmem::Q * q;
+    float *cq = sm.c + GeoBuildSmem::C * le + GeoBuildSmem::Q * q;
+    const float2 z2 = make_float2(0.f, 0.f);
 #pragma unroll 1
     for (int j = 0; j < 8; j += 2) {
-      Df2 dwv[2], cv[2];
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const float4 u0 = sm.qt[q][j + h][0], u1 = sm.qt[q][j + h][1];
-        const Df2 N{u0.x, u0.y};
-        DfAcc aa{0.0f, 0.0f};
-        df_acc(aa, w[0], Df2{u0.z, u0.w});
-        df_acc(aa, w[1], Df2{u1.x, u1.y});
-        df_acc(aa, w[2], Df2{u1.z, u1.w});
-        const Df2 av = df_norm(aa);
-        DfAcc aw{0.0f, 0.0f};
-        df_acc_add(aw, N);
-        df_acc(aw, taud, av);
-        dwv[h] = df_mul(djq, df_norm(aw));
-        DfAcc ac{0.0f, 0.0f};
-        if constexpr (SPLIT)
-          df_acc_add(ac, av);
-        else
-          df_acc(ac, aHd, av);
-        df_acc(ac, cm, N);
-        cv[h] = df_norm(ac);
-      }
-      sts_pairs(&sm.dw[le][q][j], dwv[0], dwv[1]);
-      sts_pairs(&sm.c[le][q][j], cv[0], cv[1]);
+      const float *t = sm.qt + GeoBuildSmem::QT * q + 8 * j;
+      const Df2x2 N = lds_x2(t);
+      DfAccx2 aa{z2, z2};
+      df_acc2(aa, w0, lds_x2(t + 4));
+      df_acc2(aa, w1, lds_x2(t + 8));
+      df_acc2(aa, w2, lds_x2(t + 12));
+      const Df2x2 av = df_norm2(aa);
+      DfAccx2 aw{z2, z2};
+      df_acc_add2(aw, N);
+      df_acc2(aw, tau2, av);
+      const Df2x2 dw = df_mul2(dj2, df_norm2(aw));
+      DfAccx2 ac{z2, z2};
+      if constexpr (SPLIT)
+        df_acc_add2(ac, av);
+      else
+        df_acc2(ac, df_dup(aHd), av);
+      df_acc2(ac, cm, N);
+      const Df2x2 cv = df_norm2(ac);
+      *reinterpret_cast<float4 *>(dwq + 2 * j) = make_float4(dw.h.x, dw.l.x, dw.h.y, dw.l.y);
+      *reinterpret_cast<float2 *>(cq + j) = cv.h;
+      *reinterpret_cast<float2 *>(cq + 8 + j) = cv.l;
     }
     // element volume as a pair (the same sum in every lane: TwoSum is exact
     // in either order)
@@ -1225,38 +1247,55 @@ __global__ void __launch_bounds__(64, SPLIT ? 12 : 16) elem_build_geo_kernel(OpA
     __syncwarp();
     // ---- lane i = row i
     const int i = lane8;
-    DfAcc accH[8], accM[SPLIT ? 8 : 1];
+    DfAccx2 aH2[4], aM2[SPLIT ? 4 : 1];
 #pragma unroll
-    for (int j = 0; j < 8; j++) accH[j] = DfAcc{0.0f, 0.0f};
+    for (int j = 0; j < 4; j++) aH2[j] = DfAccx2{z2, z2};
 #pragma unroll
-    for (int j = 0; j < (SPLIT ? 8 : 1); j++) accM[j] = DfAcc{0.0f, 0.0f};
+    for (int j = 0; j < (SPLIT ? 4 : 1); j++) aM2[j] = DfAccx2{z2, z2};
     DfAcc fw{0.0f, 0.0f};
     if (need_rows) {
       const Df2 lamd = ld_pair(sc + 3 * E + p);
-      const Df2 lk = SPLIT ? lamd : df_mul(aHd, lamd);
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const int t = (j >= i) ? i * (15 - i) / 2 + j : j * (15 - j) / 2 + i;
-        df_acc(accH[j], lk, ld_pair(ba.gK + (size_t)t * E + p));
-      }
-    }
-#pragma unroll 1
-    for (int r = 0; r < 8; r++) {
-      const Df2 dwi = sm.dw[le][r][i];
-      df_acc_add(fw, dwi);
-      if (!need_rows) continue;
+      const DfDup lk = df_dup(SPLIT ? lamd : df_mul(aHd, lamd));
 #pragma unroll
       for (int j = 0; j < 8; j += 2) {
-        Df2 c0, c1;
-        lds_pairs(&sm.c[le][r][j], c0, c1);
-        df_acc(accH[j], dwi, c0);
-        df_acc(accH[j + 1], dwi, c1);
+        const int t = (j >= i) ? i * (15 - i) / 2 + j : j * (15 - j) / 2 + i;
+        const int u = (j + 1 >= i) ? i * (15 - i) / 2 + j + 1 : (j + 1) * (14 - j) / 2 + i;
+        const Df2 k0 = ld_pair(ba.gK + (size_t)t * E + p);
+        const Df2 k1 = ld_pair(ba.gK + (size_t)u * E + p);
+        df_acc2(aH2[j / 2], lk, Df2x2{make_float2(k0.h, k1.h), make_float2(k0.l, k1.l)});
+      }
+    }
+    const float *dwr = sm.dw + GeoBuildSmem::DW * le + 2 * i;
+    const float *cr = sm.c + GeoBuildSmem::C * le;
+#pragma unroll 1
+    for (int r = 0; r < 8; r++) {
+      const float2 dv = *reinterpret_cast<const float2 *>(dwr + GeoBuildSmem::Q * r);
+      const Df2 dwi{dv.x, dv.y};
+      df_acc_add(fw, dwi);
+      if (!need_rows) continue;
+      const DfDup d2 = df_dup(dwi);
+#pragma unroll
+      for (int j = 0; j < 8; j += 4) {
+        Df2x2 c0, c1;
+        lds_x4(cr + GeoBuildSmem::Q * r + j, c0, c1);
+        df_acc2(aH2[j / 2], d2, c0);
+        df_acc2(aH2[j / 2 + 1], d2, c1);
         if constexpr (SPLIT) {
-          Df2 n0, n1;
-          lds_pairs(&sm.nt[r][j], n0, n1);
-          df_acc(accM[j], dwi, n0);
-          df_acc(accM[j + 1], dwi, n1);
+          Df2x2 n0, n1;
+          lds_x4(sm.nt[r] + j, n0, n1);
+          df_acc2(aM2[j / 2], d2, n0);
+          df_acc2(aM2[j / 2 + 1], d2, n1);
         }
+      }
+    }
+    DfAcc accH[8], accM[SPLIT ? 8 : 1];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      accH[2 * j] = DfAcc{aH2[j].s.x, aH2[j].c.x};
+      accH[2 * j + 1] = DfAcc{aH2[j].s.y, aH2[j].c.y};
+      if constexpr (SPLIT) {
+        accM[2 * j] = DfAcc{aM2[j].s.x, aM2[j].c.x};
+        accM[2 * j + 1] = DfAcc{aM2[j].s.y, aM2[j].c.y};
       }
     }
     if (!valid) continue;
@@ -1504,7 +1543,7 @@ cudaError_t launch_build(const OpArgs &a, const BuildArgs &ba, bool fp32,
                            cudaFuncAttributePreferredSharedMemoryCarveout, 100);
       cudaFuncSetAttribute(elem_build_df_kernel<false>,
                            cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-      // 12 / 16 blocks of 10.5 KB
+      // 10 / 12 blocks of 11.9 KB
       cudaFuncSetAttribute(elem_build_geo_kernel<true>,
                            cudaFuncAttributePreferredSharedMemoryCarveout, 100);
       cudaFuncSetAttribute(elem_build_geo_kernel<false>,
