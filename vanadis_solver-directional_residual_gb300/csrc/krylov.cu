@@ -571,13 +571,16 @@ __global__ void __launch_bounds__(RED_THREADS, 4) bst_t(Vec a, StencilView w) {
     } else {
       st->omega = o[0] / o[1];
       st->rho_next = st->rhs - st->omega * o[2];
+      st->beta = (st->rho_next / st->rho) * (st->alpha / st->omega);
     }
   }
 }
 
 // Two nodes in flight per thread and 64 registers: the pass is bound by the
 // FP64 pipe (nine operations a node) about as much as by its 97 bytes, and
-// wants warps more than loads per thread.
+// wants warps more than loads per thread.  beta comes from bst_t's last
+// block: two divisions in every thread were a third of the pipe's work here
+// (1.08 M nodes 34 -> 30 us, 8.5 M 157 -> 151).
 __global__ void __launch_bounds__(RED_THREADS, 4) bst_p(Vec a) {
   KState *stc = a.st;
   if (stc->done) return;
@@ -599,7 +602,7 @@ __global__ void __launch_bounds__(RED_THREADS, 4) bst_p(Vec a) {
     return;
   }
   const double om = stc->omega, rho1 = stc->rho_next;
-  const double beta = (rho1 / stc->rho) * (al / om);
+  const double beta = stc->beta;
   const int e = stc->pmax, shift = e - 1023;
   int em = 0;
   double v[2] = {0.0, 0.0};

@@ -38,7 +38,7 @@ struct KState {
   // the assembled-operator iteration: (rh, s), the next rho, the exponent that
   // its pair vectors are scaled by, the largest exponents of the last
   // direction, of the one being formed and of the first residual
-  double rhs, rho_next;
+  double rhs, rho_next, beta;
   int pexp, pmax, pmax_next, rmax;
 };
 
