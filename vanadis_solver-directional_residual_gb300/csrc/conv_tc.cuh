@@ -115,7 +115,7 @@ struct Args {
   int tiles_x, tiles_y, ntiles;  // ntiles = tiles_x tiles_y ceil(D / G)
   const __nv_bfloat16 *wpk;  // [27][KC][COUT][8]
   const float *bias;         // [COUT]
-  __nv_bfloat16 *out;        // [V][COUT]
+  void *out;                 // [V][COUT], BF16 or (RAW) FP32
   int relu;
   int *err;                  // bit 0: a wait ran out
   const int *skip, *skip2;
@@ -144,9 +144,11 @@ struct Shape {
   static_assert(COUT % 16 == 0 && COUT >= 16 && COUT <= 256, "M = 128 needs N % 16 == 0");
   static_assert(G >= 1 && ACC <= 512, "a plane group fits the TMEM and shared memory");
   static_assert(SMEM <= 227 * 1024, "shared memory");
+  static_assert(!RES || 3 * COUT <= 256, "three taps side by side are one MMA");
 };
 
-template <int CIN1, int CIN2, int COUT>
+// RAW: the sums as they are, in FP32 (the backward data pass).
+template <int CIN1, int CIN2, int COUT, bool RAW = false>
 __global__ void __launch_bounds__(THREADS, 1)
     conv3_tc_kernel(const __grid_constant__ CUtensorMap map1,
                     const __grid_constant__ CUtensorMap map2, Args a) {
@@ -375,9 +377,9 @@ __global__ void __launch_bounds__(THREADS, 1)
     // ------------------------------------------------ epilogue
     const int q = warp & 3;  // TMEM sub-partition: lanes 32q .. 32q + 31
     const int row = 32 * q + lane;
-    float bias[COUT];
+    float bias[RAW ? 1 : COUT];
 #pragma unroll
-    for (int c = 0; c < COUT; c++) bias[c] = a.bias ? __ldg(a.bias + c) : 0.f;
+    for (int c = 0; c < (RAW ? 1 : COUT); c++) bias[c] = a.bias ? __ldg(a.bias + c) : 0.f;
     int it = 0;
     for (int t = blockIdx.x; t < a.ntiles; t += gridDim.x, it++) {
       const int b = it & 1;
@@ -397,35 +399,52 @@ __global__ void __launch_bounds__(THREADS, 1)
       for (int g = 0; g < S::G; g++) {
         const int z = tz * S::G + g;
         if (z >= a.D) break;  // uniform over the warp
-        uint32_t v[COUT];
-#pragma unroll
-        for (int c0 = 0; c0 < COUT; c0 += 16) {
-          uint32_t r16[16];
-          tc::tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) +
-                            (uint32_t)((b * S::G + g) * COUT + c0),
-                        r16);
-          tc::tmem_wait_ld();
-#pragma unroll
-          for (int k = 0; k < 16; k++) v[c0 + k] = r16[k];
-        }
-        if (x >= a.W || y >= a.H) continue;
+        const bool in = x < a.W && y < a.H;
         const long vox = (long)x + (long)a.W * ((long)y + (long)a.H * z);
-        uint4 *o = reinterpret_cast<uint4 *>(a.out + vox * COUT);
+        if constexpr (RAW) {
+#pragma unroll 1
+          for (int c0 = 0; c0 < COUT; c0 += 16) {
+            uint32_t r16[16];
+            tc::tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) +
+                              (uint32_t)((b * S::G + g) * COUT + c0),
+                          r16);
+            tc::tmem_wait_ld();
+            if (!in) continue;
+            uint4 *o = reinterpret_cast<uint4 *>(static_cast<float *>(a.out) + vox * COUT + c0);
 #pragma unroll
-        for (int c8 = 0; c8 < COUT / 8; c8++) {
-          uint32_t pk[4];
-#pragma unroll
-          for (int k = 0; k < 4; k++) {
-            float f0 = __uint_as_float(v[8 * c8 + 2 * k]) + bias[8 * c8 + 2 * k];
-            float f1 = __uint_as_float(v[8 * c8 + 2 * k + 1]) + bias[8 * c8 + 2 * k + 1];
-            if (a.relu) {
-              f0 = fmaxf(f0, 0.f);
-              f1 = fmaxf(f1, 0.f);
-            }
-            __nv_bfloat162 h = __floats2bfloat162_rn(f0, f1);
-            pk[k] = *reinterpret_cast<uint32_t *>(&h);
+            for (int k = 0; k < 4; k++)
+              o[k] = make_uint4(r16[4 * k], r16[4 * k + 1], r16[4 * k + 2], r16[4 * k + 3]);
           }
-          o[c8] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        } else {
+          uint32_t v[COUT];
+#pragma unroll
+          for (int c0 = 0; c0 < COUT; c0 += 16) {
+            uint32_t r16[16];
+            tc::tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) +
+                              (uint32_t)((b * S::G + g) * COUT + c0),
+                          r16);
+            tc::tmem_wait_ld();
+#pragma unroll
+            for (int k = 0; k < 16; k++) v[c0 + k] = r16[k];
+          }
+          if (!in) continue;
+          uint4 *o = reinterpret_cast<uint4 *>(static_cast<__nv_bfloat16 *>(a.out) + vox * COUT);
+#pragma unroll
+          for (int c8 = 0; c8 < COUT / 8; c8++) {
+            uint32_t pk[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+              float f0 = __uint_as_float(v[8 * c8 + 2 * k]) + bias[8 * c8 + 2 * k];
+              float f1 = __uint_as_float(v[8 * c8 + 2 * k + 1]) + bias[8 * c8 + 2 * k + 1];
+              if (a.relu) {
+                f0 = fmaxf(f0, 0.f);
+                f1 = fmaxf(f1, 0.f);
+              }
+              __nv_bfloat162 h = __floats2bfloat162_rn(f0, f1);
+              pk[k] = *reinterpret_cast<uint32_t *>(&h);
+            }
+            o[c8] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+          }
         }
       }
       tc::fence_before();

@@ -341,10 +341,11 @@ struct WgArgs {
 // row W + x; zero in the rows' padding x in [W, Wp) (the buffer is shared
 // by layers of other shapes).  One block per x row, one thread per padded
 // voxel: its C channels in 16-byte loads, and per channel a coalesced store
-// across the row.
+// across the row.  dyc (may be null): the same values channels-last, [V][C].
 template <int C>
 __global__ void mask_transpose(const float *__restrict__ dy, const bf16 *__restrict__ y,
-                               bf16 *__restrict__ dyt, int W, int Wp, long Vp) {
+                               bf16 *__restrict__ dyt, bf16 *__restrict__ dyc, int W, int Wp,
+                               long Vp) {
   static_assert(C % 8 == 0, "channels");
   const long row = blockIdx.x;
   for (int x = threadIdx.x; x < Wp; x += blockDim.x) {
@@ -363,12 +364,17 @@ __global__ void mask_transpose(const float *__restrict__ dy, const bf16 *__restr
       const float4 d0 = dp[2 * c8], d1 = dp[2 * c8 + 1];
       const uint32_t yw[4] = {ym.x, ym.y, ym.z, ym.w};
       const float dv[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+      float mv[8];
 #pragma unroll
       for (int k = 0; k < 8; k++) {
         const uint32_t h16 = (k & 1) ? (yw[k >> 1] >> 16) : (yw[k >> 1] & 0xffffu);
-        out[(long)(8 * c8 + k) * Vp] =
-            __float2bfloat16_rn(__uint_as_float(h16 << 16) > 0.f ? dv[k] : 0.f);
+        mv[k] = __uint_as_float(h16 << 16) > 0.f ? dv[k] : 0.f;
+        out[(long)(8 * c8 + k) * Vp] = __float2bfloat16_rn(mv[k]);
       }
+      if (dyc)
+        reinterpret_cast<uint4 *>(dyc + v * C)[c8] =
+            make_uint4(pack2(mv[0], mv[1]), pack2(mv[2], mv[3]), pack2(mv[4], mv[5]),
+                       pack2(mv[6], mv[7]));
     }
   }
 }
@@ -733,9 +739,10 @@ __global__ void adam_kernel(float *th, const float *g, float *m, float *v, long 
 // [27][CIN][COUT] with the tap flipped (the backward data pass).
 // wb[tap][co][ci] (forward), wbt[26 - tap][ci][co] (backward data pass) and
 // wtc[tap][ci/8][co][ci%8], or with the three z taps side by side (stack)
-// wtc[dy, dx][ci/8][2 - dz][co][ci%8] (the tensor-core kernel's orders).
-__global__ void pack_weights(const float *th, bf16 *wb, bf16 *wbt, bf16 *wtc, int cin,
-                             int cout, int stack) {
+// wtc[dy, dx][ci/8][2 - dz][co][ci%8] (the tensor-core kernel's orders), wtcb
+// in the same way the backward pass's, its inputs co and its outputs ci.
+__global__ void pack_weights(const float *th, bf16 *wb, bf16 *wbt, bf16 *wtc, bf16 *wtcb,
+                             int cin, int cout, int stack, int stack_b) {
   const long total = 27L * cin * cout;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long)gridDim.x * blockDim.x) {
@@ -747,6 +754,9 @@ __global__ void pack_weights(const float *th, bf16 *wb, bf16 *wbt, bf16 *wtc, in
     wbt[((long)(26 - tap) * cin + ci) * cout + co] = b;
     const long chunk = (long)(stack ? tap % 9 : tap) * (cin / 8) + ci / 8;
     wtc[((stack ? chunk * 3 + 2 - tap / 9 : chunk) * cout + co) * 8 + (ci & 7)] = b;
+    const int tb = 26 - tap;
+    const long cb = (long)(stack_b ? tb % 9 : tb) * (cout / 8) + co / 8;
+    wtcb[((stack_b ? cb * 3 + 2 - tb / 9 : cb) * cin + ci) * 8 + (co & 7)] = b;
   }
 }
 
@@ -1069,12 +1079,13 @@ struct Net {
   bool features_set = false;
   // tcgen05 forward convolutions: packed weights, the decoders' upsampled
   // inputs on the fine grid, and per layer the TMA maps of its inputs
-  bf16 *wtc = nullptr;
+  bf16 *wtc = nullptr, *wtcb = nullptr;
+  bf16 *dyc = nullptr;  // [V][C] masked output gradient (the backward data pass's input)
   bf16 *up0 = nullptr, *up1 = nullptr;  // up(u1) on level 0, up(b2) on level 1
   int *tc_err = nullptr;                // bit 0: a tcgen05 kernel wait ran out
   int conv_mode = VDR_NET_CONV_MMA;
   bool tc_ok = false;                   // every map could be made
-  CUtensorMap tmap[NLAYER][2];
+  CUtensorMap tmap[NLAYER][2], bmap[NLAYER];
   std::vector<void *> allocs;
 };
 
@@ -1116,6 +1127,8 @@ cudaError_t conv_launch(const ConvArgs &a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+bool tc_mode(const Net &n) { return n.conv_mode == VDR_NET_CONV_TCGEN05 && n.tc_ok; }
+
 template <int CIN1, int CIN2, int COUT>
 cudaError_t wgrad_launch(const Net &n, WgArgs a, const float *dy, const bf16 *y,
                          cudaStream_t s) {
@@ -1129,7 +1142,8 @@ cudaError_t wgrad_launch(const Net &n, WgArgs a, const float *dy, const bf16 *y,
   // (scratch sized for the largest layer)
   a.Wp = (a.W + 15) & ~15;
   a.Vp = (long)a.H * a.D * a.Wp;
-  mask_transpose<COUT><<<(unsigned)((long)a.H * a.D), 128, 0, s>>>(dy, y, n.dyt, a.W, a.Wp, a.Vp);
+  mask_transpose<COUT><<<(unsigned)((long)a.H * a.D), 128, 0, s>>>(
+      dy, y, n.dyt, tc_mode(n) ? n.dyc : nullptr, a.W, a.Wp, a.Vp);
   a.dyt = n.dyt;
   const long nks = (long)a.H * a.D * (a.Wp / 16);  // 16-voxel x-row segments
   const long target = std::max<long>(1, (long)device_sm_count() * 8 / (9 * NGROUPS));
@@ -1192,7 +1206,7 @@ const float *bs(const Net &n, int l) { return n.theta + n.boff[l]; }
 // kernels of one forward pass: 10 convolutions, 2 pools, the head, and on
 // the tensor-core path the 2 upsampled copies
 int fwd_launches(const Net &n) {
-  return (n.conv_mode == VDR_NET_CONV_TCGEN05 && n.tc_ok) ? 15 : 13;
+  return tc_mode(n) ? 15 : 13;
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link
@@ -1257,37 +1271,63 @@ bool make_tmaps(Net &n) {
     if (!make_tmap(&n.tmap[i.l][0], i.in1, L.cin1, planes, d)) return false;
     n.tmap[i.l][1] = n.tmap[i.l][0];
     if (i.in2 && !make_tmap(&n.tmap[i.l][1], i.in2, L.cin2, planes, d)) return false;
+    if (!make_tmap(&n.bmap[i.l], n.dyc, L.cout,
+                   convtc::group_of(L.cout, 0, L.cin1 + L.cin2) + 2, d))
+      return false;
   }
   return true;
 }
 
-template <int CIN1, int CIN2, int COUT>
-cudaError_t conv_tc_launch(const Net &n, int l, bf16 *out, const int *sk,
-                           const int *sk2, cudaStream_t s) {
+template <int CIN1, int CIN2, int COUT, bool RAW>
+cudaError_t conv_tc_run(const Net &n, int l, const CUtensorMap &m1, const CUtensorMap &m2,
+                        convtc::Args a, cudaStream_t s) {
   using Sh = convtc::Shape<CIN1, CIN2, COUT>;
-  auto kern = convtc::conv3_tc_kernel<CIN1, CIN2, COUT>;
+  auto kern = convtc::conv3_tc_kernel<CIN1, CIN2, COUT, RAW>;
   static const cudaError_t attr =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::SMEM);
   if (attr) return attr;
   const Dims &d = n.d[DEFS[l].level];
-  convtc::Args a;
   a.W = d.W;
   a.H = d.H;
   a.D = d.D;
   a.tiles_x = (d.W + convtc::TX - 1) / convtc::TX;
   a.tiles_y = (d.H + convtc::TY - 1) / convtc::TY;
   a.ntiles = a.tiles_x * a.tiles_y * ((d.D + Sh::G - 1) / Sh::G);
+  a.err = n.tc_err;
+  const int grid = std::min(a.ntiles, device_sm_count());
+  kern<<<grid, convtc::THREADS, Sh::SMEM, s>>>(m1, m2, a);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+template <int CIN1, int CIN2, int COUT>
+cudaError_t conv_tc_launch(const Net &n, int l, bf16 *out, const int *sk,
+                           const int *sk2, cudaStream_t s) {
+  convtc::Args a{};
   a.wpk = n.wtc + n.woff[l];
   a.bias = n.theta + n.boff[l];
   a.out = out;
   a.relu = 1;
-  a.err = n.tc_err;
   a.skip = sk;
   a.skip2 = sk2;
-  const int grid = std::min(a.ntiles, device_sm_count());
-  kern<<<grid, convtc::THREADS, Sh::SMEM, s>>>(n.tmap[l][0], n.tmap[l][1], a);
-  count_launches(1);
-  return cudaGetLastError();
+  return conv_tc_run<CIN1, CIN2, COUT, false>(n, l, n.tmap[l][0], n.tmap[l][1], a, s);
+}
+
+// Layer l's backward data pass: the gradient of its CIN inputs, in FP32, from
+// the masked gradient of its COUT outputs (mask1 applied to dy).  On the
+// tensor cores from n.dyc, which the layer's weight gradient has just
+// written; 65 x 65 x 33 voxels, all nine passes: 290 -> 117 us.
+template <int COUT, int CIN>
+cudaError_t bwd_data(const Net &n, int l, const float *dy, const bf16 *y, float *out,
+                     cudaStream_t s) {
+  if (!tc_mode(n))
+    return conv_launch<COUT, 0, CIN, true, true>(
+        conv_args(n, DEFS[l].level, dy, y, nullptr, wt(n, l), nullptr, out, false, nullptr,
+                  nullptr), s);
+  convtc::Args a{};
+  a.wpk = n.wtcb + n.woff[l];
+  a.out = out;
+  return conv_tc_run<COUT, 0, CIN, true>(n, l, n.bmap[l], n.bmap[l], a, s);
 }
 
 // The forward pass's ten convolutions on the tensor cores (tcgen05).
@@ -1323,7 +1363,7 @@ cudaError_t net_forward_tc(Net &n, const int *sk, const int *sk2, cudaStream_t s
 
 // Forward pass from the prepared input x0 to the head output c.
 cudaError_t net_forward(Net &n, const int *sk, const int *sk2, cudaStream_t s) {
-  if (n.conv_mode == VDR_NET_CONV_TCGEN05 && n.tc_ok) return net_forward_tc(n, sk, sk2, s);
+  if (tc_mode(n)) return net_forward_tc(n, sk, sk2, s);
   cudaError_t e;
 #define VDR_CONV(CI1, CI2, CO, LVL, IN1, IN2, L, OUT)                              \
   if ((e = conv_launch<CI1, CI2, CO, false, false>(                                \
@@ -1358,59 +1398,41 @@ cudaError_t net_backward(Net &n, cudaStream_t s) {
   const Dims &f0 = n.d[0], &f1 = n.d[1], &f2 = n.d[2];
   // d0b: u0 = relu(conv(a4))
   if ((e = wgrad_launch<16, 0, 16>(n, wg_args(n, L_D0B, n.a4, nullptr), n.g_u0, n.u0, s))) return e;
-  if ((e = conv_launch<16, 0, 16, true, true>(
-           conv_args(n, 0, n.g_u0, n.u0, nullptr, wt(n, L_D0B), nullptr, n.g_a4, false,
-                     nullptr, nullptr), s))) return e;
+  if ((e = bwd_data<16, 16>(n, L_D0B, n.g_u0, n.u0, n.g_a4, s))) return e;
   // d0a: a4 = relu(conv([s0 | up(u1)]))
   if ((e = wgrad_launch<16, 32, 16>(n, wg_args(n, L_D0A, n.s0, n.u1), n.g_a4, n.a4, s))) return e;
-  if ((e = conv_launch<16, 0, 48, true, true>(
-           conv_args(n, 0, n.g_a4, n.a4, nullptr, wt(n, L_D0A), nullptr, n.g_cat0, false,
-                     nullptr, nullptr), s))) return e;
+  if ((e = bwd_data<16, 48>(n, L_D0A, n.g_a4, n.a4, n.g_cat0, s))) return e;
   upcat_bwd_skip<<<grid_for(f0.V * 16, 256), 256, 0, s>>>(n.g_cat0, n.g_s0, f0.V, 16, 32);
   upcat_bwd_coarse<<<grid_for(f1.V * 32, 256), 256, 0, s>>>(n.g_cat0, n.g_u1, f0, f1, 16, 32);
   count_launches(2);
   // d1b: u1 = relu(conv(a3))
   if ((e = wgrad_launch<32, 0, 32>(n, wg_args(n, L_D1B, n.a3, nullptr), n.g_u1, n.u1, s))) return e;
-  if ((e = conv_launch<32, 0, 32, true, true>(
-           conv_args(n, 1, n.g_u1, n.u1, nullptr, wt(n, L_D1B), nullptr, n.g_a3, false,
-                     nullptr, nullptr), s))) return e;
+  if ((e = bwd_data<32, 32>(n, L_D1B, n.g_u1, n.u1, n.g_a3, s))) return e;
   // d1a: a3 = relu(conv([s1 | up(b2)]))
   if ((e = wgrad_launch<32, 64, 32>(n, wg_args(n, L_D1A, n.s1, n.b2), n.g_a3, n.a3, s))) return e;
-  if ((e = conv_launch<32, 0, 96, true, true>(
-           conv_args(n, 1, n.g_a3, n.a3, nullptr, wt(n, L_D1A), nullptr, n.g_cat1, false,
-                     nullptr, nullptr), s))) return e;
+  if ((e = bwd_data<32, 96>(n, L_D1A, n.g_a3, n.a3, n.g_cat1, s))) return e;
   upcat_bwd_skip<<<grid_for(f1.V * 32, 256), 256, 0, s>>>(n.g_cat1, n.g_s1, f1.V, 32, 64);
   upcat_bwd_coarse<<<grid_for(f2.V * 64, 256), 256, 0, s>>>(n.g_cat1, n.g_b2, f1, f2, 32, 64);
   count_launches(2);
   // btb: b2 = relu(conv(a2))
   if ((e = wgrad_launch<64, 0, 64>(n, wg_args(n, L_BTB, n.a2, nullptr), n.g_b2, n.b2, s))) return e;
-  if ((e = conv_launch<64, 0, 64, true, true>(
-           conv_args(n, 2, n.g_b2, n.b2, nullptr, wt(n, L_BTB), nullptr, n.g_a2, false,
-                     nullptr, nullptr), s))) return e;
+  if ((e = bwd_data<64, 64>(n, L_BTB, n.g_b2, n.b2, n.g_a2, s))) return e;
   // bta: a2 = relu(conv(p1))
   if ((e = wgrad_launch<32, 0, 64>(n, wg_args(n, L_BTA, n.p1, nullptr), n.g_a2, n.a2, s))) return e;
-  if ((e = conv_launch<64, 0, 32, true, true>(
-           conv_args(n, 2, n.g_a2, n.a2, nullptr, wt(n, L_BTA), nullptr, n.g_p1, false,
-                     nullptr, nullptr), s))) return e;
+  if ((e = bwd_data<64, 32>(n, L_BTA, n.g_a2, n.a2, n.g_p1, s))) return e;
   pool_bwd_add<<<grid_for(f1.V * 32, 256), 256, 0, s>>>(n.g_p1, n.g_s1, f1, f2, 32);
   count_launches(1);
   // e1b: s1 = relu(conv(a1))
   if ((e = wgrad_launch<32, 0, 32>(n, wg_args(n, L_E1B, n.a1, nullptr), n.g_s1, n.s1, s))) return e;
-  if ((e = conv_launch<32, 0, 32, true, true>(
-           conv_args(n, 1, n.g_s1, n.s1, nullptr, wt(n, L_E1B), nullptr, n.g_a1, false,
-                     nullptr, nullptr), s))) return e;
+  if ((e = bwd_data<32, 32>(n, L_E1B, n.g_s1, n.s1, n.g_a1, s))) return e;
   // e1a: a1 = relu(conv(p0))
   if ((e = wgrad_launch<16, 0, 32>(n, wg_args(n, L_E1A, n.p0, nullptr), n.g_a1, n.a1, s))) return e;
-  if ((e = conv_launch<32, 0, 16, true, true>(
-           conv_args(n, 1, n.g_a1, n.a1, nullptr, wt(n, L_E1A), nullptr, n.g_p0, false,
-                     nullptr, nullptr), s))) return e;
+  if ((e = bwd_data<32, 16>(n, L_E1A, n.g_a1, n.a1, n.g_p0, s))) return e;
   pool_bwd_add<<<grid_for(f0.V * 16, 256), 256, 0, s>>>(n.g_p0, n.g_s0, f0, f1, 16);
   count_launches(1);
   // e0b: s0 = relu(conv(a0))
   if ((e = wgrad_launch<16, 0, 16>(n, wg_args(n, L_E0B, n.a0, nullptr), n.g_s0, n.s0, s))) return e;
-  if ((e = conv_launch<16, 0, 16, true, true>(
-           conv_args(n, 0, n.g_s0, n.s0, nullptr, wt(n, L_E0B), nullptr, n.g_a0, false,
-                     nullptr, nullptr), s))) return e;
+  if ((e = bwd_data<16, 16>(n, L_E0B, n.g_s0, n.s0, n.g_a0, s))) return e;
   // e0a: a0 = relu(conv(x0)); the input needs no gradient
   if ((e = wgrad_launch<16, 0, 16>(n, wg_args(n, L_E0A, n.x0, nullptr), n.g_a0, n.a0, s))) return e;
   return cudaGetLastError();
@@ -1420,8 +1442,10 @@ cudaError_t pack_all(Net &n, cudaStream_t s) {
   for (int l = 0; l < L_HEAD; l++) {
     const int cin = DEFS[l].cin1 + DEFS[l].cin2, cout = DEFS[l].cout;
     pack_weights<<<grid_for(layer_wsize(l), 256), 256, 0, s>>>(
-        n.theta + n.woff[l], n.wb + n.woff[l], n.wbt + n.woff[l], n.wtc + n.woff[l], cin,
-        cout, convtc::weights_resident(DEFS[l].cin1, DEFS[l].cin2, cout));
+        n.theta + n.woff[l], n.wb + n.woff[l], n.wbt + n.woff[l], n.wtc + n.woff[l],
+        n.wtcb + n.woff[l], cin, cout,
+        convtc::weights_resident(DEFS[l].cin1, DEFS[l].cin2, cout),
+        convtc::weights_resident(cout, 0, cin));
   }
   count_launches(L_HEAD);
   return cudaGetLastError();
@@ -1590,6 +1614,8 @@ extern "C" int vdr_net_create(vdr_handle *H, unsigned long long seed, vdr_net **
         (e = nalloc(n, &n.scal, 8)) || (e = nalloc(n, &n.partials, 2L * n.red_grid)) ||
         (e = nalloc(n, &n.ticket, 1)) || (e = nalloc(n, &n.wtc, off)) ||
         (e = nalloc(n, &n.up0, V0 * 32)) || (e = nalloc(n, &n.up1, V1 * 64)) ||
+        (e = nalloc(n, &n.wtcb, off)) ||
+        (e = nalloc(n, &n.dyc, std::max(std::max(V0 * 16, V1 * 32), V2 * 64))) ||
         (e = nalloc(n, &n.tc_err, 1))) {
       st = cuda_fail(e, "network allocation");
       break;
