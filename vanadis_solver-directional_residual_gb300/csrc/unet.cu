@@ -397,8 +397,11 @@ __device__ __forceinline__ void ldsm_x4_trans(const bf16 *p, uint32_t &r0, uint3
 // volume), NG units of 8 channels each (16-byte loads of channels-last
 // rows), into a padded shared tile, and tap dx reads its B fragments from
 // tile rows 1 + dx .. 16 + dx with ldmatrix .trans: one staging and one set
-// of A fragments for three taps.  The next k-step's rows are loaded while
-// the current one multiplies.
+// of A fragments for three taps.  The next k-step's rows and A fragments are
+// loaded while the current one multiplies (bound by that latency and by the
+// atomics at the end: ten layers at 65 x 65 x 33 voxels 455 us with the A
+// fragments loaded at use and every warp adding its own sums, 230 so; with
+// half and twice the blocks 230 and 260).
 template <int CIN1, int CIN2, int COUT, int NG>
 __global__ void __launch_bounds__(128) conv3_wgrad_tc(WgArgs a) {
   constexpr int CIN = CIN1 + CIN2, MT = COUT / 16, NT = CIN / 8;
@@ -408,6 +411,7 @@ __global__ void __launch_bounds__(128) conv3_wgrad_tc(WgArgs a) {
   constexpr int RSTR = NG * 8 + 8;  // bf16 per row
   constexpr int TROWS = 18, ITEMS = TROWS * NG, PER_LANE = (ITEMS + 31) / 32;
   __shared__ __align__(16) bf16 tile[4][TROWS * RSTR];
+  __shared__ float sums[4][MT * NG * 4 * 32];
   const int pair = blockIdx.y;  // 3 (dz + 1) + (dy + 1)
   const int dyy = pair % 3 - 1, dz = pair / 3 - 1;
   const int ntile0 = blockIdx.z * NG;
@@ -463,11 +467,32 @@ __global__ void __launch_bounds__(128) conv3_wgrad_tc(WgArgs a) {
       sv[k] = v;
     }
   };
+  // A fragments: dyt[co][vb + (2t, 2t+1)] and [vb + (2t+8, 2t+9)], vb the
+  // k-step's first voxel in the padded gradient rows: aligned pairs (zero in
+  // the rows' padding)
+  auto load_a = [&](int sg, int yy, int zz, uint32_t (&af)[MT][4]) {
+    const long vb = ((long)yy + (long)H * zz) * a.Wp + ((long)sg << 4);
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {  // rows g, g+8
+        const bf16 *rp = a.dyt + (long)(mt * 16 + g + 8 * h) * a.Vp + vb;
+        af[mt][h] = ld2(rp + 2 * t);          // a0 (row g) / a1 (row g+8): k = 2t, 2t+1
+        af[mt][2 + h] = ld2(rp + 2 * t + 8);  // a2 / a3: k = 2t+8, 2t+9
+      }
+  };
   uint4 sv[PER_LANE];
-  if (ks < ks1) load_rows(seg, y, z, sv);
+  uint32_t an[MT][4];
+  if (ks < ks1) {
+    load_rows(seg, y, z, sv);
+    load_a(seg, y, z, an);
+  }
   for (; ks < ks1; ks += 4) {
-    // the k-step's first voxel in the padded gradient rows
-    const long vb = ((long)y + (long)H * z) * a.Wp + ((long)seg << 4);
+    uint32_t af[MT][4];
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+      for (int k = 0; k < 4; k++) af[mt][k] = an[mt][k];
     __syncwarp();  // the previous k-step's ldmatrix reads are done
 #pragma unroll
     for (int k = 0; k < PER_LANE; k++) {
@@ -484,21 +509,17 @@ __global__ void __launch_bounds__(128) conv3_wgrad_tc(WgArgs a) {
         ++z;
       }
     }
-    if (ks + 4 < ks1) load_rows(seg, y, z, sv);  // in flight during the MMAs
-    // A fragments: dyt[co][vb + (2t, 2t+1)] and [vb + (2t+8, 2t+9)], aligned
-    // pairs (zero in the rows' padding)
-    uint32_t af[MT][4];
+    if (ks + 4 < ks1) {  // in flight during the MMAs
+      load_rows(seg, y, z, sv);
+      load_a(seg, y, z, an);
+    }
+    if (pair == 4 && blockIdx.z == 0)
 #pragma unroll
-    for (int mt = 0; mt < MT; mt++)
+      for (int mt = 0; mt < MT; mt++)
 #pragma unroll
-      for (int h = 0; h < 2; h++) {  // rows g, g+8
-        const bf16 *rp = a.dyt + (long)(mt * 16 + g + 8 * h) * a.Vp + vb;
-        const uint32_t lo = ld2(rp + 2 * t), hi = ld2(rp + 2 * t + 8);
-        af[mt][h] = lo;      // a0 (row g) / a1 (row g+8): k = 2t, 2t+1
-        af[mt][2 + h] = hi;  // a2 / a3: k = 2t+8, 2t+9
-        if (pair == 4 && blockIdx.z == 0)
-          dbs[mt][h] += bf_lo(lo) + bf_hi(lo) + bf_lo(hi) + bf_hi(hi);
-      }
+        for (int h = 0; h < 2; h++)
+          dbs[mt][h] += bf_lo(af[mt][h]) + bf_hi(af[mt][h]) + bf_lo(af[mt][2 + h]) +
+                        bf_hi(af[mt][2 + h]);
     // tap dx = tx - 1: B rows tx .. tx + 15; matrices (rows 0-7, j),
     // (rows 8-15, j), (rows 0-7, j+1), (rows 8-15, j+1)
 #pragma unroll
@@ -520,22 +541,29 @@ __global__ void __launch_bounds__(128) conv3_wgrad_tc(WgArgs a) {
         }
       }
   }
-  // D fragments: rows co = g (c0, c1), g+8 (c2, c3); cols ci = 2t, 2t+1
+  // D fragments: rows co = g (c0, c1), g+8 (c2, c3); cols ci = 2t, 2t+1.  The
+  // four warps' sums meet in shared memory, one tap at a time: a quarter of
+  // the atomics on the few addresses that every block adds to.
 #pragma unroll
   for (int tx = 0; tx < 3; tx++) {
     const int tap = 3 * pair + tx;
+    __syncthreads();
 #pragma unroll
     for (int mt = 0; mt < MT; mt++)
 #pragma unroll
-      for (int j = 0; j < NG; j++) {
-        const int nt = ntile0 + j;
-        if (nt >= NT) break;
+      for (int j = 0; j < NG; j++)
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-          const int co = mt * 16 + g + 8 * (q >> 1), ci = nt * 8 + 2 * t + (q & 1);
-          atomicAdd(a.dw + ((size_t)tap * COUT + co) * CIN + ci, acc[tx][mt][j][q]);
-        }
-      }
+        for (int q = 0; q < 4; q++)
+          sums[warp][((mt * NG + j) * 4 + q) * 32 + lane] = acc[tx][mt][j][q];
+    __syncthreads();
+    for (int f = warp; f < MT * NG * 4; f += 4) {
+      const int q = f & 3, j = (f >> 2) % NG, mt = (f >> 2) / NG, nt = ntile0 + j;
+      if (nt >= NT) continue;
+      const int k = f * 32 + lane;
+      const float v = (sums[0][k] + sums[1][k]) + (sums[2][k] + sums[3][k]);
+      const int co = mt * 16 + g + 8 * (q >> 1), ci = nt * 8 + 2 * t + (q & 1);
+      atomicAdd(a.dw + ((size_t)tap * COUT + co) * CIN + ci, v);
+    }
   }
   if (pair == 4 && blockIdx.z == 0) {
 #pragma unroll
@@ -806,6 +834,53 @@ __global__ void node_feature_fin(const float *acc, float *feat, long N) {
   }
 }
 
+// Two sums over the grid (256 threads a block), true in thread 0 of the last
+// block with the totals: its threads add the blocks' partials in a fixed
+// order (one thread adding 545 of them took 45 of the 55 us).
+__device__ __forceinline__ bool grid_sum2(double v0, double v1, double *partials, unsigned *ticket,
+                                          double &o0, double &o1) {
+  __shared__ double sm[2][8];
+  __shared__ bool last;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const auto block_sum = [&](double a, double b) {
+    for (int off = 16; off; off >>= 1) {
+      a += __shfl_xor_sync(FULLM, a, off);
+      b += __shfl_xor_sync(FULLM, b, off);
+    }
+    __syncthreads();
+    if (l == 0) {
+      sm[0][w] = a;
+      sm[1][w] = b;
+    }
+    __syncthreads();
+    o0 = o1 = 0.0;
+    if (threadIdx.x == 0)
+      for (int j = 0; j < 8; j++) {
+        o0 += sm[0][j];
+        o1 += sm[1][j];
+      }
+  };
+  block_sum(v0, v1);
+  if (threadIdx.x == 0) {
+    partials[2 * blockIdx.x] = o0;
+    partials[2 * blockIdx.x + 1] = o1;
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  v0 = v1 = 0.0;
+  for (unsigned b = threadIdx.x; b < gridDim.x; b += 256) {
+    v0 += __ldcg(partials + 2 * b);
+    v1 += __ldcg(partials + 2 * b + 1);
+  }
+  block_sum(v0, v1);
+  if (threadIdx.x != 0) return false;
+  *ticket = 0u;
+  return true;
+}
+
 // Deterministic sum over free nodes of f(v), f = x^2 (RMS) or diag (mean).
 template <int MODE, typename T = double>  // 0: rms over free nodes; 1: mean; 2: sum x^2
 __global__ void __launch_bounds__(256) free_sum(const T *x,
@@ -823,38 +898,8 @@ __global__ void __launch_bounds__(256) free_sum(const T *x,
       c += 1.0;
     }
   }
-  __shared__ double sm[2][8];
-  __shared__ bool last;
-  for (int off = 16; off; off >>= 1) {
-    s += __shfl_xor_sync(FULLM, s, off);
-    c += __shfl_xor_sync(FULLM, c, off);
-  }
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) {
-    sm[0][w] = s;
-    sm[1][w] = c;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double a0 = 0.0, a1 = 0.0;
-    for (int j = 0; j < 8; j++) {
-      a0 += sm[0][j];
-      a1 += sm[1][j];
-    }
-    partials[2 * blockIdx.x] = a0;
-    partials[2 * blockIdx.x + 1] = a1;
-    __threadfence();
-    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last || threadIdx.x != 0) return;
-  __threadfence();
-  double a0 = 0.0, a1 = 0.0;
-  for (unsigned b = 0; b < gridDim.x; b++) {
-    a0 += __ldcg(partials + 2 * b);
-    a1 += __ldcg(partials + 2 * b + 1);
-  }
-  *ticket = 0u;
+  double a0, a1;
+  if (!grid_sum2(s, c, partials, ticket, a0, a1)) return;
   if (MODE == 0) {
     out[0] = a1 > 0.0 ? sqrt(a0 / a1) : 0.0;  // rms
   } else if (MODE == 1) {
@@ -947,38 +992,8 @@ __global__ void __launch_bounds__(256) res_rho(const float *rhat, const double *
     a0 += pv * pv;
     a1 += rv * rv;
   }
-  __shared__ double sm[2][8];
-  __shared__ bool last;
-  for (int off = 16; off; off >>= 1) {
-    a0 += __shfl_xor_sync(FULLM, a0, off);
-    a1 += __shfl_xor_sync(FULLM, a1, off);
-  }
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) {
-    sm[0][w] = a0;
-    sm[1][w] = a1;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double s0 = 0.0, s1 = 0.0;
-    for (int j = 0; j < 8; j++) {
-      s0 += sm[0][j];
-      s1 += sm[1][j];
-    }
-    partials[2 * blockIdx.x] = s0;
-    partials[2 * blockIdx.x + 1] = s1;
-    __threadfence();
-    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last || threadIdx.x != 0) return;
-  __threadfence();
-  double s0 = 0.0, s1 = 0.0;
-  for (unsigned b = 0; b < gridDim.x; b++) {
-    s0 += __ldcg(partials + 2 * b);
-    s1 += __ldcg(partials + 2 * b + 1);
-  }
-  *ticket = 0u;
+  double s0, s1;
+  if (!grid_sum2(a0, a1, partials, ticket, s0, s1)) return;
   out[0] = s1 > 0.0 ? s0 / s1 : 0.0;
   out[1] = s1;
 }
