@@ -21,7 +21,7 @@
 // seven kernels and 26 passes (clearing v and t among them).  The FP64
 // residual of the refinement runs the same way on the pair rows.  At 1.08 M
 // nodes and 64 columns an iteration takes 923 us instead of 1346, a residual
-// 2.3 ms instead of 3.9 + 0.35; a whole solve 128 -> 86 ms, and 4.1 -> 3.5 ms
+// 1.8 ms instead of 3.9 + 0.35; a whole solve 128 -> 86 ms, and 4.1 -> 3.5 ms
 // at 343 nodes.
 #include <cuda_runtime.h>
 #include <math.h>
@@ -44,7 +44,7 @@ struct Tile {
   static constexpr int L = K / 4, TX = K == 16 ? 16 : 8, TY = PT / L / (TX / 2);
   static constexpr int SX = TX + 2, SY = TY + 2;
   static constexpr int XB = SX * SY * K * 4, RB = TX * TY * 112;  // bytes of a plane
-  static constexpr int STAGE = XB + RB, PRODUCT = STAGES * STAGE, RESIDUAL = 2 * 2 * XB;
+  static constexpr int STAGE = XB + RB, PRODUCT = STAGES * STAGE, RESIDUAL = 4 * XB + 2 * 27 * TX * TY * 8;
 };
 
 // Per-column sums of NQ quantities over the grid; true in every thread of
@@ -558,8 +558,10 @@ __global__ void __launch_bounds__(BT, 2) br_update(const BVec a, const BlockOute
 // above infinity).  The march of br_apply with pairs: a plane's tile is split
 // as it is put into shared memory, the column scaled by one power of two;
 // what does not fit becomes infinite.  Bound by issue: 27 pair products of 12
-// instructions an output.  Every thread splitting what it gathered took 2.9
-// ms at 1.08 M nodes and 64 columns, the element matrices 3.9; this 2.3.
+// instructions an output, two columns at once.  At 1.08 M nodes and 64 columns
+// the element matrices took 3.9 ms, every thread splitting what it gathered
+// 2.9, the split tiles 2.3 (waiting for the rows), packed products 2.1, and
+// with the next plane's rows copied ahead into shared memory 1.8.
 template <int K, bool PROD>
 __global__ void __launch_bounds__(PT, 2) br_residual(const BVec a, const BlockRows g,
                                                      const BlockOuter o,
@@ -570,6 +572,9 @@ __global__ void __launch_bounds__(PT, 2) br_residual(const BVec a, const BlockRo
   constexpr int L = T::L, CELLS = T::SX * T::SY, NP = (CELLS * L + PT - 1) / PT;
   extern __shared__ __align__(128) unsigned char stage[];
   float4 *sx = reinterpret_cast<float4 *>(stage);  // [2][cell][hi, lo][lane]
+  // the entries that multiply a plane, [2][9 j + c][node], j as in br_rows
+  constexpr int NODES = T::TX * T::TY;
+  float2 *se = reinterpret_cast<float2 *>(stage + 4 * T::XB);
   const int l = threadIdx.x % L, pair = threadIdx.x / L;
   unsigned long long rm[4] = {0, 0, 0, 0}, bm[4] = {0, 0, 0, 0};
   if (!PROD) {
@@ -614,28 +619,44 @@ __global__ void __launch_bounds__(PT, 2) br_residual(const BVec a, const BlockRo
           }
         }
       };
+      const auto fetch_rows = [&](int z) {
+        float2 *dst = se + ((z - zb) & 1) * 27 * NODES;
+        for (int i = threadIdx.x; i < 27 * NODES; i += PT) {
+          const int k = i / NODES, j = k / 9, x = x0 + i % T::TX, y = y0 + i % NODES / T::TX;
+          const int zr = z + j - 1;
+          const bool in = x < g.nax && y < g.nay && zr >= 0 && zr < g.naz;
+          const float2 *src =
+              g.S + (in ? (size_t)(9 * (2 - j) + k % 9) * g.N + ((long)zr * g.nay + y) * g.nax + x
+                        : 0);
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(tc::smem_u32(dst + i)),
+                       "l"(src), "r"(in ? 8 : 0)
+                       : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      };
       const bool in0 = x0 + px < g.nax && y0 + py < g.nay, in1 = in0 && x0 + px + 1 < g.nax;
-      DfAcc lo[2][4], mid[2][4], up[2][4];
-      clear<2>(lo);
-      clear<2>(mid);
+      DfAccx2 lo[2][2], mid[2][2], up[2][2];
+      const DfAccx2 none{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+      for (int u = 0; u < 2; u++)
+        lo[u][0] = lo[u][1] = mid[u][0] = mid[u][1] = none;
       __syncthreads();  // the stages of the segment before are read
+      fetch_rows(zb);
       load(zb);
       store(zb);
       long n = ((long)zb * g.nay + y0 + py) * g.nax + x0 + px;
       for (int z = zb; z <= ze; z++, n += pl) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
         if (z < ze) {
+          fetch_rows(z + 1);
           load(z + 1);
           store(z + 1);
         }
         if (in0) {
-          clear<2>(up);
+          up[0][0] = up[0][1] = up[1][0] = up[1][1] = none;
           const float4 *xs = sx + (((z - zb) & 1) * CELLS + py * T::SX + px) * 2 * L + l;
-          // rows of planes and nodes that do not exist are never written:
-          // any entries do for them
-          const float2 *row[3] = {g.S + (z > 0 ? n - pl : n), g.S + n,
-                                  g.S + (z < g.naz - 1 ? n + pl : n)};
-          const int u1 = in1 ? 1 : 0;
+          const float2 *es = se + ((z - zb) & 1) * 27 * NODES + py * T::TX + px;
 #pragma unroll 1
           for (int dy = 0; dy < 3; dy++) {
 #pragma unroll
@@ -646,15 +667,18 @@ __global__ void __launch_bounds__(PT, 2) br_residual(const BVec a, const BlockRo
               for (int u = 0; u < 2; u++) {
                 const int dx = i - u;
                 if (dx < 0 || dx > 2) continue;
-                float2 e[3];
+                DfDup e[3];
 #pragma unroll
-                for (int j = 0; j < 3; j++)
-                  e[j] = __ldg(row[j] + (size_t)(9 * (2 - j) + 3 * dy + dx) * g.N + (u ? u1 : 0));
+                for (int j = 0; j < 3; j++) {
+                  const float2 v = es[(9 * j + 3 * dy + dx) * NODES + u];
+                  e[j] = df_dup(Df2{v.x, v.y});
+                }
 #pragma unroll
-                for (int c = 0; c < 4; c++) {
-                  df_fma_acc(lo[u][c], e[0].x, e[0].y, f4(xh, c), f4(xl, c));
-                  df_fma_acc(mid[u][c], e[1].x, e[1].y, f4(xh, c), f4(xl, c));
-                  df_fma_acc(up[u][c], e[2].x, e[2].y, f4(xh, c), f4(xl, c));
+                for (int c = 0; c < 2; c++) {
+                  const Df2x2 xp{half_of(xh, c), half_of(xl, c)};
+                  df_acc2(lo[u][c], e[0], xp);
+                  df_acc2(mid[u][c], e[1], xp);
+                  df_acc2(up[u][c], e[2], xp);
                 }
               }
             }
@@ -670,7 +694,8 @@ __global__ void __launch_bounds__(PT, 2) br_residual(const BVec a, const BlockRo
                 ld4d(B, at, b);
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
-                  double ax = df_to_double(lo[u][c].s, lo[u][c].c);
+                  const DfAccx2 &t = lo[u][c / 2];
+                  double ax = c & 1 ? df_to_double(t.s.y, t.c.y) : df_to_double(t.s.x, t.c.x);
                   if (!df_scale(ax, shift[c])) ax = ldexp(ax, shift[c]);
                   r[c] = b[c] - ax;
                   bm[c] = max(bm[c], magnitude(b[c]));
@@ -683,7 +708,7 @@ __global__ void __launch_bounds__(PT, 2) br_residual(const BVec a, const BlockRo
 #pragma unroll
               for (int u = 0; u < 2; u++)
 #pragma unroll
-                for (int c = 0; c < 4; c++) {
+                for (int c = 0; c < 2; c++) {
                   lo[u][c] = mid[u][c];
                   mid[u][c] = up[u][c];
                 }
