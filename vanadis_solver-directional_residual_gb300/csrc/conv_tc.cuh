@@ -63,6 +63,7 @@ constexpr int SX = TX + 2, SY = TY + 2;    // halo slab extents in x, y
 constexpr int PROWS = SX * SY;             // 180 voxel rows per slab plane
 constexpr int THREADS = 192;
 constexpr int BUDGET = 200 * 1024;         // shared memory for slabs + weights
+constexpr int LIMIT = 225 * 1024;          // the same where that doubles the slabs
 constexpr long long WAIT_LIMIT = 2000000000LL;  // ~1 s of clocks per wait
 
 // Slab bytes of a part with C channels for G planes (1024-aligned for the
@@ -71,9 +72,15 @@ __host__ __device__ constexpr int slab_bytes(int C, int G) {
   return C == 0 ? 0 : (PROWS * (G + 2) * 2 * C + 1023) / 1024 * 1024;
 }
 __host__ __device__ constexpr int tap_bytes(int cin, int cout) { return cin / 8 * cout * 16; }
+// Taps in the ring of streamed weights beside slabs of `slabs` bytes.
+__host__ __device__ constexpr int ring_of(int wt, int slabs) {
+  return 8 * wt + slabs <= BUDGET ? 8 : (LIMIT - slabs) / wt;
+}
 // Largest G in {8, 4, 2, 1} whose two accumulator sets fit the 512 TMEM
 // columns and whose `ns` slab stages plus weights (all 27 taps resident, or
-// an 8-tap ring) fit the budget; 0 if none.
+// an 8-tap ring) fit the budget; 0 if none.  Weights too many ever to be
+// resident make do with a shorter ring beside two pairs of planes (64 -> 64
+// channels: 20.4 us with one stage and eight taps, 14.5 with two and five).
 __host__ __device__ constexpr int fit_group(int cin1, int cin2, int cout, int ns) {
   for (int G = 8; G >= 1; G /= 2) {
     if (2 * G * cout > 512) continue;
@@ -81,6 +88,7 @@ __host__ __device__ constexpr int fit_group(int cin1, int cin2, int cout, int ns
     const int wt = tap_bytes(cin1 + cin2, cout);
     const int w = (27 * wt + ns * slab <= BUDGET) ? 27 * wt : 8 * wt;
     if (ns * slab + w <= BUDGET) return G;
+    if (G == 2 && ns == 2 && 27 * wt > BUDGET && ns * slab + 5 * wt <= LIMIT) return G;
   }
   return 0;
 }
@@ -131,7 +139,7 @@ struct Shape {
   static constexpr int TXB = PROWS * (G + 2) * 2 * (CIN1 + CIN2);  // bytes the boxes land
   static constexpr int WTAP = tap_bytes(CIN1 + CIN2, COUT);  // one tap's weights
   static constexpr bool RES = weights_resident(CIN1, CIN2, COUT);
-  static constexpr int NW = RES ? 27 : 8;       // weight slots
+  static constexpr int NW = RES ? 27 : ring_of(WTAP, NS * SLAB);  // weight slots
   static constexpr int ACC = 2 * G * COUT;      // columns of the two accumulator sets
   static constexpr int TMEM_COLS =
       ACC <= 32 ? 32 : (ACC <= 64 ? 64 : (ACC <= 128 ? 128 : (ACC <= 256 ? 256 : 512)));
