@@ -637,48 +637,65 @@ __device__ __forceinline__ int child_count(int X, int Y, int Z, const Dims &f) {
 
 // gf[v][c] += gc[parent(v)][c] / count(parent)
 __global__ void pool_bwd_add(const float *gc, float *gf, Dims f, Dims c, int C) {
-  const long total = f.V * C;
+  const int c4 = C / 4;
+  const long total = f.V * c4;
   for (long idx = (long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += (long)gridDim.x * blockDim.x) {
-    const int ch = (int)(idx % C);
-    const long v = idx / C;
-    const int x = (int)(v % f.W), y = (int)((v / f.W) % f.H),
-              z = (int)(v / ((long)f.W * f.H));
+    const int ch = (int)((unsigned)idx % (unsigned)c4);
+    const unsigned v = (unsigned)(idx / c4);
+    const int x = (int)(v % (unsigned)f.W), r = (int)(v / (unsigned)f.W);
+    const int y = r % f.H, z = r / f.H;
     const int X = x >> 1, Y = y >> 1, Z = z >> 1;
     const long P = (long)X + (long)c.W * (Y + (long)c.H * Z);
-    gf[idx] += gc[P * C + ch] / (float)child_count(X, Y, Z, f);
+    const float n = (float)child_count(X, Y, Z, f);
+    const float4 g = __ldg(reinterpret_cast<const float4 *>(gc) + P * c4 + ch);
+    float4 o = reinterpret_cast<const float4 *>(gf)[idx];
+    o.x += g.x / n;
+    o.y += g.y / n;
+    o.z += g.z / n;
+    o.w += g.w / n;
+    reinterpret_cast<float4 *>(gf)[idx] = o;
   }
 }
 
 // Splits the gradient of a [skip | up(coarse)] input: gskip = first C1
 // channels; gcoarse[P] = sum over the children of the last C2 channels.
+// Four channels a thread.
 __global__ void upcat_bwd_skip(const float *gcat, float *gskip, long V, int C1, int C2) {
-  const long total = V * C1;
+  const int c4 = C1 / 4, t4 = (C1 + C2) / 4;
+  const long total = V * c4;
   for (long idx = (long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += (long)gridDim.x * blockDim.x) {
-    const long v = idx / C1;
-    const int ch = (int)(idx % C1);
-    gskip[idx] = gcat[v * (C1 + C2) + ch];
+    const long v = idx / c4;
+    const int ch = (int)((unsigned)idx % (unsigned)c4);
+    reinterpret_cast<float4 *>(gskip)[idx] =
+        __ldg(reinterpret_cast<const float4 *>(gcat) + v * t4 + ch);
   }
 }
 __global__ void upcat_bwd_coarse(const float *gcat, float *gc, Dims f, Dims c,
                                  int C1, int C2) {
-  const long total = c.V * C2;
+  const int c4 = C2 / 4, t4 = (C1 + C2) / 4;
+  const long total = c.V * c4;
   for (long idx = (long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += (long)gridDim.x * blockDim.x) {
-    const int ch = (int)(idx % C2);
-    const long vc = idx / C2;
-    const int X = (int)(vc % c.W), Y = (int)((vc / c.W) % c.H),
-              Z = (int)(vc / ((long)c.W * c.H));
-    float s = 0.f;
-    for (int k = 0; k < 2; k++)
-      for (int j = 0; j < 2; j++)
-        for (int i = 0; i < 2; i++) {
-          const int x = 2 * X + i, y = 2 * Y + j, z = 2 * Z + k;
-          if (x < f.W && y < f.H && z < f.D)
-            s += gcat[((long)x + (long)f.W * (y + (long)f.H * z)) * (C1 + C2) + C1 + ch];
-        }
-    gc[idx] = s;
+    const int ch = (int)((unsigned)idx % (unsigned)c4);
+    const unsigned vc = (unsigned)(idx / c4);
+    const int X = (int)(vc % (unsigned)c.W), r = (int)(vc / (unsigned)c.W);
+    const int Y = r % c.H, Z = r / c.H;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int t = 0; t < 8; t++) {
+      const int x = 2 * X + (t & 1), y = 2 * Y + ((t >> 1) & 1), z = 2 * Z + (t >> 2);
+      if (x < f.W && y < f.H && z < f.D) {
+        const float4 g = __ldg(reinterpret_cast<const float4 *>(gcat) +
+                               ((long)x + (long)f.W * (y + (long)f.H * z)) * t4 + C1 / 4 + ch);
+        s.x += g.x;
+        s.y += g.y;
+        s.z += g.z;
+        s.w += g.w;
+      }
+    }
+    reinterpret_cast<float4 *>(gc)[idx] = s;
   }
 }
 
@@ -789,23 +806,28 @@ __global__ void pack_weights(const float *th, bf16 *wb, bf16 *wbt, bf16 *wtc, bf
 }
 
 // Nearest upsampling of a coarse [Vc][C] BF16 tensor to the fine grid
-// (fine voxel (x, y, z) reads coarse (x/2, y/2, z/2)), 16 bytes a thread.
-__global__ void upsample_bf16(const bf16 *__restrict__ in, bf16 *__restrict__ out,
-                              int W, int H, long V, int Wc, int Hc, int C,
-                              const int *skip, const int *skip2) {
+// (fine voxel (x, y, z) reads coarse (x/2, y/2, z/2)): a thread copies 16
+// bytes of a coarse voxel to its up to eight fine ones (one thread per fine
+// unit, with its 64-bit divisions: 24 us at 129 x 129 x 65 voxels and 32
+// channels, so 15).
+__global__ void upsample_bf16(const bf16 *__restrict__ in, bf16 *__restrict__ out, Dims f, Dims c,
+                              int C, const int *skip, const int *skip2) {
   if (skipped(skip, skip2)) return;
   const int c8 = C / 8;
-  const long total = V * c8;
+  const long total = c.V * c8;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long)gridDim.x * blockDim.x) {
-    const long v = i / c8;
-    const int k = (int)(i - v * c8);
-    const int x = (int)(v % W);
-    const long r = v / W;
-    const int y = (int)(r % H), z = (int)(r / H);
-    const long vc = (long)(x >> 1) + (long)Wc * ((long)(y >> 1) + (long)Hc * (z >> 1));
-    reinterpret_cast<uint4 *>(out)[v * c8 + k] =
-        __ldg(reinterpret_cast<const uint4 *>(in) + vc * c8 + k);
+    const int k = (int)((unsigned)i % (unsigned)c8);
+    const unsigned vc = (unsigned)(i / c8);
+    const int X = (int)(vc % (unsigned)c.W), r = (int)(vc / (unsigned)c.W);
+    const int Y = r % c.H, Z = r / c.H;
+    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(in) + i);
+#pragma unroll
+    for (int t = 0; t < 8; t++) {
+      const int x = 2 * X + (t & 1), y = 2 * Y + ((t >> 1) & 1), z = 2 * Z + (t >> 2);
+      if (x < f.W && y < f.H && z < f.D)
+        reinterpret_cast<uint4 *>(out)[((long)x + (long)f.W * (y + (long)f.H * z)) * c8 + k] = v;
+    }
   }
 }
 
@@ -1346,7 +1368,7 @@ cudaError_t bwd_data(const Net &n, int l, const float *dy, const bf16 *y, float 
 }
 
 // The forward pass's ten convolutions on the tensor cores (tcgen05).
-cudaError_t net_forward_tc(Net &n, const int *sk, const int *sk2, cudaStream_t s) {
+cudaError_t net_forward_tc(Net &n, const int *sk, const int *sk2, cudaStream_t s, float *out) {
   cudaError_t e;
   const Dims &f0 = n.d[0], &f1 = n.d[1], &f2 = n.d[2];
   if ((e = conv_tc_launch<16, 0, 16>(n, L_E0A, n.a0, sk, sk2, s)) ||
@@ -1360,25 +1382,23 @@ cudaError_t net_forward_tc(Net &n, const int *sk, const int *sk2, cudaStream_t s
   if ((e = conv_tc_launch<32, 0, 64>(n, L_BTA, n.a2, sk, sk2, s)) ||
       (e = conv_tc_launch<64, 0, 64>(n, L_BTB, n.b2, sk, sk2, s)))
     return e;
-  upsample_bf16<<<grid_for(f1.V * 8, 256), 256, 0, s>>>(n.b2, n.up1, f1.W, f1.H, f1.V,
-                                                         f2.W, f2.H, 64, sk, sk2);
+  upsample_bf16<<<grid_for(f2.V * 8, 256), 256, 0, s>>>(n.b2, n.up1, f1, f2, 64, sk, sk2);
   if ((e = conv_tc_launch<32, 64, 32>(n, L_D1A, n.a3, sk, sk2, s)) ||
       (e = conv_tc_launch<32, 0, 32>(n, L_D1B, n.u1, sk, sk2, s)))
     return e;
-  upsample_bf16<<<grid_for(f0.V * 4, 256), 256, 0, s>>>(n.u1, n.up0, f0.W, f0.H, f0.V,
-                                                         f1.W, f1.H, 32, sk, sk2);
+  upsample_bf16<<<grid_for(f1.V * 4, 256), 256, 0, s>>>(n.u1, n.up0, f0, f1, 32, sk, sk2);
   if ((e = conv_tc_launch<16, 32, 16>(n, L_D0A, n.a4, sk, sk2, s)) ||
       (e = conv_tc_launch<16, 0, 16>(n, L_D0B, n.u0, sk, sk2, s)))
     return e;
-  head_fwd<<<grid_for(f0.V, 256), 256, 0, s>>>(n.u0, n.theta + n.woff[L_HEAD], n.c, f0.V,
+  head_fwd<<<grid_for(f0.V, 256), 256, 0, s>>>(n.u0, n.theta + n.woff[L_HEAD], out, f0.V,
                                                 sk, sk2);
   count_launches(5);
   return cudaGetLastError();
 }
 
 // Forward pass from the prepared input x0 to the head output c.
-cudaError_t net_forward(Net &n, const int *sk, const int *sk2, cudaStream_t s) {
-  if (tc_mode(n)) return net_forward_tc(n, sk, sk2, s);
+cudaError_t net_forward(Net &n, const int *sk, const int *sk2, cudaStream_t s, float *out) {
+  if (tc_mode(n)) return net_forward_tc(n, sk, sk2, s, out);
   cudaError_t e;
 #define VDR_CONV(CI1, CI2, CO, LVL, IN1, IN2, L, OUT)                              \
   if ((e = conv_launch<CI1, CI2, CO, false, false>(                                \
@@ -1400,7 +1420,7 @@ cudaError_t net_forward(Net &n, const int *sk, const int *sk2, cudaStream_t s) {
   VDR_CONV(16, 0, 16, 0, n.a4, nullptr, L_D0B, n.u0)
 #undef VDR_CONV
   head_fwd<<<grid_for(n.d[0].V, 256), 256, 0, s>>>(n.u0, n.theta + n.woff[L_HEAD],
-                                                   n.c, n.d[0].V, sk, sk2);
+                                                   out, n.d[0].V, sk, sk2);
   count_launches(3);
   return cudaGetLastError();
 }
@@ -1417,8 +1437,8 @@ cudaError_t net_backward(Net &n, cudaStream_t s) {
   // d0a: a4 = relu(conv([s0 | up(u1)]))
   if ((e = wgrad_launch<16, 32, 16>(n, wg_args(n, L_D0A, n.s0, n.u1), n.g_a4, n.a4, s))) return e;
   if ((e = bwd_data<16, 48>(n, L_D0A, n.g_a4, n.a4, n.g_cat0, s))) return e;
-  upcat_bwd_skip<<<grid_for(f0.V * 16, 256), 256, 0, s>>>(n.g_cat0, n.g_s0, f0.V, 16, 32);
-  upcat_bwd_coarse<<<grid_for(f1.V * 32, 256), 256, 0, s>>>(n.g_cat0, n.g_u1, f0, f1, 16, 32);
+  upcat_bwd_skip<<<grid_for(f0.V * 4, 256), 256, 0, s>>>(n.g_cat0, n.g_s0, f0.V, 16, 32);
+  upcat_bwd_coarse<<<grid_for(f1.V * 8, 256), 256, 0, s>>>(n.g_cat0, n.g_u1, f0, f1, 16, 32);
   count_launches(2);
   // d1b: u1 = relu(conv(a3))
   if ((e = wgrad_launch<32, 0, 32>(n, wg_args(n, L_D1B, n.a3, nullptr), n.g_u1, n.u1, s))) return e;
@@ -1426,8 +1446,8 @@ cudaError_t net_backward(Net &n, cudaStream_t s) {
   // d1a: a3 = relu(conv([s1 | up(b2)]))
   if ((e = wgrad_launch<32, 64, 32>(n, wg_args(n, L_D1A, n.s1, n.b2), n.g_a3, n.a3, s))) return e;
   if ((e = bwd_data<32, 96>(n, L_D1A, n.g_a3, n.a3, n.g_cat1, s))) return e;
-  upcat_bwd_skip<<<grid_for(f1.V * 32, 256), 256, 0, s>>>(n.g_cat1, n.g_s1, f1.V, 32, 64);
-  upcat_bwd_coarse<<<grid_for(f2.V * 64, 256), 256, 0, s>>>(n.g_cat1, n.g_b2, f1, f2, 32, 64);
+  upcat_bwd_skip<<<grid_for(f1.V * 8, 256), 256, 0, s>>>(n.g_cat1, n.g_s1, f1.V, 32, 64);
+  upcat_bwd_coarse<<<grid_for(f2.V * 16, 256), 256, 0, s>>>(n.g_cat1, n.g_b2, f1, f2, 32, 64);
   count_launches(2);
   // btb: b2 = relu(conv(a2))
   if ((e = wgrad_launch<64, 0, 64>(n, wg_args(n, L_BTB, n.a2, nullptr), n.g_b2, n.b2, s))) return e;
@@ -1435,7 +1455,7 @@ cudaError_t net_backward(Net &n, cudaStream_t s) {
   // bta: a2 = relu(conv(p1))
   if ((e = wgrad_launch<32, 0, 64>(n, wg_args(n, L_BTA, n.p1, nullptr), n.g_a2, n.a2, s))) return e;
   if ((e = bwd_data<64, 32>(n, L_BTA, n.g_a2, n.a2, n.g_p1, s))) return e;
-  pool_bwd_add<<<grid_for(f1.V * 32, 256), 256, 0, s>>>(n.g_p1, n.g_s1, f1, f2, 32);
+  pool_bwd_add<<<grid_for(f1.V * 8, 256), 256, 0, s>>>(n.g_p1, n.g_s1, f1, f2, 32);
   count_launches(1);
   // e1b: s1 = relu(conv(a1))
   if ((e = wgrad_launch<32, 0, 32>(n, wg_args(n, L_E1B, n.a1, nullptr), n.g_s1, n.s1, s))) return e;
@@ -1443,7 +1463,7 @@ cudaError_t net_backward(Net &n, cudaStream_t s) {
   // e1a: a1 = relu(conv(p0))
   if ((e = wgrad_launch<16, 0, 32>(n, wg_args(n, L_E1A, n.p0, nullptr), n.g_a1, n.a1, s))) return e;
   if ((e = bwd_data<32, 16>(n, L_E1A, n.g_a1, n.a1, n.g_p0, s))) return e;
-  pool_bwd_add<<<grid_for(f0.V * 16, 256), 256, 0, s>>>(n.g_p0, n.g_s0, f0, f1, 16);
+  pool_bwd_add<<<grid_for(f0.V * 4, 256), 256, 0, s>>>(n.g_p0, n.g_s0, f0, f1, 16);
   count_launches(1);
   // e0b: s0 = relu(conv(a0))
   if ((e = wgrad_launch<16, 0, 16>(n, wg_args(n, L_E0B, n.a0, nullptr), n.g_s0, n.s0, s))) return e;
@@ -1473,7 +1493,7 @@ cudaError_t net_loss_grad(Net &n, const float *rhat, const float *tg, cudaStream
   prep_input<float><<<grid_for(V, 256), 256, 0, s>>>(rhat, nullptr, n.feat, n.x0, V,
                                                        nullptr, nullptr);
   count_launches(1);
-  if ((e = net_forward(n, nullptr, nullptr, s))) return e;
+  if ((e = net_forward(n, nullptr, nullptr, s, n.c))) return e;
   if ((e = cudaMemsetAsync(n.grad, 0, sizeof(float) * n.nparam, s))) return e;
   if ((e = cudaMemsetAsync(n.scal + 1, 0, sizeof(double), s))) return e;
   free_sum<2, float><<<n.red_grid, 256, 0, s>>>(tg, n.h->mask, V, n.partials, n.ticket,
@@ -1495,7 +1515,7 @@ cudaError_t net_residual_loss_grad(Net &n, const float *rhat, cudaStream_t s) {
   prep_input<float><<<grid_for(V, 256), 256, 0, s>>>(rhat, nullptr, n.feat, n.x0, V,
                                                        nullptr, nullptr);
   count_launches(1);
-  if ((e = net_forward(n, nullptr, nullptr, s))) return e;
+  if ((e = net_forward(n, nullptr, nullptr, s, n.c))) return e;
   res_z<<<grid_for(V, 256), 256, 0, s>>>(rhat, n.c, h.dinv, h.mask, n.scal + 2, n.zbuf, V);
   count_launches(1);
   if ((e = cudaMemsetAsync(n.qbuf, 0, sizeof(double) * V, s)) ||
@@ -1526,7 +1546,7 @@ cudaError_t net_enqueue(void *ctx, const double *in, double *out, const int *ski
   prep_input<double><<<grid_for(V, 256), 256, 0, s>>>(in, n.scal, n.feat, n.x0, V,
                                                         skip, skip2);
   count_launches(2);
-  cudaError_t e = net_forward(n, skip, skip2, s);
+  cudaError_t e = net_forward(n, skip, skip2, s, n.c);
   if (e) return e;
   combine_out<<<grid_for(V, 256), 256, 0, s>>>(n.c, n.scal, n.scal + 2, n.h->mask,
                                                out, V, skip, skip2);
@@ -1852,8 +1872,7 @@ extern "C" int vdr_net_forward_device(vdr_net *N, const float *d_rhat, float *d_
   prep_input<float><<<grid_for(V, 256), 256, 0, s>>>(d_rhat, nullptr, n.feat, n.x0, V,
                                                        nullptr, nullptr);
   count_launches(1);
-  cudaError_t e = net_forward(n, nullptr, nullptr, s);
-  if (!e) e = cudaMemcpyAsync(d_out, n.c, sizeof(float) * V, cudaMemcpyDeviceToDevice, s);
+  const cudaError_t e = net_forward(n, nullptr, nullptr, s, d_out);
   return e ? cuda_fail(e, "network forward") : VDR_OK;
 }
 
