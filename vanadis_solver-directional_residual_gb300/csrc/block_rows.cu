@@ -20,8 +20,8 @@
 // with rho' = (rh, s) - omega (rh, t), where the element-wise form takes
 // seven kernels and 26 passes (clearing v and t among them).  The FP64
 // residual of the refinement runs the same way on the pair rows.  At 1.08 M
-// nodes and 64 columns an iteration takes 923 us instead of 1346, a residual
-// 1.8 ms instead of 3.9 + 0.35; a whole solve 128 -> 86 ms, and 4.1 -> 3.5 ms
+// nodes and 64 columns an iteration takes 905 us instead of 1346, a residual
+// 1.8 ms instead of 3.9 + 0.35; a whole solve 128 -> 83 ms, and 4.1 -> 3.5 ms
 // at 343 nodes.
 #include <cuda_runtime.h>
 #include <math.h>
@@ -160,28 +160,43 @@ __global__ void br_rows(const float2 *__restrict__ S, const float *__restrict__ 
   }
 }
 
-// A block's share of the tiles' planes, in one sequence along z, then over
-// the tiles: segments [z0, z1) of a tile, read from the plane before to the
-// plane after.
+// A block's share of the tiles' planes: whole columns in rounds while there is
+// one for every block, so that neighbouring tiles march side by side and find
+// their common nodes in L2, then an equal part of the columns left, taken as
+// one sequence along z, then over the tiles.  Segments [z0, z1) of a tile,
+// read from the plane before to the plane after.
 struct Share {
+  int round, rounds, first;  // columns taken in rounds, all of them
   long at, end;
   int x0, y0, z0, z1, zb, ze;
   __device__ Share(const BlockRows &g) {
-    const long total = (long)g.nxt * g.nyt * g.naz;
-    at = total * blockIdx.x / gridDim.x;
-    end = total * (blockIdx.x + 1) / gridDim.x;
+    const int tiles = g.nxt * g.nyt, G = (int)gridDim.x;
+    round = 0;
+    rounds = tiles / G;
+    first = rounds * G;
+    const long total = (long)(tiles - first) * g.naz;
+    at = total * blockIdx.x / G;
+    end = total * (blockIdx.x + 1) / G;
   }
   template <class T>
   __device__ bool next(const BlockRows &g) {
-    if (at >= end) return false;
-    const int t = (int)(at / g.naz);
-    z0 = (int)(at - (long)t * g.naz);
-    z1 = (int)min((long)g.naz, z0 + (end - at));
+    int t;
+    if (round < rounds) {
+      t = (round++) * (int)gridDim.x + (int)blockIdx.x;
+      z0 = 0;
+      z1 = g.naz;
+    } else {
+      if (at >= end) return false;
+      t = (int)(at / g.naz);
+      z0 = (int)(at - (long)t * g.naz);
+      z1 = (int)min((long)g.naz, z0 + (end - at));
+      at += z1 - z0;
+      t += first;
+    }
     x0 = t % g.nxt * T::TX;
     y0 = t / g.nxt * T::TY;
     zb = max(z0 - 1, 0);
     ze = min(z1, g.naz - 1);
-    at += z1 - z0;
     return true;
   }
 };
@@ -200,8 +215,10 @@ struct Maps {
 // 16-byte loads a node, 254 and 437 us (latency); tiles fetched by the
 // threads' own asynchronous copies 264 and 355 (as many instructions for
 // addresses as for products); by tensor copies 212 and 280; with the inner
-// products packed and rh prefetched to L2 190 and 272 (HBM:
-// 140 each; issue is 60 % busy).  Forming s in the second product's tiles
+// products packed and rh prefetched to L2 190 and 272; with
+// the columns taken side by side (Share) 167 and 270 (HBM: 140 each; the
+// second is bound by issue, 60 % busy with its four products).  Three blocks
+// an SM for the first: no change.  Forming s in the second product's tiles
 // instead of in br_s (130 us) took 594: the registers do not suffice.
 template <int K, bool SECOND>
 __global__ void __launch_bounds__(PT, 2) br_apply(const BVec a, const BlockRows g,
