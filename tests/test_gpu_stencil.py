@@ -298,3 +298,30 @@ def test_block_solve_launch_shapes(vdr, oracle, gpu_lib, dims, K):
         ax, _ = oracle.matvec0(m.iss, bb, prob.bc, x / scale)
         assert np.linalg.norm(b / scale - ax) <= 1.01 * tol * np.linalg.norm(b / scale), k
         assert rel_l2(x / scale, got["atomic"][:, k] / scale) < 1e-8, k
+
+
+def test_recorded_apply_follows_the_operator(vdr, oracle, gpu_lib):
+    """An apply recorded by its caller, after applies that already run on
+    assembled rows, and replayed after the operator was built anew gives the
+    new operator's product."""
+    torch = pytest.importorskip("torch")
+    prob = vdr.problems.rotation_shear(13, 6, 5, seed=97)
+    m = prob.mesh
+    x = np.random.default_rng(5).standard_normal(m.nnode)
+    with vdr.Solver(prob, aH=2.0, aM=7.0) as s:
+        for _ in range(3):
+            s.apply(x)
+        xd = torch.tensor(x, device="cuda")
+        yd = torch.empty_like(xd)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=torch.cuda.ExternalStream(s.stream()),
+                              capture_error_mode="thread_local"):
+            assert s.lib.vdr_apply_device(s.h, xd.data_ptr(), yd.data_ptr(), 0) == 0
+        for aM in (7.0, 19.0):
+            s.set_operator(2.0, aM)
+            s.apply(x)  # builds it
+            graph.replay()
+            torch.cuda.synchronize()
+            ref, _ = oracle.matvec0(m.iss, oracle_bb(oracle, prob, 2.0, aM), prob.bc, x)
+            assert rel_l2(yd.cpu().numpy(), ref) < TOL, aM

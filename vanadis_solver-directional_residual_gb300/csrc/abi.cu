@@ -380,6 +380,7 @@ void invalidate(Handle &h) {
 // Summing them moves 732 bytes a node where an apply then saves 308, so the
 // third apply has paid for it; one apply per operator stays element-wise.
 cudaError_t rows_for_apply(Handle &h) {
+  if (foreign_capture(h, h.stream)) return cudaSuccess;
   return ++h.st_applies >= 2 ? ensure_stencil(h) : cudaSuccess;
 }
 
@@ -741,7 +742,7 @@ int vdr_apply_device(vdr_handle *H, const double *x, double *y, int transpose) {
   }
   if ((st = ensure_operator(h))) return st;
   cudaError_t e = rows_for_apply(h);
-  if (!e && stencil_ready(h)) {
+  if (!e && stencil_ready(h) && !foreign_capture(h, h.stream)) {
     e = launch_stencil_apply(h, transpose != 0, false, x, y, nullptr, nullptr, h.stream);
     return e ? cuda_fail(e, "apply") : VDR_OK;
   }

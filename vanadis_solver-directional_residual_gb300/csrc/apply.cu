@@ -964,7 +964,8 @@ cudaError_t launch_apply(const Handle &h, bool transpose, const double *x,
                          cudaStream_t s) {
   if (h.apply_mode == VDR_APPLY_MATRIX_FREE)
     return launch_mf_apply(op_args(h), h.apply_fp32, transpose, x, y, skip, skip2, s);
-  if (stencil_ready(h)) return launch_stencil_apply(h, transpose, true, x, y, skip, skip2, s);
+  if (stencil_ready(h) && !foreign_capture(h, s))
+    return launch_stencil_apply(h, transpose, true, x, y, skip, skip2, s);
   return launch_stored_apply(h, h.apply_fp32, transpose, x, y, skip, skip2, s);
 }
 

@@ -840,6 +840,7 @@ int solve_segmented_device(Handle &h, const double *b, double *x, double tol, in
     cudaGraph_t graph;
     if ((e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal)))
       return cuda_fail(e, "begin capture");
+    const OwnCapture own(h);
     const long long before = launches_so_far();
     for (int k = 0; k < K && !e; k++) {
       if (rows) {

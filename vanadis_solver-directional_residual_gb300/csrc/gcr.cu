@@ -379,6 +379,7 @@ int solve_gcr_device(Handle &h, const double *b, double *x, double tol,
     cudaGraph_t graph;
     if ((e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal)))
       return cuda_fail(e, "begin capture");
+    const OwnCapture own(h);
     const long long before = launches_so_far();
     for (int k = 0; k < m && !e; k++) e = gcr_step(h, a, g, k, prec);
     per_cycle = (long)(launches_so_far() - before);

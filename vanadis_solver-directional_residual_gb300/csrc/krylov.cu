@@ -867,6 +867,7 @@ int solve_device(Handle &h, int method, const double *b, double *x,
     cudaGraph_t graph;
     if ((e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal)))
       return cuda_fail(e, "begin capture");
+    const OwnCapture own(h);
     const long long before = launches_so_far();
     for (int k = 0; k < K; k++) {
       e = launch_iteration(h, method, a, prec);
@@ -1838,6 +1839,7 @@ int solve32_inner(Handle &h, double tol, int itmax, int *iter, double *err) {
     cudaGraph_t graph;
     if ((e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal)))
       return cuda_fail(e, "begin capture");
+    const OwnCapture own(h);
     const long long before = launches_so_far();
     for (int k = 0; k < K && !e; k++) e = launch_iteration32(h, a);
     count_launches(before - launches_so_far());  // captured, not launched

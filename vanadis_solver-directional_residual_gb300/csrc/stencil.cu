@@ -143,6 +143,15 @@ bool stencil_ready(const Handle &h) {
          !h.gate_active && h.storage == VDR_STORE_DF;
 }
 
+// Whether a caller records on the stream: what it replays later is to follow
+// the operator as it is then, and rows are summed anew by solves and applies
+// that are called, not replayed.  The element matrices are rebuilt in place.
+bool foreign_capture(const Handle &h, cudaStream_t s) {
+  if (h.own_capture) return false;
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(s, &c) != cudaSuccess || c != cudaStreamCaptureStatusNone;
+}
+
 // Room for the rows of the handle's nodes and for `len` pairs in *x (its
 // present length in *have; a new one is not zeroed).  False where the device
 // has no room for them: the element-wise apply stays.

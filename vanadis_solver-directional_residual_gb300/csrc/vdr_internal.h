@@ -233,6 +233,7 @@ struct Handle {
   size_t st_rows = 0, st_len = 0;  // nodes and pairs that they hold room for
   int st_nax = 0, st_pl = 0;    // the strides that st_x's pads are zero for
   int st_state = 0, st_applies = 0;
+  bool own_capture = false;
   // its binary16 rows for the mixed solve (half_rows.cu): 27 half planes, a
   // scale per row, FP32 vectors; hr_state as st_state, 2 = out of range
   void *hr_H = nullptr;
@@ -339,6 +340,15 @@ struct Handle {
 // table).
 ConnView conn_view(const Handle &h);
 cudaError_t launch_emask(Handle &h);
+
+// While a solve records its own iterations, whose rows it keeps current.
+struct OwnCapture {
+  Handle &h;
+  explicit OwnCapture(Handle &handle) : h(handle) { h.own_capture = true; }
+  ~OwnCapture() { h.own_capture = false; }
+};
+
+bool foreign_capture(const Handle &h, cudaStream_t s);
 
 // SM count of the current device, cached once (thread-safe).
 int device_sm_count();
