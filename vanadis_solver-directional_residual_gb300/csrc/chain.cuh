@@ -1,0 +1,32 @@
+// chain.cuh -- kernels of an iteration that follow one another directly: the
+// next one's blocks are brought up while the last ones of the one before are
+// still running (programmatic dependent launch), instead of after them.
+// Every kernel launched so begins with chain_wait, which returns when the
+// kernel before is complete and what it wrote is visible; nothing is read
+// before it.  At 40 to 50 us a kernel it gives about one per cent (mixed loop at
+// 3.6 M nodes 34.8 -> 34.3 ms, a step at 1.08 M 9.20 -> 8.92).
+#pragma once
+#include <cuda_runtime.h>
+
+namespace vdr {
+
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <class... P, class... A>
+cudaError_t chain_launch(void (*kernel)(P...), int grid, int block, cudaStream_t s, A... args) {
+  cudaLaunchAttribute after;
+  after.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  after.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3((unsigned)block);
+  c.stream = s;
+  c.attrs = &after;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
+}  // namespace vdr
