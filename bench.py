@@ -16,7 +16,9 @@ element matrices + Jacobi diagonal (DR recompute), right-hand side, solve.
             events on the library's stream)
   e2e       the same step through the C ABI with host arrays: fields
             uploaded, right-hand side downloaded, solution downloaded
-  roofline  the dominant kernel, the stored-matrix EBE apply, timed alone
+  roofline  the dominant kernels, a BiCGStab iteration on the assembled
+            rows (--scatter atomic or color: the stored-matrix EBE apply,
+            timed alone)
   --impl reference   the reference's CPU algorithm (the C oracle port of
             vanadis_full_DR_OpenMP_timing.for) on this host's cores
 """
@@ -50,7 +52,9 @@ def args_parse(argv=None):
     ap.add_argument("--nex", type=int, default=256)
     ap.add_argument("--ney", type=int, default=256)
     ap.add_argument("--nez", type=int, default=128)
-    ap.add_argument("--scatter", default="atomic", choices=["atomic", "color"])
+    ap.add_argument("--scatter", default="auto", choices=["auto", "atomic", "color"],
+                    help="auto: the library's default (assembled rows on this "
+                         "mesh); atomic, color: element by element")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-batched", action="store_true",
                     help="skip the many-right-hand-side section")
@@ -108,9 +112,11 @@ def workload_config(a, prob):
         "dirichlet_nodes": int(prob.bc.sum()),
         "apply": "stored element matrices, double-float pairs (built on GPU "
                  "each step from the fields and the mesh's geometric factors, "
-                 "which the handle forms once)",
+                 "which the handle forms once)" +
+                 (", summed into 27-point rows each step" if a.scatter == "auto" else ""),
         "scatter": a.scatter, "solver": "bicgstab", "precision": "fp64",
-        "l2": "inputs larger than L2 (element matrices 4.3 GB per apply)",
+        "l2": "inputs larger than L2 (assembled rows 1.8 GB, element matrices "
+              "4.3 GB per apply)",
     }
 
 
@@ -282,6 +288,27 @@ def run_reference(a):
 
 
 # --------------------------------------------------------------- GPU arm
+# Bytes a node of one BiCGStab iteration on the assembled rows: the products
+# v = A p^ (rows 216, p^ 8, r, 1/diag, r^ 24, mask 1; v, s, s^ written 24) and
+# t = A s^ (216, s^ 8, s, r^ 16; t written 8), and the direction (x, p, s, t,
+# v, 1/diag, w 56, mask 1; x, r, p, p^ written 32).
+ROW_ITERATION_BYTES = 273.0 + 248.0 + 89.0
+
+
+def apply_ms(s, stream, x, y, reps):
+    """One y += A x of the handle, in ms."""
+    import torch
+    for _ in range(3):
+        s.apply_accumulate_device(x, y)
+    e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    e0.record(stream)
+    for _ in range(reps):
+        s.apply_accumulate_device(x, y)
+    e1.record(stream)
+    torch.cuda.synchronize()
+    return e0.elapsed_time(e1) / reps
+
+
 def timed_steps(s, stream, b, x, aH, aM, cf, rM, solve, reps=3):
     """One theta step on handle `s`, timed on its stream: the operator
     invalidated, element matrices + Jacobi diagonal + right-hand side in one
@@ -897,23 +924,33 @@ def run_native(a):
     t_build, t_krylov = t_build_s * 1e3, t_krylov_s * 1e3
     y = torch.zeros_like(b)
 
-    # ---- roofline of the dominant kernel: stored EBE apply ----
+    # ---- roofline of the dominant kernels: one iteration on the assembled
+    # rows (its share of the solve), or the stored EBE apply timed alone ----
     xr = torch.randn(N, dtype=torch.float64, device="cuda")
     torch.cuda.synchronize()
     reps = 20
-    for _ in range(3):
-        s.apply_accumulate_device(xr, y)
-    r0, r1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    r0.record(stream)
-    for _ in range(reps):
-        s.apply_accumulate_device(xr, y)
-    r1.record(stream)
-    torch.cuda.synchronize()
-    t_apply_ms = r0.elapsed_time(r1) / reps
     alg_bytes = 544.0 * E + 24.0 * N
     peak, peak_kind = measured_peak()
-    achieved = alg_bytes / (t_apply_ms * 1e-3) / 1e9
-    traffic = profile_traffic()
+    if a.scatter == "auto":
+        dom = {"kernel": "bst_v + bst_t + bst_p (one BiCGStab iteration on the "
+                         "assembled 27-point rows of double-float pairs)",
+               "bytes": ROW_ITERATION_BYTES * N,
+               "ms": t_krylov / max(1, fp64_out[0]),
+               "traffic": None,
+               "traffic_kind": "the solve's time over its iterations (its start, "
+                               "the assembly of the rows and its last, idle "
+                               "iterations included) against the bytes of one "
+                               "iteration: two products of 216 bytes of rows and "
+                               "5 or 4 vectors a node, 11 vectors for the direction"}
+    else:
+        t_apply_ms = apply_ms(s, stream, xr, y, reps)
+        dom = {"kernel": "stored_apply_df (EBE apply, double-float element "
+                         "matrices, %s scatter)" % a.scatter,
+               "bytes": alg_bytes, "ms": t_apply_ms, "traffic": profile_traffic(),
+               "traffic_kind": "ncu DRAM bytes of a 1,048,576-element capture "
+                               "scaled to this size by elements and nodes "
+                               "(profiles/stored_apply_df_rotation_shear.md)"}
+    achieved = dom["bytes"] / (dom["ms"] * 1e-3) / 1e9
 
     # ---- element build: roofline against the SMs' instruction issue rate ----
     inst_per_elem = profile_value(BUILD_PROFILE, "warp_instructions_per_element")
@@ -1010,13 +1047,14 @@ def run_native(a):
     mixed["fp32_rounded_variant"] = rounded
     mixed["fp32_recompute_variant"] = recompute
 
-    # ---- the other scatter forms of the same step: colour by colour (no
-    # atomics) and warp-aggregated atomics ----
+    # ---- the other scatter forms of the same step: element by element with
+    # atomics, colour by colour (no atomics) and warp-aggregated atomics ----
     scatter_variants = {
-        "atomic": {"step_s": ms / 1e3, "solve_s": t_krylov_s,
-                   "apply_ms": t_apply_ms, "apply_gbs": achieved,
-                   "iterations": fp64_out[0]}}
-    for form in ("color", "warp"):
+        a.scatter: {"step_s": ms / 1e3, "solve_s": t_krylov_s,
+                    "iterations": fp64_out[0]}}
+    if a.scatter != "auto":
+        scatter_variants[a.scatter].update(apply_ms=dom["ms"], apply_gbs=achieved)
+    for form in [f for f in ("atomic", "color", "warp") if f != a.scatter]:
         sc = vdr.Solver(prob, vdr.Options(apply_mode="stored", scatter=form,
                                           solver="bicgstab", device=local),
                         aH=aH, aM=aM)
@@ -1027,20 +1065,12 @@ def run_native(a):
             sc, cstream, bcv, xc, aH, aM, cf, rM,
             lambda: sc.solve_device(bcv, xc, tol=TOL, itmax=20000))
         yc = torch.zeros_like(b)
-        for _ in range(3):
-            sc.apply_accumulate_device(xr, yc)
-        c2e, c3e = (torch.cuda.Event(enable_timing=True) for _ in range(2))
-        c2e.record(cstream)
-        for _ in range(reps):
-            sc.apply_accumulate_device(xr, yc)
-        c3e.record(cstream)
-        torch.cuda.synchronize()
-        a_ms = c2e.elapsed_time(c3e) / reps
+        a_ms = apply_ms(sc, cstream, xr, yc, reps)
         scatter_variants[form] = {
             "step_s": c_step, "solve_s": c_solve, "apply_ms": a_ms,
             "apply_gbs": alg_bytes / (a_ms * 1e-3) / 1e9,
             "iterations": c_out[0], "status": c_out[2],
-            "rel_l2_vs_atomic_solution":
+            "rel_l2_vs_step_solution":
                 float(torch.linalg.norm(xc - x) / torch.linalg.norm(x))}
         sc.close()
         del xc, bcv, yc
@@ -1048,6 +1078,10 @@ def run_native(a):
         "FP64 atomics after neighbouring lanes add their shared x-face nodes "
         "by shuffles (4 instead of 8 atomics per element)")
     scatter_variants["color"]["what"] = "8 launches per apply, no atomics"
+    if a.scatter == "auto":
+        scatter_variants["auto"]["what"] = (
+            "the library's default: 27-point rows summed once per operator, "
+            "products by gathering")
 
     # ---- the launch shapes the handle chose by measurement (the binary16
     # apply's after the mixed steps above) ----
@@ -1131,16 +1165,11 @@ def run_native(a):
                              "step": step_s * 1e3},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak,
                          "unit": "GB/s", "frac": achieved / peak,
-                         "traffic": traffic,
-                         "traffic_kind": "ncu DRAM bytes of a 1,048,576-"
-                                         "element capture scaled to this "
-                                         "size by elements and nodes "
-                                         "(profiles/stored_apply_df_"
-                                         "rotation_shear.md)",
-                         "kernel": "stored_apply_df (EBE apply, double-float "
-                                   "element matrices, atomic scatter)",
-                         "algorithmic_bytes_per_launch": alg_bytes,
-                         "launch_ms": t_apply_ms, "peak_kind": peak_kind},
+                         "traffic": dom["traffic"],
+                         "traffic_kind": dom["traffic_kind"],
+                         "kernel": dom["kernel"],
+                         "algorithmic_bytes_per_launch": dom["bytes"],
+                         "launch_ms": dom["ms"], "peak_kind": peak_kind},
             "roofline_build": {"bound": "issue", "achieved": build_issue,
                                "peak": issue_peak,
                                "unit": "G warp instructions/s",
@@ -1201,6 +1230,7 @@ def summary_keys(line, step_s, solve_s):
         "fp64_iters": line.get("iterations"),
         "fp64store_step_s": _r(f64.get("step_s")),
         "fp64store_solve_s": _r(f64.get("solve_s")),
+        "atomic_step_s": _r(g(sv, "atomic", "step_s")),
         "color_step_s": _r(g(sv, "color", "step_s")),
         "warp_step_s": _r(g(sv, "warp", "step_s")),
         "apply_ms": _r(g(sv, "atomic", "apply_ms")),
@@ -1242,8 +1272,8 @@ def run_case(a):
     """Small fixed workloads for profiler captures (not benchmarks): the
     stored double-float apply (--case apply), the K=64 block solve
     (--case block_apply), four K=64 block applies on the tcgen05 box form
-    (--case block_apply_tc), a BiCG solve (--case bicg, fused A/A^T apply), a
-    mixed-precision solve (--case mixed, FP32-vector inner apply) and
+    (--case block_apply_tc), a BiCG solve (--case bicg, fused A/A^T apply;
+    both element by element), a mixed-precision solve (--case mixed) and
     learned-network training steps (--case unet_train), each on the
     --nex x --ney x --nez mesh."""
     import torch
@@ -1263,7 +1293,8 @@ def run_case(a):
             s.set_operator(2.0, 3.0 / dt)
             s.assemble_rhs_device(b, 3.0, 3.0 / dt, None)
     elif a.case == "apply":
-        s = vdr.Solver(prob, vdr.Options(apply_mode="stored"), aH=2.0, aM=3.0 / dt)
+        s = vdr.Solver(prob, vdr.Options(apply_mode="stored", scatter="atomic"),
+                       aH=2.0, aM=3.0 / dt)
         x = torch.randn(prob.mesh.nnode, dtype=torch.float64, device="cuda")
         y = torch.zeros_like(x)
         torch.cuda.synchronize()
@@ -1288,7 +1319,8 @@ def run_case(a):
             s.apply_block_accumulate_device(X, Y, "tf32x3")
     elif a.case == "bicg":
         # BiCG: the fused A p / A^T p~ apply over the double-float store
-        s = vdr.Solver(prob, vdr.Options(apply_mode="stored", solver="bicg"),
+        s = vdr.Solver(prob, vdr.Options(apply_mode="stored", solver="bicg",
+                                         scatter="atomic"),
                        aH=2.0, aM=3.0 / dt)
         b = torch.empty(prob.mesh.nnode, dtype=torch.float64, device="cuda")
         s.assemble_rhs_device(b, 3.0, 0.0, None)

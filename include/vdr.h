@@ -58,7 +58,11 @@ extern "C" {
 #define VDR_DR_VF 2
 
 /* ---- scatter of element results to nodes ---- */
-#define VDR_SCATTER_AUTO 0   /* measured choice: atomic */
+#define VDR_SCATTER_AUTO 0   /* measured choice: on the structured numbering
+                                (natural order, double-float store) solves,
+                                and applies from an operator's second on, sum
+                                the element matrices into 27-point rows and
+                                gather; atomic elsewhere */
 #define VDR_SCATTER_ATOMIC 1 /* fp64 atomics, elements in natural order */
 #define VDR_SCATTER_COLOR 2  /* colour by colour, no atomics, deterministic */
 #define VDR_SCATTER_WARP 3   /* fp64 atomics aggregated within a warp: on the
@@ -322,7 +326,9 @@ int vdr_apply_block_accumulate_device(vdr_handle *h, int K, const void *d_X,
 /* Solves A X = B for K columns (K = 16, 32 or 64): FP64 refinement per
  * column (residual with the FP64-accurate operator, FP64 update) around K
  * simultaneous FP32 Jacobi-BiCGStab inner solves with the tensor-core apply
- * (precision VDR_BLOCK_TF32 or VDR_BLOCK_TF32X3), column k to
+ * (precision VDR_BLOCK_TF32 or VDR_BLOCK_TF32X3; under
+ * VDR_BLOCK_APPLY_AUTO, on the structured numbering, with FP32 products on
+ * assembled 27-point rows for either), column k to
  * max(inner_tol, 0.5 tol / err_k) relative to its residual (err_k its FP64
  * relative residual); columns already at tol sit out.
  * d_X holds the initial guess.  Returns VDR_OK when every column's FP64
@@ -451,7 +457,8 @@ int vdr_solve_record_device(vdr_handle *h, const double *d_b, double *d_x,
  * Jacobi-BiCGStab with per-mesh scalars and per-mesh convergence (a mesh
  * that converges freezes), all meshes advancing together in one CUDA graph.
  * The tile shape of the per-mesh reductions is chosen by measurement at the
- * first segmented solve (vdr_segment_tuning reports it).  No counterpart in
+ * first segmented solve, or by the number of rows where every mesh is in the
+ * structured numbering (vdr_segment_tuning reports it).  No counterpart in
  * the reference, which solves one mesh per call. */
 int vdr_set_segments(vdr_handle *h, int nseg, const int *node_off);
 /* iters, errs, statuses: host arrays of nseg (nullable).  Returns VDR_OK

@@ -27,7 +27,7 @@
 // threads, in shared memory (216 bytes a thread) above.  Per iteration,
 // cluster / grid: 8.1 us at 448 nodes, 9.6 / 12 at 1,170, 11 / 12.5 at 2,800,
 // 19.5 / 12.8 at 7,000 (reads across a cluster are slow in number), then 14.1
-// at 18,500, 20 at 75,000, 26 at 100,000, 31 at 148,000; four kernels per
+// at 18,500, 20 at 75,000, 24 at 100,000, 29 at 148,000; four kernels per
 // iteration: 31 at 2,800, 53 at 100,000.
 #include <cuda_runtime.h>
 #include <math.h>
