@@ -848,10 +848,10 @@ int solve_segmented_device(Handle &h, const double *b, double *x, double tol, in
     const long long before = launches_so_far();
     for (int k = 0; k < K && !e; k++) {
       if (rows) {
-        if ((e = chain_launch(keep ? sgr_v<true> : sgr_v<false>, nt, th, s, a)) ||
-            (e = chain_launch(keep ? sgr_t<true> : sgr_t<false>, nt, th, s, a)))
+        if ((e = chain_launch(keep ? sgr_v<true> : sgr_v<false>, nt, th, 0, s, a)) ||
+            (e = chain_launch(keep ? sgr_t<true> : sgr_t<false>, nt, th, 0, s, a)))
           break;
-        e = chain_launch(sgr_p, nt, th, s, a);
+        e = chain_launch(sgr_p, nt, th, 0, s, a);
         count_launches(3);
         continue;
       }

@@ -53,6 +53,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "chain.cuh"
 #include "tc_ptx.cuh"
 
 namespace vdr {
@@ -161,6 +162,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     conv3_tc_kernel(const __grid_constant__ CUtensorMap map1,
                     const __grid_constant__ CUtensorMap map2, Args a) {
   using S = Shape<CIN1, CIN2, COUT>;
+  chain_wait();
   if ((a.skip && *(volatile const int *)a.skip) ||
       (a.skip2 && *(volatile const int *)a.skip2))
     return;

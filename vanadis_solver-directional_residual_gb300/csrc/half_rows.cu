@@ -775,9 +775,9 @@ int solve_half_rows(Handle &h, const double *res, double rnorm, double *x, doubl
     if ((e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal)))
       return cuda_fail(e, "begin capture");
     for (int k = 0; k < K && !e; k++)
-      if (!(e = chain_launch(keep ? hb_v<true> : hb_v<false>, g, HT, s, a)) &&
-          !(e = chain_launch(keep ? hb_t<true> : hb_t<false>, g, HT, s, a)))
-        e = chain_launch(hb_p, g, HT, s, a);
+      if (!(e = chain_launch(keep ? hb_v<true> : hb_v<false>, g, HT, 0, s, a)) &&
+          !(e = chain_launch(keep ? hb_t<true> : hb_t<false>, g, HT, 0, s, a)))
+        e = chain_launch(hb_p, g, HT, 0, s, a);
     const cudaError_t e2 = cudaStreamEndCapture(s, &graph);
     if (e || e2) return cuda_fail(e ? e : e2, "capture");
     e = cudaGraphInstantiate(&h.hr_graph, graph, 0);

@@ -688,10 +688,10 @@ cudaError_t launch_stencil_iteration(Handle &h, const Vec &a, cudaStream_t s) {
   const bool keep = stencil_keep(h);
   const int gs = std::min(red_grid(h.N), device_sm_count() * 4);
   cudaError_t e;
-  if ((e = chain_launch(keep ? bst_v<true> : bst_v<false>, gs, RED_THREADS, s, a, w)) ||
-      (e = chain_launch(keep ? bst_t<true> : bst_t<false>, gs, RED_THREADS, s, a, w)))
+  if ((e = chain_launch(keep ? bst_v<true> : bst_v<false>, gs, RED_THREADS, 0, s, a, w)) ||
+      (e = chain_launch(keep ? bst_t<true> : bst_t<false>, gs, RED_THREADS, 0, s, a, w)))
     return e;
-  return chain_launch(bst_p, gs, RED_THREADS, s, a);
+  return chain_launch(bst_p, gs, RED_THREADS, 0, s, a);
 }
 
 // The fused FP64 BiCGStab iteration (defined below with the fused kernels).

@@ -51,6 +51,7 @@
 #include <cstring>
 #include <vector>
 
+#include "chain.cuh"
 #include "conv_tc.cuh"
 #include "vdr_internal.h"
 
@@ -160,6 +161,7 @@ __device__ __forceinline__ void ldsm_x4(const bf16 *p, uint32_t &r0, uint32_t &r
 // weight loads through L1 (measured faster for those layers).
 template <int CIN1, int CIN2, int COUT, int MS, bool F32IN, bool F32OUT>
 __global__ void __launch_bounds__(128) conv3_kernel(ConvArgs a) {
+  chain_wait();
   if (skipped(a.skip, a.skip2)) return;
   constexpr int CIN = CIN1 + CIN2, KC = CIN / 16, NT = COUT / 8;
   static_assert(CIN1 % 16 == 0 && CIN2 % 16 == 0 && COUT % 16 == 0, "shape");
@@ -346,6 +348,7 @@ template <int C>
 __global__ void mask_transpose(const float *__restrict__ dy, const bf16 *__restrict__ y,
                                bf16 *__restrict__ dyt, bf16 *__restrict__ dyc, int W, int Wp,
                                long Vp) {
+  chain_wait();
   static_assert(C % 8 == 0, "channels");
   const long row = blockIdx.x;
   for (int x = threadIdx.x; x < Wp; x += blockDim.x) {
@@ -404,6 +407,7 @@ __device__ __forceinline__ void ldsm_x4_trans(const bf16 *p, uint32_t &r0, uint3
 // half and twice the blocks 230 and 260).
 template <int CIN1, int CIN2, int COUT, int NG>
 __global__ void __launch_bounds__(128) conv3_wgrad_tc(WgArgs a) {
+  chain_wait();
   constexpr int CIN = CIN1 + CIN2, MT = COUT / 16, NT = CIN / 8;
   static_assert(COUT % 16 == 0 && CIN % 8 == 0 && CIN1 % 8 == 0 && NG % 2 == 0, "shape");
   // B tile per warp: 18 rows (voxels) x NG units, rows padded by one unit so
@@ -597,6 +601,7 @@ __host__ __device__ inline Dims coarse_of(const Dims &f) {
 // Eight channels (16 bytes) a thread.
 __global__ void pool_fwd(const bf16 *in, bf16 *out, Dims f, Dims c, int C,
                          const int *skip, const int *skip2) {
+  chain_wait();
   if (skipped(skip, skip2)) return;
   const int c8 = C / 8;
   const long total = c.V * c8;
@@ -637,6 +642,7 @@ __device__ __forceinline__ int child_count(int X, int Y, int Z, const Dims &f) {
 
 // gf[v][c] += gc[parent(v)][c] / count(parent)
 __global__ void pool_bwd_add(const float *gc, float *gf, Dims f, Dims c, int C) {
+  chain_wait();
   const int c4 = C / 4;
   const long total = f.V * c4;
   for (long idx = (long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -662,6 +668,7 @@ __global__ void pool_bwd_add(const float *gc, float *gf, Dims f, Dims c, int C) 
 // channels; gcoarse[P] = sum over the children of the last C2 channels.
 // Four channels a thread.
 __global__ void upcat_bwd_skip(const float *gcat, float *gskip, long V, int C1, int C2) {
+  chain_wait();
   const int c4 = C1 / 4, t4 = (C1 + C2) / 4;
   const long total = V * c4;
   for (long idx = (long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -674,6 +681,7 @@ __global__ void upcat_bwd_skip(const float *gcat, float *gskip, long V, int C1, 
 }
 __global__ void upcat_bwd_coarse(const float *gcat, float *gc, Dims f, Dims c,
                                  int C1, int C2) {
+  chain_wait();
   const int c4 = C2 / 4, t4 = (C1 + C2) / 4;
   const long total = c.V * c4;
   for (long idx = (long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -702,6 +710,7 @@ __global__ void upcat_bwd_coarse(const float *gcat, float *gc, Dims f, Dims c,
 // ---------------------------------------------------------- head / loss
 __global__ void head_fwd(const bf16 *u0, const float *wh, float *c, long V,
                          const int *skip, const int *skip2) {
+  chain_wait();
   if (skipped(skip, skip2)) return;
   for (long v = (long)blockIdx.x * blockDim.x + threadIdx.x; v < V;
        v += (long)gridDim.x * blockDim.x) {
@@ -723,6 +732,7 @@ __global__ void __launch_bounds__(256) head_bwd(const bf16 *u0, const float *wh,
                                                 const unsigned char *mask,
                                                 const double *tt, float *gu0,
                                                 float *dwh, double *loss, long V) {
+  chain_wait();
   const float inv_n = (float)(*tt > 0.0 ? 1.0 / *tt : 1.0 / (double)V);
   float lw[17];
 #pragma unroll
@@ -769,6 +779,7 @@ __global__ void __launch_bounds__(256) head_bwd(const bf16 *u0, const float *wh,
 __global__ void adam_kernel(float *th, const float *g, float *m, float *v, long n,
                             float lr, float b1, float b2, float eps, float bc1,
                             float bc2) {
+  chain_wait();
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (long)gridDim.x * blockDim.x) {
     const float gi = g[i];
@@ -788,6 +799,7 @@ __global__ void adam_kernel(float *th, const float *g, float *m, float *v, long 
 // in the same way the backward pass's, its inputs co and its outputs ci.
 __global__ void pack_weights(const float *th, bf16 *wb, bf16 *wbt, bf16 *wtc, bf16 *wtcb,
                              int cin, int cout, int stack, int stack_b) {
+  chain_wait();
   const long total = 27L * cin * cout;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long)gridDim.x * blockDim.x) {
@@ -812,6 +824,7 @@ __global__ void pack_weights(const float *th, bf16 *wb, bf16 *wbt, bf16 *wtc, bf
 // channels, so 15).
 __global__ void upsample_bf16(const bf16 *__restrict__ in, bf16 *__restrict__ out, Dims f, Dims c,
                               int C, const int *skip, const int *skip2) {
+  chain_wait();
   if (skipped(skip, skip2)) return;
   const int c8 = C / 8;
   const long total = c.V * c8;
@@ -836,6 +849,7 @@ __global__ void upsample_bf16(const bf16 *__restrict__ in, bf16 *__restrict__ ou
 // node v; acc[v][4] counts the elements.
 __global__ void node_feature_acc(const int *conn, const double *vel,
                                  const double *lam, int E, float *acc) {
+  chain_wait();
   for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < 8L * E;
        t += (long)gridDim.x * blockDim.x) {
     const long e = t % E;
@@ -848,6 +862,7 @@ __global__ void node_feature_acc(const int *conn, const double *vel,
   }
 }
 __global__ void node_feature_fin(const float *acc, float *feat, long N) {
+  chain_wait();
   for (long v = (long)blockIdx.x * blockDim.x + threadIdx.x; v < N;
        v += (long)gridDim.x * blockDim.x) {
     const float c = fmaxf(acc[v * 5 + 4], 1.f);
@@ -910,6 +925,7 @@ __global__ void __launch_bounds__(256) free_sum(const T *x,
                                                 double *partials, unsigned *ticket,
                                                 double *out, const int *skip,
                                                 const int *skip2) {
+  chain_wait();
   if (skipped(skip, skip2)) return;
   double s = 0.0, c = 0.0;
   for (long v = (long)blockIdx.x * blockDim.x + threadIdx.x; v < N;
@@ -935,6 +951,7 @@ __global__ void __launch_bounds__(256) free_sum(const T *x,
 template <typename T>
 __global__ void prep_input(const T *r, const double *rms, const float *feat,
                            bf16 *x0, long V, const int *skip, const int *skip2) {
+  chain_wait();
   if (skipped(skip, skip2)) return;
   const double rm = rms ? *rms : 1.0;
   const double inv = rm > 0.0 ? 1.0 / rm : 0.0;
@@ -958,6 +975,7 @@ __global__ void prep_input(const T *r, const double *rms, const float *feat,
 __global__ void combine_out(const float *c, const double *rms, const double *dbar,
                             const unsigned char *mask, double *out, long V,
                             const int *skip, const int *skip2) {
+  chain_wait();
   if (skipped(skip, skip2)) return;
   const double sc = *rms / *dbar;
   for (long v = (long)blockIdx.x * blockDim.x + threadIdx.x; v < V;
@@ -967,6 +985,7 @@ __global__ void combine_out(const float *c, const double *rms, const double *dba
 
 // r = b - r (r holds A x_k).
 __global__ void residual_inplace(const double *b, double *r, long V) {
+  chain_wait();
   for (long v = (long)blockIdx.x * blockDim.x + threadIdx.x; v < V;
        v += (long)gridDim.x * blockDim.x)
     r[v] = b[v] - r[v];
@@ -978,6 +997,7 @@ __global__ void make_pair(const double *r, const double *xs, const double *xk,
                           const double *dinv, const unsigned char *mask,
                           const double *rms, const double *dbar, float *rhat,
                           float *tg, long V) {
+  chain_wait();
   const double rm = *rms;
   const double inv = rm > 0.0 ? 1.0 / rm : 0.0;
   for (long v = (long)blockIdx.x * blockDim.x + threadIdx.x; v < V;
@@ -992,6 +1012,7 @@ __global__ void make_pair(const double *r, const double *xs, const double *xk,
 __global__ void res_z(const float *rhat, const float *c, const double *dinv,
                       const unsigned char *mask, const double *dbar, double *z,
                       long V) {
+  chain_wait();
   const double inv = 1.0 / *dbar;
   for (long v = (long)blockIdx.x * blockDim.x + threadIdx.x; v < V;
        v += (long)gridDim.x * blockDim.x)
@@ -1005,6 +1026,7 @@ __global__ void __launch_bounds__(256) res_rho(const float *rhat, const double *
                                                const unsigned char *mask, double *rho,
                                                long V, double *partials,
                                                unsigned *ticket, double *out) {
+  chain_wait();
   double a0 = 0.0, a1 = 0.0;
   for (long v = (long)blockIdx.x * blockDim.x + threadIdx.x; v < V;
        v += (long)gridDim.x * blockDim.x) {
@@ -1023,6 +1045,7 @@ __global__ void __launch_bounds__(256) res_rho(const float *rhat, const double *
 // dL/dc = -2 (A^T rho) / (dbar ||rhat||^2) on free nodes (g holds A^T rho).
 __global__ void res_dc(const double *g, const unsigned char *mask, const double *dbar,
                        const double *rr, float *dc, long V) {
+  chain_wait();
   const double sc = *rr > 0.0 ? -2.0 / (*dbar * *rr) : 0.0;
   for (long v = (long)blockIdx.x * blockDim.x + threadIdx.x; v < V;
        v += (long)gridDim.x * blockDim.x)
@@ -1034,6 +1057,7 @@ __global__ void res_dc(const double *g, const unsigned char *mask, const double 
 __global__ void __launch_bounds__(256) head_bwd_dc(const bf16 *u0, const float *wh,
                                                    const float *dc, float *gu0,
                                                    float *dwh, long V) {
+  chain_wait();
   float lw[17];
 #pragma unroll
   for (int k = 0; k < 17; k++) lw[k] = 0.f;
@@ -1067,6 +1091,7 @@ __global__ void __launch_bounds__(256) head_bwd_dc(const bf16 *u0, const float *
 __global__ void smooth_out(const double *in, const double *ax, const double *dinv,
                            const unsigned char *mask, double omega, double *out,
                            long V, const int *skip, const int *skip2) {
+  chain_wait();
   if (skipped(skip, skip2)) return;
   for (long v = (long)blockIdx.x * blockDim.x + threadIdx.x; v < V;
        v += (long)gridDim.x * blockDim.x)
@@ -1076,6 +1101,7 @@ __global__ void smooth_out(const double *in, const double *ax, const double *din
 // Jacobi part of the preconditioner (used by the standalone apply).
 __global__ void jacobi_out(const double *in, const double *dinv,
                            const unsigned char *mask, double *out, long V) {
+  chain_wait();
   for (long v = (long)blockIdx.x * blockDim.x + threadIdx.x; v < V;
        v += (long)gridDim.x * blockDim.x)
     out[v] = mask[v] ? 0.0 : in[v] * dinv[v];
@@ -1159,7 +1185,8 @@ cudaError_t conv_launch(const ConvArgs &a, cudaStream_t s) {
   const long nseg = (long)a.H * a.D * ((a.W + 15) / 16);
   const long groups = (nseg + MS - 1) / MS;
   const long blocks = std::min<long>((groups + 3) / 4, (long)device_sm_count() * 16);
-  conv3_kernel<CIN1, CIN2, COUT, MS, F32IN, F32OUT><<<(unsigned)blocks, 128, 0, s>>>(a);
+  chain_launch(conv3_kernel<CIN1, CIN2, COUT, MS, F32IN, F32OUT>, (unsigned)blocks, 128, 0, s,
+               a);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -1179,8 +1206,8 @@ cudaError_t wgrad_launch(const Net &n, WgArgs a, const float *dy, const bf16 *y,
   // (scratch sized for the largest layer)
   a.Wp = (a.W + 15) & ~15;
   a.Vp = (long)a.H * a.D * a.Wp;
-  mask_transpose<COUT><<<(unsigned)((long)a.H * a.D), 128, 0, s>>>(
-      dy, y, n.dyt, tc_mode(n) ? n.dyc : nullptr, a.W, a.Wp, a.Vp);
+  chain_launch(mask_transpose<COUT>, (unsigned)((long)a.H * a.D), 128, 0, s, dy, y, n.dyt,
+               tc_mode(n) ? n.dyc : nullptr, a.W, a.Wp, a.Vp);
   a.dyt = n.dyt;
   const long nks = (long)a.H * a.D * (a.Wp / 16);  // 16-voxel x-row segments
   const long target = std::max<long>(1, (long)device_sm_count() * 8 / (9 * NGROUPS));
@@ -1188,7 +1215,8 @@ cudaError_t wgrad_launch(const Net &n, WgArgs a, const float *dy, const bf16 *y,
   chunk = std::max<long>(16, ((chunk + 3) / 4) * 4);
   a.chunk = chunk;
   const long nchunk = (nks + chunk - 1) / chunk;
-  conv3_wgrad_tc<CIN1, CIN2, COUT, NG><<<dim3((unsigned)nchunk, 9, NGROUPS), 128, 0, s>>>(a);
+  chain_launch(conv3_wgrad_tc<CIN1, CIN2, COUT, NG>, dim3((unsigned)nchunk, 9, NGROUPS), 128, 0,
+               s, a);
   count_launches(2);
   return cudaGetLastError();
 }
@@ -1332,7 +1360,7 @@ cudaError_t conv_tc_run(const Net &n, int l, const CUtensorMap &m1, const CUtens
   a.ntiles = a.tiles_x * a.tiles_y * ((d.D + Sh::G - 1) / Sh::G);
   a.err = n.tc_err;
   const int grid = std::min(a.ntiles, device_sm_count());
-  kern<<<grid, convtc::THREADS, Sh::SMEM, s>>>(m1, m2, a);
+  chain_launch(kern, grid, convtc::THREADS, Sh::SMEM, s, m1, m2, a);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -1374,24 +1402,26 @@ cudaError_t net_forward_tc(Net &n, const int *sk, const int *sk2, cudaStream_t s
   if ((e = conv_tc_launch<16, 0, 16>(n, L_E0A, n.a0, sk, sk2, s)) ||
       (e = conv_tc_launch<16, 0, 16>(n, L_E0B, n.s0, sk, sk2, s)))
     return e;
-  pool_fwd<<<grid_for(f1.V * 2, 256), 256, 0, s>>>(n.s0, n.p0, f0, f1, 16, sk, sk2);
+  chain_launch(pool_fwd, grid_for(f1.V * 2, 256), 256, 0, s, n.s0, n.p0, f0, f1, 16, sk, sk2);
   if ((e = conv_tc_launch<16, 0, 32>(n, L_E1A, n.a1, sk, sk2, s)) ||
       (e = conv_tc_launch<32, 0, 32>(n, L_E1B, n.s1, sk, sk2, s)))
     return e;
-  pool_fwd<<<grid_for(f2.V * 4, 256), 256, 0, s>>>(n.s1, n.p1, f1, f2, 32, sk, sk2);
+  chain_launch(pool_fwd, grid_for(f2.V * 4, 256), 256, 0, s, n.s1, n.p1, f1, f2, 32, sk, sk2);
   if ((e = conv_tc_launch<32, 0, 64>(n, L_BTA, n.a2, sk, sk2, s)) ||
       (e = conv_tc_launch<64, 0, 64>(n, L_BTB, n.b2, sk, sk2, s)))
     return e;
-  upsample_bf16<<<grid_for(f2.V * 8, 256), 256, 0, s>>>(n.b2, n.up1, f1, f2, 64, sk, sk2);
+  chain_launch(upsample_bf16, grid_for(f2.V * 8, 256), 256, 0, s, n.b2, n.up1, f1, f2, 64, sk,
+               sk2);
   if ((e = conv_tc_launch<32, 64, 32>(n, L_D1A, n.a3, sk, sk2, s)) ||
       (e = conv_tc_launch<32, 0, 32>(n, L_D1B, n.u1, sk, sk2, s)))
     return e;
-  upsample_bf16<<<grid_for(f1.V * 4, 256), 256, 0, s>>>(n.u1, n.up0, f0, f1, 32, sk, sk2);
+  chain_launch(upsample_bf16, grid_for(f1.V * 4, 256), 256, 0, s, n.u1, n.up0, f0, f1, 32, sk,
+               sk2);
   if ((e = conv_tc_launch<16, 32, 16>(n, L_D0A, n.a4, sk, sk2, s)) ||
       (e = conv_tc_launch<16, 0, 16>(n, L_D0B, n.u0, sk, sk2, s)))
     return e;
-  head_fwd<<<grid_for(f0.V, 256), 256, 0, s>>>(n.u0, n.theta + n.woff[L_HEAD], out, f0.V,
-                                                sk, sk2);
+  chain_launch(head_fwd, grid_for(f0.V, 256), 256, 0, s, n.u0, n.theta + n.woff[L_HEAD], out,
+               f0.V, sk, sk2);
   count_launches(5);
   return cudaGetLastError();
 }
@@ -1408,10 +1438,12 @@ cudaError_t net_forward(Net &n, const int *sk, const int *sk2, cudaStream_t s, f
     return e;
   VDR_CONV(16, 0, 16, 0, n.x0, nullptr, L_E0A, n.a0)
   VDR_CONV(16, 0, 16, 0, n.a0, nullptr, L_E0B, n.s0)
-  pool_fwd<<<grid_for(n.d[1].V * 2, 256), 256, 0, s>>>(n.s0, n.p0, n.d[0], n.d[1], 16, sk, sk2);
+  chain_launch(pool_fwd, grid_for(n.d[1].V * 2, 256), 256, 0, s, n.s0, n.p0, n.d[0], n.d[1], 16,
+               sk, sk2);
   VDR_CONV(16, 0, 32, 1, n.p0, nullptr, L_E1A, n.a1)
   VDR_CONV(32, 0, 32, 1, n.a1, nullptr, L_E1B, n.s1)
-  pool_fwd<<<grid_for(n.d[2].V * 4, 256), 256, 0, s>>>(n.s1, n.p1, n.d[1], n.d[2], 32, sk, sk2);
+  chain_launch(pool_fwd, grid_for(n.d[2].V * 4, 256), 256, 0, s, n.s1, n.p1, n.d[1], n.d[2], 32,
+               sk, sk2);
   VDR_CONV(32, 0, 64, 2, n.p1, nullptr, L_BTA, n.a2)
   VDR_CONV(64, 0, 64, 2, n.a2, nullptr, L_BTB, n.b2)
   VDR_CONV(32, 64, 32, 1, n.s1, n.b2, L_D1A, n.a3)
@@ -1419,8 +1451,8 @@ cudaError_t net_forward(Net &n, const int *sk, const int *sk2, cudaStream_t s, f
   VDR_CONV(16, 32, 16, 0, n.s0, n.u1, L_D0A, n.a4)
   VDR_CONV(16, 0, 16, 0, n.a4, nullptr, L_D0B, n.u0)
 #undef VDR_CONV
-  head_fwd<<<grid_for(n.d[0].V, 256), 256, 0, s>>>(n.u0, n.theta + n.woff[L_HEAD],
-                                                   out, n.d[0].V, sk, sk2);
+  chain_launch(head_fwd, grid_for(n.d[0].V, 256), 256, 0, s, n.u0, n.theta + n.woff[L_HEAD],
+               out, n.d[0].V, sk, sk2);
   count_launches(3);
   return cudaGetLastError();
 }
@@ -1437,8 +1469,10 @@ cudaError_t net_backward(Net &n, cudaStream_t s) {
   // d0a: a4 = relu(conv([s0 | up(u1)]))
   if ((e = wgrad_launch<16, 32, 16>(n, wg_args(n, L_D0A, n.s0, n.u1), n.g_a4, n.a4, s))) return e;
   if ((e = bwd_data<16, 48>(n, L_D0A, n.g_a4, n.a4, n.g_cat0, s))) return e;
-  upcat_bwd_skip<<<grid_for(f0.V * 4, 256), 256, 0, s>>>(n.g_cat0, n.g_s0, f0.V, 16, 32);
-  upcat_bwd_coarse<<<grid_for(f1.V * 8, 256), 256, 0, s>>>(n.g_cat0, n.g_u1, f0, f1, 16, 32);
+  chain_launch(upcat_bwd_skip, grid_for(f0.V * 4, 256), 256, 0, s, n.g_cat0, n.g_s0, f0.V, 16,
+               32);
+  chain_launch(upcat_bwd_coarse, grid_for(f1.V * 8, 256), 256, 0, s, n.g_cat0, n.g_u1, f0, f1,
+               16, 32);
   count_launches(2);
   // d1b: u1 = relu(conv(a3))
   if ((e = wgrad_launch<32, 0, 32>(n, wg_args(n, L_D1B, n.a3, nullptr), n.g_u1, n.u1, s))) return e;
@@ -1446,8 +1480,10 @@ cudaError_t net_backward(Net &n, cudaStream_t s) {
   // d1a: a3 = relu(conv([s1 | up(b2)]))
   if ((e = wgrad_launch<32, 64, 32>(n, wg_args(n, L_D1A, n.s1, n.b2), n.g_a3, n.a3, s))) return e;
   if ((e = bwd_data<32, 96>(n, L_D1A, n.g_a3, n.a3, n.g_cat1, s))) return e;
-  upcat_bwd_skip<<<grid_for(f1.V * 8, 256), 256, 0, s>>>(n.g_cat1, n.g_s1, f1.V, 32, 64);
-  upcat_bwd_coarse<<<grid_for(f2.V * 16, 256), 256, 0, s>>>(n.g_cat1, n.g_b2, f1, f2, 32, 64);
+  chain_launch(upcat_bwd_skip, grid_for(f1.V * 8, 256), 256, 0, s, n.g_cat1, n.g_s1, f1.V, 32,
+               64);
+  chain_launch(upcat_bwd_coarse, grid_for(f2.V * 16, 256), 256, 0, s, n.g_cat1, n.g_b2, f1, f2,
+               32, 64);
   count_launches(2);
   // btb: b2 = relu(conv(a2))
   if ((e = wgrad_launch<64, 0, 64>(n, wg_args(n, L_BTB, n.a2, nullptr), n.g_b2, n.b2, s))) return e;
@@ -1455,7 +1491,7 @@ cudaError_t net_backward(Net &n, cudaStream_t s) {
   // bta: a2 = relu(conv(p1))
   if ((e = wgrad_launch<32, 0, 64>(n, wg_args(n, L_BTA, n.p1, nullptr), n.g_a2, n.a2, s))) return e;
   if ((e = bwd_data<64, 32>(n, L_BTA, n.g_a2, n.a2, n.g_p1, s))) return e;
-  pool_bwd_add<<<grid_for(f1.V * 8, 256), 256, 0, s>>>(n.g_p1, n.g_s1, f1, f2, 32);
+  chain_launch(pool_bwd_add, grid_for(f1.V * 8, 256), 256, 0, s, n.g_p1, n.g_s1, f1, f2, 32);
   count_launches(1);
   // e1b: s1 = relu(conv(a1))
   if ((e = wgrad_launch<32, 0, 32>(n, wg_args(n, L_E1B, n.a1, nullptr), n.g_s1, n.s1, s))) return e;
@@ -1463,7 +1499,7 @@ cudaError_t net_backward(Net &n, cudaStream_t s) {
   // e1a: a1 = relu(conv(p0))
   if ((e = wgrad_launch<16, 0, 32>(n, wg_args(n, L_E1A, n.p0, nullptr), n.g_a1, n.a1, s))) return e;
   if ((e = bwd_data<32, 16>(n, L_E1A, n.g_a1, n.a1, n.g_p0, s))) return e;
-  pool_bwd_add<<<grid_for(f0.V * 4, 256), 256, 0, s>>>(n.g_p0, n.g_s0, f0, f1, 16);
+  chain_launch(pool_bwd_add, grid_for(f0.V * 4, 256), 256, 0, s, n.g_p0, n.g_s0, f0, f1, 16);
   count_launches(1);
   // e0b: s0 = relu(conv(a0))
   if ((e = wgrad_launch<16, 0, 16>(n, wg_args(n, L_E0B, n.a0, nullptr), n.g_s0, n.s0, s))) return e;
@@ -1476,11 +1512,10 @@ cudaError_t net_backward(Net &n, cudaStream_t s) {
 cudaError_t pack_all(Net &n, cudaStream_t s) {
   for (int l = 0; l < L_HEAD; l++) {
     const int cin = DEFS[l].cin1 + DEFS[l].cin2, cout = DEFS[l].cout;
-    pack_weights<<<grid_for(layer_wsize(l), 256), 256, 0, s>>>(
-        n.theta + n.woff[l], n.wb + n.woff[l], n.wbt + n.woff[l], n.wtc + n.woff[l],
-        n.wtcb + n.woff[l], cin, cout,
-        convtc::weights_resident(DEFS[l].cin1, DEFS[l].cin2, cout),
-        convtc::weights_resident(cout, 0, cin));
+    chain_launch(pack_weights, grid_for(layer_wsize(l), 256), 256, 0, s, n.theta + n.woff[l],
+                 n.wb + n.woff[l], n.wbt + n.woff[l], n.wtc + n.woff[l], n.wtcb + n.woff[l],
+                 cin, cout, convtc::weights_resident(DEFS[l].cin1, DEFS[l].cin2, cout),
+                 convtc::weights_resident(cout, 0, cin));
   }
   count_launches(L_HEAD);
   return cudaGetLastError();
@@ -1490,17 +1525,16 @@ cudaError_t pack_all(Net &n, cudaStream_t s) {
 cudaError_t net_loss_grad(Net &n, const float *rhat, const float *tg, cudaStream_t s) {
   cudaError_t e;
   const long V = n.d[0].V;
-  prep_input<float><<<grid_for(V, 256), 256, 0, s>>>(rhat, nullptr, n.feat, n.x0, V,
-                                                       nullptr, nullptr);
+  chain_launch(prep_input<float>, grid_for(V, 256), 256, 0, s, rhat, nullptr, n.feat, n.x0, V,
+               nullptr, nullptr);
   count_launches(1);
   if ((e = net_forward(n, nullptr, nullptr, s, n.c))) return e;
   if ((e = cudaMemsetAsync(n.grad, 0, sizeof(float) * n.nparam, s))) return e;
   if ((e = cudaMemsetAsync(n.scal + 1, 0, sizeof(double), s))) return e;
-  free_sum<2, float><<<n.red_grid, 256, 0, s>>>(tg, n.h->mask, V, n.partials, n.ticket,
-                                                n.scal + 3, nullptr, nullptr);
-  head_bwd<<<grid_for(V, 256, 4), 256, 0, s>>>(n.u0, n.theta + n.woff[L_HEAD], n.c, tg,
-                                               n.h->mask, n.scal + 3, n.g_u0,
-                                               n.grad + n.woff[L_HEAD], n.scal + 1, V);
+  chain_launch(free_sum<2, float>, n.red_grid, 256, 0, s, tg,
+               n.h->mask, V, n.partials, n.ticket, n.scal + 3, nullptr, nullptr);
+  chain_launch(head_bwd, grid_for(V, 256, 4), 256, 0, s, n.u0, n.theta + n.woff[L_HEAD], n.c,
+               tg, n.h->mask, n.scal + 3, n.g_u0, n.grad + n.woff[L_HEAD], n.scal + 1, V);
   count_launches(2);
   return net_backward(n, s);
 }
@@ -1512,26 +1546,28 @@ cudaError_t net_residual_loss_grad(Net &n, const float *rhat, cudaStream_t s) {
   cudaError_t e;
   Handle &h = *n.h;
   const long V = n.d[0].V;
-  prep_input<float><<<grid_for(V, 256), 256, 0, s>>>(rhat, nullptr, n.feat, n.x0, V,
-                                                       nullptr, nullptr);
+  chain_launch(prep_input<float>, grid_for(V, 256), 256, 0, s, rhat, nullptr, n.feat, n.x0, V,
+               nullptr, nullptr);
   count_launches(1);
   if ((e = net_forward(n, nullptr, nullptr, s, n.c))) return e;
-  res_z<<<grid_for(V, 256), 256, 0, s>>>(rhat, n.c, h.dinv, h.mask, n.scal + 2, n.zbuf, V);
+  chain_launch(res_z, grid_for(V, 256), 256, 0, s, rhat, n.c, h.dinv, h.mask, n.scal + 2,
+               n.zbuf, V);
   count_launches(1);
   if ((e = cudaMemsetAsync(n.qbuf, 0, sizeof(double) * V, s)) ||
       (e = launch_apply(h, false, n.zbuf, n.qbuf, nullptr, nullptr, s)))
     return e;
-  res_rho<<<n.red_grid, 256, 0, s>>>(rhat, n.qbuf, h.mask, n.pbuf, V, n.partials,
-                                     n.ticket, n.scal + 4);
+  chain_launch(res_rho, n.red_grid, 256, 0, s, rhat, n.qbuf, h.mask, n.pbuf, V, n.partials,
+               n.ticket, n.scal + 4);
   count_launches(1);
   if ((e = cudaMemsetAsync(n.gbuf, 0, sizeof(double) * V, s)) ||
       (e = launch_apply(h, true, n.pbuf, n.gbuf, nullptr, nullptr, s)))
     return e;
-  res_dc<<<grid_for(V, 256), 256, 0, s>>>(n.gbuf, h.mask, n.scal + 2, n.scal + 5, n.dc, V);
+  chain_launch(res_dc, grid_for(V, 256), 256, 0, s, n.gbuf, h.mask, n.scal + 2, n.scal + 5,
+               n.dc, V);
   count_launches(1);
   if ((e = cudaMemsetAsync(n.grad, 0, sizeof(float) * n.nparam, s))) return e;
-  head_bwd_dc<<<grid_for(V, 256, 4), 256, 0, s>>>(n.u0, n.theta + n.woff[L_HEAD], n.dc,
-                                                  n.g_u0, n.grad + n.woff[L_HEAD], V);
+  chain_launch(head_bwd_dc, grid_for(V, 256, 4), 256, 0, s, n.u0, n.theta + n.woff[L_HEAD],
+               n.dc, n.g_u0, n.grad + n.woff[L_HEAD], V);
   count_launches(1);
   return net_backward(n, s);
 }
@@ -1541,15 +1577,15 @@ cudaError_t net_enqueue(void *ctx, const double *in, double *out, const int *ski
                         const int *skip2, cudaStream_t s) {
   Net &n = *static_cast<Net *>(ctx);
   const long V = n.d[0].V;
-  free_sum<0><<<n.red_grid, 256, 0, s>>>(in, n.h->mask, V, n.partials, n.ticket,
-                                         n.scal, skip, skip2);
-  prep_input<double><<<grid_for(V, 256), 256, 0, s>>>(in, n.scal, n.feat, n.x0, V,
-                                                        skip, skip2);
+  chain_launch(free_sum<0>, n.red_grid, 256, 0, s, in,
+               n.h->mask, V, n.partials, n.ticket, n.scal, skip, skip2);
+  chain_launch(prep_input<double>, grid_for(V, 256), 256, 0, s, in, n.scal, n.feat, n.x0, V,
+               skip, skip2);
   count_launches(2);
   cudaError_t e = net_forward(n, skip, skip2, s, n.c);
   if (e) return e;
-  combine_out<<<grid_for(V, 256), 256, 0, s>>>(n.c, n.scal, n.scal + 2, n.h->mask,
-                                               out, V, skip, skip2);
+  chain_launch(combine_out, grid_for(V, 256), 256, 0, s, n.c, n.scal, n.scal + 2,
+               n.h->mask, out, V, skip, skip2);
   count_launches(1);
   // The network's output is accurate at long wavelengths only (BF16
   // activations leave noise that A amplifies); Jacobi steps remove the
@@ -1558,8 +1594,8 @@ cudaError_t net_enqueue(void *ctx, const double *in, double *out, const int *ski
     if ((e = cudaMemsetAsync(n.rbuf, 0, sizeof(double) * V, s)) ||
         (e = launch_apply(*n.h, false, out, n.rbuf, skip, skip2, s)))
       return e;
-    smooth_out<<<grid_for(V, 256), 256, 0, s>>>(in, n.rbuf, n.h->dinv, n.h->mask,
-                                                n.smooth_omega, out, V, skip, skip2);
+    chain_launch(smooth_out, grid_for(V, 256), 256, 0, s, in, n.rbuf,
+                 n.h->dinv, n.h->mask, n.smooth_omega, out, V, skip, skip2);
     count_launches(1);
   }
   return cudaGetLastError();
@@ -1793,10 +1829,11 @@ extern "C" int vdr_net_update_features(vdr_net *N, float *d_feat_out, double *db
   const long V = n.d[0].V;
   cudaError_t e;
   if ((e = cudaMemsetAsync(n.facc, 0, sizeof(float) * V * 5, s))) return cuda_fail(e, "memset");
-  node_feature_acc<<<grid_for(8L * h.E, 256), 256, 0, s>>>(h.conn, h.vel, h.lam, h.E, n.facc);
-  node_feature_fin<<<grid_for(V, 256), 256, 0, s>>>(n.facc, n.feat, V);
-  free_sum<1><<<n.red_grid, 256, 0, s>>>(h.diag, h.mask, V, n.partials, n.ticket,
-                                         n.scal + 2, nullptr, nullptr);
+  chain_launch(node_feature_acc, grid_for(8L * h.E, 256), 256, 0, s, h.conn, h.vel, h.lam, h.E,
+               n.facc);
+  chain_launch(node_feature_fin, grid_for(V, 256), 256, 0, s, n.facc, n.feat, V);
+  chain_launch(free_sum<1>, n.red_grid, 256, 0, s, h.diag, h.mask, V, n.partials, n.ticket,
+               n.scal + 2, nullptr, nullptr);
   count_launches(3);
   if ((e = cudaGetLastError())) return cuda_fail(e, "features");
   if (d_feat_out &&
@@ -1849,11 +1886,11 @@ extern "C" int vdr_net_make_pair_device(vdr_net *N, const double *d_b,
   if ((e = cudaMemsetAsync(n.rbuf, 0, sizeof(double) * V, s)) ||
       (e = launch_apply(h, false, d_xk, n.rbuf, nullptr, nullptr, s)))
     return cuda_fail(e, "pair residual");
-  residual_inplace<<<grid_for(V, 256), 256, 0, s>>>(d_b, n.rbuf, V);
-  free_sum<0><<<n.red_grid, 256, 0, s>>>(n.rbuf, h.mask, V, n.partials, n.ticket, n.scal,
-                                         nullptr, nullptr);
-  make_pair<<<grid_for(V, 256), 256, 0, s>>>(n.rbuf, d_xstar, d_xk, h.dinv, h.mask, n.scal,
-                                             n.scal + 2, d_rhat, d_target, V);
+  chain_launch(residual_inplace, grid_for(V, 256), 256, 0, s, d_b, n.rbuf, V);
+  chain_launch(free_sum<0>, n.red_grid, 256, 0, s, n.rbuf, h.mask, V, n.partials, n.ticket,
+               n.scal, nullptr, nullptr);
+  chain_launch(make_pair, grid_for(V, 256), 256, 0, s, n.rbuf, d_xstar, d_xk, h.dinv, h.mask,
+               n.scal, n.scal + 2, d_rhat, d_target, V);
   count_launches(3);
   e = cudaGetLastError();
   return e ? cuda_fail(e, "pair") : VDR_OK;
@@ -1869,8 +1906,8 @@ extern "C" int vdr_net_forward_device(vdr_net *N, const float *d_rhat, float *d_
   }
   const long V = n.d[0].V;
   cudaStream_t s = n.h->stream;
-  prep_input<float><<<grid_for(V, 256), 256, 0, s>>>(d_rhat, nullptr, n.feat, n.x0, V,
-                                                       nullptr, nullptr);
+  chain_launch(prep_input<float>, grid_for(V, 256), 256, 0, s, d_rhat, nullptr, n.feat, n.x0, V,
+               nullptr, nullptr);
   count_launches(1);
   const cudaError_t e = net_forward(n, nullptr, nullptr, s, d_out);
   return e ? cuda_fail(e, "network forward") : VDR_OK;
@@ -1936,8 +1973,8 @@ extern "C" int vdr_net_adam_step(vdr_net *N, float lr, float beta1, float beta2,
   n.adam_t += 1;
   const float bc1 = 1.f - powf(beta1, (float)n.adam_t);
   const float bc2 = 1.f - powf(beta2, (float)n.adam_t);
-  adam_kernel<<<grid_for(n.nparam, 256), 256, 0, s>>>(n.theta, n.grad, n.am, n.av, n.nparam,
-                                                      lr, beta1, beta2, eps, bc1, bc2);
+  chain_launch(adam_kernel, grid_for(n.nparam, 256), 256, 0, s, n.theta, n.grad, n.am, n.av,
+               n.nparam, lr, beta1, beta2, eps, bc1, bc2);
   count_launches(1);
   cudaError_t e = cudaGetLastError();
   if (!e) e = pack_all(n, s);
@@ -1983,7 +2020,8 @@ extern "C" int vdr_net_precondition_device(vdr_net *N, const double *d_in, doubl
     return VDR_BAD_ARGUMENT;
   }
   if ((st = prepare_operator(h))) return st;
-  jacobi_out<<<grid_for(h.N, 256), 256, 0, h.stream>>>(d_in, h.dinv, h.mask, d_out, h.N);
+  chain_launch(jacobi_out, grid_for(h.N, 256), 256, 0, h.stream, d_in, h.dinv, h.mask, d_out,
+               h.N);
   count_launches(1);
   cudaError_t e = net_enqueue(&n, d_in, d_out, nullptr, nullptr, h.stream);
   return e ? cuda_fail(e, "precondition") : VDR_OK;
