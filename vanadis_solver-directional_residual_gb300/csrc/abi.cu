@@ -25,8 +25,6 @@ struct vdr_handle {
   double *io = nullptr;  // [3][N]: x, y / b, scratch
   double *mass_partials = nullptr;
   double *mass_out = nullptr;
-  double *step_masses = nullptr;  // one per step of a time loop
-  int step_masses_n = 0;
 };
 
 namespace vdr {
@@ -1220,16 +1218,13 @@ int vdr_time_steps(vdr_handle *H, int nsteps, double cf, double rM,
   double *b = H->io + (size_t)h.N;
   double *dmass = nullptr;
   if (masses && nsteps > 0) {
-    if (H->step_masses_n < nsteps) {
-      dfree(H->step_masses);
-      H->step_masses = nullptr;
-      H->step_masses_n = 0;
-      if ((e = dalloc(&H->step_masses, nsteps))) return cuda_fail(e, "vdr_time_steps: alloc");
-      H->step_masses_n = nsteps;
-    }
-    dmass = H->step_masses;
+    if ((e = cudaMalloc(&dmass, sizeof(double) * nsteps)))
+      return cuda_fail(e, "vdr_time_steps: alloc");
   }
-  if ((e = dalloc(&H->mass_partials, 8192))) return cuda_fail(e, "alloc");
+  if ((e = dalloc(&H->mass_partials, 8192))) {
+    if (dmass) cudaFree(dmass);
+    return cuda_fail(e, "alloc");
+  }
   const int method = h.opt.solver == VDR_SOLVER_BICG ? VDR_SOLVER_BICG
                                                      : VDR_SOLVER_BICGSTAB;
   // With the stored operator the first step keeps M and F; every later step
@@ -1238,15 +1233,18 @@ int vdr_time_steps(vdr_handle *H, int nsteps, double cf, double rM,
   const bool keep_mass = h.apply_mode == VDR_APPLY_STORED && h.aH != 0.0;
   if (keep_mass &&
       ((e = dalloc(&h.Mhi, (size_t)h.E * 16)) || (e = dalloc(&h.Mlo, (size_t)h.E * 16)) ||
-       (e = dalloc(&h.Fvec, h.N)) || (e = dalloc(&h.rhs_tmp, 2 * (size_t)h.N))))
+       (e = dalloc(&h.Fvec, h.N)) || (e = dalloc(&h.rhs_tmp, 2 * (size_t)h.N)))) {
+    if (dmass) cudaFree(dmass);
     return cuda_fail(e, "vdr_time_steps: alloc");
+  }
   int status = VDR_OK, done = 0;
-  // A step's mass and the next one's right-hand side follow its solve on the
-  // stream without the host's word; after a solve that failed the latter is
-  // not used (20 us of a 400 us step at 2,800 nodes).
-  bool rhs_queued = false;
   for (int k = 0; k < nsteps; k++) {
-    if (!rhs_queued) {
+    if (k > 0 && keep_mass && h.mass_valid && h.op64_valid) {
+      if ((e = launch_rhs_from_mass(h, cf, rM, t, b, h.stream))) {
+        status = cuda_fail(e, "rhs");
+        break;
+      }
+    } else {
       BuildArgs rhs;
       rhs.cf = cf;
       rhs.rM = rM;
@@ -1262,29 +1260,14 @@ int vdr_time_steps(vdr_handle *H, int nsteps, double cf, double rM,
         break;
       }
     }
-    rhs_queued = false;
-    const auto behind = [&]() {
-      cudaError_t q = cudaSuccess;
-      if (dmass) q = launch_mass(h, t, H->mass_partials, dmass + k, h.stream);
-      if (!q && k + 1 < nsteps && keep_mass && h.mass_valid && h.op64_valid) {
-        q = launch_rhs_from_mass(h, cf, rM, t, b, h.stream);
-        rhs_queued = true;
-      }
-      return q;
-    };
     int it = 0;
     double err = 0.0;
-    if (h.opt.precision != VDR_PRECISION_MIXED) h.behind = std::ref(behind);
-    const bool taken = (bool)h.behind;
     st = solve_by_option(h, method, b, t, tol, itmax, &it, &err);
     if (iters) iters[k] = it;
     if (errs) errs[k] = err;
-    if (!taken || h.behind) {
-      h.behind = nullptr;
-      if ((e = behind())) {
-        status = cuda_fail(e, "mass and right-hand side");
-        break;
-      }
+    if (dmass && (e = launch_mass(h, t, H->mass_partials, dmass + k, h.stream))) {
+      status = cuda_fail(e, "mass");
+      break;
     }
     if (st != VDR_OK) {
       status = st;
@@ -1296,6 +1279,7 @@ int vdr_time_steps(vdr_handle *H, int nsteps, double cf, double rM,
     e = cudaMemcpyAsync(masses, dmass, sizeof(double) * nsteps,
                         cudaMemcpyDeviceToHost, h.stream);
     if (!e) e = cudaStreamSynchronize(h.stream);
+    cudaFree(dmass);
     if (e && status == VDR_OK) status = cuda_fail(e, "masses");
   }
   if (steps_done) *steps_done = done;
@@ -1367,7 +1351,6 @@ int vdr_destroy(vdr_handle *H) {
   dfree(H->io);
   dfree(H->mass_partials);
   dfree(H->mass_out);
-  dfree(H->step_masses);
   free_handle(H->h);
   delete H;
   return VDR_OK;

@@ -795,13 +795,9 @@ int solve_device(Handle &h, int method, const double *b, double *x,
 
   if (!prec && !hist && resident_fits(h)) {
     if (!(e = launch_resident(h, method, b, x, tol, itmax, stall_window))) {
-      e = cudaMemcpyAsync(&h.h_st[0], h.st, sizeof(KState), cudaMemcpyDeviceToHost, s);
-      if (!e) e = cudaEventRecord(h.ev[0], s);
-      if (!e && h.behind) {
-        e = h.behind();
-        h.behind = nullptr;
-      }
-      if (e || (e = cudaEventSynchronize(h.ev[0]))) return cuda_fail(e, "solve");
+      if ((e = cudaMemcpyAsync(&h.h_st[0], h.st, sizeof(KState), cudaMemcpyDeviceToHost, s)) ||
+          (e = cudaStreamSynchronize(s)))
+        return cuda_fail(e, "solve");
       const KState &fin = h.h_st[0];
       const int status = fin.done ? fin.status : VDR_NOT_CONVERGED;
       h.last.iterations = fin.iter;

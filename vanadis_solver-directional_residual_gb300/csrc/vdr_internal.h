@@ -1,7 +1,6 @@
 // vdr_internal.h -- host-side internals shared by the translation units of
 // libvdr.so.  Not installed; the public surface is include/vdr.h.
 #pragma once
-#include <functional>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -235,9 +234,6 @@ struct Handle {
   int st_nax = 0, st_pl = 0;    // the strides that st_x's pads are zero for
   int st_state = 0, st_applies = 0;
   bool own_capture = false;
-  // Work that a time loop wants enqueued behind a solve before the host waits
-  // for its outcome (taken by the solves that are one launch).
-  std::function<cudaError_t()> behind;
   // its binary16 rows for the mixed solve (half_rows.cu): 27 half planes, a
   // scale per row, FP32 vectors; hr_state as st_state, 2 = out of range
   void *hr_H = nullptr;
