@@ -35,7 +35,6 @@
 #include <cstring>
 #include <vector>
 
-#include "chain.cuh"
 #include "reduce.cuh"
 #include "stencil.cuh"
 #include "vdr_internal.h"
@@ -376,7 +375,6 @@ __global__ void __launch_bounds__(512, 2) sgr_w(SegVec a) {
 
 template <bool KEEP>
 __global__ void __launch_bounds__(512, 2) sgr_v(SegVec a) {
-  chain_wait();
   if (*a.s.done) return;
   const int tile = blockIdx.x;
   const SegTile tl = a.tiles[tile];
@@ -409,7 +407,6 @@ __global__ void __launch_bounds__(512, 2) sgr_v(SegVec a) {
 
 template <bool KEEP>
 __global__ void __launch_bounds__(512, 2) sgr_t(SegVec a) {
-  chain_wait();
   if (*a.s.done) return;
   const int tile = blockIdx.x;
   const SegTile tl = a.tiles[tile];
@@ -441,7 +438,6 @@ __global__ void __launch_bounds__(512, 2) sgr_t(SegVec a) {
 }
 
 __global__ void __launch_bounds__(512, 2) sgr_p(SegVec a) {
-  chain_wait();
   if (*a.s.done) return;
   const int tile = blockIdx.x;
   const SegTile tl = a.tiles[tile];
@@ -848,11 +844,13 @@ int solve_segmented_device(Handle &h, const double *b, double *x, double tol, in
     const long long before = launches_so_far();
     for (int k = 0; k < K && !e; k++) {
       if (rows) {
-        if ((e = chain_launch(keep ? sgr_v<true> : sgr_v<false>, nt, th, 0, s, a)) ||
-            (e = chain_launch(keep ? sgr_t<true> : sgr_t<false>, nt, th, 0, s, a)))
-          break;
-        e = chain_launch(sgr_p, nt, th, 0, s, a);
+        if (keep) sgr_v<true><<<nt, th, 0, s>>>(a);
+        else sgr_v<false><<<nt, th, 0, s>>>(a);
+        if (keep) sgr_t<true><<<nt, th, 0, s>>>(a);
+        else sgr_t<false><<<nt, th, 0, s>>>(a);
+        sgr_p<<<nt, th, 0, s>>>(a);
         count_launches(3);
+        e = cudaGetLastError();
         continue;
       }
       sg_p<<<nt, th, 0, s>>>(a);

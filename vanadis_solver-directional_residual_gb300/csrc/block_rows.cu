@@ -29,7 +29,6 @@
 #include <algorithm>
 
 #include "block_cols.cuh"
-#include "chain.cuh"
 #include "stencil.cuh"
 #include "tc_ptx.cuh"
 
@@ -224,7 +223,6 @@ struct Maps {
 template <int K, bool SECOND>
 __global__ void __launch_bounds__(PT, 2) br_apply(const BVec a, const BlockRows g,
                                                   const __grid_constant__ Maps maps) {
-  chain_wait();
   using T = Tile<K>;
   constexpr int NQ = SECOND ? 4 : 1, L = T::L, ST = STAGES;
   extern __shared__ __align__(128) unsigned char stage[];
@@ -401,7 +399,6 @@ __global__ void __launch_bounds__(PT, 2) br_apply(const BVec a, const BlockRows 
 // s = r - alpha v, ||s|| per column.
 template <int K>
 __global__ void __launch_bounds__(BT, 2) br_s(const BVec a) {
-  chain_wait();
   if (a.st->done) return;
   const int k0 = 4 * (threadIdx.x % (K / 4));
   DfAcc d[1][4];
@@ -432,7 +429,6 @@ __global__ void __launch_bounds__(BT, 2) br_s(const BVec a) {
 // Columns that have finished keep x and r.
 template <int K>
 __global__ void __launch_bounds__(BT, 2) br_xp(const BVec a) {
-  chain_wait();
   if (a.st->done) return;
   const int k0 = 4 * (threadIdx.x % (K / 4));
   DfAcc d[1][4];
@@ -955,10 +951,10 @@ cudaError_t block_rows_iterations(const BVec &a, const BlockRows &g, int count, 
   VDR_BY_K((made = make_maps<K>(g, a.p, &mp) && make_maps<K>(g, a.s, &ms)));
   if (!made) return cudaErrorInvalidValue;
   for (int it = 0; it < count; it++) {
-    VDR_BY_K((chain_launch(br_apply<K, false>, g.grid, PT, Tile<K>::PRODUCT, s, a, g, mp)));
-    VDR_BY_K((chain_launch(br_s<K>, grid, BT, 0, s, a)));
-    VDR_BY_K((chain_launch(br_apply<K, true>, g.grid, PT, Tile<K>::PRODUCT, s, a, g, ms)));
-    VDR_BY_K((chain_launch(br_xp<K>, grid, BT, 0, s, a)));
+    VDR_BY_K((br_apply<K, false><<<g.grid, PT, Tile<K>::PRODUCT, s>>>(a, g, mp)));
+    VDR_BY_K((br_s<K><<<grid, BT, 0, s>>>(a)));
+    VDR_BY_K((br_apply<K, true><<<g.grid, PT, Tile<K>::PRODUCT, s>>>(a, g, ms)));
+    VDR_BY_K((br_xp<K><<<grid, BT, 0, s>>>(a)));
   }
   return cudaGetLastError();
 }

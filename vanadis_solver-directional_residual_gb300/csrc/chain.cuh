@@ -1,12 +1,13 @@
-// chain.cuh -- kernels of an iteration that follow one another directly: the
+// chain.cuh -- short kernels that follow one another directly: the
 // next one's blocks are brought up while the last ones of the one before are
 // still running (programmatic dependent launch), instead of after them.
 // Every kernel launched so begins with chain_wait, which returns when the
 // kernel before is complete and what it wrote is visible; nothing is read
-// before it.  At 40 to 50 us a kernel it gives about one per cent (mixed loop at
-// 3.6 M nodes 34.8 -> 34.3 ms, a step at 1.08 M 9.20 -> 8.92, the block solve
-// 84.5 -> 83.5), at 10 us more: the network's training pass (62 launches) 859
-// -> 742 us, its forward pass 452 -> 425.
+// before it.
+// It pays where a kernel takes about 10 us: the network's training pass (62
+// launches) 859 -> 742 us, its forward pass 452 -> 425.  The Krylov iterations'
+// kernels of 30 to 350 us, the block solve's among them, gained 0.3 per cent
+// or lost 0.2, and stay plain.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -18,7 +18,6 @@
 #include <algorithm>
 #include <cstring>
 
-#include "chain.cuh"
 #include "meet.cuh"
 #include "stencil.cuh"
 
@@ -263,7 +262,6 @@ __device__ __forceinline__ void row_pair(const VecH &a, long n, const float *xp,
 
 template <bool KEEP>
 __global__ void __launch_bounds__(HT, 4) hb_v(VecH a) {
-  chain_wait();
   if (a.st->done) return;
   const float al = (float)a.st->alpha;
   DfAcc d[2] = {{0.f, 0.f}, {0.f, 0.f}};
@@ -290,7 +288,6 @@ __global__ void __launch_bounds__(HT, 4) hb_v(VecH a) {
 
 template <bool KEEP>
 __global__ void __launch_bounds__(HT, 4) hb_t(VecH a) {
-  chain_wait();
   if (a.st->done || a.st->sconv) return;
   DfAcc d[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
   PAIRS_OF(a) {
@@ -321,7 +318,6 @@ __global__ void __launch_bounds__(HT, 4) hb_t(VecH a) {
 }
 
 __global__ void __launch_bounds__(HT) hb_p(VecH a) {
-  chain_wait();
   KState *st = a.st;
   if (st->done) return;
   const float al = (float)st->alpha;
@@ -774,10 +770,17 @@ int solve_half_rows(Handle &h, const double *res, double rnorm, double *x, doubl
     cudaGraph_t graph;
     if ((e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal)))
       return cuda_fail(e, "begin capture");
-    for (int k = 0; k < K && !e; k++)
-      if (!(e = chain_launch(keep ? hb_v<true> : hb_v<false>, g, HT, 0, s, a)) &&
-          !(e = chain_launch(keep ? hb_t<true> : hb_t<false>, g, HT, 0, s, a)))
-        e = chain_launch(hb_p, g, HT, 0, s, a);
+    for (int k = 0; k < K; k++) {
+      if (keep) {
+        hb_v<true><<<g, HT, 0, s>>>(a);
+        hb_t<true><<<g, HT, 0, s>>>(a);
+      } else {
+        hb_v<false><<<g, HT, 0, s>>>(a);
+        hb_t<false><<<g, HT, 0, s>>>(a);
+      }
+      hb_p<<<g, HT, 0, s>>>(a);
+    }
+    e = cudaGetLastError();
     const cudaError_t e2 = cudaStreamEndCapture(s, &graph);
     if (e || e2) return cuda_fail(e ? e : e2, "capture");
     e = cudaGraphInstantiate(&h.hr_graph, graph, 0);

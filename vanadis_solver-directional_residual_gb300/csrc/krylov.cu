@@ -26,7 +26,6 @@
 
 #include "dfloat.cuh"
 #include "reduce.cuh"
-#include "chain.cuh"
 #include "stencil.cuh"
 #include "vdr_internal.h"
 
@@ -523,7 +522,6 @@ __global__ void __launch_bounds__(RED_THREADS, 4) bst_w(Vec a, StencilView w) {
 
 template <bool KEEP>
 __global__ void __launch_bounds__(RED_THREADS, 4) bst_v(Vec a, StencilView w) {
-  chain_wait();
   if (a.st->done) return;
   const int shift = a.st->pexp - 1023;
   const double al = a.st->alpha;
@@ -551,7 +549,6 @@ __global__ void __launch_bounds__(RED_THREADS, 4) bst_v(Vec a, StencilView w) {
 
 template <bool KEEP>
 __global__ void __launch_bounds__(RED_THREADS, 4) bst_t(Vec a, StencilView w) {
-  chain_wait();
   if (a.st->done || a.st->sconv) return;
   const int shift = a.st->pexp - 1023;
   double v[3] = {0.0, 0.0, 0.0};
@@ -585,7 +582,6 @@ __global__ void __launch_bounds__(RED_THREADS, 4) bst_t(Vec a, StencilView w) {
 // block: two divisions in every thread were a third of the pipe's work here
 // (1.08 M nodes 34 -> 30 us, 8.5 M 157 -> 151).
 __global__ void __launch_bounds__(RED_THREADS, 4) bst_p(Vec a) {
-  chain_wait();
   KState *stc = a.st;
   if (stc->done) return;
   const double al = stc->alpha;
@@ -687,11 +683,12 @@ cudaError_t launch_stencil_iteration(Handle &h, const Vec &a, cudaStream_t s) {
   const StencilView w = stencil_view(h);
   const bool keep = stencil_keep(h);
   const int gs = std::min(red_grid(h.N), device_sm_count() * 4);
-  cudaError_t e;
-  if ((e = chain_launch(keep ? bst_v<true> : bst_v<false>, gs, RED_THREADS, 0, s, a, w)) ||
-      (e = chain_launch(keep ? bst_t<true> : bst_t<false>, gs, RED_THREADS, 0, s, a, w)))
-    return e;
-  return chain_launch(bst_p, gs, RED_THREADS, 0, s, a);
+  if (keep) bst_v<true><<<gs, RED_THREADS, 0, s>>>(a, w);
+  else bst_v<false><<<gs, RED_THREADS, 0, s>>>(a, w);
+  if (keep) bst_t<true><<<gs, RED_THREADS, 0, s>>>(a, w);
+  else bst_t<false><<<gs, RED_THREADS, 0, s>>>(a, w);
+  bst_p<<<gs, RED_THREADS, 0, s>>>(a);
+  return cudaGetLastError();
 }
 
 // The fused FP64 BiCGStab iteration (defined below with the fused kernels).
