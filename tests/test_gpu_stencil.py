@@ -325,3 +325,25 @@ def test_recorded_apply_follows_the_operator(vdr, oracle, gpu_lib):
             torch.cuda.synchronize()
             ref, _ = oracle.matvec0(m.iss, oracle_bb(oracle, prob, 2.0, aM), prob.bc, x)
             assert rel_l2(yd.cpu().numpy(), ref) < TOL, aM
+
+
+def test_block_solve_of_unaligned_arrays(vdr, gpu_lib):
+    """B or X starting off a 16-byte boundary is solved as aligned ones are."""
+    torch = pytest.importorskip("torch")
+    prob = vdr.problems.rotation_shear(7, 6, 5, seed=98)
+    N, K = prob.mesh.nnode, 16
+    B = np.random.default_rng(6).standard_normal((N, K))
+    B[prob.bc == 1] = 0.0
+    with vdr.Solver(prob, aH=2.0, aM=10.0) as s:
+        got = []
+        for ob, ox in ((0, 0), (1, 0), (0, 1)):
+            Bd = torch.zeros(N * K + 1, dtype=torch.float64, device="cuda")[ob:ob + N * K]
+            Xd = torch.zeros(N * K + 1, dtype=torch.float64, device="cuda")[ox:ox + N * K]
+            Bd, Xd = Bd.view(N, K), Xd.view(N, K)
+            Bd.copy_(torch.tensor(B, device="cuda"))
+            torch.cuda.synchronize()
+            _, _, errs, st = s.solve_block_device(Bd, Xd, tol=1e-11, inner_tol=1e-4)
+            torch.cuda.synchronize()
+            assert st == 0 and np.all(errs <= 1e-11)
+            got.append(Xd.cpu().numpy().copy())
+    assert rel_l2(got[1], got[0]) < 1e-9 and rel_l2(got[2], got[0]) < 1e-9

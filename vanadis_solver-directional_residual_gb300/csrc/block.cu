@@ -1578,14 +1578,12 @@ int solve_block_device(Handle &h, int K, int precision, const double *B,
   dinv_to_f32<<<grid_n(h.N, 256, 8), 256, 0, s>>>(h.dinv, h.dinv32, h.N);
   count_launches(1);
   if ((e = cudaGetLastError())) return cuda_fail(e, "block setup");
-  // the canonical structured numbering: the iteration on assembled rows
-  BlockRows rows{};
-  const bool on_rows = block_rows_usable(h, K, &rows);
-  // The apply's operator copy carries the Jacobi scale (A D^-1).
+  // The apply's operator copy carries the Jacobi scale (A D^-1).  It comes
+  // before the rows, which take only what room is left.
   float4 *Aaos = nullptr;
-  if ((!on_rows || (K == 64 && !h.blk_tuned)) && (e = ensure_aos(h, true, &Aaos)))
-    return cuda_fail(e, "block operator copy");
-  if (K == 64 && !h.blk_tuned) {  // launch shape by measurement, before capture
+  const bool tune = K == 64 && !h.blk_tuned;
+  if (tune) {  // launch shape by measurement, before capture
+    if ((e = ensure_aos(h, true, &Aaos))) return cuda_fail(e, "block operator copy");
     if ((e = cudaMemsetAsync(a.p, 0, sizeof(float) * 2 * n, s)))
       return cuda_fail(e, "block tuning");
     const int tst = tune_block_apply(h, a.p, a.v, Aaos);
@@ -1593,6 +1591,11 @@ int solve_block_device(Handle &h, int K, int precision, const double *B,
     if (h.bk_graph) cudaGraphExecDestroy(h.bk_graph);
     h.bk_graph = nullptr;
   }
+  // the canonical structured numbering: the iteration on assembled rows
+  BlockRows rows{};
+  const bool on_rows = !((reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(X)) & 15) &&
+                       block_rows_usable(h, K, &rows);  // 16-byte accesses
+  if (!on_rows && (e = ensure_aos(h, true, &Aaos))) return cuda_fail(e, "block operator copy");
   const int gv = std::min(BK_MAX_GRID, grid_n(on_rows ? n / 4 : n, BT, 2));  // one wave
   if (on_rows) a.rh = bf;  // x = 0, so the right-hand side is the shadow residual too
   const int gm = grid_n(n, 256, 8);
