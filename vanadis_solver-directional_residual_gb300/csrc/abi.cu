@@ -1410,7 +1410,7 @@ int legacy_prepare(Legacy &L, int N, int E) {
     for (int k = 0; k < Handle::NGRAPH; k++) {
       if (h.graph_exec[k]) cudaGraphExecDestroy(h.graph_exec[k]);
       h.graph_exec[k] = nullptr;
-      h.graph_key[k] = nullptr;
+      h.graph_key[k] = {};
     }
     for (int k = 0; k < 2; k++) {
       if (h.ev[k]) cudaEventDestroy(h.ev[k]);

@@ -829,11 +829,8 @@ int solve_segmented_device(Handle &h, const double *b, double *x, double tol, in
   const int K = h.opt.iters_per_graph > 0 ? h.opt.iters_per_graph : 8;
   uintptr_t tol_bits;  // the captured kernels carry the tolerance and itmax
   std::memcpy(&tol_bits, &tol, sizeof tol_bits);
-  const void *key = (const void *)((uintptr_t)b ^ ((uintptr_t)x << 1) ^
-                                   ((uintptr_t)h.work << 2) ^ (uintptr_t)K ^
-                                   ((uintptr_t)h.seg_tile << 16) ^ (uintptr_t)th ^
-                                   ((uintptr_t)rows << 12) ^ tol_bits ^
-                                   ((uintptr_t)itmax << 24));
+  const GraphKey key{key_of(b), key_of(x), key_of(h.work), (uintptr_t)K, (uintptr_t)h.seg_tile,
+                     (uintptr_t)th, (uintptr_t)rows, tol_bits, (uintptr_t)itmax};
   if (!h.seg_graph || h.seg_key != key) {
     if (h.seg_graph) cudaGraphExecDestroy(h.seg_graph);
     h.seg_graph = nullptr;

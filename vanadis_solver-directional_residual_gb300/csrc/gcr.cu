@@ -366,12 +366,9 @@ int solve_gcr_device(Handle &h, const double *b, double *x, double tol,
       }
     }
   } else {
-  const void *key = (const void *)((uintptr_t)b ^ ((uintptr_t)x << 1) ^
-                                   ((uintptr_t)h.gcr_work << 2) ^ (uintptr_t)m ^
-                                   ((uintptr_t)(prec ? prec->ctx : nullptr) << 3) ^
-                                   ((uintptr_t)h.apply_mode << 8) ^
-                                   ((uintptr_t)h.scatter << 12) ^
-                                   ((uintptr_t)stencil_ready(h) << 16));
+  const GraphKey key{key_of(b), key_of(x), key_of(h.gcr_work), (uintptr_t)m,
+                     key_of(prec ? prec->ctx : nullptr), (uintptr_t)h.apply_mode,
+                     (uintptr_t)h.scatter, (uintptr_t)h.storage, (uintptr_t)stencil_ready(h)};
   long per_cycle = 0;
   if (!h.gcr_graph || h.gcr_key != key) {
     if (h.gcr_graph) cudaGraphExecDestroy(h.gcr_graph);

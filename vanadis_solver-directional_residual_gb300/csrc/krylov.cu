@@ -743,7 +743,7 @@ cudaError_t ensure_solver_workspace(Handle &h, int nvec) {
     for (int k = 0; k < Handle::NGRAPH; k++) {
       if (h.graph_exec[k]) cudaGraphExecDestroy(h.graph_exec[k]);
       h.graph_exec[k] = nullptr;
-      h.graph_key[k] = nullptr;
+      h.graph_key[k] = {};
     }
   }
   if (!h.st) {
@@ -844,24 +844,18 @@ int solve_device(Handle &h, int method, const double *b, double *x,
     return VDR_BAD_ARGUMENT;
   }
   const int slot = (method & 1) | (h.apply_fp32 ? 2 : 0) | (prec ? 4 : 0);
-  const void *key = (const void *)((uintptr_t)b ^ ((uintptr_t)x << 1) ^
-                                   ((uintptr_t)h.work << 2) ^ (uintptr_t)K ^
-                                   ((uintptr_t)h.apply_mode << 8) ^
-                                   ((uintptr_t)h.scatter << 12) ^
-                                   ((uintptr_t)h.storage << 16) ^
-                                   ((uintptr_t)(prec ? prec->ctx : nullptr) << 3));
+  const bool rows = stencil_ready(h);
   // the kernels' arguments carry N, E and the work-vector offsets, so a
   // graph captured for other sizes (buffers reused by a smaller mesh) is
   // captured again
-  const long long size_key = ((long long)h.N << 32) | (unsigned)h.E;
-  const bool rows = stencil_ready(h);
+  GraphKey key{key_of(b), key_of(x), key_of(h.work), (uintptr_t)K, (uintptr_t)h.apply_mode,
+               (uintptr_t)h.scatter, (uintptr_t)h.storage, key_of(prec ? prec->ctx : nullptr),
+               (uintptr_t)h.N << 32 | (unsigned)h.E};
   const bool fusable = method == VDR_SOLVER_BICGSTAB && !prec;
   for (int attempt = 0; attempt < 2; attempt++) {
     const bool fused = fusable && h.fused64;
-    const void *fkey = (const void *)((uintptr_t)key ^ ((uintptr_t)fused << 20) ^
-                                      ((uintptr_t)rows << 21));
-    if (h.graph_exec[slot] && h.graph_key[slot] == fkey && h.graph_size[slot] == size_key)
-      break;
+    key[9] = (uintptr_t)fused | (uintptr_t)rows << 1;
+    if (h.graph_exec[slot] && h.graph_key[slot] == key) break;
     if (h.graph_exec[slot]) cudaGraphExecDestroy(h.graph_exec[slot]);
     h.graph_exec[slot] = nullptr;
     cudaGraph_t graph;
@@ -879,8 +873,7 @@ int solve_device(Handle &h, int method, const double *b, double *x,
       e = cudaGraphInstantiate(&h.graph_exec[slot], graph, 0);
       cudaGraphDestroy(graph);
       if (!e) {
-        h.graph_key[slot] = fkey;
-        h.graph_size[slot] = size_key;
+        h.graph_key[slot] = key;
         break;
       }
       h.graph_exec[slot] = nullptr;
@@ -1829,10 +1822,8 @@ int solve32_inner(Handle &h, double tol, int itmax, int *iter, double *err) {
   const int K = h.opt.iters_per_graph > 0 ? h.opt.iters_per_graph : 8;
   for (int attempt = 0; attempt < 2; attempt++) {
     const bool fused = h.use_half && h.fused32;
-    const void *key = (const void *)((uintptr_t)h.work32 ^ ((uintptr_t)h.A32v << 1) ^
-                                     (uintptr_t)K ^ ((uintptr_t)h.scatter << 12) ^
-                                     ((uintptr_t)h.use_half << 20) ^
-                                     ((uintptr_t)h.A16 << 2) ^ ((uintptr_t)fused << 21));
+    const GraphKey key{key_of(h.work32), key_of(h.A32v), (uintptr_t)K, (uintptr_t)h.scatter,
+                       (uintptr_t)h.use_half, key_of(h.A16), (uintptr_t)fused};
     if (h.graph32 && h.graph32_key == key) break;
     if (h.graph32) cudaGraphExecDestroy(h.graph32);
     h.graph32 = nullptr;

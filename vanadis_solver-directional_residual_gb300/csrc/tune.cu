@@ -121,7 +121,7 @@ int tune_stored_apply(Handle &h) {
   for (int k = 0; k < Handle::NGRAPH; k++) {
     if (h.graph_exec[k]) cudaGraphExecDestroy(h.graph_exec[k]);
     h.graph_exec[k] = nullptr;
-    h.graph_key[k] = nullptr;
+    h.graph_key[k] = {};
   }
   return st;
 }

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <array>
 #include <string>
 #include <vector>
 
@@ -41,6 +42,12 @@ struct KState {
   double rhs, rho_next, beta;
   int pexp, pmax, pmax_next, rmax;
 };
+
+// What a recorded graph's kernels hold, one value a place.  Compared place by
+// place: folded into one word, two pairs of arrays can meet (b ^ 2 x is the
+// same for a second pair 2^k bytes away in x and 2^(k+1) in b).
+using GraphKey = std::array<uintptr_t, 10>;
+inline uintptr_t key_of(const void *p) { return reinterpret_cast<uintptr_t>(p); }
 
 // A right preconditioner for BiCGStab beyond Jacobi: `enqueue` adds
 // (M(in) - D^-1 in) to `out`, which already holds D^-1 in (zero on
@@ -251,7 +258,7 @@ struct Handle {
   // rh, p, v, ph, s, sh, t) and its captured iterations
   float *work32 = nullptr;
   cudaGraphExec_t graph32 = nullptr;
-  const void *graph32_key = nullptr;
+  GraphKey graph32_key{};
   // the FP32 inner iteration with the binary16 operator, and the FP64
   // Jacobi-BiCGStab iteration, as two fused cooperative vector kernels each
   // (krylov.cu); off after a failed capture
@@ -262,8 +269,7 @@ struct Handle {
   int red_blocks = 0;
   static constexpr int NGRAPH = 8;
   cudaGraphExec_t graph_exec[NGRAPH] = {};
-  long long graph_size[NGRAPH] = {};  // (N << 32) | E the graph was captured for
-  const void *graph_key[NGRAPH] = {};
+  GraphKey graph_key[NGRAPH] = {};
   cudaEvent_t ev[2] = {nullptr, nullptr};
 
   // host staging
@@ -313,7 +319,7 @@ struct Handle {
   unsigned *seg_ticket = nullptr;
   int seg_ticket_n = 0;
   cudaGraphExec_t seg_graph = nullptr;
-  const void *seg_key = nullptr;
+  GraphKey seg_key{};
   long seg_graph_launches = 0;
   int *seg_of_elem = nullptr;         // [E] storage order
   // every mesh in the canonical numbering: their grids, the assembled rows
@@ -330,7 +336,7 @@ struct Handle {
   double *gcr_work = nullptr;
   size_t gcr_words = 0;
   cudaGraphExec_t gcr_graph = nullptr;
-  const void *gcr_key = nullptr;
+  GraphKey gcr_key{};
   long gcr_cycle_launches = 0;
 };
 
