@@ -367,7 +367,7 @@ int solve_gcr_device(Handle &h, const double *b, double *x, double tol,
     }
   } else {
   const GraphKey key{key_of(b), key_of(x), key_of(h.gcr_work), (uintptr_t)m,
-                     key_of(prec ? prec->ctx : nullptr), (uintptr_t)h.apply_mode,
+                     (uintptr_t)(prec ? prec->version : 0), (uintptr_t)h.apply_mode,
                      (uintptr_t)h.scatter, (uintptr_t)h.storage, (uintptr_t)stencil_ready(h)};
   long per_cycle = 0;
   if (!h.gcr_graph || h.gcr_key != key) {

@@ -849,7 +849,7 @@ int solve_device(Handle &h, int method, const double *b, double *x,
   // graph captured for other sizes (buffers reused by a smaller mesh) is
   // captured again
   GraphKey key{key_of(b), key_of(x), key_of(h.work), (uintptr_t)K, (uintptr_t)h.apply_mode,
-               (uintptr_t)h.scatter, (uintptr_t)h.storage, key_of(prec ? prec->ctx : nullptr),
+               (uintptr_t)h.scatter, (uintptr_t)h.storage, (uintptr_t)(prec ? prec->version : 0),
                (uintptr_t)h.N << 32 | (unsigned)h.E};
   const bool fusable = method == VDR_SOLVER_BICGSTAB && !prec;
   for (int attempt = 0; attempt < 2; attempt++) {

@@ -48,6 +48,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <vector>
 
@@ -1110,6 +1111,11 @@ __global__ void jacobi_out(const double *in, const double *dinv,
 }  // namespace
 
 // ================================================================ host
+unsigned long long next_version() {
+  static std::atomic<unsigned long long> last{0};
+  return ++last;
+}
+
 struct Net {
   Handle *h = nullptr;
   Dims d[3];
@@ -1139,6 +1145,7 @@ struct Net {
   int adam_t = 0;
   int smooth_steps = 1;   // Jacobi post-smoothing steps after the network
   double smooth_omega = 1.0;
+  unsigned long long version = next_version();  // changes with the settings above and conv_mode
   bool features_set = false;
   // tcgen05 forward convolutions: packed weights, the decoders' upsampled
   // inputs on the fine grid, and per layer the TMA maps of its inputs
@@ -1747,6 +1754,7 @@ extern "C" int vdr_net_set_conv(vdr_net *N, int mode) {
     return VDR_BAD_ARGUMENT;
   }
   n.conv_mode = mode;
+  n.version = next_version();
   return VDR_OK;
 }
 
@@ -2007,6 +2015,7 @@ extern "C" int vdr_net_set_smoothing(vdr_net *N, int steps, double omega) {
   }
   N->n.smooth_steps = steps;
   N->n.smooth_omega = omega;
+  N->n.version = next_version();
   return VDR_OK;
 }
 
@@ -2040,7 +2049,7 @@ extern "C" int vdr_solve_learned_device(vdr_handle *H, vdr_net *N, const double 
   }
   Handle &h = *n.h;
   if ((st = prepare_operator(h))) return st;
-  Precond pc{net_enqueue, &n, net_enqueue_launches(n)};
+  Precond pc{net_enqueue, &n, net_enqueue_launches(n), n.version};
   int it1 = 0;
   double e1 = 0.0;
   st = solve_device(h, VDR_SOLVER_BICGSTAB, d_b, d_x, tol, itmax, &it1, &e1, &pc,
@@ -2078,7 +2087,8 @@ extern "C" int vdr_solve_gcr_device(vdr_handle *H, vdr_net *N, const double *d_b
   }
   int st = prepare_operator(h);
   if (st) return st;
-  Precond pc{net_enqueue, N ? &N->n : nullptr, N ? net_enqueue_launches(N->n) : 0};
+  Precond pc{net_enqueue, N ? &N->n : nullptr, N ? net_enqueue_launches(N->n) : 0,
+             N ? N->n.version : 0};
   int it1 = 0;
   double e1 = 0.0;
   st = solve_gcr_device(h, d_b, d_x, tol, itmax, restart, N ? &pc : nullptr,
@@ -2115,7 +2125,7 @@ extern "C" int vdr_solve_learned_hybrid_device(vdr_handle *H, vdr_net *N,
   }
   int st = prepare_operator(h);
   if (st) return st;
-  Precond pc{net_enqueue, &N->n, net_enqueue_launches(N->n)};
+  Precond pc{net_enqueue, &N->n, net_enqueue_launches(N->n), N->n.version};
   int it1 = 0, it2 = 0;
   double e1 = 0.0;
   st = solve_gcr_device(h, d_b, d_x, tol, std::min(learned_steps, itmax), learned_steps,
@@ -2146,7 +2156,8 @@ extern "C" int vdr_solve_gcr_record_device(vdr_handle *H, vdr_net *N, const doub
   }
   int st = prepare_operator(h);
   if (st) return st;
-  Precond pc{net_enqueue, N ? &N->n : nullptr, N ? net_enqueue_launches(N->n) : 0};
+  Precond pc{net_enqueue, N ? &N->n : nullptr, N ? net_enqueue_launches(N->n) : 0,
+             N ? N->n.version : 0};
   return solve_gcr_device(h, d_b, d_x, tol, itmax, restart, N ? &pc : nullptr, 0, iter,
                           err, d_hist, max_hist, n_hist);
 }

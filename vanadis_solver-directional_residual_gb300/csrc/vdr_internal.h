@@ -58,6 +58,9 @@ struct Precond {
                          const int *skip, const int *skip2, cudaStream_t s);
   void *ctx;
   int launches;  // kernels per enqueue
+  // unlike any other preconditioner's and any other settings' of this one: a
+  // graph that holds its kernels is recorded anew when it changes
+  unsigned long long version;
 };
 
 struct DeviceOp;  // forward
