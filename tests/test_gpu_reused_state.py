@@ -1,9 +1,39 @@
 """Calls that reuse what an earlier call left behind -- recorded graphs,
-buffers, rows -- give the answers that first calls give."""
+buffers, rows -- give the answers that first calls give.
+
+Bars: solutions to 1e-9 where both sides are solved to 1e-11 or below (the
+operators' condition is below 1e2 here)."""
 import numpy as np
 import pytest
 
+from helpers import rel_l2
+
 pytestmark = pytest.mark.gpu
+
+
+def system(vdr, oracle, dims, seed, aM=10.0):
+    """A theta step on a ragged mesh: problem, element matrices, right-hand
+    side, diagonal, start and the oracle's solution."""
+    prob = vdr.problems.rotation_shear(*dims, seed=seed)
+    m = prob.mesh
+    told = np.cos(0.37 * np.arange(m.nnode))
+    bb, b, diag = oracle.assemble(prob.variant, m.xx, m.yy, m.zz, m.iss, prob.vel, prob.lam,
+                                  prob.pdec, prob.q, kod=m.kod, robin_alpha=0.0, aH=2.0, aM=aM,
+                                  cf=3.0, rM=aM, t_old=told, nthreads=8)
+    b[prob.bc == 1] = 0.0
+    diag[prob.bc == 1] = 1.0
+    x0 = np.where(prob.bc == 1, 0.0, told)
+    ref, _, _, st = oracle.bicgstab(b, x0, bb, m.iss, diag, prob.bc, tol=1e-12, itmax=5000)
+    assert st == 0
+    return prob, bb, b, diag, x0, ref
+
+
+def dropin(vdr, sys_, x0=None, tol=1e-11, scale=1.0):
+    prob, bb, b, diag, start, _ = sys_
+    m = prob.mesh
+    d = np.where(prob.bc == 1, 1.0, diag * scale)
+    return vdr.kernel_dbcg_simple(m.nnode, b * scale, start if x0 is None else x0, tol, 5000,
+                                  bb * scale, m.iss, d, m.nax, m.nay, m.naz, prob.bc)
 
 
 def test_recorded_graphs_belong_to_their_arrays(vdr, gpu_lib):
@@ -96,3 +126,32 @@ def test_recorded_graphs_follow_the_network(vdr, gpu_lib, solver, change):
     assert n == launches
     if change != "conv":
         assert abs(before - want) > 0.02 * want
+
+
+def test_dropin_after_a_nonfinite_call(vdr, oracle, gpu_lib):
+    """A start that holds a NaN spoils its own call only: the next, on the
+    same planes but fewer of them, solves."""
+    tall = system(vdr, oracle, (9, 8, 19), 32)
+    low = system(vdr, oracle, (9, 8, 9), 33)
+    m = tall[0].mesh
+    plane = np.arange(m.nnode) // (m.nax * m.nay)
+    bad = tall[4].copy()
+    bad[np.flatnonzero((tall[0].bc == 0) & (plane == 10))] = np.nan
+    for _ in range(2):
+        _, _, err = dropin(vdr, tall, x0=bad)
+        assert not err <= 1e-11
+        x, _, err = dropin(vdr, low)
+        assert err <= 1e-11 and rel_l2(x, low[5]) < 1e-9
+        x, _, err = dropin(vdr, tall)
+        assert err <= 1e-11 and rel_l2(x, tall[5]) < 1e-9
+
+
+def test_dropin_sizes_up_and_down(vdr, oracle, gpu_lib):
+    """Tall, low, tall meshes on the same planes and others of the same node
+    count, below and above the one-launch limit: rows, pair vectors and pads
+    at other offsets in the same buffers."""
+    for dims in ((12, 9, 30), (12, 9, 5), (12, 9, 30), (9, 12, 30), (30, 9, 12), (75, 63, 32),
+                 (75, 63, 31), (75, 63, 4), (63, 75, 32), (12, 9, 5)):
+        sys_ = system(vdr, oracle, dims, 36)
+        x, _, err = dropin(vdr, sys_)
+        assert err <= 1e-11 and rel_l2(x, sys_[5]) < 1e-9, dims

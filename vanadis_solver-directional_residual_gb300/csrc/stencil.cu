@@ -202,10 +202,14 @@ cudaError_t ensure_stencil(Handle &h) {
   const size_t N = (size_t)h.N, len = 2 * (N + 2 * stencil_pad(h));
   if (!row_storage(h, &h.st_x, &h.st_len, len)) return cudaSuccess;
   cudaError_t e;
-  if (h.st_nax != h.nax || h.st_pl != h.nax * h.nay) {
+  // the pads lie before, between and behind the vectors: where they lie
+  // depends on the strides and on N, and their zeros meet other planes'
+  // entries (A^T) or a stored infinity (0 x inf) when they are not zero
+  if (h.st_nax != h.nax || h.st_pl != h.nax * h.nay || h.st_n != h.N) {
     if ((e = cudaMemsetAsync(h.st_x, 0, sizeof(float2) * h.st_len, h.stream))) return e;
     h.st_nax = h.nax;
     h.st_pl = h.nax * h.nay;
+    h.st_n = h.N;
   }
   const long need = (h.N + 255L) / 256;
   const int grid = (int)std::min<long>(need, (long)device_sm_count() * 32);

@@ -241,7 +241,7 @@ struct Handle {
   unsigned *st_nm = nullptr;    // [N]
   float2 *st_x = nullptr;       // two padded pair vectors: p^ and s^
   size_t st_rows = 0, st_len = 0;  // nodes and pairs that they hold room for
-  int st_nax = 0, st_pl = 0;    // the strides that st_x's pads are zero for
+  int st_nax = 0, st_pl = 0, st_n = 0;  // the mesh that st_x's pads are zero for
   int st_state = 0, st_applies = 0;
   bool own_capture = false;
   // its binary16 rows for the mixed solve (half_rows.cu): 27 half planes, a
