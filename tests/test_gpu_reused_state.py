@@ -155,3 +155,43 @@ def test_dropin_sizes_up_and_down(vdr, oracle, gpu_lib):
         sys_ = system(vdr, oracle, dims, 36)
         x, _, err = dropin(vdr, sys_)
         assert err <= 1e-11 and rel_l2(x, sys_[5]) < 1e-9, dims
+
+
+# entries just below the store's 2^120, in the middle, just above its 2^-100
+@pytest.mark.parametrize("power", [119, 60, -60, -95])
+@pytest.mark.parametrize("dims", [(12, 9, 8), (75, 63, 32)])
+def test_systems_across_the_stores_range(vdr, oracle, gpu_lib, dims, power):
+    """The system times a power of two has the same solution, whether it runs
+    as one launch or as kernels: by the drop-in (BiCG), by BiCGStab, in mixed
+    precision, as a segment and as columns."""
+    torch = pytest.importorskip("torch")
+    sys_ = system(vdr, oracle, dims, 34)
+    prob, bb, b = sys_[:3]
+    big = np.abs(bb).max()
+    small = np.abs(bb[bb != 0]).min()
+    e = power - int(np.ceil(np.log2(big))) if power > 0 else power - int(np.floor(np.log2(small)))
+    if power > 0 and np.log2(small) + e < -99:
+        pytest.skip("the entries' own range")
+    scale = 2.0 ** e
+    x, _, err = dropin(vdr, sys_, scale=scale)
+    assert err <= 1e-11 and rel_l2(x, sys_[5]) < 1e-9
+    bd = torch.tensor(b, device="cuda")
+    for precision in ("fp64", "mixed"):
+        with vdr.Solver(prob, vdr.Options(precision=precision), aH=2.0, aM=10.0) as s:
+            for f in (1.0, scale):
+                s.set_operator(2.0 * f, 10.0 * f)
+                xd = torch.tensor(sys_[4], device="cuda")
+                it, err, st = s.solve_device(bd * f, xd, tol=1e-11, itmax=2000)
+                assert st == 0 and err <= 1e-11, (precision, f, it, err, st)
+                assert rel_l2(xd.cpu().numpy(), sys_[5]) < 1e-9
+                if precision == "mixed":
+                    continue
+                if dims == (12, 9, 8):
+                    X = torch.zeros(s.N, 16, dtype=torch.float64, device="cuda")
+                    _, _, errs, st = s.solve_block_device((bd * f)[:, None].repeat(1, 16), X,
+                                                          tol=1e-11)
+                    assert st == 0 and rel_l2(X[:, 3].cpu().numpy(), sys_[5]) < 1e-9
+            s.set_segments(np.array([0, s.N]))
+            xd.zero_()
+            _, _, _, st = s.solve_segmented_device(bd * scale, xd, tol=1e-11, itmax=2000)
+            assert st == 0 and rel_l2(xd.cpu().numpy(), sys_[5]) < 1e-9

@@ -322,13 +322,13 @@ __global__ void __launch_bounds__(512, 2) sgr_first(SegVec a) {
   const int s = tl.seg;
   if (!a.s.active[s]) return;
   const long at = a.mesh[s].shift;
-  const int e = a.s.pmax[s], er = a.s.rmax[s];
+  const int e = a.s.pmax[s], er = a.s.rmax[s], base = pair_base(a.rows.top);
   TLOOP(i) {
     const double ri = a.r[i];
     const bool m = a.m[i] != 0;
     a.p[i] = ri;
-    a.php[i + at] = m ? make_float2(0.f, 0.f) : stencil_pair(ri * a.dinv[i], e - 1023);
-    a.shp[i + at] = m ? make_float2(0.f, 0.f) : stencil_pair(ri, er - 1023);
+    a.php[i + at] = m ? make_float2(0.f, 0.f) : stencil_pair(ri * a.dinv[i], e - base);
+    a.shp[i + at] = m ? make_float2(0.f, 0.f) : stencil_pair(ri, er - base);
   }
   if (tl.start == a.mesh[s].n0 && threadIdx.x == 0) a.s.pexp[s] = e;
 }
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(512, 2) sgr_w(SegVec a) {
   const SegMesh g = a.mesh[s];
   const StencilView v = mesh_rows(a, g);
   const float2 *xp = a.shp + g.shift;
-  const int shift = a.s.rmax[s] - 1023;
+  const int shift = a.s.rmax[s] - pair_base(v.top);
   double q[1] = {0.0};
   TLOOP(i) {
     const unsigned m = v.nm[i];
@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(512, 2) sgr_v(SegVec a) {
   if (!a.s.active[s]) return;
   const SegMesh g = a.mesh[s];
   const StencilView v = mesh_rows(a, g);
-  const int shift = a.s.pexp[s] - 1023;
+  const int shift = a.s.pexp[s] - pair_base(v.top);
   const double al = a.s.alpha[s];
   double q[2] = {0.0, 0.0};
   TLOOP(i) {
@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(512, 2) sgr_t(SegVec a) {
   if (!a.s.active[s] || a.s.sconv[s]) return;
   const SegMesh g = a.mesh[s];
   const StencilView v = mesh_rows(a, g);
-  const int shift = a.s.pexp[s] - 1023;
+  const int shift = a.s.pexp[s] - pair_base(v.top);
   double q[3] = {0.0, 0.0, 0.0};
   TLOOP(i) {
     const double si = a.sv[i], hi = a.rh[i];
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(512, 2) sgr_p(SegVec a) {
   }
   const double om = a.s.omega[s], rho1 = a.s.rho_next[s];
   const double beta = a.s.beta[s];
-  const int e = a.s.pmax[s], shift = e - 1023;
+  const int e = a.s.pmax[s], shift = e - pair_base(a.rows.top);
   const long at = a.mesh[s].shift;
   int em = 0;
   TLOOP(i) {
@@ -709,6 +709,7 @@ cudaError_t seg_layout(Handle &h, int tile, int threads, const double *b, double
   if (h.seg_rows) {
     a.rows.S = h.st_S;
     a.rows.nm = h.st_nm;
+    a.rows.top = h.st_nm + h.st_rows;
     a.rows.N = h.N;
     a.mesh = h.seg_mesh;
     a.php = h.seg_x;

@@ -77,6 +77,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
   const int N = a.w.N, n = (int)(blockIdx.x * T + threadIdx.x);
   const bool on = n < N;
   unsigned target = 0;
+  const int base = pair_base(a.w.top);
   const int none[1] = {0};
   const auto nothing = [](int) {};
   double x = 0.0, r = 0.0, p = 0.0, v = 0.0, s = 0.0, t = 0.0, rh = 0.0, wn = 0.0;
@@ -140,11 +141,11 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
   }
   const int ex = sh.etot[0];
   if (ex) {
-    put(0, masked_pair(msk, x, ex - 1023));
+    put(0, masked_pair(msk, x, ex - base));
     const double z[1] = {0.0};
     if (!meet<MODE, T, 1, 0, 0, AT_D, AT_D, 0>(sh, a.mt, z, none, target, nothing))
       return res_timeout(a.st);
-    v = row(0, ex - 1023);
+    v = row(0, ex - base);
   }
   {
     const double bi = msk ? 0.0 : a.b[n];
@@ -187,8 +188,8 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
   };
   if (!done) {
     // p^ = D^-1 r, and w = A^T rh (the neighbours' rows, from L2)
-    put(0, masked_pair(msk, p * di, pexp - 1023));
-    put(1, masked_pair(msk, rh, er - 1023));
+    put(0, masked_pair(msk, p * di, pexp - base));
+    put(1, masked_pair(msk, rh, er - base));
     double q[1] = {0.0};
     if (!meet<MODE, T, 1, 0, 0, AT_C, AT_C, 0>(sh, a.mt, q, none, target, nothing))
       return res_timeout(a.st);
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
           xv = __ldcg(a.shp + o);
         df_fma_acc(acc, e.x, e.y, xv.x, xv.y);
       }
-    wn = row_value(acc, er - 1023);
+    wn = row_value(acc, er - base);
     if (!msk) q[0] = wn * (p * di);
     if (!meet<MODE, T, 1, 0, 1, AT_D, AT_D, 0>(sh, a.mt, q, none, target,
                                             [&](int lane) { alpha_of(lane, sh.tot[0]); }))
@@ -221,7 +222,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
   }
   int pmax = pexp;
   while (!done) {
-    const int shift = pexp - 1023;
+    const int shift = pexp - base;
     v = row(0, shift);
     s = r - al * v;
     put(1, masked_pair(msk, s * di, shift));
@@ -268,7 +269,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
     r = s - om * t;
     p = r + beta * (p - om * v);
     const double ph = msk ? 0.0 : p * di;
-    put(0, stencil_pair(ph, pmax - 1023));
+    put(0, stencil_pair(ph, pmax - base));
     rho = rho1;
     {
       const double q[2] = {r * r, wn * ph};
@@ -336,6 +337,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicg(ResArgs a) {
   const int N = a.w.N, n = (int)(blockIdx.x * T + threadIdx.x);
   const bool on = n < N;
   unsigned target = 0;
+  const int base = pair_base(a.w.top);
   const int none[1] = {0};
   const auto nothing = [](int) {};
   const auto column = [&](int k) {  // A's entry of neighbour k with this node
@@ -395,11 +397,11 @@ __global__ void __launch_bounds__(T, 1) resident_bicg(ResArgs a) {
   }
   const int ex = sh.etot[0];
   if (ex) {
-    if (on) a.php[n] = masked_pair(msk, x, ex - 1023);
+    if (on) a.php[n] = masked_pair(msk, x, ex - base);
     const double q[1] = {0.0};
     if (!meet<MODE, T, 1, 0, 0, AT_D, AT_D, 0>(sh, a.mt, q, none, target, nothing))
       return res_timeout(a.st);
-    z = row(ex - 1023);
+    z = row(ex - base);
   }
   {
     const double bi = on ? a.b[n] : 0.0;
@@ -434,16 +436,16 @@ __global__ void __launch_bounds__(T, 1) resident_bicg(ResArgs a) {
     p = msk ? 0.0 : r * di + bk * p;
     pp = msk ? 0.0 : rr * di + bk * pp;
     if (on) {
-      a.php[n] = stencil_pair(p, pexp - 1023);
-      a.shp[n] = stencil_pair(pp, qexp - 1023);
+      a.php[n] = stencil_pair(p, pexp - base);
+      a.shp[n] = stencil_pair(pp, qexp - base);
     }
     {
       const double q[1] = {0.0};
       if (!meet<MODE, T, 1, 0, 0, AT_C, AT_C, 0>(sh, a.mt, q, none, target, nothing))
         return res_timeout(a.st);
     }
-    z = row(pexp - 1023);
-    zz = trans(qexp - 1023);
+    z = row(pexp - base);
+    zz = trans(qexp - base);
     {
       const double q[1] = {z * pp};
       const int em[2] = {df_exp(p), df_exp(pp)};

@@ -25,7 +25,8 @@ __device__ __forceinline__ void acc_pair(DfAcc &acc, float h, float l) {
 // row i is read by exactly one thread, so the store is read once (512 E
 // bytes) and 220 N written: 1.23 ms at 8.4M elements (5.0 TB/s).  The mesh's
 // elements lie from e0 on in the store of E, `l` is the node's number in it.
-__device__ __forceinline__ void assemble_node(const float4 *__restrict__ Ahi,
+// Returns the largest entry's magnitude bits.
+__device__ __forceinline__ unsigned assemble_node(const float4 *__restrict__ Ahi,
                                               const float4 *__restrict__ Alo,
                                               const unsigned char *__restrict__ emask, int E,
                                               long e0, int nax, int nay, int naz, unsigned l,
@@ -66,35 +67,47 @@ __device__ __forceinline__ void assemble_node(const float4 *__restrict__ Ahi,
       }
     }
   }
+  unsigned big = 0u;
 #pragma unroll
   for (int t = 0; t < 27; t++) {
     const Df2 a = df_norm(acc[t]);
     S[(size_t)t * N + n] = make_float2(a.h, a.l);
+    big = max(big, __float_as_uint(a.h) & 0x7fffffffu);
   }
   nm[n] = m;
+  return big;
+}
+
+__device__ __forceinline__ void raise_top(unsigned big, unsigned *top) {
+  const unsigned e = __reduce_max_sync(0xffffffffu, big) >> 23;
+  if ((threadIdx.x & 31) == 0 && e > *(volatile unsigned *)top) atomicMax(top, e);
 }
 
 __global__ void __launch_bounds__(256, 2) stencil_assemble(
     const float4 *__restrict__ Ahi, const float4 *__restrict__ Alo,
     const unsigned char *__restrict__ emask, int nax, int nay, int naz, float2 *S,
-    unsigned *nm) {
+    unsigned *nm, unsigned *top) {
+  unsigned big = 0u;
   const int E = (nax - 1) * (nay - 1) * (naz - 1), N = nax * nay * naz;
   for (long n = (long)blockIdx.x * blockDim.x + threadIdx.x; n < N;
        n += (long)gridDim.x * blockDim.x)
-    assemble_node(Ahi, Alo, emask, E, 0, nax, nay, naz, (unsigned)n, n, N, S, nm);
+    big = max(big, assemble_node(Ahi, Alo, emask, E, 0, nax, nay, naz, (unsigned)n, n, N, S, nm));
+  raise_top(big, top);
 }
 
 // The same for many meshes side by side (one row of blocks per mesh).
 __global__ void __launch_bounds__(256, 2) stencil_assemble_meshes(
     const float4 *__restrict__ Ahi, const float4 *__restrict__ Alo,
     const unsigned char *__restrict__ emask, int E, long N,
-    const SegMesh *__restrict__ meshes, float2 *S, unsigned *nm) {
+    const SegMesh *__restrict__ meshes, float2 *S, unsigned *nm, unsigned *top) {
+  unsigned big = 0u;
   const SegMesh g = meshes[blockIdx.y];
   const int count = g.nax * g.nay * g.naz;
   for (int l = (int)(blockIdx.x * blockDim.x + threadIdx.x); l < count;
        l += (int)(gridDim.x * blockDim.x))
-    assemble_node(Ahi, Alo, emask, E, g.e0, g.nax, g.nay, g.naz, (unsigned)l, g.n0 + (long)l,
-                  N, S, nm);
+    big = max(big, assemble_node(Ahi, Alo, emask, E, g.e0, g.nax, g.nay, g.naz, (unsigned)l,
+                                 g.n0 + (long)l, N, S, nm));
+  raise_top(big, top);
 }
 
 // y = A x or A^T x, or y += with ACC, any FP64 x.  Here every thread splits
@@ -130,6 +143,7 @@ StencilView stencil_view(const Handle &h) {
   StencilView v;
   v.S = h.st_S;
   v.nm = h.st_nm;
+  v.top = h.st_nm + h.st_rows;
   v.N = h.N;
   v.nax = h.nax;
   v.pl = h.nax * h.nay;
@@ -176,7 +190,7 @@ static bool row_storage(Handle &h, float2 **x, size_t *have, size_t len) {
   if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
       (rows ? 220 * N : 0) + (vec ? sizeof(float2) * len : 0) <= free_b / 2 &&
       (!rows || (!cudaMalloc(&h.st_S, sizeof(float2) * 27 * N) &&
-                 !cudaMalloc(&h.st_nm, sizeof(unsigned) * N))) &&
+                 !cudaMalloc(&h.st_nm, sizeof(unsigned) * (N + 1)))) &&
       (!vec || !cudaMalloc(x, sizeof(float2) * len))) {
     if (rows) h.st_rows = N;
     if (vec) *have = len;
@@ -213,8 +227,10 @@ cudaError_t ensure_stencil(Handle &h) {
   }
   const long need = (h.N + 255L) / 256;
   const int grid = (int)std::min<long>(need, (long)device_sm_count() * 32);
+  unsigned *top = h.st_nm + h.st_rows;
+  if ((e = cudaMemsetAsync(top, 0, sizeof(unsigned), h.stream))) return e;
   stencil_assemble<<<grid, 256, 0, h.stream>>>(h.Ahi, h.Alo, h.emask, h.nax, h.nay, h.naz,
-                                               h.st_S, h.st_nm);
+                                               h.st_S, h.st_nm, top);
   count_launches(1);
   e = cudaGetLastError();
   if (!e) h.st_state = 1;
@@ -234,9 +250,11 @@ cudaError_t ensure_segment_rows(Handle &h) {
   if (fresh && (e = cudaMemsetAsync(h.seg_x, 0, sizeof(float2) * have, h.stream))) return e;
   if ((e = launch_element_masks(h))) return e;
   const int per = (int)std::max<long>(1, std::min<long>(64, (h.seg_largest + 255) / 256));
+  unsigned *top = h.st_nm + h.st_rows;
+  if ((e = cudaMemsetAsync(top, 0, sizeof(unsigned), h.stream))) return e;
   stencil_assemble_meshes<<<dim3((unsigned)per, (unsigned)(h.seg_off.size() - 1)), 256, 0,
                             h.stream>>>(h.Ahi, h.Alo, h.emask, h.E, h.N, h.seg_mesh, h.st_S,
-                                        h.st_nm);
+                                        h.st_nm, top);
   count_launches(1);
   if (!(e = cudaGetLastError())) h.seg_rows = true;
   return e;

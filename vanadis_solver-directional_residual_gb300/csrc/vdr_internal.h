@@ -238,7 +238,7 @@ struct Handle {
   // st_state 0 not formed, 1 valid for the current operator, -1 no device
   // memory for it; st_applies: single applies of the current operator
   float2 *st_S = nullptr;       // [27][N]
-  unsigned *st_nm = nullptr;    // [N]
+  unsigned *st_nm = nullptr;    // [N], and the largest entry's exponent at [st_rows]
   float2 *st_x = nullptr;       // two padded pair vectors: p^ and s^
   size_t st_rows = 0, st_len = 0;  // nodes and pairs that they hold room for
   int st_nax = 0, st_pl = 0, st_n = 0;  // the mesh that st_x's pads are zero for
