@@ -307,6 +307,11 @@ int vdr_diag_wait_timeout(vdr_handle *h);
  * state.  Returns VDR_TIMEOUT when that path works (the handle stays
  * usable). */
 int vdr_diag_barrier_timeout(vdr_handle *h);
+/* Diagnostic of the bounded meetings of the whole-solve launches: one block
+ * of three never arrives, the others give up after ~1 ms, and one of them
+ * stores a solve's success all the same.  Returns VDR_TIMEOUT when that is
+ * what a solve would have returned (the handle stays usable). */
+int vdr_diag_meeting_timeout(vdr_handle *h);
 
 /* B[n*K + k] = cf * f(Q_k): the right-hand sides of K source fields at once.
  * d_Q is K x E (row k = per-element source of column k, kg/s, the caller's

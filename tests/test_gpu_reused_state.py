@@ -195,3 +195,24 @@ def test_systems_across_the_stores_range(vdr, oracle, gpu_lib, dims, power):
             xd.zero_()
             _, _, _, st = s.solve_segmented_device(bd * scale, xd, tol=1e-11, itmax=2000)
             assert st == 0 and rel_l2(xd.cpu().numpy(), sys_[5]) < 1e-9
+
+
+def test_meeting_times_out_and_recovers(vdr, oracle, gpu_lib):
+    """The meetings of the whole-solve launches are bounded: with one block of
+    three absent the others give up after ~1 ms, the call's outcome is the
+    timeout although one of them stores a success after it, and solves on the
+    same handle, cluster and grid forms of FP64 and mixed, run as before."""
+    import importlib
+    torch = pytest.importorskip("torch")
+    L = importlib.import_module(vdr.__name__ + "._lib")
+    for dims in ((12, 9, 8), (32, 24, 12)):
+        sys_ = system(vdr, oracle, dims, 37)
+        prob, _, b, _, x0, ref = sys_
+        for precision in ("fp64", "mixed"):
+            with vdr.Solver(prob, vdr.Options(precision=precision), aH=2.0, aM=10.0) as s:
+                for _ in range(2):
+                    assert s.lib.vdr_diag_meeting_timeout(s.h) == L.TIMEOUT
+                    x = torch.tensor(x0, device="cuda")
+                    _, err, st = s.solve_device(torch.tensor(b, device="cuda"), x, tol=1e-11,
+                                                itmax=2000)
+                    assert st == 0 and err <= 1e-11 and rel_l2(x.cpu().numpy(), ref) < 1e-9

@@ -406,13 +406,6 @@ __global__ void __launch_bounds__(T, 1) resident_half(ResHArgs a) {
   const int N = a.h.N, none[1] = {0};
   unsigned target = 0;
   const auto nothing = [](int) {};
-  const auto late = [&]() {
-    if (threadIdx.x == 0) {
-      a.st->status = VDR_TIMEOUT;
-      a.st->reason = 7;
-      a.st->done = 1;
-    }
-  };
   float x[PAIRS][2], r[PAIRS][2], p[PAIRS][2], v[PAIRS][2], t[PAIRS][2], rh[PAIRS][2],
       w[PAIRS][2], sc[PAIRS][2];  // r holds s between the two products
   const auto node = [&](int i) { return 2L * ((long)blockIdx.x * M + i * T + threadIdx.x); };
@@ -451,7 +444,7 @@ __global__ void __launch_bounds__(T, 1) resident_half(ResHArgs a) {
   {
     const double q[1] = {dot_val(d0)};
     if (!meet<IN_REGS, T, 1, 0, 1, AT_A, AT_A, 0>(sh, a.mt, q, none, target, nothing))
-      return late();
+      return;
   }
   const double bnrm2 = sh.tot[0];
   double rho = bnrm2, rr2 = bnrm2, al64 = 0.0, iwp = 0.0;
@@ -487,7 +480,7 @@ __global__ void __launch_bounds__(T, 1) resident_half(ResHArgs a) {
     const double q[1] = {dot_val(d0)};
     if (!meet<IN_REGS, T, 1, 0, 1, AT_D, AT_D, 0>(
             sh, a.mt, q, none, target, [&](int lane) { alpha_of(lane, sh.tot[0]); }))
-      return late();
+      return;
     if (sh.tot[0] == 0.0 || !isfinite(sh.tot[0])) {
       status = VDR_BREAKDOWN;
       reason = 2;
@@ -514,7 +507,7 @@ __global__ void __launch_bounds__(T, 1) resident_half(ResHArgs a) {
     {
       const double q[2] = {dot_val(d0), dot_val(d1)};
       if (!meet<IN_REGS, T, 2, 0, 0, AT_C, AT_C, 0>(sh, a.mt, q, none, target, nothing))
-        return late();
+        return;
     }
     clear();
 #pragma unroll
@@ -541,7 +534,7 @@ __global__ void __launch_bounds__(T, 1) resident_half(ResHArgs a) {
               sh.tot[5] = e;
             }
           }))
-        return late();
+        return;
     }
     const double ss = sh.tot[0], omega = sh.tot[1], ts = sh.tot[2], tt = sh.tot[3],
                  rho1 = sh.tot[4];
@@ -581,7 +574,7 @@ __global__ void __launch_bounds__(T, 1) resident_half(ResHArgs a) {
       const double q[2] = {dot_val(d0), dot_val(d1)};
       if (!meet<IN_REGS, T, 2, 0, 2, AT_A, AT_A, 0>(
               sh, a.mt, q, none, target, [&](int lane) { alpha_of(lane, sh.tot[1]); }))
-        return late();
+        return;
     }
     rr2 = sh.tot[0];
     const double wp = sh.tot[1];
@@ -729,8 +722,7 @@ int solve_half_rows(Handle &h, const double *res, double rnorm, double *x, doubl
   if (h.resident && h.N <= 4096 * sms) {
     ResHArgs ra{a.h, res, h.dinv, 1.0 / rnorm, rnorm, x, a.p, a.s, h.st, meet_args(h),
                 tol, itmax};
-    if ((e = cudaMemsetAsync(&h.st->bar_count, 0, sizeof(unsigned), s)))
-      return cuda_fail(e, "inner solve");
+    if ((e = meet_reset(h, s))) return cuda_fail(e, "inner solve");
     if (h.N <= 256 * sms) e = launch_resident_half<128, 1>(h.N, ra, s);
     else if (h.N <= 512 * sms) e = launch_resident_half<256, 1>(h.N, ra, s);
     else if (h.N <= 1024 * sms) e = launch_resident_half<512, 1>(h.N, ra, s);
@@ -742,9 +734,10 @@ int solve_half_rows(Handle &h, const double *res, double rnorm, double *x, doubl
       if ((e = cudaMemcpyAsync(&h.h_st[0], h.st, sizeof(KState), cudaMemcpyDeviceToHost, s)) ||
           (e = cudaStreamSynchronize(s)))
         return cuda_fail(e, "inner solve");
-      if (iter) *iter = h.h_st[0].iter;
-      if (err) *err = h.h_st[0].err;
-      return h.h_st[0].done ? h.h_st[0].status : VDR_NOT_CONVERGED;
+      const KState &fin = h.h_st[0];
+      if (iter) *iter = fin.late ? 0 : fin.iter;
+      if (err) *err = fin.late ? INFINITY : fin.err;
+      return outcome(fin);
     }
     cudaGetLastError();
     h.resident = false;

@@ -796,13 +796,14 @@ int solve_device(Handle &h, int method, const double *b, double *x,
           (e = cudaStreamSynchronize(s)))
         return cuda_fail(e, "solve");
       const KState &fin = h.h_st[0];
-      const int status = fin.done ? fin.status : VDR_NOT_CONVERGED;
-      h.last.iterations = fin.iter;
+      const int status = outcome(fin), n = fin.late ? 0 : fin.iter;
+      h.last.iterations = n;
       h.last.status = status;
       h.last.kernel_launches = 1;
-      h.last.breakdown = (status == VDR_BREAKDOWN || fin.reason == 6) ? fin.reason : 0;
-      if (iter) *iter = fin.iter;
-      if (err) *err = fin.err;
+      h.last.breakdown =
+          !fin.late && (status == VDR_BREAKDOWN || fin.reason == 6) ? fin.reason : 0;
+      if (iter) *iter = n;
+      if (err) *err = fin.late ? INFINITY : fin.err;
       return status;
     }
     cudaGetLastError();  // no cooperative launch here: the iteration as kernels
@@ -1963,6 +1964,10 @@ int solve_mixed_device(Handle &h, int method, const double *b, double *x,
       if (!(1.0 / rr[1] < INFINITY)) break;  // ||r|| at the denormal floor
       const int ist = solve_half_rows(h, r, rr[1], x, itol, inner_itmax, &it, &ierr);
       if (ist == VDR_CUDA_ERROR || ist == VDR_BAD_ARGUMENT) return ist;
+      if (ist == VDR_TIMEOUT) {  // x may lack a part of the correction
+        status = ist;
+        break;
+      }
     } else if (f32v) {
       // d solves A32 d = r / ||r|| on FP32 vectors; x += ||r|| d in FP64
       if (!(1.0 / rr[1] < INFINITY)) break;  // ||r|| at the denormal floor
@@ -1974,6 +1979,10 @@ int solve_mixed_device(Handle &h, int method, const double *b, double *x,
       const int ist = solve32_inner(h, itol, inner_itmax, &it, &ierr);
       h.apply_fp32 = false;
       if (ist == VDR_CUDA_ERROR || ist == VDR_BAD_ARGUMENT) return ist;
+      if (ist == VDR_TIMEOUT) {  // x may lack a part of the correction
+        status = ist;
+        break;
+      }
       k32_out<<<g, RED_THREADS, 0, s>>>(a32, x, rr[1],
                                         h.use_half ? h.dinv : nullptr);
       count_launches(1);
@@ -1984,6 +1993,10 @@ int solve_mixed_device(Handle &h, int method, const double *b, double *x,
       const int ist = solve_device(h, method, r, d, itol, inner_itmax, &it, &ierr);
       h.apply_fp32 = false;
       if (ist == VDR_CUDA_ERROR || ist == VDR_BAD_ARGUMENT) return ist;
+      if (ist == VDR_TIMEOUT) {  // x may lack a part of the correction
+        status = ist;
+        break;
+      }
       k_axpy1<<<g, RED_THREADS, 0, s>>>(a, d);
       count_launches(1);
     }

@@ -2,6 +2,7 @@
 // cooperative grid) that leave grid-wide sums behind.
 #pragma once
 #include <cuda_runtime.h>
+#include <stddef.h>
 
 #include "reduce.cuh"
 #include "vdr_internal.h"
@@ -21,6 +22,8 @@ struct MeetArgs {
   double *part;   // [SLOTS][gridDim]
   int *ipart;     // [3][gridDim]: largest exponents
   unsigned *bar;  // arrivals, zero at launch
+  unsigned *late;  // where a wait ran out
+  long long limit;  // clocks that a wait may take
 };
 
 struct ResShared {
@@ -130,7 +133,7 @@ __device__ __forceinline__ bool meet(ResShared &sh, const MeetArgs &a, const dou
         if (lane == 0) __stcg(a.ipart + (size_t)(ES + k) * B + blockIdx.x, e);
       }
       __syncwarp();
-            if (lane == 0)
+      if (lane == 0)
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
       __syncwarp();
       // the whole warp polls: with one lane polling, what followed ran split
@@ -139,11 +142,15 @@ __device__ __forceinline__ bool meet(ResShared &sh, const MeetArgs &a, const dou
       bool met, late = false;
       do {
         unsigned seen;
+        late = clock64() - t0 > a.limit;  // before the count is read: a pause
+                                          // of this CTA is not another's delay
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.bar) : "memory");
         met = (int)(seen - target) >= 0;
-        late = clock64() - t0 > RES_LIMIT;
       } while (!__all_sync(FULLR, met || late));
-      if (lane == 0) sh.ok = met;
+      if (lane == 0) {
+        sh.ok = met;
+        if (!met) *(volatile unsigned *)a.late = 1u;
+      }
       if (R > 0) {
         double in[RES_NB][RP];  // every load before the first add
 #pragma unroll
@@ -194,7 +201,12 @@ __device__ __forceinline__ bool meet(ResShared &sh, const MeetArgs &a, const dou
 
 inline MeetArgs meet_args(const Handle &h) {
   return MeetArgs{h.partials, reinterpret_cast<int *>(h.partials + SLOTS * 32 * RES_NB),
-                  &h.st->bar_count};
+                  &h.st->bar_count, &h.st->late, RES_LIMIT};
+}
+// No arrivals and nobody late.
+inline cudaError_t meet_reset(Handle &h, cudaStream_t s) {
+  static_assert(offsetof(KState, late) == offsetof(KState, bar_count) + sizeof(unsigned), "one fill");
+  return cudaMemsetAsync(&h.st->bar_count, 0, 2 * sizeof(unsigned), s);
 }
 
 }  // namespace vdr

@@ -23,7 +23,7 @@
 // partials lie in shared memory and are read across the cluster, the
 // meetings are cluster barriers.  IN_REGS, IN_SMEM: a cooperative grid, one
 // CTA per SM, p^ and s^ through L2, meetings at a counter (bounded waits:
-// VDR_TIMEOUT, reason 7); a node's 27 pairs stay in registers up to 512
+// VDR_TIMEOUT); a node's 27 pairs stay in registers up to 512
 // threads, in shared memory (216 bytes a thread) above.  Per iteration,
 // cluster / grid: 8.1 us at 448 nodes, 9.6 / 12 at 1,170, 11 / 12.5 at 2,800,
 // 19.5 / 12.8 at 7,000 (reads across a cluster are slow in number), then 14.1
@@ -51,14 +51,6 @@ struct ResArgs {
   double tol;
   int itmax, window;
 };
-
-__device__ __forceinline__ void res_timeout(KState *st) {
-  if (threadIdx.x == 0) {
-    st->status = VDR_TIMEOUT;
-    st->reason = 7;
-    st->done = 1;
-  }
-}
 
 __device__ __forceinline__ double row_value(const DfAcc &acc, int shift) {
   double o = df_to_double(acc.s, acc.c);
@@ -137,14 +129,14 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
     const double z[1] = {0.0};
     const int e1[1] = {df_exp(x)};
     if (!meet<MODE, T, 1, 1, 0, AT_C, AT_C, 2>(sh, a.mt, z, e1, target, nothing))
-      return res_timeout(a.st);
+      return;
   }
   const int ex = sh.etot[0];
   if (ex) {
     put(0, masked_pair(msk, x, ex - base));
     const double z[1] = {0.0};
     if (!meet<MODE, T, 1, 0, 0, AT_D, AT_D, 0>(sh, a.mt, z, none, target, nothing))
-      return res_timeout(a.st);
+      return;
     v = row(0, ex - base);
   }
   {
@@ -154,7 +146,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
     const double q[2] = {bi * bi, r * r};
     const int em[2] = {df_exp(r), df_exp(msk ? 0.0 : r * di)};
     if (!meet<MODE, T, 2, 2, 2, AT_A, AT_A, 0>(sh, a.mt, q, em, target, nothing))
-      return res_timeout(a.st);
+      return;
   }
   const double bnrm2 = sh.tot[0];
   double rho = sh.tot[1], rr2 = rho;
@@ -192,7 +184,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
     put(1, masked_pair(msk, rh, er - base));
     double q[1] = {0.0};
     if (!meet<MODE, T, 1, 0, 0, AT_C, AT_C, 0>(sh, a.mt, q, none, target, nothing))
-      return res_timeout(a.st);
+      return;
     DfAcc acc{0.f, 0.f};
     for (int z = 0; z < 27; z += 9)
 #pragma unroll
@@ -211,7 +203,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
     if (!msk) q[0] = wn * (p * di);
     if (!meet<MODE, T, 1, 0, 1, AT_D, AT_D, 0>(sh, a.mt, q, none, target,
                                             [&](int lane) { alpha_of(lane, sh.tot[0]); }))
-      return res_timeout(a.st);
+      return;
     if (sh.tot[0] == 0.0 || !isfinite(sh.tot[0])) {
       status = VDR_BREAKDOWN;
       reason = 2;
@@ -229,7 +221,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
     {
       const double q[2] = {s * s, rh * s};
       if (!meet<MODE, T, 2, 0, 0, AT_C, AT_C, 0>(sh, a.mt, q, none, target, nothing))
-        return res_timeout(a.st);
+        return;
     }
     t = row(1, shift);
     // omega = ts / tt and beta = (rho' / rho) (alpha / omega) = (rhs tt / ts -
@@ -249,7 +241,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
               sh.tot[5] = e;
             }
           }))
-        return res_timeout(a.st);
+        return;
     }
     const double ss = sh.tot[0], om = sh.tot[1], ts = sh.tot[2], tt = sh.tot[3],
                  rho1 = sh.tot[4], beta = sh.tot[5];
@@ -276,7 +268,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
       const int em[1] = {df_exp(ph)};
       if (!meet<MODE, T, 2, 1, 2, AT_A, AT_A, 0>(sh, a.mt, q, em, target,
                                               [&](int lane) { alpha_of(lane, sh.tot[1]); }))
-        return res_timeout(a.st);
+        return;
     }
     pexp = pmax;
     pmax = sh.etot[0];
@@ -393,14 +385,14 @@ __global__ void __launch_bounds__(T, 1) resident_bicg(ResArgs a) {
     const double q[1] = {0.0};
     const int e1[1] = {df_exp(x)};
     if (!meet<MODE, T, 1, 1, 0, AT_C, AT_C, 2>(sh, a.mt, q, e1, target, nothing))
-      return res_timeout(a.st);
+      return;
   }
   const int ex = sh.etot[0];
   if (ex) {
     if (on) a.php[n] = masked_pair(msk, x, ex - base);
     const double q[1] = {0.0};
     if (!meet<MODE, T, 1, 0, 0, AT_D, AT_D, 0>(sh, a.mt, q, none, target, nothing))
-      return res_timeout(a.st);
+      return;
     z = row(ex - base);
   }
   {
@@ -410,7 +402,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicg(ResArgs a) {
     const double q[3] = {bi * bi, r * r, (r * di) * rr};
     const int e1[1] = {df_exp(msk ? 0.0 : r * di)};
     if (!meet<MODE, T, 3, 1, 3, AT_A - 1, AT_A - 1, 0>(sh, a.mt, q, e1, target, nothing))
-      return res_timeout(a.st);
+      return;
   }
   const double bnrm2 = sh.tot[0], thr = a.tol * a.tol * bnrm2;
   double rr2 = sh.tot[1], bknum = sh.tot[2], bk = 0.0;
@@ -442,7 +434,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicg(ResArgs a) {
     {
       const double q[1] = {0.0};
       if (!meet<MODE, T, 1, 0, 0, AT_C, AT_C, 0>(sh, a.mt, q, none, target, nothing))
-        return res_timeout(a.st);
+        return;
     }
     z = row(pexp - base);
     zz = trans(qexp - base);
@@ -453,7 +445,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicg(ResArgs a) {
             const double d = bknum / sh.tot[0];
             if (lane == 0) sh.tot[1] = d;
           }))
-        return res_timeout(a.st);
+        return;
     }
     const double ak = sh.tot[1];
     pexp = sh.etot[0];
@@ -472,7 +464,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicg(ResArgs a) {
             const double d = sh.tot[1] / bknum;
             if (lane == 0) sh.tot[2] = d;
           }))
-        return res_timeout(a.st);
+        return;
     }
     rr2 = sh.tot[0];
     bknum = sh.tot[1];
@@ -496,6 +488,22 @@ __global__ void __launch_bounds__(T, 1) resident_bicg(ResArgs a) {
     st->err = bnrm2 > 0.0 ? sqrt(rr2) / sqrt(bnrm2) : 0.0;
     st->status = status;
     st->reason = reason;
+    st->done = 1;
+  }
+}
+
+// A meeting that one CTA of three never comes to, with a short limit; CTA 2
+// stores a solve's end all the same.
+__global__ void __launch_bounds__(32, 1) absent_kernel(MeetArgs mt, KState *st) {
+  __shared__ ResShared sh;
+  if (blockIdx.x == 1) return;
+  unsigned target = 0;
+  const double q[1] = {0.0};
+  const int none[1] = {0};
+  const bool met =
+      meet<IN_REGS, 32, 1, 0, 0, AT_C, AT_C, 0>(sh, mt, q, none, target, [](int) {});
+  if (blockIdx.x == 2 && threadIdx.x == 0) {
+    st->status = met ? VDR_BREAKDOWN : VDR_OK;
     st->done = 1;
   }
 }
@@ -544,6 +552,37 @@ int cluster_ctas(int N, int T) {
 
 }  // namespace
 
+// VDR_TIMEOUT when the meeting's waits ran out of their (about 1 ms) limit and
+// that, not the status stored after them, is what a solve would return.
+int diag_meeting_timeout(Handle &h) {
+  cudaError_t e = ensure_solver_workspace(h, 8);
+  cudaStream_t s = h.stream;
+  if (e || (e = cudaMemsetAsync(h.st, 0, sizeof(KState), s))) return cuda_fail(e, "diag");
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(3);
+  cfg.blockDim = dim3(32);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  MeetArgs mt = meet_args(h);
+  mt.limit = 2000000LL;
+  if ((e = cudaLaunchKernelEx(&cfg, absent_kernel, mt, h.st))) return cuda_fail(e, "diag launch");
+  count_launches(1);
+  KState fin;
+  if ((e = cudaMemcpyAsync(&fin, h.st, sizeof(KState), cudaMemcpyDeviceToHost, s)) ||
+      (e = cudaStreamSynchronize(s)))
+    return cuda_fail(e, "diag");
+  if (fin.done && fin.status == VDR_OK && outcome(fin) == VDR_TIMEOUT) {
+    set_error("diag: the meeting's wait ran out (as intended)");
+    return VDR_TIMEOUT;
+  }
+  set_error("diag: the meeting did not report its timeout");
+  return VDR_CUDA_ERROR;
+}
+
 bool resident_fits(const Handle &h) {
   return h.resident && stencil_ready(h) &&
          h.N <= 1024L * std::min(device_sm_count(), 32 * RES_NB);
@@ -552,7 +591,7 @@ bool resident_fits(const Handle &h) {
 cudaError_t launch_resident(Handle &h, int method, const double *b, double *x, double tol,
                             int itmax, int stall_window) {
   cudaError_t e;
-  if ((e = cudaMemsetAsync(&h.st->bar_count, 0, sizeof(unsigned), h.stream))) return e;
+  if ((e = meet_reset(h, h.stream))) return e;
   ResArgs a{};
   a.w = stencil_view(h);
   a.b = b;

@@ -35,7 +35,9 @@ struct KState {
   int x_zero;  // the initial guess is zero (its apply is skipped)
   unsigned int ticket;
   unsigned int pad2;
-  unsigned int bar_count, bar_gen;  // grid barrier of the fused inner kernels
+  unsigned int bar_count;  // arrivals: grid barriers, meetings of a whole-solve launch
+  unsigned int late;       // set where a meeting's wait ran out, cleared before a launch only
+  unsigned int bar_gen;
   // the assembled-operator iteration: (rh, s), the next rho, the exponent that
   // its pair vectors are scaled by, the largest exponents of the last
   // direction, of the one being formed and of the first residual
@@ -48,6 +50,13 @@ struct KState {
 // same for a second pair 2^k bytes away in x and 2^(k+1) in b).
 using GraphKey = std::array<uintptr_t, 10>;
 inline uintptr_t key_of(const void *p) { return reinterpret_cast<uintptr_t>(p); }
+
+// The outcome of a launch whose CTAs meet.  A CTA that gives up in the last
+// meeting has arrived there: the others finish, and their status stands in
+// the state while that CTA's part of x is not written.
+inline int outcome(const KState &k) {
+  return k.late ? VDR_TIMEOUT : k.done ? k.status : VDR_NOT_CONVERGED;
+}
 
 // A right preconditioner for BiCGStab beyond Jacobi: `enqueue` adds
 // (M(in) - D^-1 in) to `out`, which already holds D^-1 in (zero on
@@ -428,6 +437,7 @@ cudaError_t launch_apply_both(const Handle &h, const double *x1, double *y1,
 int diag_wait_timeout(Handle &h);
 // The same for the grid barrier of the fused inner kernels (krylov.cu).
 int diag_barrier_timeout(Handle &h);
+int diag_meeting_timeout(Handle &h);
 // The FP32 operator (A32v) on FP32 vectors, y += A x (stored mode only).
 cudaError_t launch_stored_apply32v(const Handle &h, const float *x, float *y,
                                    const int *skip, const int *skip2,
