@@ -216,3 +216,61 @@ def test_meeting_times_out_and_recovers(vdr, oracle, gpu_lib):
                     _, err, st = s.solve_device(torch.tensor(b, device="cuda"), x, tol=1e-11,
                                                 itmax=2000)
                     assert st == 0 and err <= 1e-11 and rel_l2(x.cpu().numpy(), ref) < 1e-9
+
+
+CLUSTER, WHOLE_SOLVE, ROWS = 1, 2, 4
+
+
+def test_segmented_solve_after_rows_were_refused(vdr, oracle, gpu_lib):
+    """Rows formed by a segmented solve, then a plain solve for whose pair
+    vectors there is no room (all rows go), then the segmented solve again."""
+    torch = pytest.importorskip("torch")
+    sys_ = system(vdr, oracle, (12, 9, 8), 38)
+    prob, _, b, _, x0, ref = sys_
+    bd = torch.tensor(b, device="cuda")
+    with vdr.Solver(prob, aH=2.0, aM=10.0) as s:
+        s.set_segments(np.array([0, s.N]))
+
+        def segmented():
+            x = torch.tensor(x0, device="cuda")
+            _, _, _, st = s.solve_segmented_device(bd, x, tol=1e-11, itmax=2000)
+            assert st == 0 and rel_l2(x.cpu().numpy(), ref) < 1e-9
+
+        segmented()
+        assert s.lib.vdr_diag_without(s.h, ROWS) == 0
+        x = torch.tensor(x0, device="cuda")
+        _, _, st = s.solve_device(bd, x, tol=1e-11, itmax=2000)
+        assert st == 0 and rel_l2(x.cpu().numpy(), ref) < 1e-9
+        for without in (ROWS, 0):
+            assert s.lib.vdr_diag_without(s.h, without) == 0
+            segmented()
+            s.set_operator(2.0, 10.0)
+
+
+@pytest.mark.parametrize("without", [CLUSTER, WHOLE_SOLVE, CLUSTER | WHOLE_SOLVE, ROWS,
+                                     CLUSTER | WHOLE_SOLVE | ROWS])
+@pytest.mark.parametrize("dims", [(12, 9, 8), (32, 24, 12)])
+def test_solves_without(vdr, oracle, gpu_lib, dims, without):
+    """What the solves fall back to where the device refuses clusters, whole
+    solves in one launch, or memory for rows: the same solutions."""
+    torch = pytest.importorskip("torch")
+    sys_ = system(vdr, oracle, dims, 39)
+    prob, _, b, _, x0, ref = sys_
+    bd = torch.tensor(b, device="cuda")
+    for opts in ({}, {"solver": "bicg"}, {"precision": "mixed"}):
+        with vdr.Solver(prob, vdr.Options(**opts), aH=2.0, aM=10.0) as s:
+            assert s.lib.vdr_diag_without(s.h, without) == 0
+            s.set_segments(np.array([0, s.N]))
+            calls = [lambda x: s.solve_device(bd, x, tol=1e-11, itmax=2000)[2]]
+            if not opts:
+                calls += [lambda x: s.solve_segmented_device(bd, x, tol=1e-11, itmax=2000)[3],
+                          lambda x: s.solve_gcr_device(bd, x, tol=1e-11, itmax=2000)[2]]
+            for call in calls:
+                for start in (np.zeros_like(x0), x0):
+                    x = torch.tensor(start, device="cuda")
+                    assert call(x) == 0
+                    assert rel_l2(x.cpu().numpy(), ref) < 1e-9
+            if not opts:
+                X = torch.tensor(x0, device="cuda")[:, None].repeat(1, 16)
+                _, _, errs, st = s.solve_block_device(bd[:, None].repeat(1, 16), X, tol=1e-11)
+                assert st == 0 and rel_l2(X[:, 7].cpu().numpy(), ref) < 1e-9

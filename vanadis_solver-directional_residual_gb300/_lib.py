@@ -80,6 +80,7 @@ SIGNATURES = {
     "vdr_diag_wait_timeout": (_i, [_P]),
     "vdr_diag_barrier_timeout": (_i, [_P]),
     "vdr_diag_meeting_timeout": (_i, [_P]),
+    "vdr_diag_without": (_i, [_P, _i]),
     "vdr_set_mixed_operator": (_i, [_P, _i]),
     "vdr_set_build_mode": (_i, [_P, _i]),
     "vdr_diag_beta_vf": (_i, [_i, _D, _D]),

@@ -1106,6 +1106,19 @@ int vdr_diag_wait_timeout(vdr_handle *H) {
   return diag_wait_timeout(H->h);
 }
 
+int vdr_diag_without(vdr_handle *H, int what) {
+  int st = check_handle(H);
+  if (st) return st;
+  if (what < 0 || what > (VDR_WITHOUT_CLUSTER | VDR_WITHOUT_WHOLE_SOLVE | VDR_WITHOUT_ROWS)) {
+    set_error("vdr_diag_without: unknown bits");
+    return VDR_BAD_ARGUMENT;
+  }
+  H->h.resident_cluster = !(what & VDR_WITHOUT_CLUSTER);
+  H->h.resident = !(what & VDR_WITHOUT_WHOLE_SOLVE);
+  H->h.rows_room = !(what & VDR_WITHOUT_ROWS);
+  return VDR_OK;
+}
+
 int vdr_diag_meeting_timeout(vdr_handle *H) {
   int st = check_handle(H);
   if (st) return st;

@@ -885,7 +885,7 @@ bool block_rows_usable(Handle &h, int K, BlockRows *g) {
     cudaFree(h.br_rows);
     h.br_rows = nullptr;
     h.br_words = 0;
-    if (cudaMalloc(&h.br_rows, sizeof(float) * words)) {
+    if (!h.rows_room || cudaMalloc(&h.br_rows, sizeof(float) * words)) {
       cudaGetLastError();
       return false;
     }

@@ -666,7 +666,7 @@ int ensure_half_rows(Handle &h) {
   if (!h.hr_H) {
     const size_t need = 54 * Np + Np + sizeof(float) * (6 * Np + 2 * V);
     size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || need > free_b / 2 ||
+    if (!h.rows_room || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || need > free_b / 2 ||
         cudaMalloc(&h.hr_H, 54 * Np) || cudaMalloc(&h.hr_e, Np) ||
         cudaMalloc(&h.hr_vec, sizeof(float) * (6 * Np + 2 * V)) ||
         cudaMemsetAsync(h.hr_vec, 0, sizeof(float) * (6 * Np + 2 * V), h.stream)) {

@@ -187,7 +187,7 @@ static bool row_storage(Handle &h, float2 **x, size_t *have, size_t len) {
     h.st_nax = 0;  // its pads are to be zeroed
   }
   size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
+  if (h.rows_room && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
       (rows ? 220 * N : 0) + (vec ? sizeof(float2) * len : 0) <= free_b / 2 &&
       (!rows || (!cudaMalloc(&h.st_S, sizeof(float2) * 27 * N) &&
                  !cudaMalloc(&h.st_nm, sizeof(unsigned) * (N + 1)))) &&
@@ -205,6 +205,7 @@ static bool row_storage(Handle &h, float2 **x, size_t *have, size_t len) {
   *x = nullptr;
   *have = h.st_rows = 0;
   h.st_state = -1;
+  h.seg_rows = false;  // they were these rows
   return false;
 }
 

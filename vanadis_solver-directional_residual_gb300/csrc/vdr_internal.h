@@ -262,6 +262,7 @@ struct Handle {
   cudaGraphExec_t hr_graph = nullptr;
   bool resident = true;  // whole solves in one launch (resident.cu) ...
   bool resident_cluster = true;  // ... of one cluster where they fit
+  bool rows_room = true;  // false: as if no memory were left for assembled rows
 
   // solver workspace
   double *work = nullptr;
