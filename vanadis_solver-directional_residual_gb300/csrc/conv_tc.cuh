@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int row = 32 * q + lane;
     float bias[RAW ? 1 : COUT];
 #pragma unroll
-    for (int c = 0; c < (RAW ? 1 : COUT); c++) bias[c] = a.bias ? __ldg(a.bias + c) : 0.f;
+    for (int c = 0; c < (RAW ? 1 : COUT); c++) bias[c] = a.bias ? a.bias[c] : 0.f;
     int it = 0;
     for (int t = blockIdx.x; t < a.ntiles; t += gridDim.x, it++) {
       const int b = it & 1;

@@ -343,12 +343,11 @@ struct WgArgs {
 // dyt[c][row][x] = dY[v][c] where Y[v][c] > 0 (the ReLU's derivative), v =
 // row W + x; zero in the rows' padding x in [W, Wp) (the buffer is shared
 // by layers of other shapes).  One block per x row, one thread per padded
-// voxel: its C channels in 16-byte loads, and per channel a coalesced store
-// across the row.  dyc (may be null): the same values channels-last, [V][C].
+// voxel: its C channels in 16-byte loads, up to 32 of them before the first
+// store, and per channel a coalesced store across the row.  dyc (may be null): the same values channels-last, [V][C].
 template <int C>
-__global__ void mask_transpose(const float *__restrict__ dy, const bf16 *__restrict__ y,
-                               bf16 *__restrict__ dyt, bf16 *__restrict__ dyc, int W, int Wp,
-                               long Vp) {
+__global__ void mask_transpose(const float *dy, const bf16 *y, bf16 *dyt, bf16 *dyc, int W,
+                               int Wp, long Vp) {
   chain_wait();
   static_assert(C % 8 == 0, "channels");
   const long row = blockIdx.x;
@@ -362,11 +361,22 @@ __global__ void mask_transpose(const float *__restrict__ dy, const bf16 *__restr
     const long v = row * W + x;
     const float4 *dp = reinterpret_cast<const float4 *>(dy + v * C);
     const uint4 *yp = reinterpret_cast<const uint4 *>(y + v * C);
+    constexpr int A = C / 8 < 4 ? C / 8 : 4;
+    uint4 ym[A];
+    float4 dm[2 * A];
 #pragma unroll
     for (int c8 = 0; c8 < C / 8; c8++) {
-      const uint4 ym = yp[c8];
-      const float4 d0 = dp[2 * c8], d1 = dp[2 * c8 + 1];
-      const uint32_t yw[4] = {ym.x, ym.y, ym.z, ym.w};
+      if (c8 % A == 0) {
+#pragma unroll
+        for (int k = 0; k < A; k++) {
+          ym[k] = yp[c8 + k];
+          dm[2 * k] = dp[2 * (c8 + k)];
+          dm[2 * k + 1] = dp[2 * (c8 + k) + 1];
+        }
+      }
+      const uint4 yv = ym[c8 % A];
+      const float4 d0 = dm[2 * (c8 % A)], d1 = dm[2 * (c8 % A) + 1];
+      const uint32_t yw[4] = {yv.x, yv.y, yv.z, yv.w};
       const float dv[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
       float mv[8];
 #pragma unroll
@@ -618,8 +628,8 @@ __global__ void pool_fwd(const bf16 *in, bf16 *out, Dims f, Dims c, int C,
     for (int t = 0; t < 8; t++) {
       const int x = 2 * X + (t & 1), y = 2 * Y + ((t >> 1) & 1), z = 2 * Z + (t >> 2);
       if (x < f.W && y < f.H && z < f.D) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(
-                                  in + ((long)x + (long)f.W * (y + (long)f.H * z)) * C) + ch);
+        const uint4 v = reinterpret_cast<const uint4 *>(
+            in + ((long)x + (long)f.W * (y + (long)f.H * z)) * C)[ch];
         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int k = 0; k < 4; k++) {
@@ -655,7 +665,7 @@ __global__ void pool_bwd_add(const float *gc, float *gf, Dims f, Dims c, int C) 
     const int X = x >> 1, Y = y >> 1, Z = z >> 1;
     const long P = (long)X + (long)c.W * (Y + (long)c.H * Z);
     const float n = (float)child_count(X, Y, Z, f);
-    const float4 g = __ldg(reinterpret_cast<const float4 *>(gc) + P * c4 + ch);
+    const float4 g = reinterpret_cast<const float4 *>(gc)[P * c4 + ch];
     float4 o = reinterpret_cast<const float4 *>(gf)[idx];
     o.x += g.x / n;
     o.y += g.y / n;
@@ -677,7 +687,7 @@ __global__ void upcat_bwd_skip(const float *gcat, float *gskip, long V, int C1, 
     const long v = idx / c4;
     const int ch = (int)((unsigned)idx % (unsigned)c4);
     reinterpret_cast<float4 *>(gskip)[idx] =
-        __ldg(reinterpret_cast<const float4 *>(gcat) + v * t4 + ch);
+        reinterpret_cast<const float4 *>(gcat)[v * t4 + ch];
   }
 }
 __global__ void upcat_bwd_coarse(const float *gcat, float *gc, Dims f, Dims c,
@@ -696,8 +706,8 @@ __global__ void upcat_bwd_coarse(const float *gcat, float *gc, Dims f, Dims c,
     for (int t = 0; t < 8; t++) {
       const int x = 2 * X + (t & 1), y = 2 * Y + ((t >> 1) & 1), z = 2 * Z + (t >> 2);
       if (x < f.W && y < f.H && z < f.D) {
-        const float4 g = __ldg(reinterpret_cast<const float4 *>(gcat) +
-                               ((long)x + (long)f.W * (y + (long)f.H * z)) * t4 + C1 / 4 + ch);
+        const float4 g = reinterpret_cast<const float4 *>(
+            gcat)[((long)x + (long)f.W * (y + (long)f.H * z)) * t4 + C1 / 4 + ch];
         s.x += g.x;
         s.y += g.y;
         s.z += g.z;
@@ -823,8 +833,8 @@ __global__ void pack_weights(const float *th, bf16 *wb, bf16 *wbt, bf16 *wtc, bf
 // bytes of a coarse voxel to its up to eight fine ones (one thread per fine
 // unit, with its 64-bit divisions: 24 us at 129 x 129 x 65 voxels and 32
 // channels, so 15).
-__global__ void upsample_bf16(const bf16 *__restrict__ in, bf16 *__restrict__ out, Dims f, Dims c,
-                              int C, const int *skip, const int *skip2) {
+__global__ void upsample_bf16(const bf16 *in, bf16 *out, Dims f, Dims c, int C, const int *skip,
+                              const int *skip2) {
   chain_wait();
   if (skipped(skip, skip2)) return;
   const int c8 = C / 8;
@@ -835,7 +845,7 @@ __global__ void upsample_bf16(const bf16 *__restrict__ in, bf16 *__restrict__ ou
     const unsigned vc = (unsigned)(i / c8);
     const int X = (int)(vc % (unsigned)c.W), r = (int)(vc / (unsigned)c.W);
     const int Y = r % c.H, Z = r / c.H;
-    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(in) + i);
+    const uint4 v = reinterpret_cast<const uint4 *>(in)[i];
 #pragma unroll
     for (int t = 0; t < 8; t++) {
       const int x = 2 * X + (t & 1), y = 2 * Y + ((t >> 1) & 1), z = 2 * Z + (t >> 2);
