@@ -59,10 +59,10 @@ extern "C" {
 
 /* ---- scatter of element results to nodes ---- */
 #define VDR_SCATTER_AUTO 0   /* measured choice: on the structured numbering
-                                (natural order, double-float store) solves,
-                                and applies from an operator's second on, sum
-                                the element matrices into 27-point rows and
-                                gather; atomic elsewhere */
+                                (natural order, double-float store) solves
+                                sum the element matrices into 27-point rows
+                                and gather; atomic elsewhere and for
+                                vdr_apply* */
 #define VDR_SCATTER_ATOMIC 1 /* fp64 atomics, elements in natural order */
 #define VDR_SCATTER_COLOR 2  /* colour by colour, no atomics, deterministic */
 #define VDR_SCATTER_WARP 3   /* fp64 atomics aggregated within a warp: on the

@@ -274,3 +274,55 @@ def test_solves_without(vdr, oracle, gpu_lib, dims, without):
                 X = torch.tensor(x0, device="cuda")[:, None].repeat(1, 16)
                 _, _, errs, st = s.solve_block_device(bd[:, None].repeat(1, 16), X, tol=1e-11)
                 assert st == 0 and rel_l2(X[:, 7].cpu().numpy(), ref) < 1e-9
+
+
+def test_applies_leave_no_rows_behind(vdr, oracle, gpu_lib):
+    """A caller's applies take one kernel and no memory each, however many
+    they are, and their products do not change when a solve has formed rows:
+    each against the oracle's element matrices to 1e-13 (FP64 sums of pair
+    products, 2^-47 each)."""
+    torch = pytest.importorskip("torch")
+    prob, bb, b = system(vdr, oracle, (33, 17, 21), 40)[:3]
+    m = prob.mesh
+    x = np.random.default_rng(8).standard_normal(m.nnode)
+    xd, bd = torch.tensor(x, device="cuda"), torch.tensor(b, device="cuda")
+    y = torch.empty_like(xd)
+    ref = [oracle.matvec0(m.iss, bb, prob.bc, x, transpose=t)[0] for t in (False, True)]
+    with vdr.Solver(prob, aH=2.0, aM=10.0) as s:
+        s.apply_device(xd, y)  # builds the operator
+        s.solve_gcr_device(bd, torch.zeros_like(bd), tol=1e-8, itmax=5)
+        s.set_operator(2.0, 10.0)
+        for solved in (False, True):
+            s.apply_device(xd, y)
+            if solved:
+                s.solve_device(bd, torch.zeros_like(bd), tol=1e-8, itmax=500)
+            torch.cuda.synchronize()
+            free, launches = torch.cuda.mem_get_info()[0], vdr.kernel_launch_count()
+            for k in range(4):
+                s.apply_device(xd, y, transpose=k % 2 == 1)
+                torch.cuda.synchronize()
+                assert rel_l2(y.cpu().numpy(), ref[k % 2]) < 1e-13, (solved, k)
+                s.apply_accumulate_device(xd, y, transpose=k % 2 == 1)
+            assert vdr.kernel_launch_count() - launches == 8
+            assert torch.cuda.mem_get_info()[0] == free
+
+
+def test_products_on_rows_in_training(vdr, gpu_lib):
+    """The residual loss's gradient, A and A^T in it, before and after a solve
+    formed the operator's rows: apart by the gradient's own atomics (2e-7) and
+    what 1e-14 in the products turns over in FP32 and BF16 roundings."""
+    torch = pytest.importorskip("torch")
+    prob = vdr.problems.rotation_shear(17, 12, 9, seed=41)
+    free = torch.tensor(prob.bc == 0, device="cuda")
+    b = torch.tensor(np.cos(0.37 * np.arange(prob.mesh.nnode)), device="cuda") * free
+    with vdr.Solver(prob, aH=2.0, aM=10.0) as s, vdr.LearnedNet(s, seed=5) as net:
+        net.update_features()
+        rhat = (torch.randn(s.N, dtype=torch.float64, device="cuda") * free).float()
+        got = []
+        for solved in (False, True):
+            if solved:
+                s.solve_device(b, torch.zeros_like(b), tol=1e-10, itmax=500)
+            loss = net.residual_loss_grad(rhat)
+            got.append((loss, net.get_grads().astype(np.float64)))
+        assert abs(got[0][0] - got[1][0]) <= 1e-6 * abs(got[0][0])
+        assert rel_l2(got[1][1], got[0][1]) < 1e-4

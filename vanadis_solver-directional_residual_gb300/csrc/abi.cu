@@ -373,15 +373,6 @@ void invalidate(Handle &h) {
   if (h.st_state > 0) h.st_state = 0;
   if (h.hr_state > 0) h.hr_state = 0;
   h.seg_rows = false;
-  h.st_applies = 0;
-}
-
-// Single applies: the rows are assembled at the second apply of an operator.
-// Summing them moves 732 bytes a node where an apply then saves 308, so the
-// third apply has paid for it; one apply per operator stays element-wise.
-cudaError_t rows_for_apply(Handle &h) {
-  if (foreign_capture(h, h.stream)) return cudaSuccess;
-  return ++h.st_applies >= 2 ? ensure_stencil(h) : cudaSuccess;
 }
 
 // d64[c][p] = src[c][perm[p]] (perm null: identity), d32 the FP32 copy.
@@ -741,14 +732,10 @@ int vdr_apply_device(vdr_handle *H, const double *x, double *y, int transpose) {
     return VDR_BAD_ARGUMENT;
   }
   if ((st = ensure_operator(h))) return st;
-  cudaError_t e = rows_for_apply(h);
-  if (!e && stencil_ready(h) && !foreign_capture(h, h.stream)) {
-    e = launch_stencil_apply(h, transpose != 0, false, x, y, nullptr, nullptr, h.stream);
-    return e ? cuda_fail(e, "apply") : VDR_OK;
-  }
-  if (e || (e = cudaMemsetAsync(y, 0, sizeof(double) * h.N, h.stream)))
+  cudaError_t e;
+  if ((e = cudaMemsetAsync(y, 0, sizeof(double) * h.N, h.stream)))
     return cuda_fail(e, "memset");
-  if ((e = launch_apply(h, transpose != 0, x, y, nullptr, nullptr, h.stream)))
+  if ((e = launch_element_apply(h, transpose != 0, x, y, nullptr, nullptr, h.stream)))
     return cuda_fail(e, "apply");
   return VDR_OK;
 }
@@ -763,8 +750,7 @@ int vdr_apply_accumulate_device(vdr_handle *H, const double *x, double *y,
     return VDR_BAD_ARGUMENT;
   }
   if ((st = ensure_operator(h))) return st;
-  cudaError_t e = rows_for_apply(h);
-  if (!e) e = launch_apply(h, transpose != 0, x, y, nullptr, nullptr, h.stream);
+  cudaError_t e = launch_element_apply(h, transpose != 0, x, y, nullptr, nullptr, h.stream);
   return e ? cuda_fail(e, "apply") : VDR_OK;
 }
 

@@ -959,14 +959,19 @@ cudaError_t launch_bc_to_mask(const int *bc, unsigned char *mask, int N,
   return cudaGetLastError();
 }
 
+cudaError_t launch_element_apply(const Handle &h, bool transpose, const double *x, double *y,
+                                 const int *skip, const int *skip2, cudaStream_t s) {
+  if (h.apply_mode == VDR_APPLY_MATRIX_FREE)
+    return launch_mf_apply(op_args(h), h.apply_fp32, transpose, x, y, skip, skip2, s);
+  return launch_stored_apply(h, h.apply_fp32, transpose, x, y, skip, skip2, s);
+}
+
 cudaError_t launch_apply(const Handle &h, bool transpose, const double *x,
                          double *y, const int *skip, const int *skip2,
                          cudaStream_t s) {
-  if (h.apply_mode == VDR_APPLY_MATRIX_FREE)
-    return launch_mf_apply(op_args(h), h.apply_fp32, transpose, x, y, skip, skip2, s);
   if (stencil_ready(h) && !foreign_capture(h, s))
-    return launch_stencil_apply(h, transpose, true, x, y, skip, skip2, s);
-  return launch_stored_apply(h, h.apply_fp32, transpose, x, y, skip, skip2, s);
+    return launch_stencil_apply(h, transpose, x, y, skip, skip2, s);
+  return launch_element_apply(h, transpose, x, y, skip, skip2, s);
 }
 
 }  // namespace vdr

@@ -2019,7 +2019,8 @@ int true_residual_device(Handle &h, const double *b, const double *x,
   double *ax = a.t;
   double *out = a.sh;  // scalar scratch
   if ((e = cudaMemsetAsync(ax, 0, sizeof(double) * h.N, s))) return cuda_fail(e, "memset");
-  if ((e = launch_apply(h, false, x, ax, nullptr, nullptr, s))) return cuda_fail(e, "apply");
+  if ((e = launch_element_apply(h, false, x, ax, nullptr, nullptr, s)))
+    return cuda_fail(e, "apply");
   const int g = red_grid(h.N);
   k_true_residual<<<g, RED_THREADS, 0, s>>>(a, ax, h.partials, &h.st->ticket, out);
   count_launches(1);

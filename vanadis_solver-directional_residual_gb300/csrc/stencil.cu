@@ -110,11 +110,16 @@ __global__ void __launch_bounds__(256, 2) stencil_assemble_meshes(
   raise_top(big, top);
 }
 
-// y = A x or A^T x, or y += with ACC, any FP64 x.  Here every thread splits
-// its 27 gathered values and scales each plane by itself, which makes it
-// bound by instruction issue (0.75 ms at 8.5M nodes, 94 us at 1.08M: about
-// the element-wise apply's time); the Krylov iterations split once per node.
-template <bool TRANS, bool ACC, bool KEEP>
+// y += A x or A^T x, any FP64 x, for the products of solvers that keep FP64
+// vectors (GCR, a preconditioned BiCGStab, first residuals).  Here every
+// thread splits its 27 gathered values and scales each plane by itself, which
+// makes it bound by instruction issue: 95 / 718 us at 1.08 / 8.5 M nodes
+// where the element-wise apply takes 105 / 773; the Krylov iterations split
+// once per node.  A caller's own applies stay element-wise: summing the rows
+// (160 us, 1.23 ms) costs what 15 of them would save, and the FP64 sums over
+// the elements are closer to the exact product (3.5e-15 against 5.9e-15
+// relative, random input).
+template <bool TRANS, bool KEEP>
 __global__ void __launch_bounds__(256, 4) stencil_apply(const StencilView v,
                                                         const double *__restrict__ x,
                                                         double *__restrict__ y,
@@ -123,18 +128,8 @@ __global__ void __launch_bounds__(256, 4) stencil_apply(const StencilView v,
   if (skip2 && *(volatile const int *)skip2) return;
   for (long n = (long)blockIdx.x * blockDim.x + threadIdx.x; n < v.N;
        n += (long)gridDim.x * blockDim.x) {
-    const double o = stencil_row<TRANS, KEEP>(v, n, x);
-    y[n] = ACC ? y[n] + o : o;
+    y[n] += stencil_row<TRANS, KEEP>(v, n, x);
   }
-}
-
-template <bool TRANS, bool ACC>
-void apply_keep(const Handle &h, bool keep, int grid, const StencilView &v, const double *x,
-                double *y, const int *skip, const int *skip2, cudaStream_t s) {
-  if (keep)
-    stencil_apply<TRANS, ACC, true><<<grid, 256, 0, s>>>(v, x, y, skip, skip2);
-  else
-    stencil_apply<TRANS, ACC, false><<<grid, 256, 0, s>>>(v, x, y, skip, skip2);
 }
 
 }  // namespace
@@ -261,19 +256,13 @@ cudaError_t ensure_segment_rows(Handle &h) {
   return e;
 }
 
-cudaError_t launch_stencil_apply(const Handle &h, bool transpose, bool accumulate,
-                                 const double *x, double *y, const int *skip,
-                                 const int *skip2, cudaStream_t s) {
+cudaError_t launch_stencil_apply(const Handle &h, bool transpose, const double *x, double *y,
+                                 const int *skip, const int *skip2, cudaStream_t s) {
   const StencilView v = stencil_view(h);
   const bool keep = stencil_keep(h);
-  const int grid = (int)((h.N + 255L) / 256);
-  if (transpose) {
-    if (accumulate) apply_keep<true, true>(h, keep, grid, v, x, y, skip, skip2, s);
-    else apply_keep<true, false>(h, keep, grid, v, x, y, skip, skip2, s);
-  } else {
-    if (accumulate) apply_keep<false, true>(h, keep, grid, v, x, y, skip, skip2, s);
-    else apply_keep<false, false>(h, keep, grid, v, x, y, skip, skip2, s);
-  }
+  const auto kern = transpose ? (keep ? stencil_apply<true, true> : stencil_apply<true, false>)
+                              : (keep ? stencil_apply<false, true> : stencil_apply<false, false>);
+  kern<<<(unsigned)((h.N + 255L) / 256), 256, 0, s>>>(v, x, y, skip, skip2);
   count_launches(1);
   return cudaGetLastError();
 }

@@ -245,13 +245,13 @@ struct Handle {
 
   // the assembled 27-point operator of the structured numbering (stencil.cuh):
   // st_state 0 not formed, 1 valid for the current operator, -1 no device
-  // memory for it; st_applies: single applies of the current operator
+  // memory for it
   float2 *st_S = nullptr;       // [27][N]
   unsigned *st_nm = nullptr;    // [N], and the largest entry's exponent at [st_rows]
   float2 *st_x = nullptr;       // two padded pair vectors: p^ and s^
   size_t st_rows = 0, st_len = 0;  // nodes and pairs that they hold room for
   int st_nax = 0, st_pl = 0, st_n = 0;  // the mesh that st_x's pads are zero for
-  int st_state = 0, st_applies = 0;
+  int st_state = 0;
   bool own_capture = false;
   // its binary16 rows for the mixed solve (half_rows.cu): 27 half planes, a
   // scale per row, FP32 vectors; hr_state as st_state, 2 = out of range
@@ -443,6 +443,11 @@ int diag_meeting_timeout(Handle &h);
 cudaError_t launch_stored_apply32v(const Handle &h, const float *x, float *y,
                                    const int *skip, const int *skip2,
                                    cudaStream_t s);
+// y += A x or A^T x: by elements, whose contributions to a node are added in
+// FP64; launch_apply by the assembled rows where they are current, for the
+// products of solvers.
+cudaError_t launch_element_apply(const Handle &h, bool transpose, const double *x, double *y,
+                                 const int *skip, const int *skip2, cudaStream_t s);
 cudaError_t launch_apply(const Handle &h, bool transpose, const double *x,
                          double *y, const int *skip, const int *skip2,
                          cudaStream_t s);
@@ -482,10 +487,9 @@ bool stencil_ready(const Handle &h);
 // The same for a handle of many meshes (h.seg_rows when they are current).
 cudaError_t ensure_segment_rows(Handle &h);
 cudaError_t launch_element_masks(Handle &h);
-// y (+)= A x or A^T x from the assembled rows.
-cudaError_t launch_stencil_apply(const Handle &h, bool transpose, bool accumulate,
-                                 const double *x, double *y, const int *skip,
-                                 const int *skip2, cudaStream_t s);
+// y += A x or A^T x from the assembled rows.
+cudaError_t launch_stencil_apply(const Handle &h, bool transpose, const double *x, double *y,
+                                 const int *skip, const int *skip2, cudaStream_t s);
 
 // ---- the mixed solve's inner operator on assembled rows (half_rows.cu) ----
 // Forms the binary16 rows for the current operator where it can (the handle
