@@ -782,7 +782,10 @@ int solve_device(Handle &h, int method, const double *b, double *x,
                  const Precond *prec, int stall_window, double *hist,
                  int max_hist, int *n_hist) {
   cudaError_t e = ensure_solver_workspace(h, 8);
-  if (!e && !h.apply_fp32) e = ensure_stencil(h);
+  // BiCG beyond a whole solve's launch applies A and A^T by elements, in one
+  // pass over the store: rows would serve its first residual only
+  const bool whole = !prec && !hist && resident_size(h);
+  if (!e && !h.apply_fp32 && (method == VDR_SOLVER_BICGSTAB || whole)) e = ensure_stencil(h);
   if (e) return cuda_fail(e, "solver workspace");
   cudaStream_t s = h.stream;
   Vec a = make_vec(h, b, x);
@@ -790,7 +793,7 @@ int solve_device(Handle &h, int method, const double *b, double *x,
   const long long launches0 = launches_so_far();
   h.last = vdr_solve_stats{};
 
-  if (!prec && !hist && resident_fits(h)) {
+  if (whole && stencil_ready(h)) {
     if (!(e = launch_resident(h, method, b, x, tol, itmax, stall_window))) {
       if ((e = cudaMemcpyAsync(&h.h_st[0], h.st, sizeof(KState), cudaMemcpyDeviceToHost, s)) ||
           (e = cudaStreamSynchronize(s)))

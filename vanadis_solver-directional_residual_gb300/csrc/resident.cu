@@ -583,9 +583,8 @@ int diag_meeting_timeout(Handle &h) {
   return VDR_CUDA_ERROR;
 }
 
-bool resident_fits(const Handle &h) {
-  return h.resident && stencil_ready(h) &&
-         h.N <= 1024L * std::min(device_sm_count(), 32 * RES_NB);
+bool resident_size(const Handle &h) {
+  return h.resident && h.N <= 1024L * std::min(device_sm_count(), 32 * RES_NB);
 }
 
 cudaError_t launch_resident(Handle &h, int method, const double *b, double *x, double tol,

@@ -504,7 +504,7 @@ int solve_half_rows(Handle &h, const double *res, double rnorm, double *x, doubl
 // ---- whole solves in one launch (resident.cu) ----
 // BiCGStab or BiCG with Jacobi on the assembled rows, where a node per thread
 // fits on the device; the outcome is in h.st.  An error means that nothing ran.
-bool resident_fits(const Handle &h);
+bool resident_size(const Handle &h);
 cudaError_t launch_resident(Handle &h, int method, const double *b, double *x, double tol,
                             int itmax, int stall_window);
 
