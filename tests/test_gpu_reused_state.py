@@ -3,6 +3,8 @@ buffers, rows -- give the answers that first calls give.
 
 Bars: solutions to 1e-9 where both sides are solved to 1e-11 or below (the
 operators' condition is below 1e2 here)."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -349,3 +351,34 @@ def test_bicg_holds_rows_for_whole_solves_only(vdr, gpu_lib, dims, rows):
         assert st == 0 and err <= 1e-10
         held = free - torch.cuda.mem_get_info()[0]
     assert (held > 150 * prob.mesh.nnode) == rows, held
+
+
+@pytest.mark.parametrize("dims", [(1, 1, 1), (6, 19, 19), (13, 5, 7), (40, 39, 38)])
+@pytest.mark.parametrize("order", ["own", "permuted"])
+def test_noalloc_solve_is_the_same_every_time(vdr, oracle, gpu_lib, dims, order):
+    """vdr_bicg_noalloc_device on the reference's own numbering: the same bits
+    from call to call (its sums have one order), and the oracle's solution; with
+    the elements listed in another order (atomics) the solution."""
+    torch = pytest.importorskip("torch")
+    prob, bb, b, diag, x0, ref = system(vdr, oracle, dims, 43, aM=200.0)
+    m, E, iss = prob.mesh, prob.mesh.nelem, prob.mesh.iss
+    if order == "permuted":
+        perm = np.random.default_rng(9).permutation(E)
+        bb = np.ascontiguousarray(bb.reshape(E, 64)[perm]).ravel()
+        iss = np.ascontiguousarray(iss.reshape(8, E)[:, perm]).ravel()
+    dev = [torch.tensor(v, device="cuda") for v in (b, bb, diag)]
+    ints = [torch.tensor(np.asarray(v, dtype=np.int32), device="cuda") for v in (iss, prob.bc)]
+    got = []
+    for _ in range(6):
+        x = torch.tensor(x0, device="cuda")
+        torch.cuda.synchronize()
+        it, err = ctypes.c_int(-1), ctypes.c_double(-1.0)
+        ptr = [ctypes.c_void_p(t.data_ptr()) for t in (*dev, *ints, x)]
+        st = gpu_lib.vdr_bicg_noalloc_device(m.nnode, m.nax, m.nay, m.naz, ptr[0], ptr[5], 1e-12,
+                                             5000, ptr[1], ptr[3], ptr[2], ptr[4], None,
+                                             ctypes.byref(it), ctypes.byref(err))
+        assert st == 0 and err.value <= 1e-12
+        got.append((it.value, x.cpu().numpy()))
+        assert rel_l2(got[-1][1], ref) < 1e-9
+    if order == "own":
+        assert all(n == got[0][0] and np.array_equal(x, got[0][1]) for n, x in got)

@@ -41,6 +41,7 @@ struct NaState {
   int iter, itmax, done, status;
   unsigned int ticket;
   int bad;  // set when an ISS entry lies outside 1..n
+  int other;  // set when ISS is not the reference's own numbering
 };
 
 constexpr int NA_MAX_Q = 3;  // most sums reduced by one kernel (na_start)
@@ -54,7 +55,7 @@ constexpr long NA_TOTAL_DOUBLES =
 static __device__ __align__(256) double g_noalloc_scratch[NA_TOTAL_DOUBLES];
 
 struct NaArgs {
-  int n, E;
+  int n, E, nax, nay;
   const double *b, *diag, *bb;
   const int *iss, *bc;
   double *x, *r, *rr, *p, *pp, *z, *zz;
@@ -66,12 +67,73 @@ __device__ __forceinline__ int na_node(const NaArgs &a, int s, long e) {
   return __ldg(a.iss + (size_t)s * a.E + e) - 1;
 }
 
+__device__ __forceinline__ bool na_masked(const NaArgs &a, int node) {
+  return a.bc && __ldg(a.bc + node) == 1;
+}
+
+// Node offset of an element's local node s from its first.
+__device__ __forceinline__ int na_offset(const NaArgs &a, int s) {
+  const int s2 = s & 3;
+  return (s2 == 1 || s2 == 2) + a.nax * ((s2 >> 1) + a.nay * (s >> 2));
+}
+
+__global__ void na_numbering(NaArgs a) {
+  bool other = false;
+  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < 8L * a.E;
+       t += (long)gridDim.x * blockDim.x) {
+    const int s = (int)(t / a.E), e = (int)(t - (long)s * a.E);
+    const int r = e / (a.nax - 1), i = e - r * (a.nax - 1);
+    const int k = r / (a.nay - 1), j = r - k * (a.nay - 1);
+    other |= na_node(a, s, e) != i + a.nax * (j + a.nay * k) + na_offset(a, s);
+  }
+  if (other) a.st->other = 1;
+}
+
+// y = P A P x (TRANS: P A^T P x) on the reference's own numbering: a node's
+// up to eight elements on eight lanes, their contributions added in the order
+// of the elements, as the reference's loop adds them.  The same result every
+// time, where atomics moved the recorded case's iteration counts by up to four
+// from call to call; 2,800 nodes, 94 iterations: 5.4 -> 3.8 ms.
+template <bool TRANS>
+__device__ __forceinline__ void na_gather(const NaArgs &a, const double *xin, double *y) {
+  const int lane = threadIdx.x & 31, q = lane & 7;
+  const int warps = (int)(gridDim.x * blockDim.x) >> 5;
+  const int nex = a.nax - 1, ney = a.nay - 1, nez = a.E / (nex * ney);
+  const int dx = q & 1, dy = (q >> 1) & 1, dz = q >> 2;  // 0: the element before
+  const int own = 4 * (1 - dz) + (dy ? (dx ? 0 : 1) : (dx ? 3 : 2));
+  for (int w = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5; 4 * w < a.n; w += warps) {
+    const int node = 4 * w + (lane >> 3);
+    const int r = node / a.nax, k = r / a.nay;
+    const int i = node - r * a.nax + dx - 1, j = r - k * a.nay + dy - 1, l = k + dz - 1;
+    double acc = 0.0;
+    if (node < a.n && i >= 0 && i < nex && j >= 0 && j < ney && l >= 0 && l < nez) {
+      const double *blk = a.bb + 64L * (i + (long)nex * (j + (long)ney * l));
+      const int first = i + a.nax * (j + a.nay * l);
+#pragma unroll
+      for (int s = 0; s < 8; s++) {
+        const int nd = first + na_offset(a, s);
+        const double xv = na_masked(a, nd) ? 0.0 : xin[nd];
+        acc += __ldg(blk + (TRANS ? 8 * s + own : 8 * own + s)) * xv;
+      }
+    }
+    double sum = 0.0;
+#pragma unroll
+    for (int e = 0; e < 8; e++) sum += __shfl_sync(0xffffffffu, acc, (lane & 24) + e);
+    if (q == 0 && node < a.n) y[node] = na_masked(a, node) ? 0.0 : sum;
+  }
+}
+
 // y += P A P x (TRANS: P A^T P x) over the reference's BB layout
-// BB[64e + 8i + j]; Dirichlet columns read as 0, rows are not written.
+// BB[64e + 8i + j]; Dirichlet columns read as 0, rows are not written.  y is
+// zero before.  Elements in another order or numbering scatter by atomics.
 template <bool TRANS>
 __global__ void na_apply(NaArgs a, const double *__restrict__ xin,
                          double *__restrict__ y) {
   if (a.st->done) return;
+  if (!a.st->other) {
+    na_gather<TRANS>(a, xin, y);
+    return;
+  }
   for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < a.E;
        e += (long)gridDim.x * blockDim.x) {
     int nd[8];
@@ -85,7 +147,7 @@ __global__ void na_apply(NaArgs a, const double *__restrict__ xin,
         nd[s] = 0;
         m[s] = true;
       } else {
-        m[s] = a.bc && __ldg(a.bc + nd[s]) == 1;
+        m[s] = na_masked(a, nd[s]);
       }
       xv[s] = m[s] ? 0.0 : xin[nd[s]];
     }
@@ -293,6 +355,8 @@ extern "C" int vdr_bicg_noalloc_device(int n, int nax, int nay, int naz,
   NaArgs a;
   a.n = n;
   a.E = (int)E;
+  a.nax = nax;
+  a.nay = nay;
   a.b = b;
   a.x = x;
   a.bb = bb;
@@ -318,7 +382,8 @@ extern "C" int vdr_bicg_noalloc_device(int n, int nax, int nay, int naz,
   if (!e) e = cudaMemsetAsync(a.r, 0, sizeof(double) * n, s);
   if (e) return cuda_fail(e, "vdr_bicg_noalloc_device: reset");
   const int gv = (int)std::min<long>(NA_MAX_BLOCKS, ((long)n + NA_THREADS - 1) / NA_THREADS);
-  const int ge = (int)std::min<long>(4096, (E + NA_THREADS - 1) / NA_THREADS);
+  const int ge = (int)std::min<long>(4096, (8L * n + NA_THREADS - 1) / NA_THREADS);
+  na_numbering<<<ge, NA_THREADS, 0, s>>>(a);
   na_mask_x<<<gv, NA_THREADS, 0, s>>>(a);
   na_apply<false><<<ge, NA_THREADS, 0, s>>>(a, a.x, a.r);
   na_start<<<gv, NA_THREADS, 0, s>>>(a);
