@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(512, 2) sgr_first(SegVec a) {
   const int s = tl.seg;
   if (!a.s.active[s]) return;
   const long at = a.mesh[s].shift;
-  const int e = a.s.pmax[s], er = a.s.rmax[s], base = pair_base(a.rows.top);
+  const int e = a.s.pmax[s], er = a.s.rmax[s], base = pair_base(a.rows.nm);
   TLOOP(i) {
     const double ri = a.r[i];
     const bool m = a.m[i] != 0;
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(512, 2) sgr_w(SegVec a) {
   const SegMesh g = a.mesh[s];
   const StencilView v = mesh_rows(a, g);
   const float2 *xp = a.shp + g.shift;
-  const int shift = a.s.rmax[s] - pair_base(v.top);
+  const int shift = a.s.rmax[s] - pair_base(v.nm);
   double q[1] = {0.0};
   TLOOP(i) {
     const unsigned m = v.nm[i];
@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(512, 2) sgr_v(SegVec a) {
   if (!a.s.active[s]) return;
   const SegMesh g = a.mesh[s];
   const StencilView v = mesh_rows(a, g);
-  const int shift = a.s.pexp[s] - pair_base(v.top);
+  const int shift = a.s.pexp[s] - pair_base(v.nm);
   const double al = a.s.alpha[s];
   double q[2] = {0.0, 0.0};
   TLOOP(i) {
@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(512, 2) sgr_t(SegVec a) {
   if (!a.s.active[s] || a.s.sconv[s]) return;
   const SegMesh g = a.mesh[s];
   const StencilView v = mesh_rows(a, g);
-  const int shift = a.s.pexp[s] - pair_base(v.top);
+  const int shift = a.s.pexp[s] - pair_base(v.nm);
   double q[3] = {0.0, 0.0, 0.0};
   TLOOP(i) {
     const double si = a.sv[i], hi = a.rh[i];
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(512, 2) sgr_p(SegVec a) {
   }
   const double om = a.s.omega[s], rho1 = a.s.rho_next[s];
   const double beta = a.s.beta[s];
-  const int e = a.s.pmax[s], shift = e - pair_base(a.rows.top);
+  const int e = a.s.pmax[s], shift = e - pair_base(a.rows.nm);
   const long at = a.mesh[s].shift;
   int em = 0;
   TLOOP(i) {
@@ -708,8 +708,7 @@ cudaError_t seg_layout(Handle &h, int tile, int threads, const double *b, double
   a.t = w + 7 * N;
   if (h.seg_rows) {
     a.rows.S = h.st_S;
-    a.rows.nm = h.st_nm;
-    a.rows.top = h.st_nm + h.st_rows;
+    a.rows.nm = h.st_nm + NM_LEAD;
     a.rows.N = h.N;
     a.mesh = h.seg_mesh;
     a.php = h.seg_x;

@@ -72,7 +72,7 @@ __device__ __forceinline__ float f4(const float4 &v, int c) {
 struct BlockRows {
   const float4 *rows;  // [N][7]: 27 scaled entries and a zero
   const float2 *S;     // the FP64-accurate pairs [27][N]
-  const unsigned *top;
+  const unsigned *nm;
   int N, nax, nay, naz;
   int nxt, nyt, grid;  // tiles along x and y, blocks
   int *err;            // set where a bounded wait ran out

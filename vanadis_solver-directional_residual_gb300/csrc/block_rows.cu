@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(PT, 2) br_residual(const BVec a, const BlockRo
 #pragma unroll
     for (int c = 0; c < 4; c++) rm[c] = bm[c];
   } else {
-    const int base = pair_base(g.top);
+    const int base = pair_base(g.nm);
     int shift[4];
 #pragma unroll
     for (int c = 0; c < 4; c++) shift[c] = o.xexp[4 * l + c] - base;
@@ -896,7 +896,7 @@ bool block_rows_usable(Handle &h, int K, BlockRows *g) {
   count_launches(1);
   g->rows = reinterpret_cast<const float4 *>(h.br_rows);
   g->S = h.st_S;
-  g->top = h.st_nm + h.st_rows;
+  g->nm = h.st_nm + NM_LEAD;
   g->N = h.N;
   g->nax = h.nax;
   g->nay = h.nay;

@@ -98,7 +98,7 @@ struct Vec {
   double *x, *r, *rh, *p, *v, *ph, *s, *sh, *t;  // BiCGStab
   double *rr, *pp, *z, *zz;                      // BiCG (r, p, x shared)
   float2 *php, *shp;  // p^ and s^ as pairs (assembled operator)
-  const unsigned *top;  // for pair_base
+  const unsigned *nm;  // the rows', for pair_base
   double *w;          // A^T rh (assembled operator, in p^'s place)
 };
 
@@ -462,7 +462,7 @@ Vec make_vec(Handle &h, const double *b, double *x) {
     a.php = h.st_x + stencil_pad(h);
     a.shp = a.php + N + 2 * stencil_pad(h);
     a.w = a.ph;
-    a.top = stencil_view(h).top;
+    a.nm = stencil_view(h).nm;
   }
   return a;
 }
@@ -484,7 +484,7 @@ Vec make_vec(Handle &h, const double *b, double *x) {
 __global__ void __launch_bounds__(RED_THREADS) bst_first(Vec a) {
   KState *st = a.st;
   if (st->done) return;
-  const int e = st->pmax, er = st->rmax, base = pair_base(a.top);
+  const int e = st->pmax, er = st->rmax, base = pair_base(a.nm);
   double rv[U], dv[U];
   unsigned char mv[U];
   VLOOP(rv[u] = ok ? a.r[i] : 0.0; dv[u] = ok ? a.dinv[i] : 0.0; mv[u] = ok ? a.m[i] : 1;,
@@ -508,7 +508,7 @@ __device__ __forceinline__ void bst_alpha(KState *st, double wp) {
 // w = A^T rh with (w, p^).
 __global__ void __launch_bounds__(RED_THREADS, 4) bst_w(Vec a, StencilView w) {
   if (a.st->done) return;
-  const int shift = a.st->rmax - pair_base(w.top);
+  const int shift = a.st->rmax - pair_base(w.nm);
   double v[1] = {0.0};
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n;
        i += (long)gridDim.x * blockDim.x) {
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(RED_THREADS, 4) bst_w(Vec a, StencilView w) {
 template <bool KEEP>
 __global__ void __launch_bounds__(RED_THREADS, 4) bst_v(Vec a, StencilView w) {
   if (a.st->done) return;
-  const int shift = a.st->pexp - pair_base(w.top);
+  const int shift = a.st->pexp - pair_base(w.nm);
   const double al = a.st->alpha;
   double v[2] = {0.0, 0.0};
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n;
@@ -550,7 +550,7 @@ __global__ void __launch_bounds__(RED_THREADS, 4) bst_v(Vec a, StencilView w) {
 template <bool KEEP>
 __global__ void __launch_bounds__(RED_THREADS, 4) bst_t(Vec a, StencilView w) {
   if (a.st->done || a.st->sconv) return;
-  const int shift = a.st->pexp - pair_base(w.top);
+  const int shift = a.st->pexp - pair_base(w.nm);
   double v[3] = {0.0, 0.0, 0.0};
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n;
        i += (long)gridDim.x * blockDim.x) {
@@ -603,7 +603,7 @@ __global__ void __launch_bounds__(RED_THREADS, 4) bst_p(Vec a) {
   }
   const double om = stc->omega, rho1 = stc->rho_next;
   const double beta = stc->beta;
-  const int e = stc->pmax, shift = e - pair_base(a.top);
+  const int e = stc->pmax, shift = e - pair_base(a.nm);
   int em = 0;
   double v[2] = {0.0, 0.0};
   constexpr int UP = 2;
@@ -978,7 +978,7 @@ __global__ void __launch_bounds__(RED_THREADS) bst_xmax(Vec a, int *ex) {
   if ((threadIdx.x & 31) == 0) atomicMax(ex, em);
 }
 __global__ void __launch_bounds__(RED_THREADS) bst_xsplit(Vec a, const int *ex) {
-  const int shift = *ex - pair_base(a.top);
+  const int shift = *ex - pair_base(a.nm);
   if (*ex == 0) return;
   double xv[U];
   VLOOP(xv[u] = ok ? a.x[i] : 0.0;, a.php[i] = stencil_pair(xv[u], shift);)
@@ -986,7 +986,7 @@ __global__ void __launch_bounds__(RED_THREADS) bst_xsplit(Vec a, const int *ex) 
 __global__ void __launch_bounds__(RED_THREADS, 4) bst_residual(Vec a, StencilView w, double *r,
                                                                const int *ex, double *out) {
   const int e = *ex;  // 0: x is zero
-  const int shift = e - pair_base(w.top);
+  const int shift = e - pair_base(w.nm);
   double v[2] = {0.0, 0.0};
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n;
        i += (long)gridDim.x * blockDim.x) {

@@ -19,11 +19,10 @@ enum { CLUSTER, IN_REGS, IN_SMEM };
 enum { AT_C = 0, AT_D = 2, AT_A = 5, SLOTS = 7 };
 
 struct MeetArgs {
-  double *part;   // [SLOTS][gridDim]
-  int *ipart;     // [3][gridDim]: largest exponents
-  unsigned *bar;  // arrivals, zero at launch
-  unsigned *late;  // where a wait ran out
+  double *part;     // [SLOTS][gridDim]; behind them [3][gridDim] largest exponents
+  unsigned *bar;    // arrivals, zero at launch; the next word: where a wait ran out
   long long limit;  // clocks that a wait may take
+  __device__ int *ipart() const { return reinterpret_cast<int *>(part + SLOTS * 32 * RES_NB); }
 };
 
 struct ResShared {
@@ -130,7 +129,7 @@ __device__ __forceinline__ bool meet(ResShared &sh, const MeetArgs &a, const dou
 #pragma unroll
       for (int k = 0; k < NE; k++) {
         const int e = __reduce_max_sync(FULLR, lane < nw ? sh.e[ES + k][lane] : 0);
-        if (lane == 0) __stcg(a.ipart + (size_t)(ES + k) * B + blockIdx.x, e);
+        if (lane == 0) __stcg(a.ipart() + (size_t)(ES + k) * B + blockIdx.x, e);
       }
       __syncwarp();
       if (lane == 0)
@@ -140,16 +139,19 @@ __device__ __forceinline__ bool meet(ResShared &sh, const MeetArgs &a, const dou
       // (13 us more per iteration at 145 CTAs)
       const long long t0 = clock64();
       bool met, late = false;
-      do {
+      const auto arrived = [&]() {
         unsigned seen;
-        late = clock64() - t0 > a.limit;  // before the count is read: a pause
-                                          // of this CTA is not another's delay
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.bar) : "memory");
-        met = (int)(seen - target) >= 0;
+        return (int)(seen - target) >= 0;
+      };
+      do {
+        met = arrived();
+        late = clock64() - t0 > a.limit;
       } while (!__all_sync(FULLR, met || late));
+      if (!met) met = arrived();  // a pause of this CTA is not another's delay
       if (lane == 0) {
         sh.ok = met;
-        if (!met) *(volatile unsigned *)a.late = 1u;
+        if (!met) *(volatile unsigned *)(a.bar + 1) = 1u;
       }
       if (R > 0) {
         double in[RES_NB][RP];  // every load before the first add
@@ -171,7 +173,7 @@ __device__ __forceinline__ bool meet(ResShared &sh, const MeetArgs &a, const dou
 #pragma unroll
         for (int i = 0; i < RES_NB; i++)
           etot[k] =
-              max(etot[k], __ldcg(a.ipart + (size_t)(ES + k) * B + min(lane + 32 * i, B - 1)));
+              max(etot[k], __ldcg(a.ipart() + (size_t)(ES + k) * B + min(lane + 32 * i, B - 1)));
     }
   }
   if (w == 0) {
@@ -200,8 +202,7 @@ __device__ __forceinline__ bool meet(ResShared &sh, const MeetArgs &a, const dou
 }
 
 inline MeetArgs meet_args(const Handle &h) {
-  return MeetArgs{h.partials, reinterpret_cast<int *>(h.partials + SLOTS * 32 * RES_NB),
-                  &h.st->bar_count, &h.st->late, RES_LIMIT};
+  return MeetArgs{h.partials, &h.st->bar_count, RES_LIMIT};
 }
 // No arrivals and nobody late.
 inline cudaError_t meet_reset(Handle &h, cudaStream_t s) {

@@ -40,6 +40,11 @@
 namespace vdr {
 namespace {
 
+// (Not above 128 bytes: the compiler leaves a larger argument in constant
+// memory and resident_bicgstab forms its neighbours' addresses anew in every
+// product, 5 per cent of an iteration.  resident_bicg has no registers to hold
+// them in, and is asked to leave them there: 48 to 104 bytes of spills less
+// and 2 to 5 per cent of a solve.)
 struct ResArgs {
   StencilView w;
   const double *b, *dinv;
@@ -51,6 +56,7 @@ struct ResArgs {
   double tol;
   int itmax, window;
 };
+static_assert(sizeof(ResArgs) <= 128, "in registers");
 
 __device__ __forceinline__ double row_value(const DfAcc &acc, int shift) {
   double o = df_to_double(acc.s, acc.c);
@@ -69,7 +75,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
   const int N = a.w.N, n = (int)(blockIdx.x * T + threadIdx.x);
   const bool on = n < N;
   unsigned target = 0;
-  const int base = pair_base(a.w.top);
+  const int base = pair_base(a.w.nm);
   const int none[1] = {0};
   const auto nothing = [](int) {};
   double x = 0.0, r = 0.0, p = 0.0, v = 0.0, s = 0.0, t = 0.0, rh = 0.0, wn = 0.0;
@@ -323,13 +329,13 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
 // taken as it is (the drop-in's may be nonzero on Dirichlet rows, where x
 // stays zero).
 template <int MODE, int T>
-__global__ void __launch_bounds__(T, 1) resident_bicg(ResArgs a) {
+__global__ void __launch_bounds__(T, 1) resident_bicg(const __grid_constant__ ResArgs a) {
   extern __shared__ float2 dyn[];  // [27][T]: columns, or rows (IN_SMEM)
   __shared__ ResShared sh;
   const int N = a.w.N, n = (int)(blockIdx.x * T + threadIdx.x);
   const bool on = n < N;
   unsigned target = 0;
-  const int base = pair_base(a.w.top);
+  const int base = pair_base(a.w.nm);
   const int none[1] = {0};
   const auto nothing = [](int) {};
   const auto column = [&](int k) {  // A's entry of neighbour k with this node

@@ -86,20 +86,20 @@ __device__ __forceinline__ void raise_top(unsigned big, unsigned *top) {
 __global__ void __launch_bounds__(256, 2) stencil_assemble(
     const float4 *__restrict__ Ahi, const float4 *__restrict__ Alo,
     const unsigned char *__restrict__ emask, int nax, int nay, int naz, float2 *S,
-    unsigned *nm, unsigned *top) {
+    unsigned *nm) {
   unsigned big = 0u;
   const int E = (nax - 1) * (nay - 1) * (naz - 1), N = nax * nay * naz;
   for (long n = (long)blockIdx.x * blockDim.x + threadIdx.x; n < N;
        n += (long)gridDim.x * blockDim.x)
     big = max(big, assemble_node(Ahi, Alo, emask, E, 0, nax, nay, naz, (unsigned)n, n, N, S, nm));
-  raise_top(big, top);
+  raise_top(big, nm - 1);
 }
 
 // The same for many meshes side by side (one row of blocks per mesh).
 __global__ void __launch_bounds__(256, 2) stencil_assemble_meshes(
     const float4 *__restrict__ Ahi, const float4 *__restrict__ Alo,
     const unsigned char *__restrict__ emask, int E, long N,
-    const SegMesh *__restrict__ meshes, float2 *S, unsigned *nm, unsigned *top) {
+    const SegMesh *__restrict__ meshes, float2 *S, unsigned *nm) {
   unsigned big = 0u;
   const SegMesh g = meshes[blockIdx.y];
   const int count = g.nax * g.nay * g.naz;
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(256, 2) stencil_assemble_meshes(
        l += (int)(gridDim.x * blockDim.x))
     big = max(big, assemble_node(Ahi, Alo, emask, E, g.e0, g.nax, g.nay, g.naz, (unsigned)l,
                                  g.n0 + (long)l, N, S, nm));
-  raise_top(big, top);
+  raise_top(big, nm - 1);
 }
 
 // y += A x or A^T x, any FP64 x, for the products of solvers that keep FP64
@@ -137,8 +137,7 @@ __global__ void __launch_bounds__(256, 4) stencil_apply(const StencilView v,
 StencilView stencil_view(const Handle &h) {
   StencilView v;
   v.S = h.st_S;
-  v.nm = h.st_nm;
-  v.top = h.st_nm + h.st_rows;
+  v.nm = h.st_nm + NM_LEAD;
   v.N = h.N;
   v.nax = h.nax;
   v.pl = h.nax * h.nay;
@@ -185,7 +184,7 @@ static bool row_storage(Handle &h, float2 **x, size_t *have, size_t len) {
   if (h.rows_room && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
       (rows ? 220 * N : 0) + (vec ? sizeof(float2) * len : 0) <= free_b / 2 &&
       (!rows || (!cudaMalloc(&h.st_S, sizeof(float2) * 27 * N) &&
-                 !cudaMalloc(&h.st_nm, sizeof(unsigned) * (N + 1)))) &&
+                 !cudaMalloc(&h.st_nm, sizeof(unsigned) * (NM_LEAD + N)))) &&
       (!vec || !cudaMalloc(x, sizeof(float2) * len))) {
     if (rows) h.st_rows = N;
     if (vec) *have = len;
@@ -223,10 +222,10 @@ cudaError_t ensure_stencil(Handle &h) {
   }
   const long need = (h.N + 255L) / 256;
   const int grid = (int)std::min<long>(need, (long)device_sm_count() * 32);
-  unsigned *top = h.st_nm + h.st_rows;
-  if ((e = cudaMemsetAsync(top, 0, sizeof(unsigned), h.stream))) return e;
+  unsigned *nm = h.st_nm + NM_LEAD;
+  if ((e = cudaMemsetAsync(nm - 1, 0, sizeof(unsigned), h.stream))) return e;
   stencil_assemble<<<grid, 256, 0, h.stream>>>(h.Ahi, h.Alo, h.emask, h.nax, h.nay, h.naz,
-                                               h.st_S, h.st_nm, top);
+                                               h.st_S, nm);
   count_launches(1);
   e = cudaGetLastError();
   if (!e) h.st_state = 1;
@@ -246,11 +245,11 @@ cudaError_t ensure_segment_rows(Handle &h) {
   if (fresh && (e = cudaMemsetAsync(h.seg_x, 0, sizeof(float2) * have, h.stream))) return e;
   if ((e = launch_element_masks(h))) return e;
   const int per = (int)std::max<long>(1, std::min<long>(64, (h.seg_largest + 255) / 256));
-  unsigned *top = h.st_nm + h.st_rows;
-  if ((e = cudaMemsetAsync(top, 0, sizeof(unsigned), h.stream))) return e;
+  unsigned *nm = h.st_nm + NM_LEAD;
+  if ((e = cudaMemsetAsync(nm - 1, 0, sizeof(unsigned), h.stream))) return e;
   stencil_assemble_meshes<<<dim3((unsigned)per, (unsigned)(h.seg_off.size() - 1)), 256, 0,
                             h.stream>>>(h.Ahi, h.Alo, h.emask, h.E, h.N, h.seg_mesh, h.st_S,
-                                        h.st_nm, top);
+                                        nm);
   count_launches(1);
   if (!(e = cudaGetLastError())) h.seg_rows = true;
   return e;

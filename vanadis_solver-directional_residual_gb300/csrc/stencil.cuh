@@ -29,11 +29,12 @@ namespace vdr {
 
 struct StencilView {
   const float2 *S = nullptr;
-  const unsigned *nm = nullptr;
-  const unsigned *top = nullptr;  // biased FP32 exponent of the largest entry
+  const unsigned *nm = nullptr;  // and before it what pair_base reads
   int N = 0, nax = 0, pl = 0;
 };
 
+constexpr int NM_LEAD = 32;  // words before nm; the last: the biased FP32
+                             // exponent of the largest entry
 // A vector whose largest biased exponent is e becomes pairs by 2^-(e - base):
 // largest magnitude in [2^h, 2^(h + 1)) with h = 200 - top, at most 72.  A
 // row's 27 products then stay below 2^128 for a vector 2^48 times larger than
@@ -43,8 +44,8 @@ struct StencilView {
 // with entries around 1, values down to 2^-198 of the largest are held and
 // down to 2^-174 in full; with the largest entries that the store allows
 // (2^123 once summed) it is 2^-76 and 2^-52.
-__device__ __forceinline__ int pair_base(const unsigned *top) {
-  return 1023 - max((int)*top - 200, -72);
+__device__ __forceinline__ int pair_base(const unsigned *nm) {
+  return 1023 - max((int)nm[-1] - 200, -72);
 }
 
 __device__ __forceinline__ int stencil_off(int k, int nax, int pl) {

@@ -247,7 +247,7 @@ struct Handle {
   // st_state 0 not formed, 1 valid for the current operator, -1 no device
   // memory for it
   float2 *st_S = nullptr;       // [27][N]
-  unsigned *st_nm = nullptr;    // [N], and the largest entry's exponent at [st_rows]
+  unsigned *st_nm = nullptr;    // [NM_LEAD + N]
   float2 *st_x = nullptr;       // two padded pair vectors: p^ and s^
   size_t st_rows = 0, st_len = 0;  // nodes and pairs that they hold room for
   int st_nax = 0, st_pl = 0, st_n = 0;  // the mesh that st_x's pads are zero for
@@ -402,7 +402,6 @@ struct BuildArgs {
   const float2 *gJi = nullptr, *gDj = nullptr, *gK = nullptr;
   float2 *gsc = nullptr;  // [10][E] per-element scalars of that build, as pairs
 };
-
 
 // ---- launchers (element.cu) ----
 cudaError_t launch_build(const OpArgs &a, const BuildArgs &ba, bool fp32,
