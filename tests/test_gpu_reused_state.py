@@ -382,3 +382,37 @@ def test_noalloc_solve_is_the_same_every_time(vdr, oracle, gpu_lib, dims, order)
         assert rel_l2(got[-1][1], ref) < 1e-9
     if order == "own":
         assert all(n == got[0][0] and np.array_equal(x, got[0][1]) for n, x in got)
+
+
+@pytest.mark.parametrize("dims,robin", [((1, 1, 1), 0.0), ((2, 1, 3), 0.3), ((6, 19, 19), 0.4),
+                                        ((33, 17, 21), 0.0), ((75, 63, 31), 0.0)])
+def test_time_loop_is_the_same_every_time(vdr, oracle, gpu_lib, dims, robin):
+    """Up to the largest whole solve a step's sums have one order, from both
+    builds (by geometric factors, and with a Robin term by coordinates): the
+    right-hand side and the diagonal are the oracle's, to 1e-12, and repeat bit
+    for bit, as do the time loop's counts, masses and field."""
+    torch = pytest.importorskip("torch")
+    prob = vdr.problems.rotation_shear(*dims, seed=44)
+    prob.pdec[:] = 0.2
+    prob.robin_alpha = robin
+    if np.all(prob.bc == 1):
+        prob.bc[:] = 0
+    m, aM = prob.mesh, max(10.0, 0.3 * max(dims))
+    told = np.cos(0.37 * np.arange(m.nnode))
+    _, b, diag = oracle.assemble(prob.variant, m.xx, m.yy, m.zz, m.iss, prob.vel, prob.lam,
+                                 prob.pdec, prob.q, kod=m.kod, robin_alpha=robin, aH=2.0, aM=aM,
+                                 cf=3.0, rM=aM, t_old=told, nthreads=8)
+    b[prob.bc == 1] = 0.0
+    diag[prob.bc == 1] = 1.0
+    seen = set()
+    for solver in ("bicg", "bicgstab") * 3:
+        with vdr.Solver(prob, vdr.Options(solver=solver), aH=2.0, aM=aM) as s:
+            rhs, d = s.assemble_rhs(3.0, aM, told), s.diag()
+            assert rel_l2(rhs, b) < 1e-12 and rel_l2(d, diag) < 1e-12
+            t = torch.tensor(told * (prob.bc == 0), device="cuda")
+            torch.cuda.synchronize()
+            masses, its, errs, st, done = s.time_steps_device(t, 3, 3.0, aM, tol=1e-10, itmax=5000)
+            assert st == 0 and done == 3
+            seen.add((solver, tuple(its), masses.tobytes(), t.cpu().numpy().tobytes(),
+                      rhs.tobytes(), d.tobytes()))
+    assert len(seen) == 2

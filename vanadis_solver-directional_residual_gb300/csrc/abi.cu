@@ -190,24 +190,29 @@ int build_operator(Handle &h, const BuildArgs *rhs) {
   // The H/M rows are accumulated in double-float unless a value left the
   // pairs' safe window (flag bit 2: redo with FP64 rows), and the store is
   // double-float unless an entry left the store window (bit 1: FP64 store).
+  bool parts = false;
   for (int attempt = 0; attempt < 3; attempt++) {
     const bool df = stored && h.storage == VDR_STORE_DF;
     BuildArgs ba;
     ba.exact_fp64 = h.exact_build;
     ba.bad = h.flag;
+    if ((need_op || rhs->Mhi) && !h.exact_build && ordered_sums(h)) {
+      if ((e = dalloc(&h.build_parts, (size_t)h.E * 24))) return cuda_fail(e, "alloc build parts");
+      ba.parts = h.build_parts;
+    }
     if (rhs) {
       ba.cf = rhs->cf;
       ba.rM = rhs->rM;
       ba.told = rhs->told;
       ba.b = rhs->b;
-      if ((e = cudaMemsetAsync(ba.b, 0, sizeof(double) * h.N, h.stream)))
+      if (!ba.parts && (e = cudaMemsetAsync(ba.b, 0, sizeof(double) * h.N, h.stream)))
         return cuda_fail(e, "memset rhs");
       // time loop: keep M and F of this operator (double-float build only)
       if (rhs->Mhi && !h.exact_build) {
         ba.Mhi = rhs->Mhi;
         ba.Mlo = rhs->Mlo;
         ba.f = rhs->f;
-        if ((e = cudaMemsetAsync(ba.f, 0, sizeof(double) * h.N, h.stream)))
+        if (!ba.parts && (e = cudaMemsetAsync(ba.f, 0, sizeof(double) * h.N, h.stream)))
           return cuda_fail(e, "memset f");
       }
     }
@@ -217,7 +222,7 @@ int build_operator(Handle &h, const BuildArgs *rhs) {
       if (df && ((e = dalloc(&h.Ahi, (size_t)h.E * 16)) ||
                  (e = dalloc(&h.Alo, (size_t)h.E * 16))))
         return cuda_fail(e, "alloc element matrices");
-      if ((e = cudaMemsetAsync(h.diag, 0, sizeof(double) * h.N, h.stream)))
+      if (!ba.parts && (e = cudaMemsetAsync(h.diag, 0, sizeof(double) * h.N, h.stream)))
         return cuda_fail(e, "memset diag");
       ba.aH = h.aH;
       ba.aM = h.aM;
@@ -261,12 +266,16 @@ int build_operator(Handle &h, const BuildArgs *rhs) {
       return cuda_fail(e, "flag");
     // bit 3: the M store left its window (M is then not kept)
     h.mass_valid = ba.Mhi && !(bad & 4) && !(bad & 3);
-    if (!(bad & 3)) break;
+    if (!(bad & 3)) {
+      if (ba.parts && (e = launch_node_sums(h, ba, h.stream))) return cuda_fail(e, "node sums");
+      parts = ba.parts != nullptr;
+      break;
+    }
     if (bad & 2) h.exact_build = true;
     if ((bad & 1) && df) h.storage = VDR_STORE_FP64;
   }
   if (need_op) {
-    if ((e = launch_diag_fix(h.diag, h.dinv, h.mask, h.N, h.stream)) ||
+    if ((!parts && (e = launch_diag_fix(h.diag, h.dinv, h.mask, h.N, h.stream))) ||
         (e = launch_emask(h)))
       return cuda_fail(e, "diag");
     h.op64_valid = true;
@@ -424,7 +433,7 @@ void free_handle(Handle &h) {
   dfree(h.bk_f); dfree(h.bk_d); dfree(h.br_rows);
   if (h.bk_graph) cudaGraphExecDestroy(h.bk_graph);
   dfree(h.gcr_work); dfree(h.stage_d); dfree(h.drs); dfree(h.work32);
-  dfree(h.Mhi); dfree(h.Mlo); dfree(h.Fvec); dfree(h.rhs_tmp); dfree(h.massw);
+  dfree(h.Mhi); dfree(h.Mlo); dfree(h.Fvec); dfree(h.rhs_tmp); dfree(h.build_parts); dfree(h.massw);
   free_geometry(h);
   dfree(h.gsc);
   if (h.graph32) cudaGraphExecDestroy(h.graph32);

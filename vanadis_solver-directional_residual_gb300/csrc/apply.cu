@@ -764,6 +764,135 @@ __global__ void rhs_combine_kernel(const double *__restrict__ F,
 }
 }  // namespace
 
+// ---- a node's elements added in one order ----
+// Its up to eight elements, q = dx + 2 dy + 4 dz (0: the element before the
+// node on that axis), in the order of their numbers.  No atomics: the same
+// bits every time.  Up to the size of whole-solve launches, so that all of
+// such a step has one order: the recorded run's BiCG counts moved by up to
+// three from run to run with the atomics' order.  Above, the parts' memory
+// (192 bytes an element) and the eightfold splitting of x would cost more
+// than the atomics.
+namespace {
+struct AroundNode {
+  int p = -1, own = 0, first = 0;  // element (-1: none), the node's slot, its first node
+};
+__device__ __forceinline__ AroundNode around_node(int i, int j, int k, int q, int nax, int nay,
+                                                  int naz) {
+  AroundNode a;
+  const int dx = q & 1, dy = (q >> 1) & 1, dz = q >> 2;
+  i += dx - 1;
+  j += dy - 1;
+  k += dz - 1;
+  if (i >= 0 && i < nax - 1 && j >= 0 && j < nay - 1 && k >= 0 && k < naz - 1) {
+    a.p = i + (nax - 1) * (j + (nay - 1) * k);
+    a.own = 4 * (1 - dz) + (dy ? (dx ? 0 : 1) : (dx ? 3 : 2));
+    a.first = i + nax * (j + nay * k);
+  }
+  return a;
+}
+
+// diag (where given) with its inverse as diag_fix_kernel leaves them, f and b.
+__global__ void node_sums_kernel(const double *__restrict__ parts, int E, int N, int nax, int nay,
+                                 int naz, const unsigned char *__restrict__ mask, double *diag,
+                                 double *dinv, double *f, double *b) {
+  double *const to[3] = {diag, f, b};
+  for (int node = blockIdx.x * blockDim.x + threadIdx.x; node < N;
+       node += gridDim.x * blockDim.x) {
+    const int r = node / nax, i = node - r * nax, k = r / nay, j = r - k * nay;
+    const bool m = mask[node] != 0;
+#pragma unroll
+    for (int t = 0; t < 3; t++) {
+      if (!to[t]) continue;
+      double v[8], s = 0.0;
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const AroundNode a = around_node(i, j, k, q, nax, nay, naz);
+        v[q] = a.p >= 0 ? __ldcs(parts + (size_t)(8 * t + a.own) * E + a.p) : 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < 8; q++) s += v[q];
+      if (m) s = t == 0 ? 1.0 : 0.0;
+      to[t][node] = s;
+      if (t == 0) dinv[node] = 1.0 / s;
+    }
+  }
+}
+
+// y = P A P x from a double-float store with stored_apply_df's arithmetic: a
+// row of an element on each of a node's eight lanes, 32 nodes a block, whose
+// sums one warp forms (each lane forming its node's took eight times the
+// FP64 pipe's time).
+__global__ void __launch_bounds__(256) node_apply_df(const float4 *__restrict__ Ahi,
+                                                     const float4 *__restrict__ Alo,
+                                                     const ConnView cv, int E, int N, int naz,
+                                                     const double *__restrict__ x,
+                                                     double *__restrict__ y) {
+  __shared__ double part[8][33];
+  const int q = threadIdx.x & 7, at = threadIdx.x >> 3;
+  for (int n0 = 32 * blockIdx.x; n0 < N; n0 += 32 * gridDim.x) {
+    const int node = n0 + at, r = node / cv.nax, k = r / (cv.ney + 1);
+    const AroundNode a = around_node(node - r * cv.nax, r - k * (cv.ney + 1), k, q, cv.nax,
+                                     cv.ney + 1, naz);
+    double o = 0.0;
+    if (node < N && a.p >= 0) {
+      ElemNodes<true> c;
+      c.base = a.first;
+      c.nax = cv.nax;
+      c.pl = cv.pl;
+      c.m = __ldg(cv.emask + a.p);
+      const size_t row = (size_t)(2 * a.own) * E + a.p;
+      const float4 h0 = Ahi[row], h1 = Ahi[row + E], l0 = Alo[row], l1 = Alo[row + E];
+      const float ah[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+      const float al[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+      double xv[8];
+      int emax = 0;
+#pragma unroll
+      for (int s = 0; s < 8; s++) {
+        xv[s] = c[s] < 0 ? 0.0 : __ldg(x + c[s]);
+        emax = max(emax, df_exp(xv[s]));
+      }
+      const int shift = emax - 1023;
+      bool bad = false;
+      DfAcc acc{0.0f, 0.0f};
+#pragma unroll
+      for (int s = 0; s < 8; s++) {
+        float xh, xl;
+        df_split(xv[s], xh, xl, bad, shift);
+        df_fma_acc(acc, ah[s], al[s], xh, xl);
+      }
+      o = df_to_double(acc.s, acc.c);
+      if (!df_scale(o, shift)) o = ldexp(o, shift);
+      if (bad) {  // inf or NaN among them
+        o = 0.0;
+        for (int s = 0; s < 8; s++) o += df_to_double(ah[s], al[s]) * xv[s];
+      }
+      if ((c.m >> a.own) & 1u) o = 0.0;
+    }
+    __syncthreads();  // the sums before are read
+    part[q][at] = o;
+    __syncthreads();
+    if (threadIdx.x < 32 && n0 + (int)threadIdx.x < N) {
+      double s = 0.0;
+#pragma unroll
+      for (int e = 0; e < 8; e++) s += part[e][threadIdx.x];
+      y[n0 + threadIdx.x] = s;
+    }
+  }
+}
+}  // namespace
+
+bool ordered_sums(const Handle &h) {
+  return h.nax > 1 && h.nay > 1 && h.naz > 1 && !h.perm_d &&
+         h.N <= whole_solve_nodes();
+}
+
+cudaError_t launch_node_sums(const Handle &h, const BuildArgs &ba, cudaStream_t s) {
+  node_sums_kernel<<<grid_for(h.N, 128, 16), 128, 0, s>>>(
+      ba.parts, h.E, h.N, h.nax, h.nay, h.naz, h.mask, ba.diag, h.dinv, ba.f, ba.b);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_rhs_from_mass(Handle &h, double cf, double rM, const double *t,
                                  double *b, cudaStream_t s) {
   // H - rM M = A/aH - (aM/aH + rM) M
@@ -773,7 +902,13 @@ cudaError_t launch_rhs_from_mass(Handle &h, double cf, double rM, const double *
   if ((e = launch_apply(h, false, t, y1, nullptr, nullptr, s))) return e;
   const bool color = h.scatter == VDR_SCATTER_COLOR;
   const ConnView cv = conn_view(h);
-  const int nranges = color ? h.ncolors : 1;
+  const bool ordered = ordered_sums(h) && cv.emask;
+  if (ordered) {
+    node_apply_df<<<grid_for(8L * h.N, 256, 8), 256, 0, s>>>(h.Mhi, h.Mlo, cv, h.E, h.N, h.naz, t,
+                                                             y2);
+    count_launches(1);
+  }
+  const int nranges = ordered ? 0 : color ? h.ncolors : 1;
   for (int r = 0; r < nranges; r++) {
     const int p0 = color ? h.color_off[r] : 0;
     const int p1 = color ? h.color_off[r + 1] : h.E;

@@ -606,6 +606,10 @@ __device__ __forceinline__ void df_rows_out(const OpArgs &a, const BuildArgs &ba
                                             double qe, double vol, Df2 aHd, Df2 aMd, Df2 nrMd,
                                             const Df2 *told, int tshift) {
   const long E = a.E;
+  const auto give = [&](int q, double *to, double v) {
+    if (ba.parts) ba.parts[(size_t)(8 * q + i) * E + p] = v;
+    else if (ci >= 0) atomicAdd(to + ci, v);
+  };
   if (ba.Ahi && !ba.A64) {
     // double-float store: A_e row = aH H + aM M formed in double-float,
     // stored as its (hi, lo) pair; the store window is checked on hi
@@ -633,7 +637,7 @@ __device__ __forceinline__ void df_rows_out(const OpArgs &a, const BuildArgs &ba
           make_float4(rowd[4 * h].l, rowd[4 * h + 1].l, rowd[4 * h + 2].l, rowd[4 * h + 3].l);
     }
     if (bad) atomicOr(ba.bad, 1);  // store window (bit 1)
-    if (ba.diag && ci >= 0) atomicAdd(ba.diag + ci, df_to_double(rowd[i].h, rowd[i].l));
+    if (ba.diag) give(0, ba.diag, df_to_double(rowd[i].h, rowd[i].l));
   }
   if (!ba.Ahi && (ba.A64 || ba.diag)) {
     double row[8];
@@ -648,7 +652,7 @@ __device__ __forceinline__ void df_rows_out(const OpArgs &a, const BuildArgs &ba
       for (int jj = 0; jj < 4; jj++)
         ba.A64[(size_t)(4 * i + jj) * E + p] = make_double2(row[2 * jj], row[2 * jj + 1]);
     }
-    if (ba.diag && ci >= 0) atomicAdd(ba.diag + ci, row[i]);
+    if (ba.diag) give(0, ba.diag, row[i]);
   }
   if constexpr (SPLIT) {
     if (ba.Mhi) {
@@ -673,8 +677,8 @@ __device__ __forceinline__ void df_rows_out(const OpArgs &a, const BuildArgs &ba
   }
   const double fwd = df_to_double(fw.s, fw.c);
   if (ba.phi) ba.phi[(size_t)i * E + p] = fwd / vol;
-  if (ba.f && ci >= 0) atomicAdd(ba.f + ci, (qe / vol) * fwd);
-  if (ba.b && ci >= 0) {
+  if (ba.f) give(1, ba.f, (qe / vol) * fwd);
+  if (ba.b && (ba.parts || ci >= 0)) {
     double val = ba.cf * ((qe / vol) * fwd);
     if (SPLIT && ba.told) {
       // (H - rM M) T_old in double-float on the scaled T_old, scaled back
@@ -689,7 +693,7 @@ __device__ __forceinline__ void df_rows_out(const OpArgs &a, const BuildArgs &ba
       if (!df_scale(f, tshift)) f = ldexp(f, tshift);
       val -= f;
     }
-    atomicAdd(ba.b + ci, val);
+    give(2, ba.b, val);
   }
 }
 

@@ -589,9 +589,9 @@ int diag_meeting_timeout(Handle &h) {
   return VDR_CUDA_ERROR;
 }
 
-bool resident_size(const Handle &h) {
-  return h.resident && h.N <= 1024L * std::min(device_sm_count(), 32 * RES_NB);
-}
+long whole_solve_nodes() { return 1024L * std::min(device_sm_count(), 32 * RES_NB); }
+
+bool resident_size(const Handle &h) { return h.resident && h.N <= whole_solve_nodes(); }
 
 cudaError_t launch_resident(Handle &h, int method, const double *b, double *x, double tol,
                             int itmax, int stall_window) {

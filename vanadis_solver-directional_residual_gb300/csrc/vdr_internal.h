@@ -296,6 +296,7 @@ struct Handle {
   // right-hand side from two applies; rhs_tmp holds A T and M T
   float4 *Mhi = nullptr, *Mlo = nullptr;
   double *Fvec = nullptr, *rhs_tmp = nullptr;
+  double *build_parts = nullptr;  // BuildArgs::parts
   bool mass_valid = false;
   double *massw = nullptr;  // [8][E] integrate_mass weights (fixed geometry)
 
@@ -401,6 +402,9 @@ struct BuildArgs {
   // double-float build reads them instead of recomputing the Jacobians
   const float2 *gJi = nullptr, *gDj = nullptr, *gK = nullptr;
   float2 *gsc = nullptr;  // [10][E] per-element scalars of that build, as pairs
+  // [3][8][E]: the elements' parts of diag, f and b, to be summed by
+  // launch_node_sums, instead of atomics into them (double-float build)
+  double *parts = nullptr;
 };
 
 // ---- launchers (element.cu) ----
@@ -442,6 +446,11 @@ int diag_meeting_timeout(Handle &h);
 cudaError_t launch_stored_apply32v(const Handle &h, const float *x, float *y,
                                    const int *skip, const int *skip2,
                                    cudaStream_t s);
+// Whether builds and right-hand sides add a node's elements in one order.
+bool ordered_sums(const Handle &h);
+// diag (with h.dinv; 1 on Dirichlet nodes), f and b, those asked for, from
+// ba.parts.
+cudaError_t launch_node_sums(const Handle &h, const BuildArgs &ba, cudaStream_t s);
 // y += A x or A^T x: by elements, whose contributions to a node are added in
 // FP64; launch_apply by the assembled rows where they are current, for the
 // products of solvers.
@@ -503,6 +512,7 @@ int solve_half_rows(Handle &h, const double *res, double rnorm, double *x, doubl
 // ---- whole solves in one launch (resident.cu) ----
 // BiCGStab or BiCG with Jacobi on the assembled rows, where a node per thread
 // fits on the device; the outcome is in h.st.  An error means that nothing ran.
+long whole_solve_nodes();
 bool resident_size(const Handle &h);
 cudaError_t launch_resident(Handle &h, int method, const double *b, double *x, double tol,
                             int itmax, int stall_window);
