@@ -295,10 +295,10 @@ int vdr_time_steps(vdr_handle *h, int nsteps, double cf, double rM,
 #define VDR_BLOCK_APPLY_TCGEN05 3
 #define VDR_BLOCK_APPLY_AUTO 4
 int vdr_set_block_apply(vdr_handle *h, int variant);
-/* Diagnostic of the bounded device wait used by VDR_BLOCK_APPLY_BULK (the
- * tcgen05 box apply bounds its waits the same way): one
- * warp waits on an mbarrier that nothing completes, with a ~1 ms budget;
- * the wait gives up, flags it and returns.  Returns VDR_TIMEOUT when that
+/* Diagnostic of the bounded device waits of VDR_BLOCK_APPLY_BULK (the tcgen05
+ * box apply bounds its waits the same way) and of the block solve's products
+ * on assembled rows: one warp each waits on an mbarrier that nothing
+ * completes, with a ~1 ms budget; the wait gives up, flags it and returns.  Returns VDR_TIMEOUT when that
  * path works (the handle stays usable). */
 int vdr_diag_wait_timeout(vdr_handle *h);
 /* Diagnostic of the bounded grid barrier of the mixed solve's fused inner

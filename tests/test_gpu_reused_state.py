@@ -416,3 +416,22 @@ def test_time_loop_is_the_same_every_time(vdr, oracle, gpu_lib, dims, robin):
             seen.add((solver, tuple(its), masses.tobytes(), t.cpu().numpy().tobytes(),
                       rhs.tobytes(), d.tobytes()))
     assert len(seen) == 2
+
+
+def test_block_solve_after_copy_waits_ran_out(vdr, oracle, gpu_lib):
+    """The ring of copies of the products on rows gives up on a copy that is
+    never issued, drains and reports it; block solves on the same handle
+    before and after give the oracle's solution."""
+    import importlib
+    torch = pytest.importorskip("torch")
+    L = importlib.import_module(vdr.__name__ + "._lib")
+    sys_ = system(vdr, oracle, (12, 9, 8), 45)
+    prob, _, b, _, _, ref = sys_
+    B = torch.tensor(b, device="cuda")[:, None].repeat(1, 32)
+    with vdr.Solver(prob, aH=2.0, aM=10.0) as s:
+        for _ in range(3):
+            X = torch.zeros_like(B)
+            _, _, errs, st = s.solve_block_device(B, X, tol=1e-11)
+            assert st == 0 and np.all(errs <= 1e-11)
+            assert rel_l2(X[:, 30].cpu().numpy(), ref) < 1e-9
+            assert s.lib.vdr_diag_wait_timeout(s.h) == L.TIMEOUT

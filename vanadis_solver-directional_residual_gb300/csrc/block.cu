@@ -1468,9 +1468,10 @@ cudaError_t ensure_aos(Handle &h, bool scaled, float4 **out) {
   return cudaSuccess;
 }
 
-// The bulk-copy wait's timeout path, end to end: VDR_TIMEOUT when a wait
-// that nothing completes ran out of its (about 1 ms) budget and the flag
-// reached the host; the context stays usable.
+// The copy waits' timeout paths, end to end (bulk copies, and the ring of
+// tensor copies of the products on rows): VDR_TIMEOUT when waits that nothing
+// completes ran out of their (about 1 ms) budgets and the flags reached the
+// host; the context stays usable.
 int diag_wait_timeout(Handle &h) {
   cudaError_t e;
   if (!h.block_err && (e = cudaMalloc(&h.block_err, sizeof(int))))
@@ -1480,13 +1481,14 @@ int diag_wait_timeout(Handle &h) {
   wait_timeout_kernel<<<1, 32, 0, h.stream>>>(h.block_err, 2000000LL);
   count_launches(1);
   if ((e = cudaGetLastError()) ||
+      (e = launch_ring_timeout(h.block_err, 2, 500000LL, h.stream)) ||
       (e = cudaMemcpyAsync(&flag, h.block_err, sizeof(int), cudaMemcpyDeviceToHost,
                            h.stream)) ||
       (e = cudaMemsetAsync(h.block_err, 0, sizeof(int), h.stream)) ||
       (e = cudaStreamSynchronize(h.stream)))
     return cuda_fail(e, "diag");
-  if (!flag) {
-    set_error("diag: the wait completed although nothing arrived");
+  if (flag != 3) {
+    set_error("diag: a wait completed although nothing arrived");
     return VDR_CUDA_ERROR;
   }
   set_error("diag: the bounded wait ran out as designed");

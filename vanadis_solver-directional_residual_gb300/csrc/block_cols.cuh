@@ -88,6 +88,9 @@ struct BlockOuter {
 bool make_node_map(CUtensorMap *m, const float *base, int words, int nax, int nay, int naz,
                    int bx, int by);
 bool block_rows_usable(Handle &h, int K, BlockRows *g);
+// One warp waits for a copy that is never issued, gives up after `limit`
+// clocks, drains the ring and sets `bit` of *err.
+cudaError_t launch_ring_timeout(int *err, int bit, long long limit, cudaStream_t s);
 cudaError_t block_rows_mask(const BVec &a, const BlockOuter &o, double *X, int *nonzero, int grid,
                             cudaStream_t s);
 cudaError_t block_rows_residual(const BVec &a, const BlockRows &g, const BlockOuter &o,

@@ -203,6 +203,32 @@ struct Share {
 
 constexpr long long WAIT_LIMIT = 2000000000LL;  // ~1 s of clocks per wait
 
+// After a wait of a ring of copies ran out: says so and lets the copies on
+// their way land (each wait bounded).  One thread.
+template <int ST>
+__device__ __forceinline__ void ring_gave_up(uint64_t (&full)[ST], int *err, int bit,
+                                             long long limit) {
+  atomicOr(err, bit);
+  for (int i = 0; i < ST; i++) {
+    tc::mbar_wait(tc::smem_u32(full + i), 0u, limit);
+    tc::mbar_wait(tc::smem_u32(full + i), 1u, limit);
+  }
+}
+
+// The ring's failure path on its own: a stage announced whose copy is never
+// issued, so nothing is in flight.
+__global__ void __launch_bounds__(32) ring_timeout_kernel(int *err, int bit, long long limit) {
+  __shared__ __align__(8) uint64_t full[STAGES];
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < STAGES; i++) tc::mbar_init(tc::smem_u32(full + i), 1);
+    tc::mbar_init_fence();
+    tc::mbar_arrive_expect_tx(tc::smem_u32(full), 1024);
+  }
+  __syncthreads();
+  const bool ok = __syncthreads_and(tc::mbar_wait(tc::smem_u32(full), 0u, limit));
+  if (!ok && threadIdx.x == 0) ring_gave_up(full, err, bit, limit);
+}
+
 struct Maps {
   CUtensorMap x, rows;
 };
@@ -356,15 +382,9 @@ __global__ void __launch_bounds__(PT, 2) br_apply(const BVec a, const BlockRows 
     seen += (unsigned)count;
     ok = __syncthreads_and(ok);  // and the segment's stages are read
   }
-  if (!ok && threadIdx.x == 0) {
-    // a copy did not arrive: stop the iteration, let the copies on their way
-    // land (each wait bounded) and say so
-    atomicOr(g.err, 1);
+  if (!ok && threadIdx.x == 0) {  // a copy did not arrive: the iteration stops
     *(volatile int *)&a.st->done = 1;
-    for (int i = 0; i < ST; i++) {
-      tc::mbar_wait(tc::smem_u32(full + i), 0u, WAIT_LIMIT);
-      tc::mbar_wait(tc::smem_u32(full + i), 1u, WAIT_LIMIT);
-    }
+    ring_gave_up(full, g.err, 1, WAIT_LIMIT);
   }
   __syncthreads();
   DfAcc sums[NQ][4];
@@ -868,6 +888,12 @@ bool make_maps(const BlockRows &g, const float *x, Maps *m) {
 }
 
 }  // namespace
+
+cudaError_t launch_ring_timeout(int *err, int bit, long long limit, cudaStream_t s) {
+  ring_timeout_kernel<<<1, 32, 0, s>>>(err, bit, limit);
+  count_launches(1);
+  return cudaGetLastError();
+}
 
 // The rows of the current operator and the inverse diagonal in h.dinv32;
 // false where the element-wise form stays: another numbering, store or
