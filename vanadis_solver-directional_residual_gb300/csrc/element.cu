@@ -599,7 +599,7 @@ __device__ __forceinline__ Df2 df_point_tau(const OpArgs &a, const double *drs, 
 // store (double-float pairs, or FP64 rows), diag += A_ii, the M store, phi,
 // f and b += cf f_i - ((H - rM M) T_old)_i as the BuildArgs ask; told is the
 // element's T_old at the nodes scaled by 2^-tshift.
-template <bool SPLIT>
+template <bool SPLIT, bool PARTS>
 __device__ __forceinline__ void df_rows_out(const OpArgs &a, const BuildArgs &ba, long p,
                                             int i, int ci, DfAcc (&accH)[8],
                                             DfAcc (&accM)[SPLIT ? 8 : 1], const DfAcc &fw,
@@ -607,7 +607,7 @@ __device__ __forceinline__ void df_rows_out(const OpArgs &a, const BuildArgs &ba
                                             const Df2 *told, int tshift) {
   const long E = a.E;
   const auto give = [&](int q, double *to, double v) {
-    if (ba.parts) ba.parts[(size_t)(8 * q + i) * E + p] = v;
+    if (PARTS) ba.parts[(size_t)(8 * q + i) * E + p] = v;
     else if (ci >= 0) atomicAdd(to + ci, v);
   };
   if (ba.Ahi && !ba.A64) {
@@ -678,7 +678,7 @@ __device__ __forceinline__ void df_rows_out(const OpArgs &a, const BuildArgs &ba
   const double fwd = df_to_double(fw.s, fw.c);
   if (ba.phi) ba.phi[(size_t)i * E + p] = fwd / vol;
   if (ba.f) give(1, ba.f, (qe / vol) * fwd);
-  if (ba.b && (ba.parts || ci >= 0)) {
+  if (ba.b && (PARTS || ci >= 0)) {
     double val = ba.cf * ((qe / vol) * fwd);
     if (SPLIT && ba.told) {
       // (H - rM M) T_old in double-float on the scaled T_old, scaled back
@@ -709,7 +709,7 @@ struct BuildSmemDF {
   Df2 ftab[4][8];            // N at the 4 face-3 points
 };
 
-template <bool SPLIT>
+template <bool SPLIT, bool PARTS>
 __global__ void __launch_bounds__(64, 8) elem_build_df_kernel(OpArgs a, BuildArgs ba) {
   __shared__ BuildSmemDF sm;
   fill_df_tables(sm.tab, sm.ftab);
@@ -874,8 +874,8 @@ __global__ void __launch_bounds__(64, 8) elem_build_df_kernel(OpArgs a, BuildArg
     }
     if (!valid) continue;
     const double qe = (a.f.q && (ba.f || ba.b)) ? __ldg(a.f.q + p) : 0.0;
-    df_rows_out<SPLIT>(a, ba, p, i, ck, accH, accM, fw, qe, vol, aHd, aMd, nrMd, sm.told[le],
-                       tshift);
+    df_rows_out<SPLIT, PARTS>(a, ba, p, i, ck, accH, accM, fw, qe, vol, aHd, aMd, nrMd,
+                              sm.told[le], tshift);
   }
   // Any out-of-window value: the host redoes this build with the FP64 rows
   // (bit 2 of the flag).
@@ -1141,7 +1141,7 @@ __device__ __forceinline__ void lds_x4(const float *p, Df2x2 &a, Df2x2 &b) {
 // right-hand side from T_old 1.72 -> 1.37 ms, without one 1.22 -> 0.99; 8.4 M
 // 9.9 -> 8.4.  Blocks per SM: with the registers that 12 / 16 leave 1.40 / 8.79
 // ms (1.05 M / 8.4 M), 11 / 14 1.40 / 8.40, 10 / 12 1.37 / 8.41.
-template <bool SPLIT>
+template <bool SPLIT, bool PARTS>
 __global__ void __launch_bounds__(64, SPLIT ? 10 : 12) elem_build_geo_kernel(OpArgs a, BuildArgs ba) {
   __shared__ GeoBuildSmem sm;
   if (threadIdx.x < 8) {
@@ -1304,9 +1304,8 @@ __global__ void __launch_bounds__(64, SPLIT ? 10 : 12) elem_build_geo_kernel(OpA
     }
     if (!valid) continue;
     const double qe = (a.f.q && (ba.f || ba.b)) ? __ldg(a.f.q + p) : 0.0;
-    df_rows_out<SPLIT>(a, ba, p, i, ck, accH, accM, fw, qe, df_to_double(vol.h, vol.l), aHd,
-                       aMd, nrMd, sm.told[le],
-                       tshift);
+    df_rows_out<SPLIT, PARTS>(a, ba, p, i, ck, accH, accM, fw, qe, df_to_double(vol.h, vol.l),
+                              aHd, aMd, nrMd, sm.told[le], tshift);
   }
   if (range_bad) atomicOr(ba.bad, 2);
 }
@@ -1541,32 +1540,29 @@ cudaError_t launch_build(const OpArgs &a, const BuildArgs &ba, bool fp32,
     elem_build_kernel<double><<<grid, 64, 0, s>>>(a, ba);
   else {
     if (ba.gK ? !ba.gsc : !ba.drs) return cudaErrorInvalidValue;
+    // [from the geometric factors][H and M apart][sums left to launch_node_sums,
+    // a kernel of its own: the choice inside cost the others 2 per cent]
+    using Kern = void (*)(OpArgs, BuildArgs);
+    static const Kern kernels[2][2][2] = {
+        {{elem_build_df_kernel<false, false>, elem_build_df_kernel<false, true>},
+         {elem_build_df_kernel<true, false>, elem_build_df_kernel<true, true>}},
+        {{elem_build_geo_kernel<false, false>, elem_build_geo_kernel<false, true>},
+         {elem_build_geo_kernel<true, false>, elem_build_geo_kernel<true, true>}}};
     static std::once_flag carveout;  // 8 blocks of 27.5 KB need the full carveout,
+                                     // as do 10 / 12 blocks of 11.9 KB
     std::call_once(carveout, [] {
-      cudaFuncSetAttribute(elem_build_df_kernel<true>,
-                           cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-      cudaFuncSetAttribute(elem_build_df_kernel<false>,
-                           cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-      // 10 / 12 blocks of 11.9 KB
-      cudaFuncSetAttribute(elem_build_geo_kernel<true>,
-                           cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-      cudaFuncSetAttribute(elem_build_geo_kernel<false>,
-                           cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+      for (const auto &apart : kernels)
+        for (const auto &parts : apart)
+          for (const Kern kern : parts)
+            cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     });
     const int g2 = (int)std::min<long>(((long)a.E + 255) / 256, (long)device_sm_count() * 8);
     if (ba.gK) {  // from the mesh's geometric factors
       elem_geo_scalars_kernel<<<g2, 256, 0, s>>>(a, ba.gsc, ba.bad);
-      if (ba.told || ba.Mhi)
-        elem_build_geo_kernel<true><<<grid, 64, 0, s>>>(a, ba);
-      else
-        elem_build_geo_kernel<false><<<grid, 64, 0, s>>>(a, ba);
     } else {
       elem_dr_scalars_kernel<<<g2, 256, 0, s>>>(a, ba.drs);
-      if (ba.told || ba.Mhi)  // H and M apart
-        elem_build_df_kernel<true><<<grid, 64, 0, s>>>(a, ba);
-      else
-        elem_build_df_kernel<false><<<grid, 64, 0, s>>>(a, ba);
     }
+    kernels[ba.gK != nullptr][ba.told || ba.Mhi][ba.parts != nullptr]<<<grid, 64, 0, s>>>(a, ba);
     count_launches(1);
   }
   count_launches(1);
