@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(512, 2) sgr_first(SegVec a) {
   const int s = tl.seg;
   if (!a.s.active[s]) return;
   const long at = a.mesh[s].shift;
-  const int e = a.s.pmax[s], er = a.s.rmax[s], base = pair_base(a.rows.nm);
+  const int e = a.s.pmax[s], er = a.s.rmax[s], base = 1023 - pair_head(a.rows.nm);
   TLOOP(i) {
     const double ri = a.r[i];
     const bool m = a.m[i] != 0;
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(512, 2) sgr_first(SegVec a) {
     a.php[i + at] = m ? make_float2(0.f, 0.f) : stencil_pair(ri * a.dinv[i], e - base);
     a.shp[i + at] = m ? make_float2(0.f, 0.f) : stencil_pair(ri, er - base);
   }
-  if (tl.start == a.mesh[s].n0 && threadIdx.x == 0) a.s.pexp[s] = e;
+  if (tl.start == a.mesh[s].n0 && threadIdx.x == 0) a.s.pexp[s] = e + 1023 - base;
 }
 
 __device__ __forceinline__ void seg_alpha(const SegVec &a, int s, double wp) {
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(512, 2) sgr_w(SegVec a) {
   const SegMesh g = a.mesh[s];
   const StencilView v = mesh_rows(a, g);
   const float2 *xp = a.shp + g.shift;
-  const int shift = a.s.rmax[s] - pair_base(v.nm);
+  const int shift = a.s.rmax[s] + pair_head(v.nm) - 1023;
   double q[1] = {0.0};
   TLOOP(i) {
     const unsigned m = v.nm[i];
@@ -370,7 +370,10 @@ __global__ void __launch_bounds__(512, 2) sgr_w(SegVec a) {
     if (!a.m[i]) q[0] += o * (a.p[i] * a.dinv[i]);
   }
   double o[1];
-  if (seg_sum<1>(q, a, tile, s, o)) seg_alpha(a, s, o[0]);
+  if (seg_sum<1>(q, a, tile, s, o)) {
+    a.s.pmax[s] += pair_head(v.nm);
+    seg_alpha(a, s, o[0]);
+  }
 }
 
 template <bool KEEP>
@@ -382,7 +385,7 @@ __global__ void __launch_bounds__(512, 2) sgr_v(SegVec a) {
   if (!a.s.active[s]) return;
   const SegMesh g = a.mesh[s];
   const StencilView v = mesh_rows(a, g);
-  const int shift = a.s.pexp[s] - pair_base(v.nm);
+  const int shift = a.s.pexp[s] - 1023;
   const double al = a.s.alpha[s];
   double q[2] = {0.0, 0.0};
   TLOOP(i) {
@@ -414,7 +417,7 @@ __global__ void __launch_bounds__(512, 2) sgr_t(SegVec a) {
   if (!a.s.active[s] || a.s.sconv[s]) return;
   const SegMesh g = a.mesh[s];
   const StencilView v = mesh_rows(a, g);
-  const int shift = a.s.pexp[s] - pair_base(v.nm);
+  const int shift = a.s.pexp[s] - 1023;
   double q[3] = {0.0, 0.0, 0.0};
   TLOOP(i) {
     const double si = a.sv[i], hi = a.rh[i];
@@ -456,7 +459,7 @@ __global__ void __launch_bounds__(512, 2) sgr_p(SegVec a) {
   }
   const double om = a.s.omega[s], rho1 = a.s.rho_next[s];
   const double beta = a.s.beta[s];
-  const int e = a.s.pmax[s], shift = e - pair_base(a.rows.nm);
+  const int e = a.s.pmax[s], shift = e - 1023;
   const long at = a.mesh[s].shift;
   int em = 0;
   TLOOP(i) {
@@ -479,7 +482,7 @@ __global__ void __launch_bounds__(512, 2) sgr_p(SegVec a) {
   if (seg_sum<2>(q, a, tile, s, o)) {
     a.s.iter[s] += 1;
     a.s.pexp[s] = e;
-    a.s.pmax[s] = atomicExch(a.s.pmax_next + s, 0);
+    a.s.pmax[s] = atomicExch(a.s.pmax_next + s, 0) + pair_head(a.rows.nm);
     a.s.rho[s] = rho1;
     const double err = sqrt(o[0] / a.s.bnrm2[s]);
     a.s.err[s] = err;

@@ -624,7 +624,7 @@ __global__ void __launch_bounds__(PT, 2) br_residual(const BVec a, const BlockRo
 #pragma unroll
     for (int c = 0; c < 4; c++) rm[c] = bm[c];
   } else {
-    const int base = pair_base(g.nm);
+    const int base = 1023 - pair_head(g.nm);
     int shift[4];
 #pragma unroll
     for (int c = 0; c < 4; c++) shift[c] = o.xexp[4 * l + c] - base;

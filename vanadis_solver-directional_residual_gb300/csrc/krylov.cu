@@ -98,7 +98,7 @@ struct Vec {
   double *x, *r, *rh, *p, *v, *ph, *s, *sh, *t;  // BiCGStab
   double *rr, *pp, *z, *zz;                      // BiCG (r, p, x shared)
   float2 *php, *shp;  // p^ and s^ as pairs (assembled operator)
-  const unsigned *nm;  // the rows', for pair_base
+  const unsigned *nm;  // the rows', null where they are not current
   double *w;          // A^T rh (assembled operator, in p^'s place)
 };
 
@@ -157,6 +157,10 @@ __global__ void __launch_bounds__(RED_THREADS) k_start(Vec a) {
   double o[3];
   if (grid_sum<3>(v, a.partials, &a.st->ticket, o)) {
     KState *st = a.st;
+    if (a.nm) {
+      st->pmax += pair_head(a.nm);
+      st->rmax += pair_head(a.nm);
+    }
     st->bnrm2 = o[0];
     st->iter = 0;
     st->sconv = 0;
@@ -462,7 +466,7 @@ Vec make_vec(Handle &h, const double *b, double *x) {
     a.php = h.st_x + stencil_pad(h);
     a.shp = a.php + N + 2 * stencil_pad(h);
     a.w = a.ph;
-    a.nm = stencil_view(h).nm;
+    a.nm = stencil_ready(h) ? stencil_view(h).nm : nullptr;
   }
   return a;
 }
@@ -476,7 +480,7 @@ Vec make_vec(Handle &h, const double *b, double *x) {
 // w = A^T rh, formed once, gives alpha = rho / (w, p^) before the product it
 // scales; the next rho is (rh, s) - omega (rh, t), known before r is formed.
 // p^ and s^ exist only as the products' inputs, pairs scaled by the largest
-// exponent of the direction before (pair_base: room for 2^48 times that).  618 bytes per node and iteration against 1,024 E + ~240 N
+// exponent of the direction before (pair_head: room for 2^48 times that).  618 bytes per node and iteration against 1,024 E + ~240 N
 // element-wise; each kernel's last block adds the block partials in a fixed
 // order.
 
@@ -484,13 +488,13 @@ Vec make_vec(Handle &h, const double *b, double *x) {
 __global__ void __launch_bounds__(RED_THREADS) bst_first(Vec a) {
   KState *st = a.st;
   if (st->done) return;
-  const int e = st->pmax, er = st->rmax, base = pair_base(a.nm);
+  const int e = st->pmax, er = st->rmax;
   double rv[U], dv[U];
   unsigned char mv[U];
   VLOOP(rv[u] = ok ? a.r[i] : 0.0; dv[u] = ok ? a.dinv[i] : 0.0; mv[u] = ok ? a.m[i] : 1;,
         a.p[i] = rv[u];
-        a.shp[i] = mv[u] ? make_float2(0.f, 0.f) : stencil_pair(rv[u], er - base);
-        a.php[i] = mv[u] ? make_float2(0.f, 0.f) : stencil_pair(rv[u] * dv[u], e - base);)
+        a.shp[i] = mv[u] ? make_float2(0.f, 0.f) : stencil_pair(rv[u], er - 1023);
+        a.php[i] = mv[u] ? make_float2(0.f, 0.f) : stencil_pair(rv[u] * dv[u], e - 1023);)
   if (blockIdx.x == 0 && threadIdx.x == 0) st->pexp = e;
 }
 
@@ -508,7 +512,7 @@ __device__ __forceinline__ void bst_alpha(KState *st, double wp) {
 // w = A^T rh with (w, p^).
 __global__ void __launch_bounds__(RED_THREADS, 4) bst_w(Vec a, StencilView w) {
   if (a.st->done) return;
-  const int shift = a.st->rmax - pair_base(w.nm);
+  const int shift = a.st->rmax - 1023;
   double v[1] = {0.0};
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n;
        i += (long)gridDim.x * blockDim.x) {
@@ -523,7 +527,7 @@ __global__ void __launch_bounds__(RED_THREADS, 4) bst_w(Vec a, StencilView w) {
 template <bool KEEP>
 __global__ void __launch_bounds__(RED_THREADS, 4) bst_v(Vec a, StencilView w) {
   if (a.st->done) return;
-  const int shift = a.st->pexp - pair_base(w.nm);
+  const int shift = a.st->pexp - 1023;
   const double al = a.st->alpha;
   double v[2] = {0.0, 0.0};
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n;
@@ -550,7 +554,7 @@ __global__ void __launch_bounds__(RED_THREADS, 4) bst_v(Vec a, StencilView w) {
 template <bool KEEP>
 __global__ void __launch_bounds__(RED_THREADS, 4) bst_t(Vec a, StencilView w) {
   if (a.st->done || a.st->sconv) return;
-  const int shift = a.st->pexp - pair_base(w.nm);
+  const int shift = a.st->pexp - 1023;
   double v[3] = {0.0, 0.0, 0.0};
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n;
        i += (long)gridDim.x * blockDim.x) {
@@ -603,7 +607,7 @@ __global__ void __launch_bounds__(RED_THREADS, 4) bst_p(Vec a) {
   }
   const double om = stc->omega, rho1 = stc->rho_next;
   const double beta = stc->beta;
-  const int e = stc->pmax, shift = e - pair_base(a.nm);
+  const int e = stc->pmax, shift = e - 1023;
   int em = 0;
   double v[2] = {0.0, 0.0};
   constexpr int UP = 2;
@@ -647,7 +651,7 @@ __global__ void __launch_bounds__(RED_THREADS, 4) bst_p(Vec a) {
     KState *st = a.st;
     st->iter += 1;
     st->pexp = e;
-    st->pmax = atomicExch(&st->pmax_next, 0);
+    st->pmax = atomicExch(&st->pmax_next, 0) + pair_head(a.nm);
     st->rho_old = st->rho;
     st->rho = rho1;
     st->err = sqrt(o[0]) / sqrt(st->bnrm2);
@@ -977,21 +981,22 @@ __global__ void __launch_bounds__(RED_THREADS) bst_xmax(Vec a, int *ex) {
   em = __reduce_max_sync(FULL, em);
   if ((threadIdx.x & 31) == 0) atomicMax(ex, em);
 }
-__global__ void __launch_bounds__(RED_THREADS) bst_xsplit(Vec a, const int *ex) {
-  const int shift = *ex - pair_base(a.nm);
+// ex[1]: the exponent with the pairs' head, 0 where x is zero.
+__global__ void __launch_bounds__(RED_THREADS) bst_xsplit(Vec a, int *ex) {
+  const int e = *ex ? *ex + pair_head(a.nm) : 0, shift = e - 1023;
+  if (blockIdx.x == 0 && threadIdx.x == 0) ex[1] = e;
   if (*ex == 0) return;
   double xv[U];
   VLOOP(xv[u] = ok ? a.x[i] : 0.0;, a.php[i] = stencil_pair(xv[u], shift);)
 }
 __global__ void __launch_bounds__(RED_THREADS, 4) bst_residual(Vec a, StencilView w, double *r,
                                                                const int *ex, double *out) {
-  const int e = *ex;  // 0: x is zero
-  const int shift = e - pair_base(w.nm);
+  const int e = ex[1];  // 0: x is zero
   double v[2] = {0.0, 0.0};
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n;
        i += (long)gridDim.x * blockDim.x) {
     const double bi = a.b[i];
-    const double ax = e ? stencil_row_pairs<false, false>(w, i, a.php, shift) : 0.0;
+    const double ax = e ? stencil_row_pairs<false, false>(w, i, a.php, e - 1023) : 0.0;
     const double ri = bi - ax;
     r[i] = ri;
     v[0] += ri * ri;

@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicgstab(ResArgs a) {
   const int N = a.w.N, n = (int)(blockIdx.x * T + threadIdx.x);
   const bool on = n < N;
   unsigned target = 0;
-  const int base = pair_base(a.w.nm);
+  const int base = 1023 - pair_head(a.w.nm);
   const int none[1] = {0};
   const auto nothing = [](int) {};
   double x = 0.0, r = 0.0, p = 0.0, v = 0.0, s = 0.0, t = 0.0, rh = 0.0, wn = 0.0;
@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(T, 1) resident_bicg(const __grid_constant__ Re
   const int N = a.w.N, n = (int)(blockIdx.x * T + threadIdx.x);
   const bool on = n < N;
   unsigned target = 0;
-  const int base = pair_base(a.w.nm);
+  const int base = 1023 - pair_head(a.w.nm);
   const int none[1] = {0};
   const auto nothing = [](int) {};
   const auto column = [&](int k) {  // A's entry of neighbour k with this node

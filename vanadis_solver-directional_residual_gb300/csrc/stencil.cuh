@@ -29,14 +29,15 @@ namespace vdr {
 
 struct StencilView {
   const float2 *S = nullptr;
-  const unsigned *nm = nullptr;  // and before it what pair_base reads
+  const unsigned *nm = nullptr;  // and before it what pair_head reads
   int N = 0, nax = 0, pl = 0;
 };
 
 constexpr int NM_LEAD = 32;  // words before nm; the last: the biased FP32
                              // exponent of the largest entry
-// A vector whose largest biased exponent is e becomes pairs by 2^-(e - base):
-// largest magnitude in [2^h, 2^(h + 1)) with h = 200 - top, at most 72.  A
+// A vector whose largest biased exponent is e becomes pairs by 2^-(e + head -
+// 1023): largest magnitude in [2^h, 2^(h + 1)), h = -head = 200 - top, at most
+// 72.  (The exponents that the iterations keep have head added already.)  A
 // row's 27 products then stay below 2^128 for a vector 2^48 times larger than
 // the one that gave e: the iterations scale a direction and its s^ by the
 // direction before.  (2^53 times larger, FP64 would have nothing left of the
@@ -44,8 +45,8 @@ constexpr int NM_LEAD = 32;  // words before nm; the last: the biased FP32
 // with entries around 1, values down to 2^-198 of the largest are held and
 // down to 2^-174 in full; with the largest entries that the store allows
 // (2^123 once summed) it is 2^-76 and 2^-52.
-__device__ __forceinline__ int pair_base(const unsigned *nm) {
-  return 1023 - max((int)nm[-1] - 200, -72);
+__device__ __forceinline__ int pair_head(const unsigned *nm) {
+  return max((int)nm[-1] - 200, -72);
 }
 
 __device__ __forceinline__ int stencil_off(int k, int nax, int pl) {
@@ -114,7 +115,7 @@ __device__ __forceinline__ double stencil_row(const StencilView &v, long n,
 }
 
 // The Krylov iteration's form: the input already split into pairs, scaled by
-// one power of two per vector (pair_base), with zeros for a plane and a row beyond both
+// one power of two per vector (pair_head), with zeros for a plane and a row beyond both
 // ends (stencil_pad), so that the 27 products need no mask, no index clamp
 // and no split: the rows hold zeros wherever no coupling exists.
 // A^T reads its neighbours' rows at shifted places, which stay inside S.
