@@ -308,12 +308,15 @@ int vdr_diag_wait_timeout(vdr_handle *h);
  * usable). */
 int vdr_diag_barrier_timeout(vdr_handle *h);
 /* The handle goes on as if the device had refused: launches of one cluster,
- * whole-solve launches, further memory for assembled rows (any of the bits;
- * 0: everything again, but an operator whose rows were refused stays
- * element-wise).  For tests of the paths that are then taken. */
+ * whole-solve launches, further memory for assembled rows, any other further
+ * memory as long as the handle holds rows, which are given back for it (any
+ * of the bits; 0: everything again, but a handle whose rows were refused or
+ * given back stays element-wise).  For tests of the paths that are then
+ * taken. */
 #define VDR_WITHOUT_CLUSTER 1
 #define VDR_WITHOUT_WHOLE_SOLVE 2
 #define VDR_WITHOUT_ROWS 4
+#define VDR_WITHOUT_OTHER_ROOM 8
 int vdr_diag_without(vdr_handle *h, int what);
 /* Diagnostic of the bounded meetings of the whole-solve launches: one block
  * of three never arrives, the others give up after ~1 ms, and one of them

@@ -223,7 +223,7 @@ def test_meeting_times_out_and_recovers(vdr, oracle, gpu_lib):
                     assert st == 0 and err <= 1e-11 and rel_l2(x.cpu().numpy(), ref) < 1e-9
 
 
-CLUSTER, WHOLE_SOLVE, ROWS = 1, 2, 4
+CLUSTER, WHOLE_SOLVE, ROWS, OTHER_ROOM = 1, 2, 4, 8
 
 
 def test_segmented_solve_after_rows_were_refused(vdr, oracle, gpu_lib):
@@ -435,3 +435,58 @@ def test_block_solve_after_copy_waits_ran_out(vdr, oracle, gpu_lib):
             assert st == 0 and np.all(errs <= 1e-11)
             assert rel_l2(X[:, 30].cpu().numpy(), ref) < 1e-9
             assert s.lib.vdr_diag_wait_timeout(s.h) == L.TIMEOUT
+
+
+@pytest.mark.parametrize("call", ["block", "gcr", "loop", "mixed", "half", "network"])
+def test_rows_make_room(vdr, oracle, gpu_lib, call):
+    """Calls that need memory beside the rows of an earlier solve and find
+    none: the rows are given back for it, the call's result is the oracle's,
+    and later solves run by elements, in mixed precision too."""
+    torch = pytest.importorskip("torch")
+    sys_ = system(vdr, oracle, (12, 9, 8), 46)
+    prob, bb, b, diag, x0, ref = sys_
+    m = prob.mesh
+    bd = torch.tensor(b, device="cuda")
+
+    def solved(x):
+        return rel_l2(x.cpu().numpy(), ref) < 1e-9
+
+    with vdr.Solver(prob, aH=2.0, aM=10.0) as s:
+        x = torch.tensor(x0, device="cuda")
+        assert s.solve_device(bd, x, tol=1e-11, itmax=2000)[2] == 0 and solved(x)
+        assert s.stats()["kernel_launches"] == 1
+        assert s.lib.vdr_diag_without(s.h, OTHER_ROOM) == 0
+        x = torch.tensor(x0, device="cuda")
+        if call == "block":
+            X = torch.zeros(s.N, 16, dtype=torch.float64, device="cuda")
+            _, _, errs, st = s.solve_block_device(bd[:, None].repeat(1, 16), X, tol=1e-11)
+            assert st == 0 and solved(X[:, 9])
+        elif call == "gcr":
+            assert s.solve_gcr_device(bd, x, tol=1e-11, itmax=2000)[2] == 0 and solved(x)
+        elif call == "loop":
+            told = np.cos(0.37 * np.arange(m.nnode))
+            t = torch.tensor(told, device="cuda")
+            torch.cuda.synchronize()
+            _, its, _, st, done = s.time_steps_device(t, 1, 3.0, 10.0, tol=1e-11, itmax=2000)
+            assert st == 0 and done == 1 and solved(t)
+        elif call == "mixed":
+            s.set_mixed_operator("half")
+            assert s.solve_mixed_device(bd, x, tol=1e-11, inner_tol=1e-3)[3] == 0 and solved(x)
+        elif call == "half":
+            y = torch.empty(s.N, dtype=torch.float32, device="cuda")
+            s.apply_half_device((bd / bd.abs().max()).float(), y)
+            torch.cuda.synchronize()
+            want, _ = oracle.matvec0(m.iss, bb, prob.bc, b / np.abs(b).max() / diag)
+            assert rel_l2(y.double().cpu().numpy(), want) < 2e-3
+        else:
+            with vdr.LearnedNet(s, seed=2) as net:
+                net.update_features()
+                assert s.solve_learned_device(net, bd, x, tol=1e-9, itmax=2000)[2] == 0
+                assert rel_l2(x.cpu().numpy(), ref) < 1e-7
+        for without in (OTHER_ROOM, 0):
+            assert s.lib.vdr_diag_without(s.h, without) == 0
+            x = torch.tensor(x0, device="cuda")
+            assert s.solve_device(bd, x, tol=1e-11, itmax=2000)[2] == 0 and solved(x)
+            assert s.stats()["kernel_launches"] > 1
+            x = torch.tensor(x0, device="cuda")
+            assert s.solve_mixed_device(bd, x, tol=1e-11, inner_tol=1e-4)[3] == 0 and solved(x)

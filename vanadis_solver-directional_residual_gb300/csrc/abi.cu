@@ -197,7 +197,7 @@ int build_operator(Handle &h, const BuildArgs *rhs) {
     ba.exact_fp64 = h.exact_build;
     ba.bad = h.flag;
     if ((need_op || rhs->Mhi) && !h.exact_build && ordered_sums(h)) {
-      if ((e = dalloc(&h.build_parts, (size_t)h.E * 24))) return cuda_fail(e, "alloc build parts");
+      if ((e = take(h, &h.build_parts, (size_t)h.E * 24))) cudaGetLastError();  // by atomics
       ba.parts = h.build_parts;
     }
     if (rhs) {
@@ -217,7 +217,7 @@ int build_operator(Handle &h, const BuildArgs *rhs) {
       }
     }
     if (need_op) {
-      if (stored && !df && (e = dalloc(&h.A64, (size_t)h.E * 32)))
+      if (stored && !df && (e = take(h, &h.A64, (size_t)h.E * 32)))
         return cuda_fail(e, "alloc element matrices");
       if (df && ((e = dalloc(&h.Ahi, (size_t)h.E * 16)) ||
                  (e = dalloc(&h.Alo, (size_t)h.E * 16))))
@@ -231,7 +231,7 @@ int build_operator(Handle &h, const BuildArgs *rhs) {
       ba.Alo = df ? h.Alo : nullptr;
       ba.diag = h.diag;
       if (h.want_phi) {
-        if ((e = dalloc(&h.phi, (size_t)h.E * 8))) return cuda_fail(e, "alloc phi");
+        if ((e = take(h, &h.phi, (size_t)h.E * 8))) return cuda_fail(e, "alloc phi");
         ba.phi = h.phi;
       }
     }
@@ -244,14 +244,14 @@ int build_operator(Handle &h, const BuildArgs *rhs) {
         if (gst) return gst;
       }
       if (geo) {
-        if ((e = dalloc(&h.gsc, (size_t)h.E * 10)))
+        if ((e = take(h, &h.gsc, (size_t)h.E * 10)))
           return cuda_fail(e, "alloc element scalars");
         ba.gJi = h.geo.Ji;
         ba.gDj = h.geo.Dj;
         ba.gK = h.geo.K;
         ba.gsc = h.gsc;
       } else {
-        if ((e = dalloc(&h.drs, (size_t)h.E * 5))) return cuda_fail(e, "alloc DR scalars");
+        if ((e = take(h, &h.drs, (size_t)h.E * 5))) return cuda_fail(e, "alloc DR scalars");
         ba.drs = h.drs;
       }
     }
@@ -333,7 +333,7 @@ int ensure_operator32(Handle &h) {
     }
   }
   cudaError_t e;
-  if ((e = dalloc(&h.A32, (size_t)h.E * 16))) return cuda_fail(e, "alloc FP32 matrices");
+  if ((e = take(h, &h.A32, (size_t)h.E * 16))) return cuda_fail(e, "alloc FP32 matrices");
   BuildArgs ba;
   ba.aH = h.aH;
   ba.aM = h.aM;
@@ -350,7 +350,12 @@ int ensure_operator32(Handle &h) {
 int ensure_inner(Handle &h, int method) {
   if (method == VDR_SOLVER_BICGSTAB) {
     int st = ensure_operator(h);
-    if (st || (st = ensure_half_rows(h))) return st;
+    if (st) return st;
+    // what else the solve takes comes first: room for it is not to be made
+    // from rows that it has counted on
+    const cudaError_t e = ensure_solver_workspace(h, 11);
+    if (e) return cuda_fail(e, "solver workspace");
+    if ((st = ensure_half_rows(h))) return st;
     if (half_rows_ready(h)) return VDR_OK;
   }
   return ensure_operator32(h);
@@ -728,7 +733,7 @@ int vdr_set_operator(vdr_handle *H, double aH, double aM) {
 }
 
 static int ensure_io(vdr_handle *H) {
-  cudaError_t e = dalloc(&H->io, 3 * (size_t)H->h.N);
+  cudaError_t e = take(H->h, &H->io, 3 * (size_t)H->h.N);
   return e ? cuda_fail(e, "alloc io") : VDR_OK;
 }
 
@@ -1104,13 +1109,14 @@ int vdr_diag_wait_timeout(vdr_handle *H) {
 int vdr_diag_without(vdr_handle *H, int what) {
   int st = check_handle(H);
   if (st) return st;
-  if (what < 0 || what > (VDR_WITHOUT_CLUSTER | VDR_WITHOUT_WHOLE_SOLVE | VDR_WITHOUT_ROWS)) {
+  if (what < 0 || what >= 2 * VDR_WITHOUT_OTHER_ROOM) {
     set_error("vdr_diag_without: unknown bits");
     return VDR_BAD_ARGUMENT;
   }
   H->h.resident_cluster = !(what & VDR_WITHOUT_CLUSTER);
   H->h.resident = !(what & VDR_WITHOUT_WHOLE_SOLVE);
   H->h.rows_room = !(what & VDR_WITHOUT_ROWS);
+  H->h.other_room = !(what & VDR_WITHOUT_OTHER_ROOM);
   return VDR_OK;
 }
 
@@ -1246,8 +1252,8 @@ int vdr_time_steps(vdr_handle *H, int nsteps, double cf, double rM,
   // b = cf F - (H - rM M) T_old from two applies instead of a Gauss pass.
   const bool keep_mass = h.apply_mode == VDR_APPLY_STORED && h.aH != 0.0;
   if (keep_mass &&
-      ((e = dalloc(&h.Mhi, (size_t)h.E * 16)) || (e = dalloc(&h.Mlo, (size_t)h.E * 16)) ||
-       (e = dalloc(&h.Fvec, h.N)) || (e = dalloc(&h.rhs_tmp, 2 * (size_t)h.N)))) {
+      ((e = take(h, &h.Mhi, (size_t)h.E * 16)) || (e = take(h, &h.Mlo, (size_t)h.E * 16)) ||
+       (e = take(h, &h.Fvec, h.N)) || (e = take(h, &h.rhs_tmp, 2 * (size_t)h.N)))) {
     if (dmass) cudaFree(dmass);
     return cuda_fail(e, "vdr_time_steps: alloc");
   }
@@ -1431,13 +1437,13 @@ int legacy_prepare(Legacy &L, int N, int E) {
       h.ev[k] = nullptr;
     }
     const size_t cN = std::max(N, L.capN), cE = std::max(E, L.capE);
-    if ((e = dalloc(&h.Ahi, cE * 16)) ||
-        (e = dalloc(&h.Alo, cE * 16)) || (e = dalloc(&h.conn, cE * 8)) ||
-        (e = dalloc(&h.emask, cE)) || (e = dalloc(&h.diag, cN)) || (e = dalloc(&h.dinv, cN)) ||
-        (e = dalloc(&h.mask, cN)) ||
-        (e = dalloc(&L.bb, cE * 64)) || (e = dalloc(&L.b, cN)) ||
-        (e = dalloc(&L.x, cN)) || (e = dalloc(&L.iss, cE * 8)) ||
-        (e = dalloc(&L.bc, cN)) || (e = dalloc(&L.bad, 1))) {
+    if ((e = take(h, &h.Ahi, cE * 16)) ||
+        (e = take(h, &h.Alo, cE * 16)) || (e = take(h, &h.conn, cE * 8)) ||
+        (e = take(h, &h.emask, cE)) || (e = take(h, &h.diag, cN)) || (e = take(h, &h.dinv, cN)) ||
+        (e = take(h, &h.mask, cN)) ||
+        (e = take(h, &L.bb, cE * 64)) || (e = take(h, &L.b, cN)) ||
+        (e = take(h, &L.x, cN)) || (e = take(h, &L.iss, cE * 8)) ||
+        (e = take(h, &L.bc, cN)) || (e = take(h, &L.bad, 1))) {
       L.capN = L.capE = 0;
       return cuda_fail(e, "kernel_dbcg_simple_: alloc");
     }
@@ -1525,7 +1531,7 @@ void kernel_dbcg_simple_(int *Np, double *B, double *X, double *TOLp,
   h.nax = canonical ? (int)nax : 0;
   h.nay = canonical ? (int)nay : 0;
   h.naz = canonical ? (int)naz : 0;
-  if (h.st_state > 0) h.st_state = 0;
+  h.st_state = 0;  // whether there is room for rows is asked at every call
   if (canonical && (e = launch_emask(h))) {
     cuda_fail(e, "kernel_dbcg_simple_: masks");
     *ERRp = inf;

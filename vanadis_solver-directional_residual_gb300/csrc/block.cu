@@ -1449,7 +1449,7 @@ cudaError_t ensure_aos(Handle &h, bool scaled, float4 **out) {
     if ((e = cudaMemset(h.block_err, 0, sizeof(int)))) return e;
   }
   if (!h.Aaos) {
-    if ((e = cudaMalloc(&h.Aaos, sizeof(float4) * 16 * (size_t)h.E))) return e;
+    if ((e = take(h, &h.Aaos, 16 * (size_t)h.E))) return e;
     h.aos_valid = false;
   }
   if (!h.aos_valid || h.aos_scaled != scaled) {
@@ -1521,14 +1521,12 @@ int solve_block_device(Handle &h, int K, int precision, const double *B,
     h.bk_K = 0;
     if (h.bk_graph) cudaGraphExecDestroy(h.bk_graph);
     h.bk_graph = nullptr;
-    if ((e = cudaMalloc(&h.bk_f, sizeof(float) * 8 * (size_t)n)) ||
-        (e = cudaMalloc(&h.bk_d, sizeof(double) * ((size_t)n + BK_COLS +
-                                                   BK_PARTIALS + 8))))
+    if ((e = take(h, &h.bk_f, 8 * (size_t)n)) ||
+        (e = take(h, &h.bk_d, (size_t)n + BK_COLS + BK_PARTIALS + 8)))
       return cuda_fail(e, "block workspace");
     h.bk_K = K;
   }
-  if (!h.dinv32 && (e = cudaMalloc(&h.dinv32, sizeof(float) * (size_t)h.N)))
-    return cuda_fail(e, "block workspace");
+  if ((e = take(h, &h.dinv32, h.N))) return cuda_fail(e, "block workspace");
   float *fv = h.bk_f;
   double *R = h.bk_d;
   double *colsd = R + n;

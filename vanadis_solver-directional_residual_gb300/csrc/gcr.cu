@@ -311,7 +311,7 @@ int solve_gcr_device(Handle &h, const double *b, double *x, double tol,
     h.gcr_words = 0;
     if (h.gcr_graph) cudaGraphExecDestroy(h.gcr_graph);
     h.gcr_graph = nullptr;
-    if ((e = cudaMalloc(&h.gcr_work, sizeof(double) * need))) return cuda_fail(e, "GCR workspace");
+    if ((e = take(h, &h.gcr_work, need))) return cuda_fail(e, "GCR workspace");
     h.gcr_words = need;
   }
   GcrArgs a{};

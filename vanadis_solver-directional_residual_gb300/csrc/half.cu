@@ -244,9 +244,7 @@ bool half_store_available(const Handle &h) {
 
 cudaError_t launch_half_store(Handle &h, int *bad, cudaStream_t s) {
   cudaError_t e;
-  if (!h.A16 && (e = cudaMalloc(&h.A16, sizeof(uint4) * 8 * (size_t)h.E)))
-    return e;
-  if (!h.e16 && (e = cudaMalloc(&h.e16, (size_t)h.E))) return e;
+  if ((e = take(h, &h.A16, 8 * (size_t)h.E)) || (e = take(h, &h.e16, h.E))) return e;
   const ConnView cv = conn_view(h);
   const float4 *hi = (h.storage == VDR_STORE_DF) ? h.Ahi : nullptr;
   const double2 *a64 = hi ? nullptr : h.A64;

@@ -742,7 +742,7 @@ cudaError_t ensure_solver_workspace(Handle &h, int nvec) {
     if (h.work) cudaFree(h.work);
     h.work = nullptr;
     h.nwork = 0;
-    if ((e = cudaMalloc(&h.work, sizeof(double) * (size_t)h.N * nvec))) return e;
+    if ((e = take(h, &h.work, (size_t)h.N * nvec))) return e;
     h.nwork = nvec;
     for (int k = 0; k < Handle::NGRAPH; k++) {
       if (h.graph_exec[k]) cudaGraphExecDestroy(h.graph_exec[k]);
@@ -1814,7 +1814,7 @@ namespace {
 // relative residual; graph-captured like solve_device.
 int solve32_inner(Handle &h, double tol, int itmax, int *iter, double *err) {
   cudaError_t e;
-  if (!h.work32 && (e = cudaMalloc(&h.work32, sizeof(float) * 10 * (size_t)h.N)))
+  if ((e = take(h, &h.work32, 10 * (size_t)h.N)))
     return cuda_fail(e, "FP32 workspace");
   cudaStream_t s = h.stream;
   Vec32 a = make_vec32(h);
@@ -1926,10 +1926,9 @@ int solve_mixed_device(Handle &h, int method, const double *b, double *x,
   // The stored FP32 operator runs its inner BiCGStab on FP32 vectors.
   const bool f32v = h.apply_mode == VDR_APPLY_STORED && method == VDR_SOLVER_BICGSTAB;
   const bool hr = f32v && half_rows_ready(h);
-  if (f32v && !hr && !h.dinv32 && (e = cudaMalloc(&h.dinv32, sizeof(float) * (size_t)h.N)))
+  if (f32v && !hr && (e = take(h, &h.dinv32, h.N)))
     return cuda_fail(e, "FP32 diagonal");
-  if (f32v && !hr && !h.work32 &&
-      (e = cudaMalloc(&h.work32, sizeof(float) * 10 * (size_t)h.N)))
+  if (f32v && !hr && (e = take(h, &h.work32, 10 * (size_t)h.N)))
     return cuda_fail(e, "FP32 workspace");
   for (int outer = 0; outer <= max_outer; outer++) {
     h.apply_fp32 = false;

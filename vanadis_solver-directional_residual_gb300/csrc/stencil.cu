@@ -203,6 +203,39 @@ static bool row_storage(Handle &h, float2 **x, size_t *have, size_t len) {
   return false;
 }
 
+cudaError_t take_memory(Handle &h, void **p, size_t bytes) {
+  const bool held = h.st_S || h.hr_H || h.br_rows;
+  cudaError_t e = cudaErrorMemoryAllocation;
+  if ((h.other_room || !held) && !(e = cudaMalloc(p, bytes))) return cudaSuccess;
+  *p = nullptr;
+  if (!held) return e;
+  cudaGetLastError();
+  cudaFree(h.st_S);
+  cudaFree(h.st_nm);
+  cudaFree(h.st_x);
+  cudaFree(h.seg_x);
+  h.st_S = h.st_x = h.seg_x = nullptr;
+  h.st_nm = nullptr;
+  h.st_rows = h.st_len = 0;
+  h.st_nax = 0;
+  h.st_state = -1;
+  h.seg_rows = false;
+  cudaFree(h.hr_H);
+  cudaFree(h.hr_e);
+  cudaFree(h.hr_vec);
+  if (h.hr_graph) cudaGraphExecDestroy(h.hr_graph);
+  h.hr_H = nullptr;
+  h.hr_e = nullptr;
+  h.hr_vec = nullptr;
+  h.hr_graph = nullptr;
+  h.hr_state = -1;
+  cudaFree(h.br_rows);
+  h.br_rows = nullptr;
+  h.br_words = 0;
+  if ((e = cudaMalloc(p, bytes))) *p = nullptr;
+  return e;
+}
+
 cudaError_t ensure_stencil(Handle &h) {
   if (h.st_state != 0 || !h.op64_valid || h.apply_mode != VDR_APPLY_STORED ||
       h.storage != VDR_STORE_DF || h.opt.scatter != VDR_SCATTER_AUTO || h.perm_d || !h.Ahi ||

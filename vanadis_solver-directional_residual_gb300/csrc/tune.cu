@@ -131,7 +131,7 @@ int tune_half_apply(Handle &h) {
   if (!h.use_half || h.E < TUNE_MIN_ELEMENTS || capturing(h.stream)) return VDR_OK;
   h.half_tuned = true;
   cudaError_t e;
-  if (!h.work32 && (e = cudaMalloc(&h.work32, sizeof(float) * 10 * (size_t)h.N)))
+  if ((e = take(h, &h.work32, 10 * (size_t)h.N)))
     return cuda_fail(e, "tuning workspace");
   const float *x = h.work32;
   float *y = h.work32 + h.N;

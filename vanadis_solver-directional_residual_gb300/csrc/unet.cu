@@ -1173,7 +1173,7 @@ namespace {
 
 template <typename T>
 cudaError_t nalloc(Net &n, T **p, size_t count) {
-  cudaError_t e = cudaMalloc((void **)p, sizeof(T) * std::max<size_t>(count, 1));
+  cudaError_t e = take(*n.h, p, count);
   if (!e) n.allocs.push_back((void *)*p);
   return e;
 }

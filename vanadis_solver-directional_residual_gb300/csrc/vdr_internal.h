@@ -263,6 +263,7 @@ struct Handle {
   bool resident = true;  // whole solves in one launch (resident.cu) ...
   bool resident_cluster = true;  // ... of one cluster where they fit
   bool rows_room = true;  // false: as if no memory were left for assembled rows
+  bool other_room = true;  // false: as if none were left for anything beside them
 
   // solver workspace
   double *work = nullptr;
@@ -369,6 +370,16 @@ struct OwnCapture {
 };
 
 bool foreign_capture(const Handle &h, cudaStream_t s);
+
+// cudaMalloc for what a call cannot do without: where there is no room, the
+// handle's assembled rows (up to half of what was free when they were formed)
+// make it, and its solves go on element-wise.  Not while rows are in use.
+cudaError_t take_memory(Handle &h, void **p, size_t bytes);
+template <typename T>
+cudaError_t take(Handle &h, T **p, size_t n) {
+  if (*p) return cudaSuccess;
+  return take_memory(h, reinterpret_cast<void **>(p), sizeof(T) * (n ? n : 1));
+}
 
 // SM count of the current device, cached once (thread-safe).
 int device_sm_count();
