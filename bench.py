@@ -19,7 +19,8 @@ element matrices + Jacobi diagonal (DR recompute), right-hand side, solve.
   roofline  the dominant kernels, a BiCGStab iteration on the assembled
             rows (--scatter atomic or color: the stored-matrix EBE apply,
             timed alone)
-  --impl reference   the reference's CPU algorithm (the C oracle port of
+  --impl reference   unavailable: says why
+  --impl cpu-port    the reference's CPU algorithm (the C oracle port of
             vanadis_full_DR_OpenMP_timing.for) on this host's cores
 """
 from __future__ import annotations
@@ -48,7 +49,7 @@ def args_parse(argv=None):
     ap.add_argument("--gpus", type=int, default=1)
     ap.add_argument("--steps", type=int, default=5)
     ap.add_argument("--warmup", type=int, default=3)
-    ap.add_argument("--impl", default="native", choices=["native", "reference"])
+    ap.add_argument("--impl", default="native", choices=["native", "reference", "cpu-port"])
     ap.add_argument("--nex", type=int, default=256)
     ap.add_argument("--ney", type=int, default=256)
     ap.add_argument("--nez", type=int, default=128)
@@ -250,6 +251,18 @@ def cpu_solve_sample(prob, dt, iters, full=False):
     t_sol = time.perf_counter() - t0
     return {"t_asm": t_asm, "t_solve": t_sol, "iters": it, "err": err,
             "status": st, "threads": threads}
+
+
+def reference_unavailable():
+    """The reference itself cannot be run here, and a port's time is not its
+    time (run_reference: --impl cpu-port)."""
+    if dist_info()[0] == 0:
+        print(json.dumps({
+            "impl": "reference",
+            "unavailable": "Fortran and CUDA sources without package metadata (pip: neither "
+                           "setup.py nor pyproject.toml), no Fortran compiler here, and its GPU "
+                           "reductions spin on a mutex that they have freed"}), flush=True)
+    return 0
 
 
 def run_reference(a):
@@ -1369,6 +1382,8 @@ def main():
     if a.case:
         return run_case(a)
     if a.impl == "reference":
+        return reference_unavailable()
+    if a.impl == "cpu-port":
         return run_reference(a)
     return run_native(a)
 
