@@ -133,8 +133,9 @@ __device__ __forceinline__ bool group_active(const BVec &a) {
 
 // The rows in the order in which the march reads them: node n = (x, y, z)
 // holds the entries that multiply plane z around (x, y), for the rows one
-// plane down, in the plane and one plane up: rows[28 n + 9 j + c] = entry
-// 9 (2 - j) + c of node n + (j - 1) planes, times D^-1 of the neighbour.
+// plane down, in the plane and one plane up: rows[28 n + 9 (c / 3) + 3 j +
+// c % 3] = entry 9 (2 - j) + c of node n + (j - 1) planes, times D^-1 of the
+// neighbour, c = 3 (dy + 1) + dx + 1.
 __global__ void br_rows(const float2 *__restrict__ S, const float *__restrict__ dinv, int N, int nax,
                         int pl, float *__restrict__ rows) {
   for (long n = (long)blockIdx.x * blockDim.x + threadIdx.x; n < N;

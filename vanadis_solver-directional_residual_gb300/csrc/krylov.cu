@@ -480,7 +480,8 @@ Vec make_vec(Handle &h, const double *b, double *x) {
 // w = A^T rh, formed once, gives alpha = rho / (w, p^) before the product it
 // scales; the next rho is (rh, s) - omega (rh, t), known before r is formed.
 // p^ and s^ exist only as the products' inputs, pairs scaled by the largest
-// exponent of the direction before (pair_head: room for 2^48 times that).  618 bytes per node and iteration against 1,024 E + ~240 N
+// exponent of the direction before (pair_head: room for 2^48 times that).
+// 610 bytes per node and iteration (273 + 248 + 89) against 1,024 E + ~240 N
 // element-wise; each kernel's last block adds the block partials in a fixed
 // order.
 
@@ -581,10 +582,10 @@ __global__ void __launch_bounds__(RED_THREADS, 4) bst_t(Vec a, StencilView w) {
 }
 
 // Two nodes in flight per thread and 64 registers: the pass is bound by the
-// FP64 pipe (nine operations a node) about as much as by its 97 bytes, and
+// FP64 pipe (nine operations a node) about as much as by its 89 bytes, and
 // wants warps more than loads per thread.  beta comes from bst_t's last
-// block: two divisions in every thread were a third of the pipe's work here
-// (1.08 M nodes 34 -> 30 us, 8.5 M 157 -> 151).
+// block, two divisions less in every thread (1.08 M nodes 26.5 -> 23.0 us,
+// 8.5 M 131 -> 126).
 __global__ void __launch_bounds__(RED_THREADS, 4) bst_p(Vec a) {
   KState *stc = a.st;
   if (stc->done) return;
@@ -1914,7 +1915,7 @@ int solve_mixed_device(Handle &h, int method, const double *b, double *x,
   cudaStream_t s = h.stream;
   double *r = h.work + 8 * (size_t)h.N;
   double *d = h.work + 9 * (size_t)h.N;
-  double *scal = h.work + 10 * (size_t)h.N;  // one double used
+  double *scal = h.work + 10 * (size_t)h.N;  // two doubles, two ints
   Vec a = make_vec(h, b, x);
   const int g = red_grid(h.N);
   MixedStats st;

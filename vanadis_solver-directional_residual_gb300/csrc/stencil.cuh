@@ -10,7 +10,7 @@
 // output vector, and inner products with it can be formed where it is.
 // Measured at 8.5M nodes (2.05 GB with the two vectors of the fused inner
 // product): 0.34 ms, 6.0 TB/s, against 0.77 ms for the 4.77 GB element-wise
-// apply; at 1.08M nodes 48 us against 80 us.
+// apply; at 1.08M nodes 41 us against 105 us.
 //
 // Layout: S[k N + n] = (hi, lo) of the coupling of node n with node n +
 // off(k), k = 9 (dz + 1) + 3 (dy + 1) + (dx + 1), off = dx + nax dy + nax
@@ -115,9 +115,9 @@ __device__ __forceinline__ double stencil_row(const StencilView &v, long n,
 }
 
 // The Krylov iteration's form: the input already split into pairs, scaled by
-// one power of two per vector (pair_head), with zeros for a plane and a row beyond both
-// ends (stencil_pad), so that the 27 products need no mask, no index clamp
-// and no split: the rows hold zeros wherever no coupling exists.
+// one power of two per vector (pair_head), with zeros for a plane and a row
+// beyond both ends (stencil_pad), so that the 27 products need no mask, no
+// index clamp and no split: the rows hold zeros wherever no coupling exists.
 // A^T reads its neighbours' rows at shifted places, which stay inside S.
 template <bool TRANS, bool KEEP>
 __device__ __forceinline__ double stencil_row_pairs(const StencilView &v, long n,

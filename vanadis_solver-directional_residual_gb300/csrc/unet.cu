@@ -831,8 +831,8 @@ __global__ void pack_weights(const float *th, bf16 *wb, bf16 *wbt, bf16 *wtc, bf
 // Nearest upsampling of a coarse [Vc][C] BF16 tensor to the fine grid
 // (fine voxel (x, y, z) reads coarse (x/2, y/2, z/2)): a thread copies 16
 // bytes of a coarse voxel to its up to eight fine ones (one thread per fine
-// unit, with its 64-bit divisions: 24 us at 129 x 129 x 65 voxels and 32
-// channels, so 15).
+// unit, with its 64-bit divisions: 29 us at 129 x 129 x 65 voxels and 32
+// channels, so 15.5).
 __global__ void upsample_bf16(const bf16 *in, bf16 *out, Dims f, Dims c, int C, const int *skip,
                               const int *skip2) {
   chain_wait();
