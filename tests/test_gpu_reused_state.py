@@ -317,7 +317,7 @@ def test_products_on_rows_in_training(vdr, gpu_lib):
     formed the operator's rows: apart by the gradient's own atomics (2e-7) and
     what 1e-14 in the products turns over in FP32 and BF16 roundings."""
     torch = pytest.importorskip("torch")
-    prob = vdr.problems.rotation_shear(17, 12, 9, seed=41)
+    prob = vdr.problems.rotation_shear(64, 32, 32, seed=41)  # large enough for rows
     free = torch.tensor(prob.bc == 0, device="cuda")
     b = torch.tensor(np.cos(0.37 * np.arange(prob.mesh.nnode)), device="cuda") * free
     with vdr.Solver(prob, aH=2.0, aM=10.0) as s, vdr.LearnedNet(s, seed=5) as net:
@@ -490,3 +490,33 @@ def test_rows_make_room(vdr, oracle, gpu_lib, call):
             assert s.stats()["kernel_launches"] > 1
             x = torch.tensor(x0, device="cuda")
             assert s.solve_mixed_device(bd, x, tol=1e-11, inner_tol=1e-4)[3] == 0 and solved(x)
+
+
+@pytest.mark.parametrize("call", ["gcr", "learned"])
+def test_few_products_form_no_rows(vdr, gpu_lib, call):
+    """GCR and preconditioned solves take the rows that another solve has
+    formed, but form none (236 bytes a node): the same residual after three
+    iterations without them and with them, to BF16 roundings in the network."""
+    torch = pytest.importorskip("torch")
+    prob = vdr.problems.rotation_shear(75, 63, 31, seed=47)
+    free_nodes = torch.tensor(prob.bc == 0, device="cuda")
+    b = torch.tensor(np.cos(0.37 * np.arange(prob.mesh.nnode)), device="cuda") * free_nodes
+    x = torch.zeros_like(b)
+    with vdr.Solver(prob, aH=2.0, aM=200.0) as s, vdr.LearnedNet(s, seed=6) as net:
+        net.update_features()
+
+        def solve():
+            x.zero_()
+            if call == "gcr":
+                return s.solve_gcr_device(b, x, tol=0.0, itmax=3)[1]
+            return s.solve_learned_device(net, b, x, tol=0.0, itmax=3)[1]
+
+        s.apply_device(b, x)
+        s.true_residual_device(b, x)  # the solver's vectors
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        first = solve()
+        vectors = 41 * 8 if call == "gcr" else 0  # GCR(20)'s own, bytes a node
+        assert free - torch.cuda.mem_get_info()[0] < (vectors + 100) * s.N
+        s.solve_device(b, torch.zeros_like(b), tol=1e-8, itmax=500)
+        assert abs(solve() - first) <= (1e-9 if call == "gcr" else 0.02) * first

@@ -898,15 +898,18 @@ cudaError_t launch_rhs_from_mass(Handle &h, double cf, double rM, const double *
   // H - rM M = A/aH - (aM/aH + rM) M
   double *y1 = h.rhs_tmp, *y2 = h.rhs_tmp + h.N;
   cudaError_t e;
-  if ((e = cudaMemsetAsync(h.rhs_tmp, 0, sizeof(double) * 2 * (size_t)h.N, s))) return e;
-  if ((e = launch_apply(h, false, t, y1, nullptr, nullptr, s))) return e;
   const bool color = h.scatter == VDR_SCATTER_COLOR;
   const ConnView cv = conn_view(h);
-  const bool ordered = ordered_sums(h) && cv.emask;
+  const bool ordered = ordered_sums(h) && cv.emask && h.storage == VDR_STORE_DF;
   if (ordered) {
-    node_apply_df<<<grid_for(8L * h.N, 256, 8), 256, 0, s>>>(h.Mhi, h.Mlo, cv, h.E, h.N, h.naz, t,
-                                                             y2);
-    count_launches(1);
+    const int grid = grid_for(8L * h.N, 256, 8);
+    node_apply_df<<<grid, 256, 0, s>>>(h.Ahi, h.Alo, cv, h.E, h.N, h.naz, t, y1);
+    node_apply_df<<<grid, 256, 0, s>>>(h.Mhi, h.Mlo, cv, h.E, h.N, h.naz, t, y2);
+    count_launches(2);
+  } else {
+    if ((e = cudaMemsetAsync(h.rhs_tmp, 0, sizeof(double) * 2 * (size_t)h.N, s)) ||
+        (e = launch_apply(h, false, t, y1, nullptr, nullptr, s)))
+      return e;
   }
   const int nranges = ordered ? 0 : color ? h.ncolors : 1;
   for (int r = 0; r < nranges; r++) {
@@ -1104,7 +1107,7 @@ cudaError_t launch_element_apply(const Handle &h, bool transpose, const double *
 cudaError_t launch_apply(const Handle &h, bool transpose, const double *x,
                          double *y, const int *skip, const int *skip2,
                          cudaStream_t s) {
-  if (stencil_ready(h) && !foreign_capture(h, s))
+  if (products_on_rows(h) && !foreign_capture(h, s))
     return launch_stencil_apply(h, transpose, x, y, skip, skip2, s);
   return launch_element_apply(h, transpose, x, y, skip, skip2, s);
 }

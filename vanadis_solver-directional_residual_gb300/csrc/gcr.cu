@@ -299,7 +299,6 @@ int solve_gcr_device(Handle &h, const double *b, double *x, double tol,
     return VDR_BAD_ARGUMENT;
   }
   cudaError_t e = ensure_solver_workspace(h, 8);  // KState, events
-  if (!e) e = ensure_stencil(h);
   if (e) return cuda_fail(e, "solver workspace");
   cudaStream_t s = h.stream;
   const int g = gcr_grid(h.N);
@@ -368,7 +367,7 @@ int solve_gcr_device(Handle &h, const double *b, double *x, double tol,
   } else {
   const GraphKey key{key_of(b), key_of(x), key_of(h.gcr_work), (uintptr_t)m,
                      (uintptr_t)(prec ? prec->version : 0), (uintptr_t)h.apply_mode,
-                     (uintptr_t)h.scatter, (uintptr_t)h.storage, (uintptr_t)stencil_ready(h)};
+                     (uintptr_t)h.scatter, (uintptr_t)h.storage, (uintptr_t)products_on_rows(h)};
   long per_cycle = 0;
   if (!h.gcr_graph || h.gcr_key != key) {
     if (h.gcr_graph) cudaGraphExecDestroy(h.gcr_graph);

@@ -111,13 +111,15 @@ __global__ void __launch_bounds__(256, 2) stencil_assemble_meshes(
 }
 
 // y += A x or A^T x, any FP64 x, for the products of solvers that keep FP64
-// vectors (GCR, a preconditioned BiCGStab, first residuals).  Here every
-// thread splits its 27 gathered values and scales each plane by itself, which
-// makes it bound by instruction issue: 95 / 718 us at 1.08 / 8.5 M nodes
-// where the element-wise apply takes 105 / 773; the Krylov iterations split
-// once per node.  A caller's own applies stay element-wise: summing the rows
-// (160 us, 1.23 ms) costs what 15 of them would save, and the FP64 sums over
-// the elements are closer to the exact product (3.5e-15 against 5.9e-15
+// vectors (GCR, a preconditioned BiCGStab, first residuals) where another
+// solve has formed the rows (products_on_rows).  Here every thread splits its
+// 27 gathered values and scales each plane by itself, which makes it bound by
+// instruction issue: 95 / 718 us at 1.08 / 8.5 M nodes where the element-wise
+// apply takes 105 / 773; the Krylov iterations split once per node.  Rows are
+// not formed for it: their sum (160 us, 1.23 ms) costs what 15 products save
+// (GCR of one to three iterations on a new operator took up to 10 per cent
+// longer).  A caller's own applies stay element-wise also because FP64 sums
+// over the elements are closer to the exact product (3.5e-15 against 5.9e-15
 // relative, random input).
 template <bool TRANS, bool KEEP>
 __global__ void __launch_bounds__(256, 4) stencil_apply(const StencilView v,
@@ -150,6 +152,11 @@ bool stencil_ready(const Handle &h) {
   return h.st_state == 1 && h.apply_mode == VDR_APPLY_STORED && !h.apply_fp32 &&
          !h.gate_active && h.storage == VDR_STORE_DF;
 }
+
+// Current rows, and a mesh on which a product with them is the faster one:
+// 18,513 nodes 57.5 us an iteration of GCR by rows, 56.7 by elements; 100,096
+// nodes 92.4 and 93.0.
+bool products_on_rows(const Handle &h) { return h.N >= 65536 && stencil_ready(h); }
 
 // Whether a caller records on the stream: what it replays later is to follow
 // the operator as it is then, and rows are summed anew by solves and applies

@@ -503,6 +503,7 @@ cudaError_t launch_bc_to_mask(const int *bc, unsigned char *mask, int N,
 // called before work that applies the operator several times.
 cudaError_t ensure_stencil(Handle &h);
 bool stencil_ready(const Handle &h);
+bool products_on_rows(const Handle &h);
 // The same for a handle of many meshes (h.seg_rows when they are current).
 cudaError_t ensure_segment_rows(Handle &h);
 cudaError_t launch_element_masks(Handle &h);
